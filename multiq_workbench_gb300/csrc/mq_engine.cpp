@@ -293,25 +293,26 @@ mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_
     const uint64_t need = max_more < b.max_steps ? (uint64_t)max_more : (uint64_t)b.max_steps;
     const uint64_t max_launches = fault == MQ_FAULT_LAUNCH_BUDGET ? 1 : (need + kF64Chunk - 1) / kF64Chunk + 1;
     const uint32_t chunk = fault == MQ_FAULT_LAUNCH_BUDGET ? 16u : kF64Chunk;
-    CK(e->misc.grow(64), "counters");
-    unsigned long long* d_steps = e->misc.as<unsigned long long>();
-    uint32_t* d_live = reinterpret_cast<uint32_t*>(d_steps + 1);
-    CK(cudaMemsetAsync(d_steps, 0, 16, e->st), "counter reset");
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev), "device attributes");
+    CK(e->misc.grow(256 + sizeof(uint2) * (size_t)mqd::f64_hand_entries(sms)), "counters");
+    mqd::F64Ctrs* ctr = e->misc.as<mqd::F64Ctrs>();
+    uint2* hand = reinterpret_cast<uint2*>(e->misc.as<char>() + 256);
+    CK(cudaMemsetAsync(ctr, 0, sizeof(mqd::F64Ctrs), e->st), "counter reset");
     const double2* rf_tab = e->tabs.as<double2>();
     const double2* ac_tab = rf_tab + tlen;
     uint64_t budget = max_more;
-    uint32_t launches = 0, live = 0;
+    uint32_t launches = 0, kernels = 0, live = 0;
     float step_ms = 0.0f;
     for (;;) {
         uint32_t L = budget < chunk ? (uint32_t)budget : chunk;
         if (L == 0 || launches >= max_launches) break;
-        CK(cudaMemsetAsync(d_live, 0, 4, e->st), "counter reset");
         CK(cudaEventRecord(e->ev[2], e->st), "event");
         CK(mqd::launch_f64_step(dev_grid(e), b, e->jobc.as<JobC>(), rf_tab, ac_tab, tlen, dev_ions(e), (uint32_t)n, L,
-                                d_steps, d_live, e->st), "FP64 step kernel");
+                                ctr, hand, e->st, &kernels), "FP64 step kernel");
         CK(cudaEventRecord(e->ev[3], e->st), "event");
         live = 0;
-        CK(cudaMemcpyAsync(&live, d_live, 4, cudaMemcpyDeviceToHost, e->st), "live count");
+        CK(cudaMemcpyAsync(&live, &ctr->live, 4, cudaMemcpyDeviceToHost, e->st), "live count");
         CK(cudaStreamSynchronize(e->st), "FP64 step kernel");
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e->ev[2], e->ev[3]);
@@ -321,13 +322,13 @@ mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_
         if (live == 0) break;
     }
     unsigned long long steps = 0;
-    CK(cudaMemcpyAsync(&steps, d_steps, 8, cudaMemcpyDeviceToHost, e->st), "step count");
+    CK(cudaMemcpyAsync(&steps, &ctr->steps, 8, cudaMemcpyDeviceToHost, e->st), "step count");
     CK(cudaStreamSynchronize(e->st), "step count");
     *steps_out = steps;
     if (stats) {
         stats->launches += launches;
-        stats->kernel_launches += launches;
-        stats->step_kernel_launches += launches;
+        stats->kernel_launches += kernels;
+        stats->step_kernel_launches += kernels - launches;   // less the counter kernel of each round
         stats->step_kernel_ms += step_ms;
     }
     if (live != 0 && max_more >= b.max_steps)

@@ -1,4 +1,4 @@
-// Plain FP64 ion-trajectory kernel: one thread per ion, FP64 state, f32 field nodes
+// Plain FP64 ion-trajectory kernel: a group of lanes per ion, FP64 state, f32 field nodes
 // promoted to f64, global phase tables, xorshift64 collision Monte Carlo.  It evaluates
 // exactly the operations of the FP64 CPU integrator in the same order and is compiled
 // with --fmad=false, so its final states equal the CPU integrator's bit for bit.
@@ -79,151 +79,457 @@ __device__ __forceinline__ void table_get(const double2* t, uint32_t tlen, doubl
     else mqp::phase_at(w, n, s, c);
 }
 
-__global__ void __launch_bounds__(128) k_f64_step(DevGrid g, Batch b, const JobC* __restrict__ jobs,
-                                                  const double2* __restrict__ rf_tab, const double2* __restrict__ ac_tab,
-                                                  uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more,
-                                                  unsigned long long* d_steps, uint32_t* d_live) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t done = 0;
-    int32_t status = 1;
-    if (i < n && io.status[i] == 0) {
-        const JobC jc = jobs[io.jid[i]];
-        const double2* tac = ac_tab + (size_t)jc.tab * tlen;
-        double x[3] = {io.x[i], io.y[i], io.z[i]};
-        double v[3] = {io.vx[i], io.vy[i], io.vz[i]};
-        uint64_t rng = io.rng[i];
-        uint32_t age = io.steps[i], ncoll = io.ncoll[i];
-        int32_t leg = io.leg[i];
-        status = 0;
-        double rs, rc, as_, ac;
-        mqp::sincos2pi(io.ph_rf[i], &rs, &rc);
-        mqp::sincos2pi(io.ph_ac[i], &as_, &ac);
-        const double dt = b.dt, qmdt = jc.qmdt, h = g.h;
-        // bit patterns of the step's positive thresholds for the integer-pipe comparisons
-        const long long lim_x = __double_as_longlong((double)(g.nx - 2)), lim_y = __double_as_longlong((double)(g.ny - 2)),
-                        lim_z = __double_as_longlong((double)(g.nz - 2));
-        const long long k_exit = __double_as_longlong(b.z_exit), k_return = __double_as_longlong(b.z_return);
-        const long long k_lim0 = __double_as_longlong(b.lim[0]), k_lim1 = __double_as_longlong(b.lim[1]),
-                        k_lim2 = __double_as_longlong(b.lim[2]);
-        const size_t nx = (size_t)g.nx, ny = (size_t)g.ny;
-        while (done < max_more) {
-            double S, Cc, Sa = 0.0, Ca = 0.0;
-            table_get(rf_tab, tlen, b.w_rf, age, &S, &Cc);
-            double srf = b.v_rf * (S * rc + Cc * rs);
-            double sac = 0.0;
-            if (jc.use_ac) {
-                table_get(tac, tlen, jc.w_ac, age, &Sa, &Ca);
-                sac = jc.v_ac * (Sa * ac + Ca * as_);
+// ---------------------------------------------------------------- the step kernel
+// What bounds it: GB300's FP64 pipe. An SM takes one FP64 warp instruction per 19 cycles (a warp that
+// has its scheduler's share to itself one per 64), however many lanes are active and however much
+// independent work the warp has. A step is about 200 FP64 operations: with one lane per ion it took
+// 9 us, and a warp lasted as long as its longest-lived ion, with 6 of 32 lanes active on average.
+// Here a group of G lanes steps one ion, so that one instruction does several of its operations:
+// each lane owns an axis (position, velocity, cell) and one of the eight cell corners (two for
+// G = 4), whose weight and products with the nine field components it forms; the nine sums over the
+// corners run side by side in nine lanes (G = 16) or three to a lane (G = 4), and the drive's
+// products ride in idle lanes. 26 (G = 16) or 59 (G = 4) FP64 instructions a step remain, and
+// groups take the next ion of a queue when theirs ends. Comparisons, conversions, corner reloads
+// and the collision test (against an FP32 bound, exact only where that does not decide) stay off
+// the pipe. Every operation is the CPU integrator's, in its order: results are its bits.
+// Which G: 16 up to the ions that one warp per scheduler holds (f64_hand_entries), where latency is all
+// that counts: 1.8 us a step for up to 1,216 ions against 3.4 with G = 4 (S14 grid, no gas). Above, the
+// pipe is full and 4 lanes waste fewer slots: 4,864 ions 3.4 us, 58,368 ions 25 us a step. The last ions of
+// a large call go on in groups of 16.
+// Measured (whole run_batch calls, before -> now): mass scan of 25,000 ions 162 -> 32 ms; S14 point with
+// 20,000 ions and up to 75,000 steps 1,098 -> 197 ms.
+constexpr unsigned FULL = 0xffffffffu;
+constexpr int kBlock = 256;            // 8 warps: two per scheduler, one to fill the other's gaps
+constexpr int kPad = 120 * 1024;       // dynamic shared memory asked for, unused
+constexpr uint32_t kPollSteps = 32;    // steps between looks at the count of open ions
+
+// 0.0 + p, on the integer pipe: p itself, but +0 for -0
+__device__ __forceinline__ double plus_zero(double p) {
+    return __double_as_longlong(p) == (long long)0x8000000000000000ULL ? 0.0 : p;
+}
+__device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(FULL, v, src); }
+// order-preserving signed key of a double's bits (NaN aside; -0 as +0)
+__device__ __forceinline__ long long order_key(long long b) {
+    if (b == (long long)0x8000000000000000ULL) b = 0;
+    return b < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)b) : b;
+}
+// FP32 upper bound of |v| from the high word of a double; from 2^127 on (infinities and NaN too) a
+// value whose square overflows
+__device__ __forceinline__ float mag_up(double v) {
+    const int hi = min(max(__double2hiint(v) & 0x7fffffff, 0x38100000), 0x47e00000);
+    return __int_as_float(((hi - 0x38000000) << 3) + 8);
+}
+__device__ __forceinline__ uint64_t xs_step(uint64_t x) {
+    x ^= x << 13;
+    x ^= x >> 7;
+    x ^= x << 17;
+    return x;
+}
+__device__ __forceinline__ double xs_unit(uint64_t x) { return (double)(x >> 11) / 9007199254740992.0; }
+
+// Shared memory of a group, in doubles: the fractions of the three axes as pairs {1 - t, t}, the
+// products of the nine sums (rows of 8 corners, 10 apart: 16-byte reads of the rows meet no bank
+// twice), and what the lanes hand each other besides: nine weighted sums, four drive products and
+// the drive amplitudes.
+constexpr int kRow = 10;
+constexpr int kSums = 6 + 9 * kRow;
+constexpr int kGroupDoubles = kSums + 16;
+
+template <int G>
+__global__ void __launch_bounds__(kBlock, 1)
+k_f64_step(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __restrict__ rf_tab,
+           const double2* __restrict__ ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more,
+           F64Ctrs* __restrict__ ctr, uint2* hand, uint32_t hand_at, int from_hand) {
+    constexpr int GPW = 32 / G;            // groups per warp
+    constexpr int NC = G == 16 ? 1 : 2;    // corners per lane
+    constexpr int NP = G == 16 ? 5 : 9;    // sums a lane has products of, per corner
+    constexpr int NS = G == 16 ? 1 : 3;    // sums a lane adds up
+    extern __shared__ __align__(16) double sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gl = lane % G, base = lane - gl;
+    const int d = gl % 3;                  // the lane's axis; lanes 0..2 own it
+    double* const tw = sm + (size_t)(threadIdx.x / G) * kGroupDoubles;
+    double* const prod = tw + 6;
+    double* const xch = tw + kSums;
+    const uint32_t count = from_hand ? ctr->handed : n;
+    // ions handed to a later launch instead of being finished: once at most hand_at are open
+    const bool hands = !from_hand && hand != nullptr;
+    uint32_t* const head = from_hand ? &ctr->head_b : &ctr->head_a;
+    // the first ions, spread so that every scheduler of every SM has work before any has two warps
+    const uint32_t first = (uint32_t)((((warp >> 2) * GPW + lane / G) * 4 + (warp & 3)) * gridDim.x + blockIdx.x);
+    const uint32_t groups = gridDim.x * (kBlock / 32) * GPW;
+
+    const double h = g.h, inv_h = g.inv_h, dt = b.dt;
+    const int32_t nd = d == 0 ? g.nx : d == 1 ? g.ny : g.nz;
+    const long long lim_c = __double_as_longlong((double)(nd - 2));
+    const size_t nx = (size_t)g.nx, ny = (size_t)g.ny;
+    [[maybe_unused]] const size_t total = nx * ny * (size_t)g.nz;   // bounds-checked build
+    // High words of the positions that no plane or face can end: strictly between the words of the
+    // limits (positive doubles order like their words), so one compare per lane clears a step
+    const int up = min(__double2hiint(b.lim[d]), d == 2 ? __double2hiint(b.z_exit) : 0x7fffffff);
+    const int in_lo = d == 2 ? __double2hiint(b.z_return) + 1 : 0;
+    const unsigned in_n = gl < 3 ? (unsigned)max(up - in_lo, 0) : 0xffffffffu;
+    // the lane's corner (G = 4: that and the one with di = 1; corner c = 4 di + 2 dj + dk) and, for
+    // G = 16, which products (lanes 0..7 sums 0..4, lanes 8..15 sums 5..8) and which sum it has
+    // (sum 3 f + d of field f: RF, AC, DC; lanes 9..15 repeat sums 0..6 and keep nothing of it)
+    const int cn = G == 16 ? gl & 7 : gl;
+    const bool upper = G == 16 && gl >= 8;
+    const int chain = G == 16 ? (gl < 9 ? gl : gl - 9) : gl % 3;
+    // Drive amplitudes amp (sin cos0 + cos sin0) of RF and AC for the next step. G = 16: lanes 9..12
+    // form the four products, sums and amplitudes in the instructions that the sums' lanes use for
+    // theirs. G = 4: even lanes RF, odd lanes AC, lanes 2 and 3 the second product.
+    const bool drives = G == 16 ? gl >= 9 : true;
+    const bool is_ac = G == 16 ? gl >= 11 : (gl & 1) != 0;
+    const bool second = G == 16 ? (gl == 10 || gl == 12) : (gl & 2) != 0;
+    // where the lane's first two addends lie: {RF, AC} sums of its axis, or the two drive products
+    const int i0 = G == 16 && gl >= 9 ? (gl >= 11 ? 11 : 9) : d, i1 = G == 16 && gl >= 9 ? i0 + 1 : d + 3;
+
+    bool have = false, drained = false, fresh = true;
+    uint32_t id = 0, age = 0, left = 1, ncoll = 0, jid = 0;
+    int32_t leg = 0;
+    uint64_t rng = 1;
+    double x = 0.0, v = 0.0, cell = 0.0, kick = 0.0, ph = 0.0, w_tone = 0.0, coef = 0.0;
+    float nsd2 = 0.0f, ub0 = 0.0f;
+    int32_t ci = -1, cj = -1, ck = -1;
+    uint32_t mask = 0;
+    double val[NC][NP];
+    const double2* tab = rf_tab;
+    bool use_ac = false;
+    double S = 0.0, Cc = 0.0;
+#pragma unroll
+    for (int k = 0; k < NC; ++k)
+#pragma unroll
+        for (int m = 0; m < NP; ++m) val[k][m] = 0.0;
+    unsigned long long steps_total = 0;
+    uint32_t live = 0;
+    bool turn = true;   // some group of the warp has no ion
+
+    // the cell of position x and its fractions t of it; refills the corner values of the groups in `upd`
+    // that changed cell. A fraction in [0, 1) of the cell it had means that the cell is the same.
+    auto refill = [&](bool upd, double gx) -> double {
+        const int32_t ca = cell_lo_bits(gx, nd, lim_c);
+        cell = i2d_bits(ca);
+        const double t = gx - cell;
+        const int32_t ni = __shfl_sync(FULL, ca, base), nj = __shfl_sync(FULL, ca, base + 1), nk = __shfl_sync(FULL, ca, base + 2);
+        const bool move = upd && (ni != ci || nj != cj || nk != ck);
+        bool c0 = false, c1 = false;
+        if (move) {
+            ci = ni; cj = nj; ck = nk;
+            // every load is asked for before the first value is used
+            float r[NC][9], solid[2] = {0.0f, 0.0f};
+#pragma unroll
+            for (int k = 0; k < NC; ++k) {
+                const int di = G == 16 ? cn >> 2 : k;
+                size_t q = (size_t)(ci + di) + nx * ((size_t)(cj + ((cn >> 1) & 1)) + ny * (size_t)(ck + (cn & 1)));
+                q = MQ_CHK(q, total, MQ_SITE_F64_FIELD);
+                const float4 a4 = __ldg(g.ac + q), o4 = __ldg((upper ? g.dc : g.rf) + q);
+                if (G == 16) {
+                    r[k][0] = upper ? a4.z : o4.x; r[k][1] = upper ? o4.x : o4.y; r[k][2] = upper ? o4.y : o4.z;
+                    r[k][3] = upper ? o4.z : a4.x; r[k][4] = a4.y;
+                } else {
+                    const float4 d4 = __ldg(g.dc + q);
+                    r[k][0] = o4.x; r[k][1] = o4.y; r[k][2] = o4.z; r[k][3] = a4.x; r[k][4] = a4.y; r[k][5] = a4.z;
+                    r[k][6] = d4.x; r[k][7] = d4.y; r[k][8] = d4.z;
+                }
+                solid[k] = upper ? 0.0f : o4.w;
             }
-            // fields_at: one pass over the 8 corners, weights (1-t, t) in order i, j, k
-            double gx = mqp::div_rn(x[0], h, g.inv_h), gy = mqp::div_rn(x[1], h, g.inv_h), gz = mqp::div_rn(x[2], h, g.inv_h);
-            int32_t ci = cell_lo_bits(gx, g.nx, lim_x), cj = cell_lo_bits(gy, g.ny, lim_y), ck = cell_lo_bits(gz, g.nz, lim_z);
-            double tx = gx - i2d_bits(ci), ty = gy - i2d_bits(cj), tz = gz - i2d_bits(ck);
-            if (b.nearest) { tx = 0.0; ty = 0.0; tz = 0.0; }
-            double er[3] = {0.0, 0.0, 0.0}, ea[3] = {0.0, 0.0, 0.0}, ed[3] = {0.0, 0.0, 0.0};
+            bool odd = false;
 #pragma unroll
-            for (int di = 0; di < 2; ++di) {
-                double wx = di ? tx : 1.0 - tx;
+            for (int k = 0; k < NC; ++k)
 #pragma unroll
-                for (int dj = 0; dj < 2; ++dj) {
-                    double wy = dj ? ty : 1.0 - ty;
+                for (int m = 0; m < NP; ++m) val[k][m] = mqp::widen_normal(r[k][m], odd);
+            if (odd)   // subnormals, infinities, NaN
 #pragma unroll
-                    for (int dk = 0; dk < 2; ++dk) {
-                        double wz = dk ? tz : 1.0 - tz;
-                        size_t q = (size_t)(ci + di) + nx * ((size_t)(cj + dj) + ny * (size_t)(ck + dk));
-                        q = MQ_CHK(q, nx * ny * (size_t)g.nz, MQ_SITE_F64_FIELD);
-                        double w = wx * wy * wz;
-                        float4 r = __ldg(g.rf + q), a = __ldg(g.ac + q), c = __ldg(g.dc + q);
-                        er[0] += w * mqp::widen(r.x); er[1] += w * mqp::widen(r.y); er[2] += w * mqp::widen(r.z);
-                        ea[0] += w * mqp::widen(a.x); ea[1] += w * mqp::widen(a.y); ea[2] += w * mqp::widen(a.z);
-                        ed[0] += w * mqp::widen(c.x); ed[1] += w * mqp::widen(c.y); ed[2] += w * mqp::widen(c.z);
+                for (int k = 0; k < NC; ++k)
+#pragma unroll
+                    for (int m = 0; m < NP; ++m) val[k][m] = (double)r[k][m];
+            c0 = solid[0] > 0.5f;
+            c1 = solid[1] > 0.5f;
+        }
+        const unsigned m0 = __ballot_sync(FULL, c0), m1 = NC == 2 ? __ballot_sync(FULL, c1) : 0u;
+        if (move) mask = NC == 2 ? (((m0 >> base) & 15u) | (((m1 >> base) & 15u) << 4)) : ((m0 >> base) & 255u);
+        return t;
+    };
+    auto put_fractions = [&](double t) {
+        if (b.nearest) t = 0.0;
+        const double omt = 1.0 - t;
+        if (gl < 3) { tw[2 * gl] = omt; tw[2 * gl + 1] = t; }
+    };
+
+    for (uint32_t iter = 1;; ++iter) {
+        if (turn) {
+            // ---- groups without an ion take the next one of the queue
+            bool got = false;
+            for (;;) {
+                const unsigned need = __ballot_sync(FULL, !have && !drained && gl == 0);
+                if (!need) break;
+                uint32_t slot = first;
+                const unsigned later = __ballot_sync(FULL, !have && !drained && gl == 0 && !fresh);
+                if (later) {
+                    uint32_t q = 0;
+                    const int leader = __ffs(later) - 1;
+                    if (lane == leader) q = atomicAdd(head, (uint32_t)__popc(later));
+                    q = __shfl_sync(FULL, q, leader) + groups;
+                    if (!fresh) slot = q + __popc(later & ((1u << base) - 1u));
+                }
+                if (!have && !drained) {
+                    fresh = false;
+                    if (slot >= count) drained = true;
+                    else {
+                        uint32_t done = 0;
+                        id = slot;
+                        if (from_hand) { const uint2 e = hand[slot]; id = e.x; done = e.y; }
+                        if (io.status[id] == 0) {
+                            have = got = true;
+                            jid = io.jid[id];
+                            const JobC& jc = jobs[jid];
+                            x = d == 0 ? io.x[id] : d == 1 ? io.y[id] : io.z[id];
+                            v = d == 0 ? io.vx[id] : d == 1 ? io.vy[id] : io.vz[id];
+                            rng = io.rng[id]; age = io.steps[id]; ncoll = io.ncoll[id]; leg = io.leg[id];
+                            // steps to the time-out (one at least) or to the end of this call's share
+                            left = age < b.max_steps ? b.max_steps - age : 1u;
+                            left = min(left, max_more - done);
+                            steps_total += gl == 0 ? left : 0u;   // corrected when the ion ends before that
+                            use_ac = jc.use_ac != 0;
+                            w_tone = is_ac ? jc.w_ac : b.w_rf;
+                            const double amp = is_ac ? jc.v_ac : b.v_rf;
+                            kick = G == 16 && drives ? amp : jc.qmdt;
+                            const float nsd_up = jc.nsd == 0.0 ? 0.0f : mag_up(jc.nsd);
+                            nsd2 = __fmul_ru(__fmul_ru(nsd_up, nsd_up), 1.00001f);
+                            ub0 = __fmul_ru(__fmul_ru(nsd_up, mag_up(6.0 * jc.s_gas)), 1.00001f);
+                            double s0, c0;
+                            mqp::sincos2pi(is_ac ? io.ph_ac[id] : io.ph_rf[id], &s0, &c0);
+                            ph = second ? s0 : c0;
+                            tab = is_ac ? ac_tab + (size_t)jc.tab * tlen : rf_tab;
+                            ci = -1;
+                            if (G == 16) {     // the amplitudes of the first step
+                                double s1, c1;
+                                table_get(tab, tlen, w_tone, age, &s1, &c1);
+                                if (drives) xch[13 + (is_ac ? 1 : 0)] = amp * (s1 * c0 + c1 * s0);
+                            } else {
+                                coef = amp;
+                            }
+                        } else if (gl == 0 && hands) atomicSub(&ctr->open, 1u);
                     }
                 }
             }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                v[d] += qmdt * (srf * er[d] + sac * ea[d] + ed[d]);
-                x[d] += v[d] * dt;
+            if (!__any_sync(FULL, have)) break;
+            if (__any_sync(FULL, got)) {
+                put_fractions(refill(have && ci < 0, mqp::div_rn(x, h, inv_h)));
+                if (G == 4 && got) table_get(tab, tlen, w_tone, age, &S, &Cc);
+                __syncwarp();
             }
-            age += 1;
-            done += 1;
+            turn = false;
+        }
+
+        // ---- one step. A group without an ion computes on stale values and keeps nothing.
+        // asked for here: the drive's sine and cosine of the next step
+        double S1 = 0.0, C1 = 0.0;
+        if (have && drives) table_get(tab, tlen, w_tone, age + 1, &S1, &C1);
+        const uint64_t r1 = xs_step(rng);   // the first draw of this step's collision, if there is one
+        double dr;
+        if (G == 16) {
+            dr = xch[13 + (chain / 3 == 1 ? 1 : 0)];
+            if (chain / 3 == 1 && !use_ac) dr = 0.0;
+        } else {
+            dr = (second ? Cc : S) * ph;
+            dr = dr + shfl_d(dr, lane ^ 2);
+            dr = coef * dr;
+        }
+        // ---- trilinear weights of the lane's corners and their products
+        {
+            const double wy = tw[2 + ((cn >> 1) & 1)], wz = tw[4 + (cn & 1)];
+#pragma unroll
+            for (int k = 0; k < NC; ++k) {
+                const double w = tw[G == 16 ? cn >> 2 : k] * wy * wz;
+#pragma unroll
+                for (int m = 0; m < NP; ++m)
+                    if (G == 4 || m < 4) prod[((upper ? 5 : 0) + m) * kRow + cn + 4 * k] = w * val[k][m];
+                    else if (!upper) prod[m * kRow + cn] = w * val[k][m];
+            }
+        }
+        __syncwarp();
+        // ---- sums over the corners in order, one per lane (G = 16) or one per field (G = 4)
+        double acc[NS];
+#pragma unroll
+        for (int f = 0; f < NS; ++f) {
+            const double2* row = reinterpret_cast<const double2*>(prod + (chain + 3 * f) * kRow);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double2 p = row[c];
+                acc[f] = c == 0 ? plus_zero(p.x) : acc[f] + p.x;
+                acc[f] = acc[f] + p.y;
+            }
+        }
+        if (G == 16) {
+            // sums times amplitudes | drive products of the next step
+            const double m = (drives ? (second ? C1 : S1) : dr) * (drives ? ph : acc[0]);
+            if (gl < 13) xch[gl] = gl >= 6 && gl < 9 ? acc[0] : m;
+            __syncwarp();
+            const double e2 = xch[i0] + xch[i1];       // RF + AC | sin cos0 + cos sin0
+            const double e = e2 + xch[6 + d];
+            const double k = kick * (drives ? e2 : e);  // velocity change | amplitude
+            if (gl == 9 || gl == 11) xch[gl == 9 ? 13 : 14] = k;
+            v += k;
+        } else {
+            const double srf = shfl_d(dr, base);
+            double sac = shfl_d(dr, base + 1);
+            if (!use_ac) sac = 0.0;
+            v += kick * (srf * acc[0] + sac * acc[NS / 2] + acc[NS - 1]);
+            S = S1;
+            Cc = C1;
+        }
+        x += v * dt;
+        age += 1;
+        left -= 1;
+        // What the end of the step may have to deal with, found while the FP64 pipe works on the new
+        // position: a collision, another cell, a limit. Most steps have none and skip it all.
+        const double gx = mqp::div_rn(x, h, inv_h);
+        double t = gx - cell;
+        bool maybe;
+        if (!b.legacy_coll) {
+            // candidate only if u < nsd (|v| + 6 s), that is u - 6 nsd s < nsd |v|: first in FP32, the
+            // left side from below, the right from above and squared
+            const float vf = mag_up(v), sq = __fmul_ru(vf, vf);
+            const float s2 = __fadd_ru(__shfl_sync(FULL, sq, base), __fadd_ru(__shfl_sync(FULL, sq, base + 1), __shfl_sync(FULL, sq, base + 2)));
+            const float du = __fadd_rd((float)(uint32_t)(r1 >> 40) * 0x1.0p-24f, -ub0);
+            rng = r1;   // one draw every step
+            maybe = have && !(du >= 0.0f && __fmul_rd(du, du) >= __fmul_ru(nsd2, s2));
+        } else {
+            leg -= 1;
+            maybe = have && leg <= 0;
+        }
+        const bool moved = have && gl < 3 && (unsigned)__double2hiint(t) >= 0x3ff00000u;
+        const bool edge = have && ((unsigned)(__double2hiint(x) - in_lo) >= in_n || mask != 0u || left == 0u);
+        bool put = false, give = false;
+        int32_t status = 0;
+        const bool some = __any_sync(FULL, maybe || moved || edge);
+        // ---- collisions
+        if (some && __any_sync(FULL, maybe)) {
+            const JobC& jc = jobs[have ? jid : 0u];
+            const double v0 = shfl_d(v, base), v1 = shfl_d(v, base + 1), v2 = shfl_d(v, base + 2);
+            const double vm = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
             if (!b.legacy_coll) {
-                double vm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-                double bound = vm + 6.0 * jc.s_gas;
-                if (mqp::xs_next(&rng) < jc.nsd * bound) {
-                    double vg[3];
+                const double bound = vm + 6.0 * jc.s_gas;
+                const bool cand = maybe && xs_unit(r1) < jc.nsd * bound;
+                if (__any_sync(FULL, cand)) {
+                    uint64_t r = r1, ra = 0, rb = 0;   // six draws: two per axis, in axis order
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        double u1 = mqp::xs_next(&rng), u2 = mqp::xs_next(&rng);
-                        vg[d] = jc.s_gas * mqp::gauss(u1, u2);
+                    for (int k = 0; k < 3; ++k) {
+                        r = xs_step(r);
+                        if (k == d) ra = r;
+                        r = xs_step(r);
+                        if (k == d) rb = r;
                     }
-                    double gv[3] = {v[0] - vg[0], v[1] - vg[1], v[2] - vg[2]};
-                    double gl = sqrt(gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2]);
-                    if (mqp::xs_next(&rng) * bound < gl) {
-                        double c = 2.0 * mqp::xs_next(&rng) - 1.0;
+                    const double vg = jc.s_gas * mqp::gauss(xs_unit(ra), xs_unit(rb));
+                    const double gv = v - vg;
+                    const double g0 = shfl_d(gv, base), g1 = shfl_d(gv, base + 1), g2 = shfl_d(gv, base + 2);
+                    const double gm = sqrt(g0 * g0 + g1 * g1 + g2 * g2);
+                    r = xs_step(r);
+                    const bool hit = cand && xs_unit(r) * bound < gm;
+                    if (cand) rng = r;
+                    if (__any_sync(FULL, hit)) {
+                        r = xs_step(r);
+                        const double c = 2.0 * xs_unit(r) - 1.0;
+                        r = xs_step(r);
                         double sp, cp;
-                        mqp::sincos2pi(mqp::xs_next(&rng), &sp, &cp);
-                        double omc = 1.0 - c * c;
-                        double sn = sqrt(omc > 0.0 ? omc : 0.0);
-                        double nn[3] = {sn * cp, sn * sp, c};
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) v[d] = v[d] - jc.mr * gv[d] + jc.mr * gl * nn[d];
-                        ncoll += 1;
+                        mqp::sincos2pi(xs_unit(r), &sp, &cp);
+                        const double omc = 1.0 - c * c;
+                        const double sn = sqrt(omc > 0.0 ? omc : 0.0);
+                        const double nn = d == 2 ? c : sn * (d == 0 ? cp : sp);
+                        const double vn = v - jc.mr * gv + jc.mr * gm * nn;
+                        if (hit) { v = vn; rng = r; ncoll += 1; }
                     }
                 }
             } else {
-                leg -= 1;
-                if (leg <= 0) {
-                    double vm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-                    if (vm > jc.floor_v) {
-                        double c = 2.0 * mqp::xs_next(&rng) - 1.0;
-                        double sp, cp;
-                        mqp::sincos2pi(mqp::xs_next(&rng), &sp, &cp);
-                        double omc = 1.0 - c * c;
-                        double sn = sqrt(omc > 0.0 ? omc : 0.0);
-                        double dd[3] = {sn * cp, sn * sp, c};
-                        double k1 = 1.0 - jc.mr, k2 = jc.mr * vm;
-#pragma unroll
-                        for (int d = 0; d < 3; ++d) v[d] = v[d] * k1 + k2 * dd[d];
-                        ncoll += 1;
-                    }
-                    double u = mqp::xs_next(&rng);
-                    double mfp = -mqp::log_(u > 1e-7 ? u : 1e-7) * jc.mfp_mean;
-                    double vn = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-                    double st = floor(mfp / (vn > 1e-3 ? vn : 1e-3) / dt);
-                    if (st < 1.0) st = 1.0;
-                    leg = !(st < 2147483647.0) ? 2147483647 : (int32_t)st;
+                uint64_t r = r1;
+                const bool hit = maybe && vm > jc.floor_v;
+                if (__any_sync(FULL, hit)) {
+                    const uint64_t r2 = xs_step(r1), r3 = xs_step(r2);
+                    const double c = 2.0 * xs_unit(r1) - 1.0;
+                    double sp, cp;
+                    mqp::sincos2pi(xs_unit(r2), &sp, &cp);
+                    const double omc = 1.0 - c * c;
+                    const double sn = sqrt(omc > 0.0 ? omc : 0.0);
+                    const double dd = d == 2 ? c : sn * (d == 0 ? cp : sp);
+                    const double k1 = 1.0 - jc.mr, k2 = jc.mr * vm;
+                    const double vn = v * k1 + k2 * dd;
+                    if (hit) { v = vn; r = r3; ncoll += 1; }
                 }
+                const double u = xs_unit(r);
+                const double mfp = -mqp::log_(u > 1e-7 ? u : 1e-7) * jc.mfp_mean;
+                const double n0 = shfl_d(v, base), n1 = shfl_d(v, base + 1), n2 = shfl_d(v, base + 2);
+                const double vn = sqrt(n0 * n0 + n1 * n1 + n2 * n2);
+                double st = floor(mfp / (vn > 1e-3 ? vn : 1e-3) / dt);
+                if (st < 1.0) st = 1.0;
+                if (maybe) { rng = r; leg = !(st < 2147483647.0) ? 2147483647 : (int32_t)st; }
             }
-            const long long bx = __double_as_longlong(x[0]), by = __double_as_longlong(x[1]), bz = __double_as_longlong(x[2]);
-            if (gt_pos(bz, k_exit)) { status = 3; break; }
-            if (lt_pos(bz, k_return)) { status = 2; break; }
-            if (lt_zero(bx) || lt_zero(by) || lt_zero(bz) || gt_pos(bx, k_lim0) || gt_pos(by, k_lim1) || gt_pos(bz, k_lim2)) {
-                status = 4;
-                break;
-            }
-            if (x[2] > b.crash_z0 && x[2] < b.crash_z1) {
-                int32_t ni = mqp::node_round(mqp::div_rn(x[0], h, g.inv_h), g.nx), nj = mqp::node_round(mqp::div_rn(x[1], h, g.inv_h), g.ny),
-                        nk = mqp::node_round(mqp::div_rn(x[2], h, g.inv_h), g.nz);
-                size_t q = (size_t)ni + nx * ((size_t)nj + ny * (size_t)nk);
-                q = MQ_CHK(q, nx * ny * (size_t)g.nz, MQ_SITE_F64_CRASH);
-                if (__ldg(&g.rf[q].w) > 0.5f) { status = 1; break; }
-            }
-            if (age >= b.max_steps) { status = 5; break; }
         }
-        io.x[i] = x[0]; io.y[i] = x[1]; io.z[i] = x[2];
-        io.vx[i] = v[0]; io.vy[i] = v[1]; io.vz[i] = v[2];
-        io.rng[i] = rng; io.steps[i] = age; io.ncoll[i] = ncoll; io.leg[i] = leg; io.status[i] = status;
+        if (some && __any_sync(FULL, moved)) t = refill(have, gx);
+        put_fractions(t);
+        // ---- termination tests: exit, return, box, conductor, time-out
+        if (some && __any_sync(FULL, edge || (have && mask != 0u))) {
+            const unsigned th = (unsigned)__double2hiint(t);
+            const long long bx = __double_as_longlong(x);
+            const long long kx = order_key(bx);
+            const bool in = !is_nan_bits(bx) && kx > order_key(__double_as_longlong(b.crash_z0)) &&
+                            kx < order_key(__double_as_longlong(b.crash_z1));
+            const unsigned own = (gt_pos(bx, __double_as_longlong(b.z_exit)) ? 1u : 0u) |
+                                 (lt_pos(bx, __double_as_longlong(b.z_return)) ? 2u : 0u) | (in ? 4u : 0u);
+            const unsigned zf = __shfl_sync(FULL, own, base + 2);
+            const unsigned out = (__ballot_sync(FULL, lt_zero(bx) || gt_pos(bx, __double_as_longlong(b.lim[d]))) >> base) & 7u;
+            const unsigned hb = (__ballot_sync(FULL, th >= 0x3fe00000u && th < 0x7ff00000u) >> base) & 7u;   // t >= 0.5
+            const unsigned near = ((hb & 1u) << 2) | (hb & 2u) | ((hb >> 2) & 1u);                             // nearest node's corner
+            if (have) {
+                status = (zf & 1u) ? 3 : (zf & 2u) ? 2 : out ? 4 : 0;
+                if (status == 0 && (zf & 4u) && ((mask >> near) & 1u)) status = 1;
+                if (status == 0 && age >= b.max_steps) status = 5;
+                put = status != 0 || left == 0u;
+            }
+        }
+        if (hands && iter % kPollSteps == 0) {   // few ions left: they go on in wider groups
+            const uint32_t open = *(volatile uint32_t*)&ctr->open, taken = *(volatile uint32_t*)head;
+            if (__shfl_sync(FULL, (open <= hand_at && (uint64_t)taken + groups >= count) ? 1 : 0, 0) != 0) {
+                give = have && !put;
+                drained = true;
+                turn = true;
+            }
+        }
+        __syncwarp();
+        if (__any_sync(FULL, put || give)) {
+            turn = true;
+            if (put || give) {
+                if (gl < 3) {
+                    (gl == 0 ? io.x : gl == 1 ? io.y : io.z)[id] = x;
+                    (gl == 0 ? io.vx : gl == 1 ? io.vy : io.vz)[id] = v;
+                }
+                if (gl == 0) {
+                    io.rng[id] = rng; io.steps[id] = age; io.ncoll[id] = ncoll; io.leg[id] = leg; io.status[id] = status;
+                    steps_total -= left;
+                    if (give) hand[atomicAdd(&ctr->handed, 1u)] = make_uint2(id, max_more - left);
+                    else {
+                        if (hands) atomicSub(&ctr->open, 1u);
+                        live += status == 0 ? 1u : 0u;
+                    }
+                }
+                have = false;
+            }
+        }
     }
-    // warp-aggregated step and live counters
-    unsigned long long s = done;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    uint32_t live = __popc(__ballot_sync(0xffffffffu, status == 0));
-    if ((threadIdx.x & 31) == 0) {
-        if (s) atomicAdd(d_steps, s);
-        if (live) atomicAdd(d_live, live);
+    for (int o = 16; o > 0; o >>= 1) {
+        steps_total += __shfl_down_sync(FULL, steps_total, o);
+        live += __shfl_down_sync(FULL, live, o);
     }
+    if (lane == 0) {
+        if (steps_total) atomicAdd(&ctr->steps, steps_total);
+        if (live) atomicAdd(&ctr->live, live);
+    }
+}
+
+// counters of one round of launches: n open ions, nothing taken or handed on
+__global__ void k_f64_begin(F64Ctrs* ctr, uint32_t n) {
+    ctr->live = ctr->head_a = ctr->head_b = ctr->handed = 0;
+    ctr->open = n;
 }
 
 __global__ void k_dc_combine(const float4* b0, const float4* b1, const float4* b2, const float4* b3,
@@ -272,9 +578,28 @@ cudaError_t launch_inject(const mqp::Batch& b, JobTable jt, DevIons io, uint32_t
 
 cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc, const double2* rf_tab,
                             const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more,
-                            unsigned long long* d_steps, uint32_t* d_live, cudaStream_t s) {
+                            F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels) {
     if (n == 0) return cudaSuccess;
-    k_f64_step<<<blocks_for(n, 128), 128, 0, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, d_steps, d_live);
+    int dev = 0, sms = 0;
+    cudaError_t e;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    // one block per SM: the shared memory asked for lets no second one in
+    if ((e = cudaFuncSetAttribute(k_f64_step<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPad)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_f64_step<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPad)) != cudaSuccess) return e;
+    k_f64_begin<<<1, 1, 0, s>>>(ctr, n);
+    const uint32_t wide = f64_hand_entries(sms);
+    if (n <= wide) {
+        k_f64_step<16><<<sms, kBlock, kPad, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr, nullptr, 0, 0);
+        *kernels += 2;
+    } else {
+        k_f64_step<4><<<sms, kBlock, kPad, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr, hand, hand ? wide : 0, 0);
+        *kernels += 2;
+        if (hand) {
+            k_f64_step<16><<<sms, kBlock, kPad, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr, hand, 0, 1);
+            *kernels += 1;
+        }
+    }
     return cudaGetLastError();
 }
 

@@ -34,11 +34,25 @@ struct JobTable {       // per-job device data for injection
 // per-job counters written by the summary kernel: [crashed, returned, transmitted, left, timeout, n, sum_coll, sum_steps]
 constexpr int kCounters = 8;
 
+// device counters of the FP64 step launches
+struct F64Ctrs {
+    unsigned long long steps;   // executed ion-steps
+    uint32_t live;              // ions still alive after the last launch
+    uint32_t bad;               // (allocation-free entry) job indices out of range
+    uint32_t head_a, head_b;    // queue heads of the narrow and the wide launch, beyond their first ions
+    uint32_t handed;            // ions the narrow launch handed to the wide one
+    uint32_t open;              // ions the narrow launch has not finished
+};
+
 // ---- mq_f64.cu
 cudaError_t launch_inject(const mqp::Batch& b, JobTable jt, DevIons io, uint32_t n, cudaStream_t s);
 cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc, const double2* rf_tab,
                             const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more,
-                            unsigned long long* d_steps, uint32_t* d_live, cudaStream_t s);
+                            F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels);
+// Ions that the 16-lane groups of one warp per scheduler hold: up to so many, a call steps them in
+// groups of 16 lanes. A larger call starts in groups of 4, which hand over the last so many of their
+// ions through a list of that length (null: they finish them themselves).
+inline uint32_t f64_hand_entries(int sms) { return 8u * (uint32_t)sms; }
 cudaError_t launch_phase_table(double w, uint32_t len, double2* out, cudaStream_t s);
 cudaError_t launch_dc_combine(const float4* b0, const float4* b1, const float4* b2, const float4* b3,
                               float v0, float v1, float v2, float v3, float4* out, size_t n, cudaStream_t s);

@@ -2,7 +2,8 @@
 // comment on mq_run_ions_device_noalloc in include/mq_engine.h).
 //
 // The FP64 step kernel needs two pieces of working memory besides the caller's inputs and
-// outputs: the per-job constant table and a pair of counters (executed steps, live ions).
+// outputs: the per-job constant table and a few counters (executed steps, live ions, queue heads).
+// It has no list for the wide groups, so groups of one width take a call from start to end.
 // Here both live in one file-scope static device array.  Host code never uses the array's
 // name as an address (on the host it only names a stand-in object): the device address is
 // looked up with cudaGetSymbolAddress with the device current, once per device and CUDA
@@ -17,7 +18,8 @@
 
 namespace {
 
-constexpr size_t kCounterBytes = 256;   // [0] u64 executed steps, [8] u32 live ions, [12] u32 bad job indices
+constexpr size_t kCounterBytes = 256;   // mqd::F64Ctrs
+static_assert(sizeof(mqd::F64Ctrs) <= kCounterBytes, "scratch layout");
 static_assert(sizeof(mqp::JobC) == 96, "scratch sizing assumes a 96-byte job record");
 static_assert(MQ_NOALLOC_SCRATCH_BYTES == kCounterBytes + MQ_NOALLOC_MAX_JOBS * sizeof(mqp::JobC), "scratch layout");
 
@@ -112,9 +114,8 @@ extern "C" mq_status mq_run_ions_device_noalloc(const mq_dev_grid* grid, const m
     unsigned char* base = nullptr;
     if (scratch_address(dev, &base) != cudaSuccess) return MQ_ERR_CUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    unsigned long long* d_steps = reinterpret_cast<unsigned long long*>(base);
-    uint32_t* d_live = reinterpret_cast<uint32_t*>(base + 8);
-    uint32_t* d_bad = reinterpret_cast<uint32_t*>(base + 12);
+    mqd::F64Ctrs* ctr = reinterpret_cast<mqd::F64Ctrs*>(base);
+    uint32_t* d_bad = &ctr->bad;
     mqp::JobC* d_jobs = reinterpret_cast<mqp::JobC*>(base + kCounterBytes);
 
     // every ion's job index must name one of the jobs: the states are device memory, so the check
@@ -149,23 +150,23 @@ extern "C" mq_status mq_run_ions_device_noalloc(const mq_dev_grid* grid, const m
     d.ph_rf = io->ph_rf; d.ph_ac = io->ph_ac; d.rng = io->rng; d.steps = io->steps; d.ncoll = io->ncoll;
     d.leg = io->leg; d.status = io->status; d.jid = io->jid;
 
-    if (cudaMemsetAsync(d_steps, 0, 8, st) != cudaSuccess) return MQ_ERR_CUDA;   // the scratch keeps old values
+    if (cudaMemsetAsync(ctr, 0, sizeof(*ctr), st) != cudaSuccess) return MQ_ERR_CUDA;   // the scratch keeps old values
     uint64_t budget = max_more;
+    uint32_t kernels = 0;
     for (;;) {
         const uint32_t L = budget < kChunk ? (uint32_t)budget : kChunk;
         if (L == 0) break;
-        if (cudaMemsetAsync(d_live, 0, 4, st) != cudaSuccess) return MQ_ERR_CUDA;
         // no phase tables (length 0): the kernel evaluates every drive phase directly
-        if (mqd::launch_f64_step(g, b, d_jobs, nullptr, nullptr, 0, d, (uint32_t)n, L, d_steps, d_live, st) != cudaSuccess)
+        if (mqd::launch_f64_step(g, b, d_jobs, nullptr, nullptr, 0, d, (uint32_t)n, L, ctr, nullptr, st, &kernels) != cudaSuccess)
             return MQ_ERR_CUDA;
         uint32_t live = 0;
-        if (cudaMemcpyAsync(&live, d_live, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
+        if (cudaMemcpyAsync(&live, &ctr->live, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
         if (cudaStreamSynchronize(st) != cudaSuccess) return MQ_ERR_CUDA;
         budget -= L;
         if (live == 0) break;
     }
     unsigned long long steps = 0;
-    if (cudaMemcpyAsync(&steps, d_steps, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
+    if (cudaMemcpyAsync(&steps, &ctr->steps, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
     if (cudaStreamSynchronize(st) != cudaSuccess) return MQ_ERR_CUDA;
     if (ion_steps) *ion_steps = steps;
     return MQ_OK;

@@ -100,6 +100,14 @@ __device__ __forceinline__ double widen(float f) {
     return __hiloint2double((int)hi, (int)(u << 29));
 }
 
+// the same without a branch for zeros and normal numbers; `odd` is set for any other value
+__device__ __forceinline__ double widen_normal(float f, bool& odd) {
+    const uint32_t u = __float_as_uint(f), m = u & 0x7FFFFFFFu;
+    odd |= m - 0x800000u >= 0x7F000000u && m != 0u;
+    const uint32_t hi = ((uint32_t)((int32_t)u >> 3) & 0x8FFFFFFFu) + (m ? 0x38000000u : 0u);
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
 // x / h correctly rounded without a division (h > 0, inv_h = RN(1/h)): q = x * inv_h, then one
 // step of Markstein's correction q + (x - q h) inv_h with fused multiply-adds (P. Markstein, IBM J.
 // Res. Dev. 34 (1990) 111-119: with a correctly rounded reciprocal and a quotient within one ulp,
