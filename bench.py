@@ -36,7 +36,7 @@ sys.path.insert(0, str(ROOT))
 METRIC = "ion-steps/s, 1 GB300: batched mixed-precision vs plain FP64 at matched outcomes"
 UNIT = "ion-steps/s"
 # Bytes the stepping kernel must move, counted by the kernel itself: every cell-cache fill reads the
-# 8 corner node records of a cell (64 or 48 B each), and every ion it takes from the queue reads its
+# 8 corners of a cell (8 narrow records of 48 B, or 4 wide ones of 96 B, each with the node above), and every ion it takes from the queue reads its
 # working state and job constants and writes them back (ION_STATE_BYTES).  The 384 B of corner
 # values an ion-step interpolates (8 corners x 3 float4) come from registers between fills.
 CORNERS = 8
@@ -45,10 +45,10 @@ ION_STATE_BYTES = 48 + 16 + 24 + 56 + 64   # double-floats, phase offsets, count
 
 def stepping_bytes(stats, wide: bool, nearest: bool = False) -> float:
     """Algorithmic bytes of the stepping kernel(s) of one call, from the kernel's own counters: cell
-    fills x 8 node records (1 record in the nearest-node field mode, which reads only the cell's
-    lowest corner), plus the state traffic of every ion taken from the work queue."""
-    rec = 64 if wide else 48
-    return float(stats.cell_loads) * (1 if nearest else CORNERS) * rec + float(stats.ions_queued) * ION_STATE_BYTES
+    fills x 8 narrow or 4 wide node records (1 record in the nearest-node field mode, which reads only
+    the cell's lowest corner), plus the state traffic of every ion taken from the work queue."""
+    rec, per_fill = (96, CORNERS // 2) if wide else (48, CORNERS)
+    return float(stats.cell_loads) * (1 if nearest else per_fill) * rec + float(stats.ions_queued) * ION_STATE_BYTES
 
 
 def cpu_model() -> str:
@@ -189,7 +189,7 @@ def run_gridstudy(args, rank: int, world: int):
             agree = float(np.mean(ions_m.status == ions_d.status))
         nodes = f.nx * f.ny * f.nz
         grids.append({"h_mm": h, "dims": [f.nx, f.ny, f.nz], "nodes": nodes,
-                      "node_records_gb": nodes * (64 if tuned["wide_records"] else 48) / 1e9, "solve_s": t_solve,
+                      "node_records_gb": nodes * (96 if tuned["wide_records"] else 48) / 1e9, "solve_s": t_solve,
                       "tuning": tuned,
                       "mixed": {"value": rate, "unit": UNIT, "ms_per_step": float(np.mean(ms)), "gpu_launches": int(launches),
                                 "e2e": steps / float(np.mean(walls)), "ion_steps": int(steps),
@@ -343,7 +343,7 @@ def run_legacy(args, rank: int, world: int):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": None, "peak_source": "measured hbm_gbs" if peaks.get("hbm_gbs") else "fallback",
                          "kernel": "k_mixed (legacy collisions, nearest-node fields)",
-                         "algorithmic_bytes": f"cell fills counted by the kernel x 1 node record ({64 if tuned['wide_records'] else 48} B) "
+                         "algorithmic_bytes": f"cell fills counted by the kernel x 1 node record ({96 if tuned['wide_records'] else 48} B) "
                                               f"+ {ION_STATE_BYTES} B per ion taken from the queue",
                          "cell_loads_per_ion_step": loads / max(steps, 1)},
             "roofline_l2": {"achieved": achieved, "peak": l2, "unit": "GB/s", "frac": achieved / l2 if l2 else None},
@@ -891,7 +891,7 @@ def main():
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                              "traffic": None, "peak_source": f"{peak_src} hbm_gbs",
                              "kernel": "k_mixed",
-                             "algorithmic_bytes": f"cell fills counted by the kernel x 8 node records ({64 if wide else 48} B) "
+                             "algorithmic_bytes": f"cell fills counted by the kernel x {'4 node records (96 B)' if wide else '8 node records (48 B)'} "
                                                   f"+ {ION_STATE_BYTES} B per ion taken from the queue",
                              "algorithmic_bytes_per_ion_step": moved / max(steps_total, 1),
                              "cell_loads_per_ion_step": loads / max(steps_total, 1)},

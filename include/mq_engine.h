@@ -136,8 +136,8 @@ typedef struct mq_tuning {
     uint32_t chunk;              /* steps per ion per launch (compaction interval)         */
     int32_t use_graph;           /* replay the launch sequence as one CUDA graph           */
     int32_t prefetch;            /* L1-prefetch the cell each ion is heading for           */
-    int32_t wide_records;        /* 64-byte node records read with 256-bit loads (else 48 B;
-                                    needs 4 x nodes below 2^32)                            */
+    int32_t wide_records;        /* 96-byte records of a node and the one above it, read with
+                                    256-bit loads (else 48 B; needs 4 x nodes below 2^32)  */
     int32_t sort_cells;          /* before every launch, put the live ions in the Morton order
                                     of their cells (a counting sort on the device)         */
 } mq_tuning;

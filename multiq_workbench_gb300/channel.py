@@ -336,7 +336,7 @@ class Engine:
 
     def set_tuning(self, blocks_per_sm: int | None = None, chunk: int | None = None, use_graph: bool | None = None,
                    prefetch: bool | None = None, wide_records: bool | None = None, sort_cells: bool | None = None) -> None:
-        """Override the mixed engine's launch shape; ``wide_records`` picks 64-byte node records read
+        """Override the mixed engine's launch shape; ``wide_records`` picks 96-byte node records read
         with 256-bit loads (the default on grids below 1 GB of 48-byte records) over 48-byte ones;
         ``sort_cells`` puts every launch's live ions in the Morton order of their cells."""
         cur = self.tuning()

@@ -70,7 +70,7 @@ __device__ __forceinline__ size_t mq_chk_span(size_t i, size_t span, size_t n, u
 // site ids
 enum MqCheckSite : unsigned {
     MQ_SITE_F64_FIELD = 1, MQ_SITE_F64_CRASH = 2,
-    MQ_SITE_MIX_CELL = 10, MQ_SITE_MIX_ION = 11, MQ_SITE_MIX_LIST_OUT = 12,
+    MQ_SITE_MIX_CELL = 10, MQ_SITE_MIX_ION = 11, MQ_SITE_MIX_LIST_OUT = 12, MQ_SITE_MIX_HAND = 13,
     MQ_SITE_TDM_CUBE = 20, MQ_SITE_TDM_PORT = 21, MQ_SITE_TDM_GATE = 22, MQ_SITE_TDM_CRASH = 23,
     MQ_SITE_TMX_CELL = 30, MQ_SITE_TMX_LIST = 31,
     MQ_SITE_SELFTEST = 99,

@@ -425,7 +425,7 @@ mq_status mq_engine_create(const mq_grid_desc* g, int32_t precision, int32_t dev
     for (int i = 0; i < 8; ++i) e->layers[i] = g->layers_mm[i];
     e->nnodes = (size_t)g->nx * g->ny * g->nz;
     auto bail = [&](mq_status s) { mq_engine_destroy(e); return s; };
-    // the mixed kernel addresses its 3 (or 4, wide) float4 of node record per node with 32-bit offsets
+    // the mixed kernels address narrow records, 3 float4 per node, with 32-bit offsets
     if (precision == MQ_PREC_MIXED && 3 * e->nnodes >= ((size_t)1 << 32)) {
         e->err = "grid too large for the mixed engine (3 x nodes must be below 2^32)";
         return bail(MQ_ERR_TOO_LARGE);

@@ -10,7 +10,9 @@
 //   * positions in grid units and velocities in cells per step, each an FP32 double-float
 //     (compensated two-sum accumulator); field nodes, interpolation and collision
 //     kinematics in FP32;
-//   * fields as interleaved node records of 64 bytes (256-bit loads) or 48 bytes, by grid size;
+//   * a second kernel with four lanes per ion for the lists that leave the chip idle: short ones, and
+//     the last ions of a long one;
+//   * fields as interleaved node records of 96 bytes (256-bit loads) or 48 bytes, by grid size;
 //     the 8 corners of the ion's cell x {RF, DC, AC} held in registers and reloaded only when
 //     the ion changes cell (the cached conductor bits of the corners give the nearest-node
 //     crash test), with an optional L1 prefetch of the cell the ion is heading for;
@@ -37,10 +39,14 @@ using namespace mqx;
 
 constexpr unsigned FULL = 0xffffffffu;
 
-struct Ctrs {                       // device counters (40 B)
+constexpr int kMaxLegs = 10;         // lane-group launches of one round
+
+struct Ctrs {                       // device counters
     uint32_t head;                  // work-queue head of the current launch
     uint32_t count[2];              // live-list lengths (ping-pong)
-    uint32_t pad;
+    uint32_t open;                  // ions the current launch has not finished
+    uint32_t head_g[kMaxLegs];      // queue heads of the lane-group launches, beyond their first ions
+    uint32_t handed[kMaxLegs + 2];  // ions handed to each of them, by k_mixed or by the one before
     unsigned long long steps;       // executed ion-steps
     unsigned long long cell_loads;  // cell-cache fills (8 node records each)
     unsigned long long queued;      // ions queued over the call's launches
@@ -80,13 +86,15 @@ __device__ __forceinline__ void rotate(float& s, float& c, float cw, float sw) {
 }
 
 // ---------------------------------------------------------------- cell cache
-// Interleaved node records: node q occupies float4 [Sq] = {RF.xyz, conductor mask},
-// [Sq+1] = {combined DC.xyz, conductor bits of the cell based at q}, [Sq+2] = {AC.xyz, 0}, with
-// a record stride S of 3 float4 (48 B) or 4 (64 B, the last float4 spare), so the 8 corners of a
-// cell are 4 runs of 2 records. Wide records are 64-byte aligned and read with two 256-bit loads
-// each (16 loads a reload instead of 24): faster where the cell reloads hit L2 (about 5% on the
-// 0.100 mm channel), slower on fine grids whose gathers reach HBM and pay for the 33% larger
-// footprint (0.050 mm: 10.7 against 17.3 G ion-steps/s).
+// Node records, interleaved by field component d (RF, combined DC, AC of one component side by side, so
+// that a lane which needs one component reads one piece), each with the conductor bits of the cell
+// based at the node:
+//   narrow  48 B: float4 [3q + d] = {RF, DC, AC, bits}: a cell is 4 runs of 2 records (x neighbours);
+//   wide    96 B: float4 [6q + 2d] = {RF, RF', DC, DC'}, [6q + 2d + 1] = {AC, AC', bits, 0}, the primes from
+//           the node above (z + 1): a cell is 2 runs of 2 records, 12 sectors and 12 256-bit loads (4 for
+//           a lane of a group), and the values come in the pairs that two-at-a-time arithmetic takes.
+// Wide records are faster where the cell reloads hit L2, slower on fine grids whose gathers reach HBM
+// and pay for twice the footprint.
 struct Cell {
     float R[3][8], D[3][8], A[3][8];   // corner values per field and component, corner q = a + 2b + 4c
     int32_t ci, cj, ck;
@@ -94,8 +102,8 @@ struct Cell {
     uint32_t mask;                      // conductor bit per corner
 };
 
-// record offsets are 32-bit (the host refuses grids with S x nodes >= 2^32): less address arithmetic
-// in the divergent reload path (measured about 1% on the sweep)
+// node indices are 32-bit (the host refuses grids with 3 x nodes >= 2^32): less address arithmetic in
+// the divergent reload path (measured about 1% on the sweep)
 __device__ __forceinline__ uint32_t node_of(const MixBatch& B, int32_t ci, int32_t cj, int32_t ck) {
     return (uint32_t)ci + (uint32_t)B.nx * ((uint32_t)cj + (uint32_t)B.ny * (uint32_t)ck);
 }
@@ -111,34 +119,39 @@ __device__ __forceinline__ void ld256_na(const float4* p, float4& a, float4& b) 
 template <bool WIDE, bool NEAREST>
 __device__ __forceinline__ void load_cell(const float4* __restrict__ nodes, const MixBatch& B, int32_t ci, int32_t cj,
                                           int32_t ck, Cell& c) {
-    constexpr uint32_t S = WIDE ? 4u : 3u;
     const uint32_t sy = (uint32_t)B.nx, sz = (uint32_t)B.nx * (uint32_t)B.ny;
     const uint32_t base = node_of(B, ci, cj, ck);
     uint32_t m = 0;
+    if (WIDE) {
 #pragma unroll
-    for (int q = 0; q < (NEAREST ? 1 : 8); ++q) {
-        uint32_t o = S * (base + (uint32_t)(q & 1) + ((q & 2) ? sy : 0u) + ((q & 4) ? sz : 0u));
-        o = (uint32_t)MQ_CHK_SPAN(o, S, S * (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
-        float4 r, d, a;
-        if (WIDE && !NEAREST) {
-            // 64-byte records: both loads are 32-byte aligned. Wide records serve the grids whose
-            // fills hit L2; left out of L1 they do not evict the lines the narrow-record grids
-            // depend on either way (5% on the sweep; the fine grids' 48-byte fills lose 3x
-            // without L1, so they keep it)
-            float4 spare;
-            ld256_na(nodes + o, r, d);
-            ld256_na(nodes + o + 2, a, spare);
-        } else if (WIDE) {
-            float4 spare;
-            ld256(nodes + o, r, d);
-            ld256(nodes + o + 2, a, spare);
-        } else {
-            r = __ldg(nodes + o); d = __ldg(nodes + o + 1); a = __ldg(nodes + o + 2);
+        for (int q = 0; q < (NEAREST ? 1 : 4); ++q) {
+            uint32_t o = base + (uint32_t)(q & 1) + ((q & 2) ? sy : 0u);
+            o = (uint32_t)MQ_CHK(o, (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
+            const float4* p = nodes + (size_t)6 * o;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                float4 u, v;
+                // left out of L1: these grids' fills hit L2, and the kernel's other data keeps the L1
+                // (5% on the sweep)
+                if (NEAREST) ld256(p + 2 * d, u, v);
+                else ld256_na(p + 2 * d, u, v);
+                c.R[d][q] = u.x; c.D[d][q] = u.z; c.A[d][q] = v.x;
+                if (!NEAREST) { c.R[d][q + 4] = u.y; c.D[d][q + 4] = u.w; c.A[d][q + 4] = v.y; }
+                if (q == 0 && d == 0) m = __float_as_uint(v.z);   // conductor bits of the cell's corners
+            }
         }
-        c.R[0][q] = r.x; c.R[1][q] = r.y; c.R[2][q] = r.z;
-        c.D[0][q] = d.x; c.D[1][q] = d.y; c.D[2][q] = d.z;
-        c.A[0][q] = a.x; c.A[1][q] = a.y; c.A[2][q] = a.z;
-        if (q == 0) m = __float_as_uint(d.w);   // conductor bits of the cell's corners
+    } else {
+#pragma unroll
+        for (int q = 0; q < (NEAREST ? 1 : 8); ++q) {
+            uint32_t o = 3u * (base + (uint32_t)(q & 1) + ((q & 2) ? sy : 0u) + ((q & 4) ? sz : 0u));
+            o = (uint32_t)MQ_CHK_SPAN(o, 3u, 3u * (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
+            // through L1, which these grids' fills depend on: neighbouring cells share a face
+            const float4 x = __ldg(nodes + o), y = __ldg(nodes + o + 1), z = __ldg(nodes + o + 2);
+            c.R[0][q] = x.x; c.R[1][q] = y.x; c.R[2][q] = z.x;
+            c.D[0][q] = x.y; c.D[1][q] = y.y; c.D[2][q] = z.y;
+            c.A[0][q] = x.z; c.A[1][q] = y.z; c.A[2][q] = z.z;
+            if (q == 0) m = __float_as_uint(x.w);
+        }
     }
     c.ci = ci; c.cj = cj; c.ck = ck; c.mask = m;
     c.fci = (float)ci; c.fcj = (float)cj; c.fck = (float)ck;
@@ -151,9 +164,15 @@ __device__ __forceinline__ void prefetch_cell(const float4* nodes, const MixBatc
     const uint32_t base = node_of(B, ci, cj, ck);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        const float4* p = nodes + (WIDE ? 4 : 3) * (base + ((r & 1) ? sy : 0) + ((r & 2) ? sz : 0));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(p + (WIDE ? 7 : 5)));
+        if (WIDE) {   // two runs of two 96-byte records
+            const float4* p = nodes + (size_t)6 * (base + ((r & 2) ? sy : 0u) + (uint32_t)(r & 1));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 5));
+        } else {
+            const float4* p = nodes + 3 * (base + ((r & 1) ? sy : 0) + ((r & 2) ? sz : 0));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 5));
+        }
     }
 }
 
@@ -177,12 +196,24 @@ __device__ __forceinline__ float df_diff(float xh, float xl, float th, float tl)
     return __fadd_rn(__fsub_rn(xh, th), __fsub_rn(xl, tl));
 }
 
+// an ion's counters to its state, its position and velocity to the working state
+__device__ __forceinline__ void put_ion(const DevIons& io, float* __restrict__ keep, uint32_t n_all, uint32_t id, uint32_t n, uint32_t ncoll,
+                                        int32_t leg, int32_t status, const float xh[3], const float xl[3], const float uh[3],
+                                        const float ul[3]) {
+    io.steps[id] = n; io.ncoll[id] = ncoll; io.leg[id] = leg; io.status[id] = status;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        keep[(size_t)(0 + d) * n_all + id] = xh[d]; keep[(size_t)(3 + d) * n_all + id] = xl[d];
+        keep[(size_t)(6 + d) * n_all + id] = uh[d]; keep[(size_t)(9 + d) * n_all + id] = ul[d];
+    }
+}
+
 // ---------------------------------------------------------------- the persistent worker
 template <bool LEGACY, bool PREFETCH, bool WIDE, bool NEAREST>
-__global__ void __launch_bounds__(128, 3)
+__global__ void __launch_bounds__(128, NEAREST ? 5 : 3)
 k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__ jobs, DevIons io,
         const uint32_t* __restrict__ list_in, uint32_t* __restrict__ list_out, Ctrs* ctr, int in_slot, uint32_t chunk,
-        float* __restrict__ keep, const uint64_t* __restrict__ kph, uint32_t n_all) {
+        float* __restrict__ keep, const uint64_t* __restrict__ kph, uint32_t n_all, uint2* __restrict__ hand, uint32_t hand_at) {
     // keep: the working state of every ion of the call in grid units, double-float position and
     // velocity (12 floats per ion, structure of arrays over n_all), filled from the FP64 states by
     // k_init_list and written back to them by k_unstage, so this kernel does no FP64 arithmetic;
@@ -193,10 +224,12 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
     __shared__ float sj_sgas[128], sj_mr[128], sj_floor[128], sj_mfp[128];
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t count = ctr->count[in_slot];
-    if (count == 0) return;
+    if (count <= hand_at) return;   // the lane-group launch takes them
     uint32_t* count_out = &ctr->count[in_slot ^ 1];
 
-    bool have = false, drained = false;
+    // lanes that take ions: all 32 when the list fills the grid, else the warp's even share of it
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    bool have = false, drained = lane >= (count + warps - 1) / warps;
     uint32_t id = 0, jid = 0, n = 0, done = 0, ncoll = 0;
     int32_t leg = 0;
     float xh[3], xl[3], uh[3], ul[3];
@@ -224,9 +257,25 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
     // the last 4 iterations are appended to the next launch's list, then lanes without an ion are
     // refilled (a lane that finished waits at most 3 iterations; 1.8% on the sweep and 3% on the
     // legacy scan against ballots every iteration).
-    bool append = false;
+    bool append = false, ended = false;
     for (;;) {
       if ((iter & 3u) == 0u) {
+        // ---- ions that ended; when the queue is empty and few are left, they go on in lane groups
+        const unsigned em = __ballot_sync(FULL, ended);
+        if (em && lane == 0) atomicSub(&ctr->open, (uint32_t)__popc(em));
+        ended = false;
+        if ((iter & 31u) == 0u && __any_sync(FULL, drained)) {
+            const uint32_t open = __shfl_sync(FULL, *(volatile uint32_t*)&ctr->open, 0);
+            if (open <= hand_at) {
+                if (have) {
+                    hand[MQ_CHK(atomicAdd(&ctr->handed[0], 1u), hand_at, MQ_SITE_MIX_HAND)] = make_uint2(id, done);
+                    put_ion(io, keep, n_all, id, n, ncoll, leg, 0, xh, xl, uh, ul);
+                    steps_total += done;
+                    have = false;
+                }
+                drained = true;
+            }
+        }
         // ---- warp-ballot compaction of survivors into the next launch's list
         const unsigned am = __ballot_sync(FULL, append);
         if (am) {
@@ -443,8 +492,8 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             // (the loss-surface planes - exit, return and the crash window - are crossed on the full
             // double-float position against the double-float thresholds; the box test is the
             // unclamped cell index leaving [0, n-2])
-            // A plane more than one cell away cannot be crossed whatever the low parts hold, so the
-            // exact test runs only within a cell of it; the crash window matters only in a cell with
+            // A plane farther away than the low parts reach cannot be crossed, so the exact test runs
+            // only close to it; the crash window matters only in a cell with
             // a conductor corner (most cells have none).
             int32_t status = 0;
             if (xh[2] > B.z_exit_near && df_diff(xh[2], xl[2], B.z_exit_h, B.z_exit_l) > 0.0f) status = 3;
@@ -466,12 +515,8 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             if (status != 0 || done >= chunk) {
                 // ---- write back: counters to the ion states, position and velocity to the working
                 //      state (k_unstage turns it into the FP64 state when the caller wants that)
-                io.steps[id] = n; io.ncoll[id] = ncoll; io.leg[id] = leg; io.status[id] = status;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    keep[(size_t)(0 + d) * n_all + id] = xh[d]; keep[(size_t)(3 + d) * n_all + id] = xl[d];
-                    keep[(size_t)(6 + d) * n_all + id] = uh[d]; keep[(size_t)(9 + d) * n_all + id] = ul[d];
-                }
+                put_ion(io, keep, n_all, id, n, ncoll, leg, status, xh, xl, uh, ul);
+                ended = true;
                 steps_total += done;
                 append = status == 0;
                 have = false;
@@ -487,26 +532,431 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
     if (lane == 0 && loads) atomicAdd(&ctr->cell_loads, (unsigned long long)loads);
 }
 
-// interleave RF | combined DC | AC into node records of `stride` float4 (once per DC configuration
-// and record width); the spare w of the DC record holds the conductor bits of the 8 corners of the
-// cell whose lowest corner is this node (bit a + 2b + 4c), so a cell reload reads its crash mask in
-// one word
+// ---------------------------------------------------------------- lane groups
+// The same steps with four lanes per ion, for lists that leave the chip idle (few ions, or the last
+// ones of a large batch): there the time of a step is what counts, not lanes. Lanes 0..2 each hold
+// one axis (position, velocity, cell, and that component of the cell's field records: one read per
+// corner pair); lane 3 repeats lane 0. The fractions and velocities that all axes need go round by
+// shuffles. What depends on the step count alone is prepared 16 steps at a time, a part in each lane,
+// and lies in shared memory: the drive amplitudes, and the candidates' uniforms or the legacy
+// collisions' directions and free paths. Every operation is k_mixed's, on the same numbers, so an
+// ion's states do not depend on which kernel steps it.
+// What bounds it: the latency of one step's chain (position -> fractions -> field -> kick -> position)
+// and, with many ions to a warp, the reload of some ion's cell on nearly every step; so the chain is kept
+// short (one vote clears most steps) and registers few. A step takes 0.27 us for up to 608 ions,
+// 0.44 for 4,864 and 0.57 for 19,456 (S14 grid), where the one-lane kernel takes 0.8 to 1.1; from there
+// on the one-lane kernel's 58,368 ions in flight win (1.15 us a step), so longer lists start with it.
+// Measured, whole run_batch calls, one-lane kernel with 64-byte records -> now: 1,000 ions at one point
+// 2.25 -> 1.04 ms; mass scan of 25,000 short-lived ions 1.26 -> 0.82; Fig. 4 legacy scan 21.2 -> 10.8;
+// S14 sweep of 62,000 ions 76.7 -> 39.9; sweep of 4.2 million ions 63.7 -> 55.6.
+// One block per SM, as many warps as the registers hold (16 at 128 a thread; 24 at 80 where the nearest
+// node's record is the whole cell).
+constexpr int group_block(bool nearest) { return nearest ? 768 : 512; }
+// Warps per SM that share the ions: two a scheduler, which hide each other's waits; more only once these
+// would hold over eight ions each (9,728 ions of the S14 grid: 0.49 us a step with 8 warps, 0.51 with 16)
+constexpr uint32_t kGroupFirst = 8;
+
+// Shared floats of a group: 16 steps x {RF, AC} amplitudes, then 16 x {uniform} or 16 x {direction, free path}
+// (and 4 more, so that the 8 groups of a warp read different banks)
+__host__ __device__ constexpr int group_floats(bool legacy) { return 36 + (legacy ? 64 : 16); }
+// two FP32 operations in one instruction, each rounded as alone
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+template <bool LEGACY, bool WIDE, bool NEAREST>
+__global__ void __launch_bounds__(group_block(NEAREST), 1)
+k_mixed_group(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__ jobs, DevIons io,
+              const uint32_t* __restrict__ list_in, uint2* __restrict__ hand, uint32_t* __restrict__ list_out, Ctrs* ctr,
+              int in_slot, uint32_t chunk, int leg_no, uint32_t leg_steps, float* __restrict__ keep,
+              const uint64_t* __restrict__ kph, uint32_t n_all, uint32_t hand_at) {
+    constexpr int NQ = NEAREST ? 1 : 4;
+    const uint32_t lane = threadIdx.x & 31u, gl = lane & 3u, base = lane & ~3u, warp = threadIdx.x >> 5;
+    // Legs of one round: each steps its ions by at most leg_steps and hands on those that are neither ended
+    // nor at the round's `chunk` steps; the next starts with full warps again. The first leg takes a short
+    // list whole, of a long one what k_mixed handed on.
+    const bool direct = leg_no == 0 && ctr->count[in_slot] <= hand_at;
+    const uint32_t count = direct ? ctr->count[in_slot] : ctr->handed[leg_no];
+    if (count == 0) return;
+    const uint2* const from = hand + (size_t)(leg_no & 1) * hand_at;
+    uint2* const to = hand + (size_t)((leg_no & 1) ^ 1) * hand_at;
+    const uint32_t groups = gridDim.x * (blockDim.x >> 2);
+    const uint32_t warps = blockDim.x >> 5, full = (count + 8u * gridDim.x - 1u) / (8u * gridDim.x);
+    const uint32_t lead = full < kGroupFirst ? kGroupFirst : full > warps ? warps : full;
+    const uint32_t first = warp < lead ? ((lane >> 2) * lead + warp) * gridDim.x + blockIdx.x
+                                       : (8u * lead + (lane >> 2) * (warps - lead) + warp - lead) * gridDim.x + blockIdx.x;
+    extern __shared__ __align__(16) float group_sm[];
+    float* const drive = group_sm + (size_t)(threadIdx.x >> 2) * group_floats(LEGACY);
+    float* const draws = drive + 32;
+    const int d = gl == 3u ? 0 : (int)gl;
+    const bool is_z = gl == 2u, is_ac = (gl & 1u) != 0u;
+    const int32_t top = (d == 0 ? B.nx : d == 1 ? B.ny : B.nz) - 2;
+    const float lim = d == 0 ? B.lim_x : d == 1 ? B.lim_y : B.lim_z;
+    const uint32_t sy = (uint32_t)B.nx, sz = (uint32_t)B.nx * (uint32_t)B.ny;
+    const uint32_t stride = gl == 0u ? 1u : gl == 1u ? sy : gl == 2u ? sz : 0u;
+    const size_t row = (size_t)(WIDE ? 6u : 3u) * sy, layer = (size_t)3 * sz;   // to the y and z neighbours' records
+    // positions that no plane or face can end: beyond them the exact tests run
+    const float in_lo = is_z ? fmaxf(B.z_ret_near, 0.0f) : 0.0f, in_hi = is_z ? fminf(B.z_exit_near, lim - 0.0625f) : lim - 0.0625f;
+
+    // Every lane of the warp runs every step together (the shuffles then need no lane masks): a group
+    // without an ion moves a particle of speed 1 that no force acts on, and keeps nothing. (Zeros,
+    // infinities and NaN would take the slow branch of the square roots, every step, for the whole warp.)
+    bool have = false, waits = false, drained = false, fresh = true;
+    bool idle = true;                    // some group of the warp has no ion under way
+    uint32_t id = 0, jid = 0, n = 0, n0 = 0, done = 0, stop = 0, ncoll = 0, k0 = 0, k1 = 0, mask = 0, loads = 0;
+    int32_t leg = 0;
+    float xh = 0.f, xl = 0.f, uh = 1.f, ul = 0.f, fc = 0.f;
+    // the component's RF, DC and AC values: corner q in the low half, q + 4 (z + 1) in the high one
+    uint64_t R[NQ], D[NQ], A[NQ];
+    uint64_t P = 0, W = 0;
+    float cw = 1.f, sw = 0.f, amp = 0.f, kick = 0.f, ca2 = 0.f, cand_b = 0.f;
+    float mr = 0.f, floor_v = 0.f, mfp_mean = 0.f;     // legacy collisions
+    unsigned long long steps_total = 0;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) R[q] = D[q] = A[q] = 0;
+
+    // node records of the cell that holds the group's position, the lane's component
+    auto fill = [&](bool go) {
+        const int32_t ci = clampi(__float2int_rd(xh), 0, top);
+        uint32_t o = (uint32_t)ci * stride;
+        o += __shfl_xor_sync(FULL, o, 1);
+        o += __shfl_xor_sync(FULL, o, 2);
+        if (!go) return;
+        fc = (float)ci;
+        ++loads;
+        o = (uint32_t)MQ_CHK(o, (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
+        const float4* const p = nodes + (size_t)(WIDE ? 6u : 3u) * o + (WIDE ? 2 : 1) * d;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const float4* pq = p + ((q & 1) ? (WIDE ? 6 : 3) : 0) + ((q & 2) ? row : 0);
+            float4 u, v;
+            if (WIDE) {
+                ld256(pq, u, v);
+                if (q == 0) mask = __float_as_uint(v.z);
+            } else {
+                const float4 r = __ldg(pq), t = NEAREST ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldg(pq + layer);
+                u = make_float4(r.x, t.x, r.y, t.y);
+                v = make_float4(r.z, t.z, 0.f, 0.f);
+                if (q == 0) mask = __float_as_uint(r.w);
+            }
+            R[q] = pack2(u.x, u.y); D[q] = pack2(u.z, u.w); A[q] = pack2(v.x, v.y);
+        }
+    };
+    // tables of the 16-step block that holds step n (P is the drive phase at its start): each lane one
+    // window of four steps of the draws, and two windows of its drive (lanes 0, 1 the first two, 2, 3 the others):
+    // exact at a window's start, then rotated
+    auto block = [&]() {
+        const uint32_t w = ((n >> 4) << 2) + gl;
+        if (LEGACY) {
+            // a collision at window step q takes words 2q and 2q + 1 of the window's two blocks: cos(theta)
+            // from the top 24 bits of the first, the free path from the top 24 of the second, phi from their low bytes
+            const uint4 ra = philox(k0, k1, w, 2u, 0u, 0u), rb = philox(k0, k1, w, 3u, 0u, 0u);
+            const uint32_t wa[4] = {ra.x, ra.z, rb.x, rb.z}, wb[4] = {ra.y, ra.w, rb.y, rb.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float cth = 2.0f * unif(wa[q]) - 1.0f;
+                float sp, cp;
+                angle_sincos(unif16(((wa[q] & 0xffu) << 8) | (wb[q] & 0xffu)), &sp, &cp);
+                const float sn = sqrtf(fmaxf(0.0f, 1.0f - cth * cth));
+                reinterpret_cast<float4*>(draws)[4u * gl + q] =
+                    make_float4(sn * cp, sn * sp, cth, -__logf(fmaxf(unif(wb[q]), 1e-7f)));
+            }
+        } else {
+            const uint4 r = philox(k0, k1, w, 0u, 0u, 0u);
+            reinterpret_cast<float4*>(draws)[gl] = make_float4(unif(r.x), unif(r.y), unif(r.z), unif(r.w));
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t q0 = ((gl & 2u) + (uint32_t)k) * 4u;
+            float s, c;
+            turn_sincos(P + (uint64_t)q0 * W, s, c);
+#pragma unroll
+            for (uint32_t q = 0; q < 4u; ++q) {
+                drive[2u * (q0 + q) + (gl & 1u)] = amp * s;
+                rotate(s, c, cw, sw);
+            }
+        }
+        P += 16u * W;
+    };
+
+    // exact termination tests: exit, return, box, conductor, time-out
+    auto test = [&](float ff) {
+        int32_t status = 0;
+        uint32_t zf = 0;
+        if (is_z) {
+            if (xh > B.z_exit_near && df_diff(xh, xl, B.z_exit_h, B.z_exit_l) > 0.0f) zf = 3;
+            else if (xh < B.z_ret_near && df_diff(xh, xl, B.z_ret_h, B.z_ret_l) < 0.0f) zf = 2;
+            if (df_diff(xh, xl, B.cz0_h, B.cz0_l) > 0.0f && df_diff(xh, xl, B.cz1_h, B.cz1_l) < 0.0f) zf |= 4;
+        }
+        zf = __shfl_sync(FULL, zf, base + 2);
+        const unsigned out = (__ballot_sync(FULL, ff < 0.0f || ff > lim - 1.0f) >> base) & 7u;
+        const unsigned corner = (__ballot_sync(FULL, __fadd_rn(__fsub_rn(xh, fc), xl) >= 0.5f) >> base) & 7u;
+        if (zf & 3u) status = (int32_t)(zf & 3u);
+        else if (out) status = 4;
+        else if (mask != 0u && (zf & 4u) && ((mask >> corner) & 1u)) status = 1;
+        else if (n >= B.max_steps) status = 5;
+        if (have && (!LEGACY || n != n0) && (status != 0 || n >= stop)) {
+            if (gl < 3u) {
+                keep[(size_t)d * n_all + id] = xh; keep[(size_t)(3 + d) * n_all + id] = xl;
+                keep[(size_t)(6 + d) * n_all + id] = uh; keep[(size_t)(9 + d) * n_all + id] = ul;
+            }
+            if (gl == 0u) {
+                io.steps[id] = n; io.ncoll[id] = ncoll; io.leg[id] = leg; io.status[id] = status;
+                done += n - n0;
+                if (status == 0 && done < chunk)
+                    to[MQ_CHK(atomicAdd(&ctr->handed[leg_no + 1], 1u), hand_at, MQ_SITE_MIX_HAND)] = make_uint2(id, done);
+                else if (status == 0)
+                    list_out[MQ_CHK(atomicAdd(&ctr->count[in_slot ^ 1], 1u), n_all, MQ_SITE_MIX_LIST_OUT)] = id;
+                steps_total += n - n0;
+            }
+            have = false;
+            kick = 0.f; uh = 1.f; xh = xl = ul = 0.f;
+        }
+        idle = __any_sync(FULL, !have);
+    };
+
+    for (uint32_t iter = 0;; ++iter) {
+        if (idle) {
+            // ---- groups without an ion take the next one of the list
+            const unsigned need = __ballot_sync(FULL, !have && !waits && !drained && gl == 0u);
+            if (need && (iter & 15u) == 0u) {
+                uint32_t slot = first;
+                const unsigned later = __ballot_sync(FULL, !have && !waits && !drained && gl == 0u && !fresh);
+                if (later) {
+                    uint32_t q = 0;
+                    const int leader = __ffs(later) - 1;
+                    if ((int)lane == leader) q = atomicAdd(&ctr->head_g[leg_no], (uint32_t)__popc(later));
+                    q = __shfl_sync(FULL, q, leader) + groups;
+                    if (!fresh) slot = q + __popc(later & ((1u << base) - 1u));
+                }
+                if (!have && !waits && !drained) {
+                    fresh = false;
+                    if (slot >= count) drained = true;
+                    else {
+                        done = 0;
+                        if (direct) id = list_in[slot];
+                        else { const uint2 e = from[slot]; id = e.x; done = e.y; }
+                        id = (uint32_t)MQ_CHK(id, n_all, MQ_SITE_MIX_ION);
+                        n = io.steps[id];
+                        waits = true;
+                    }
+                }
+            }
+            // An ion starts when its step count is congruent to the warp's counter mod 16, so that every
+            // block of words and phases begins on the same iteration for all of the warp's ions
+            const bool start = waits && ((iter ^ n) & 15u) == 0u;
+            if (__any_sync(FULL, start)) {
+                if (start) {
+                    have = true;
+                    waits = false;
+                    jid = io.jid[id];
+                    const MixJob& J = jobs[jid];
+                    kick = J.kick; ca2 = J.cand_a * J.cand_a; cand_b = J.cand_b;
+                    if (LEGACY) { mr = J.mr; floor_v = J.floor_v; mfp_mean = J.mfp_mean; }
+                    const uint64_t Wrf = ((uint64_t)B.w_rf_hi << 32) | B.w_rf_lo, Wac = ((uint64_t)J.w_ac_hi << 32) | J.w_ac_lo;
+                    W = is_ac ? Wac : Wrf;
+                    cw = is_ac ? J.cw_ac : B.cw_rf;
+                    sw = is_ac ? J.sw_ac : B.sw_rf;
+                    amp = is_ac ? (J.use_ac ? J.v_ac : 0.0f) : B.v_rf;
+                    n0 = n; ncoll = io.ncoll[id]; leg = io.leg[id];
+                    // the step to stop at: the time-out (one step at least), the end of the round or of the leg
+                    uint32_t left = n < B.max_steps ? B.max_steps - n : 1u;
+                    left = left < chunk - done ? left : chunk - done;
+                    stop = n + (left < leg_steps ? left : leg_steps);
+                    xh = keep[(size_t)d * n_all + id]; xl = keep[(size_t)(3 + d) * n_all + id];
+                    uh = keep[(size_t)(6 + d) * n_all + id]; ul = keep[(size_t)(9 + d) * n_all + id];
+                    P = kph[(is_ac ? (size_t)n_all : 0) + id] + (uint64_t)(n & ~15u) * W;
+                    const uint64_t key = io.rng[id];
+                    k0 = (uint32_t)key; k1 = (uint32_t)(key >> 32);
+                    if (n & 15u) block();
+                }
+                fill(start);
+                __syncwarp();
+            }
+            idle = __any_sync(FULL, !have && !drained);
+            if (!idle && !__any_sync(FULL, have)) break;
+        }
+        if ((iter & 15u) == 0u) {
+            __syncwarp();
+            block();
+            __syncwarp();
+        }
+        const uint32_t now = iter & 15u;
+        const float2 a2 = reinterpret_cast<const float2*>(drive)[now];
+        const float a_rf = a2.x, a_ac = a2.y;
+        // ---- field component at the current position: as field_comp, two corners an instruction
+        float E;
+        if (NEAREST) {
+            float r, di, ai, hi;
+            unpack2(R[0], r, hi); unpack2(D[0], di, hi); unpack2(A[0], ai, hi);
+            E = fmaf(a_rf, r, fmaf(a_ac, ai, di));
+        } else {
+            const float t = __fadd_rn(__fsub_rn(xh, fc), xl);
+            const float tx = __shfl_sync(FULL, t, base), ty = __shfl_sync(FULL, t, base + 1), tz = __shfl_sync(FULL, t, base + 2);
+            const uint64_t ar2 = pack2(a_rf, a_rf), aa2 = pack2(a_ac, a_ac);
+            uint64_t F[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) F[q] = fma2(ar2, R[q % NQ], fma2(aa2, A[q % NQ], D[q % NQ]));
+            const uint64_t tx2 = pack2(tx, tx), ty2 = pack2(ty, ty);
+            const uint64_t x0 = fma2(tx2, sub2(F[1], F[0]), F[0]), x1 = fma2(tx2, sub2(F[3], F[2]), F[2]);
+            float c0, c1;
+            unpack2(fma2(ty2, sub2(x1, x0), x0), c0, c1);
+            E = fmaf(tz, c1 - c0, c0);
+        }
+        // Legacy collisions come every few steps and most warps hold many ions, so nearly every step has a new
+        // cell: the tests of a position wait for its records here, where the field needs them anyway
+        if (LEGACY && __any_sync(FULL, have && n != n0 && (xh < in_lo || xh > in_hi || mask != 0u || n >= stop))) test(floorf(xh));
+        // ---- kick and drift, compensated
+        {
+            const float inc = __fadd_rn(__fmul_rn(kick, E), ul);
+            two_sum(uh, inc, uh, ul);
+            float r, e;
+            fast_two_sum(xh, uh, r, e);
+            e = __fadd_rn(e, __fadd_rn(xl, ul));
+            fast_two_sum(r, e, xh, xl);
+        }
+        n += have ? 1u : 0u;   // a waiting ion's count stays: its start is found by it
+        // ---- what the end of the step may have to deal with: a collision, another cell, a limit
+        const float ux = __shfl_sync(FULL, uh, base), uy = __shfl_sync(FULL, uh, base + 1), uz = __shfl_sync(FULL, uh, base + 2);
+        bool coll;
+        float um2 = 0.0f;
+        if (!LEGACY) {
+            const float u0 = draws[now];
+            um2 = fmaf(ux, ux, fmaf(uy, uy, uz * uz));
+            const float du = u0 - cand_b;
+            coll = have && (du < 0.0f || du * du < ca2 * um2);
+        } else {
+            leg -= 1;
+            coll = have && leg <= 0;
+        }
+        const float ff = floorf(xh);
+        const bool moved = have && ff != fc;
+        bool edge = !LEGACY && have && (xh < in_lo || xh > in_hi || mask != 0u || n >= stop);
+        if (!LEGACY && !__any_sync(FULL, coll || moved || edge)) continue;
+        if (LEGACY) {
+            const unsigned ch = __ballot_sync(FULL, moved);
+            if (ch) fill(((ch >> base) & 15u) != 0u);
+        }
+        if (__any_sync(FULL, coll)) {
+            if (!LEGACY) {
+                // the candidate's two Philox blocks, one in even lanes, one in odd
+                const uint4 r = philox(k0, k1, n - 1u, 1u + (gl & 1u), 0u, 0u);
+                uint4 r0;
+                r0.x = __shfl_sync(FULL, r.x, base); r0.y = __shfl_sync(FULL, r.y, base);
+                r0.z = __shfl_sync(FULL, r.z, base); r0.w = __shfl_sync(FULL, r.w, base);
+                const uint32_t r1x = __shfl_sync(FULL, r.x, base + 1), r1y = __shfl_sync(FULL, r.y, base + 1);
+                if (coll) {
+                    const float s_gas = jobs[jid].s_gas, mr_ = jobs[jid].mr;
+                    const float um = sqrtf(um2);
+                    const float u2v = B.u2v_f;
+                    const float v[3] = {ux * u2v, uy * u2v, uz * u2v};
+                    float gv[3], vm_sum;
+                    thermal_partner(r0, s_gas, um * u2v, v, gv, vm_sum);
+                    const float gm = sqrtf(fmaf(gv[0], gv[0], fmaf(gv[1], gv[1], gv[2] * gv[2])));
+                    if (unif16(r0.w & 0xffffu) * vm_sum < gm) {
+                        const float cth = 2.0f * unif(r1x) - 1.0f;
+                        float sp, cp;
+                        angle_sincos(unif(r1y), &sp, &cp);
+                        const float sn = sqrtf(fmaxf(0.0f, 1.0f - cth * cth));
+                        const float nn = d == 0 ? sn * cp : d == 1 ? sn * sp : cth;
+                        const float gd = d == 0 ? gv[0] : d == 1 ? gv[1] : gv[2], vd = d == 0 ? v[0] : d == 1 ? v[1] : v[2];
+                        const float vn = fmaf(mr_ * gm, nn, fmaf(-mr_, gd, vd));
+                        uh = vn * B.v2u_f;
+                        ul = 0.0f;
+                        ncoll += 1;
+                    }
+                }
+            } else {
+                const float4 dr = reinterpret_cast<const float4*>(draws)[now];   // direction, -ln u of the free path
+                const float dd[3] = {dr.x, dr.y, dr.z};
+                const float u2v = B.u2v_f;
+                float v[3] = {ux * u2v, uy * u2v, uz * u2v};
+                const float vm = sqrtf(fmaf(v[0], v[0], fmaf(v[1], v[1], v[2] * v[2])));
+                const bool hit = coll && vm > floor_v;
+                const float v2u = B.v2u_f;
+                float own_v = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float vn = fmaf(mr * vm, dd[k], v[k] * (1.0f - mr));
+                    v[k] = hit ? vn : v[k];
+                    if (k == d) own_v = vn;
+                }
+                uh = hit ? own_v * v2u : uh;
+                ul = hit ? 0.0f : ul;
+                ncoll += hit ? 1u : 0u;
+                const float mfp = dr.w * mfp_mean;
+                const float vn = sqrtf(fmaf(v[0], v[0], fmaf(v[1], v[1], v[2] * v[2])));
+                const float st = floorf(__fdividef(mfp, fmaxf(vn, 1e-3f) * B.dt_f));
+                const int32_t nl = st < 1.0f ? 1 : (st < 2147483520.0f ? (int32_t)st : 2147483647);
+                leg = coll ? nl : leg;
+            }
+        }
+        // ---- cell of the new position
+        if (!LEGACY) {
+            const unsigned ch = __ballot_sync(FULL, moved);
+            if (ch) {
+                fill(((ch >> base) & 15u) != 0u);
+                edge = edge || (have && mask != 0u);
+            }
+        }
+        // ---- termination tests
+        if (!LEGACY && __any_sync(FULL, edge)) test(ff);
+    }
+    if (gl != 0u) loads = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        steps_total += __shfl_down_sync(FULL, steps_total, o);
+        loads += __shfl_down_sync(FULL, loads, o);
+    }
+    if (lane == 0) {
+        if (steps_total) atomicAdd(&ctr->steps, steps_total);
+        if (loads) atomicAdd(&ctr->cell_loads, (unsigned long long)loads);
+    }
+}
+
+// interleave RF | combined DC | AC by component into node records of `stride` float4 (once per DC
+// configuration and record width); the spare w of each holds the conductor bits of the 8 corners of
+// the cell whose lowest corner is this node (bit a + 2b + 4c), so a cell reload reads its crash mask
+// in one word
 __global__ void k_pack_nodes(const float4* __restrict__ rf, const float4* __restrict__ dc, const float4* __restrict__ ac,
                              float4* __restrict__ nodes, size_t n, int32_t nx, int32_t ny, int32_t nz, int stride) {
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
-    nodes[stride * q] = rf[q];
-    if (stride == 4) nodes[4 * q + 3] = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 d = dc[q];
+    const float4 r = rf[q], d = dc[q], a = ac[q];
     const size_t sy = (size_t)nx, sz = (size_t)nx * (size_t)ny;
     const int32_t i = (int32_t)(q % sy), j = (int32_t)((q / sy) % (size_t)ny), k = (int32_t)(q / sz);
     uint32_t m = 0;
     if (i < nx - 1 && j < ny - 1 && k < nz - 1)
         for (int c = 0; c < 8; ++c)
             m |= (rf[q + (size_t)(c & 1) + ((c & 2) ? sy : 0) + ((c & 4) ? sz : 0)].w > 0.5f ? 1u : 0u) << c;
-    d.w = __uint_as_float(m);
-    nodes[stride * q + 1] = d;
-    nodes[stride * q + 2] = ac[q];
+    const float w = __uint_as_float(m);
+    if (stride == 3) {
+        nodes[3 * q] = make_float4(r.x, d.x, a.x, w);
+        nodes[3 * q + 1] = make_float4(r.y, d.y, a.y, w);
+        nodes[3 * q + 2] = make_float4(r.z, d.z, a.z, w);
+    } else {
+        const size_t t = k < nz - 1 ? q + sz : q;   // a cell's upper corners; the top layer bases no cell
+        const float4 rt = rf[t], dt = dc[t], at = ac[t];
+        nodes[6 * q] = make_float4(r.x, rt.x, d.x, dt.x);
+        nodes[6 * q + 1] = make_float4(a.x, at.x, w, 0.f);
+        nodes[6 * q + 2] = make_float4(r.y, rt.y, d.y, dt.y);
+        nodes[6 * q + 3] = make_float4(a.y, at.y, w, 0.f);
+        nodes[6 * q + 4] = make_float4(r.z, rt.z, d.z, dt.z);
+        nodes[6 * q + 5] = make_float4(a.z, at.z, w, 0.f);
+    }
 }
 
 // ---------------------------------------------------------------- injection for the mixed engine
@@ -746,7 +1196,10 @@ __global__ void k_sort_scatter(const uint32_t* __restrict__ list, const Ctrs* __
 // prepare launch: clear the queue head and the output count, and add the launch's queue length
 __global__ void k_prep(Ctrs* ctr, int out_slot) {
     ctr->head = 0;
+    for (int k = 0; k < kMaxLegs; ++k) ctr->head_g[k] = ctr->handed[k] = 0;
+    ctr->handed[kMaxLegs] = 0;
     ctr->count[out_slot] = 0;
+    ctr->open = ctr->count[out_slot ^ 1];
     ctr->queued += ctr->count[out_slot ^ 1];
 }
 
@@ -816,8 +1269,10 @@ MixBatch make_mix_batch(const mqp::Batch& b) {
     split(b.z_return / b.h, m.z_ret_h, m.z_ret_l);
     split(b.crash_z0 / b.h, m.cz0_h, m.cz0_l);
     split(b.crash_z1 / b.h, m.cz1_h, m.cz1_l);
-    m.z_exit_near = m.z_exit_h - 1.0f;
-    m.z_ret_near = m.z_ret_h + 1.0f;
+    // a plane farther than this cannot be crossed whatever the low part holds (below half an ulp of z)
+    const float near = fmaxf(0x1.0p-6f, (float)b.nz * 0x1.0p-20f);
+    m.z_exit_near = m.z_exit_h - near;
+    m.z_ret_near = m.z_ret_h + near;
     m.lim_x = (float)(b.nx - 1);
     m.lim_y = (float)(b.ny - 1);
     m.lim_z = (float)(b.nz - 1);
@@ -845,6 +1300,26 @@ Tuning default_tuning(int device, size_t nodes) {
     return t;
 }
 
+// Ions that the lane groups hold at once: a list of up to so many is stepped by them alone, a longer
+// one's last so many are handed to them.
+static uint32_t hand_entries(int sms, bool nearest) { return (uint32_t)sms * (uint32_t)(group_block(nearest) / 4); }
+
+// Steps of the lane-group launches of one round of `chunk` steps. Between them the ions that are left are
+// spread over full warps again: worth its 10 us where warps hold many ions each and these end one by one
+// over many thousand steps, as with legacy collisions (Fig. 4 scan of 26,000 ions: 11.9 -> 10.7 ms). Thermal
+// ions end early or not at all (S14 sweep 39.2 against 39.8 ms with such legs), and where a warp has
+// one or two ions there is nothing to pack.
+static int plan_legs(uint32_t chunk, bool many_legs, uint32_t legs[kMaxLegs]) {
+    uint32_t leg = many_legs ? 1024u : chunk, left = chunk;
+    int k = 0;
+    while (left > 0) {
+        legs[k] = k == kMaxLegs - 1 || left < leg + leg / 2 ? left : leg;
+        left -= legs[k++];
+        leg += leg / 2;
+    }
+    return k;
+}
+
 void release(Scratch& s) {
     if (s.graph) cudaGraphExecDestroy(s.graph);
     for (void* p : {s.lists, s.ctrs, s.params, s.jobs, s.nodes, s.keep, s.sort}) if (p) cudaFree(p);
@@ -866,6 +1341,16 @@ static Kernel pick_kernel(const Tuning& t, const MixBatch& mb) {
     }
     if (t.wide) return t.prefetch ? k_mixed<false, true, true, false> : k_mixed<false, false, true, false>;
     return t.prefetch ? k_mixed<false, true, false, false> : k_mixed<false, false, false, false>;
+}
+
+typedef decltype(&k_mixed_group<true, true, false>) GroupKernel;
+static GroupKernel pick_group_kernel(const Tuning& t, const MixBatch& mb) {
+    if (mb.nearest) {
+        if (mb.legacy_coll) return t.wide ? k_mixed_group<true, true, true> : k_mixed_group<true, false, true>;
+        return t.wide ? k_mixed_group<false, true, true> : k_mixed_group<false, false, true>;
+    }
+    if (mb.legacy_coll) return t.wide ? k_mixed_group<true, true, false> : k_mixed_group<true, false, false>;
+    return t.wide ? k_mixed_group<false, true, false> : k_mixed_group<false, false, false>;
 }
 
 // bins of the cell sort: the top min(22, 3 b) bits of the Morton code, b the bits of the largest
@@ -924,14 +1409,26 @@ static cudaError_t enqueue_launches(const Scratch& s, const Tuning& t, int block
             *kernels += 5;
         }
         const Kernel kern = pick_kernel(t, mb);
-        kern<<<grid, t.tpb, 0, st>>>(nodes, mb, jobs, io, li, lo, ctr, in, ch, keep, kph, n);
-        *kernels += 2;
+        const uint32_t hand_at = hand_entries(t.sms, mb.nearest != 0);
+        uint2* hand = reinterpret_cast<uint2*>(ctr + 1);
+        if (n > hand_at) {
+            kern<<<grid, t.tpb, 0, st>>>(nodes, mb, jobs, io, li, lo, ctr, in, ch, keep, kph, n, hand, hand_at);
+            *kernels += 1;
+        }
+        const int sm = group_block(mb.nearest != 0) / 4 * group_floats(mb.legacy_coll != 0) * (int)sizeof(float);
+        const GroupKernel gk = pick_group_kernel(t, mb);
+        cudaFuncSetAttribute(gk, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        uint32_t legs[kMaxLegs];
+        const int nlegs = plan_legs(ch, mb.legacy_coll && L == 0 && n > 2u * kGroupFirst * (uint32_t)t.sms, legs);
+        for (int k = 0; k < nlegs; ++k)
+            gk<<<t.sms, group_block(mb.nearest != 0), sm, st>>>(nodes, mb, jobs, io, li, hand, lo, ctr, in, ch, k, legs[k], keep, kph, n, hand_at);
+        *kernels += 1u + (uint32_t)nlegs;
     }
     return cudaGetLastError();
 }
 
 cudaError_t pack_nodes(Scratch& s, DevGrid g, uint64_t grid_gen, int wide, cudaStream_t st, uint32_t* kernels) {
-    const int stride = wide ? 4 : 3;
+    const int stride = wide ? 6 : 3;
     if (s.nodes && s.nodes_gen == grid_gen && s.nodes_stride == stride) return cudaSuccess;
     cudaError_t e;
     const size_t n = (size_t)g.nx * g.ny * g.nz;
@@ -965,7 +1462,7 @@ cudaError_t run(Scratch& s, const Tuning& t, DevGrid g, uint64_t grid_gen, const
         if ((e = cudaMalloc(&s.lists, list_bytes)) != cudaSuccess) return e;
         s.list_cap = list_bytes;
     }
-    if (!s.ctrs && (e = cudaMalloc(&s.ctrs, sizeof(Ctrs))) != cudaSuccess) return e;
+    if (!s.ctrs && (e = cudaMalloc(&s.ctrs, sizeof(Ctrs) + sizeof(uint2) * 2 * (size_t)hand_entries(t.sms, true))) != cudaSuccess) return e;
     if (s.jobs_cap < njobs * sizeof(MixJob)) {
         if (s.jobs) cudaFree(s.jobs);
         s.jobs = nullptr; s.jobs_cap = 0;

@@ -30,7 +30,7 @@ struct MixBatch {      // per-batch constants (device-resident parameter block)
     float cw_rf, sw_rf;              // cos / sin of the RF phase advance per step
     float z_exit_h, z_exit_l, z_ret_h, z_ret_l;       // grid units, double-float
     float cz0_h, cz0_l, cz1_h, cz1_l;                 // crash window, grid units
-    float z_exit_near, z_ret_near;                    // one cell inside the exit / return planes
+    float z_exit_near, z_ret_near;                    // a little inside the exit / return planes: beyond, the exact test
     float lim_x, lim_y, lim_z;                        // n - 1 (exact)
     int32_t nx, ny, nz;
     int32_t nearest, legacy_coll;
@@ -45,7 +45,7 @@ struct Tuning {
     uint32_t chunk = 20000;    // steps per ion per launch (compaction interval)
     int use_graph = 1;         // replay the launch sequence as one CUDA graph
     int prefetch = 0;          // L1-prefetch the cell an ion is heading for
-    int wide = 0;              // 64-byte node records read with 256-bit loads (else 48-byte records)
+    int wide = 0;              // 96-byte records of node pairs read with 256-bit loads (else 48-byte records)
     uint32_t max_launches = 0; // cap on launches per call (0 = as many as the step budget needs)
     int sort_cells = 0;        // put each launch's live list in the Morton order of the ions' cells
     int sms = 0;               // filled from the device
@@ -60,7 +60,7 @@ struct Scratch {
     size_t jobs_cap = 0;
     void* keep = nullptr;      // working state of the call's ions (phase offsets, double-floats, staged flags)
     size_t keep_cap = 0;
-    void* nodes = nullptr;     // interleaved RF | DC | AC node records (float4 x 3 or 4 per node)
+    void* nodes = nullptr;     // interleaved RF | DC | AC node records (float4 x 3 or 6 per node)
     size_t nodes_cap = 0;
     uint64_t nodes_gen = ~0ull; // grid generation the records were packed from
     int nodes_stride = 0;       // float4 per record of the packed records

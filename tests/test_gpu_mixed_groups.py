@@ -1,0 +1,55 @@
+"""The mixed engine's lane groups: an ion's final state does not depend on which kernel stepped it. A batch
+larger than the groups hold (19,456 or, with nearest-node fields, 29,184 ions on 152 SMs) starts in the
+one-lane kernel, is spread over its warps unevenly, and hands its last ions to the groups in the
+middle of their flights; the same jobs run alone, odd sizes down to one ion, go through the groups
+from their first step. Bit for bit the same for every physics, both node record widths, and launches of
+37 steps, which re-queue ions at every position of a 16-step block and cut the groups' legs."""
+import sys
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, str(Path(__file__).resolve().parent))
+from test_gpu_parity import FIELDS, _mq, _variants  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+DC = [0.0, 5.0, -5.0, 0.0]
+SIZES = (1, 7, 33, 1217, 4865, 23878)   # 30,001 together; the 23,878 alone are also above 19,456
+
+
+def _jobs(legacy_species):
+    mq = _mq()
+    out = []
+    for k, n in enumerate(SIZES):
+        mz = 493.0 + 2 * k
+        sp = mq.Species(mz * 5, 5.0, 0.0) if legacy_species else mq.Species(mz, 1.0, 2.95 * mz ** (2 / 3))
+        out.append(mq.Job(sp, mq.RfAc(100.0, 500e3, 0.5 if k else 0.0, 100e3 + 1e3 * k), n, 77 + k))
+    return out
+
+
+@pytest.mark.parametrize("wide", [True, False], ids=["wide", "narrow"])
+@pytest.mark.parametrize("name", ["corrected_disc", "half_kick_gauss", "legacy_all", "legacy_coll_trilinear", "thermal_nearest",
+                                  "no_gas_rf_random"])
+def test_groups_equal_one_lane_kernel(coarse, name, wide):
+    mq = _mq()
+    ph = _variants()[name]
+    jobs = _jobs(name.startswith("legacy"))
+    with mq.Engine(coarse, mq.PREC_MIXED) as e:
+        e.set_tuning(wide_records=wide)
+        whole, jid = e.run_batch_ions(jobs, DC, ph)
+        steps = e.last_stats.ion_steps
+        assert steps == int(whole.steps.astype(np.int64).sum())
+        assert (whole.status != 0).all()
+        alone = [e.run_batch_ions([j], DC, ph)[0] for j in jobs]
+        e.set_tuning(chunk=37)
+        cut, _ = e.run_batch_ions(jobs[:5], DC, ph)
+    for k in range(len(jobs)):
+        m = jid == k
+        for f in FIELDS[:-1]:
+            a, b = getattr(whole, f)[m], getattr(alone[k], f)
+            assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), f"{name}: job {k}, {f}"
+    m = jid < 5
+    for f in FIELDS:
+        assert np.array_equal(getattr(whole, f)[m].view(np.uint8), getattr(cut, f).view(np.uint8)), f"{name}: 37-step launches, {f}"
