@@ -1,4 +1,4 @@
-// Nine-channel tandem transport on the GPU: one thread per track, all tracks in lockstep on
+// Nine-channel tandem transport on the GPU: a group of lanes per track, every track on
 // the global clock, FP64 state, compiled without FMA contraction so that every track's
 // arithmetic equals the CPU restatement of trapsim::Model::advance bit for bit.
 //
@@ -6,6 +6,7 @@
 // lib.rs:176-276 (Model::advance: region fields, routing), lib.rs:338-385 (enter / leave),
 // simulation/mqviz/src/world.rs:265-314 (fields_at, gate_delta, is_crash), world.rs:471-488
 // (collide).
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <utility>
@@ -16,6 +17,7 @@
 #include "mq_tandem.h"
 #include "mq_tandem_internal.h"
 #include "mq_check.h"
+#include "mq_f64dev.h"
 
 namespace {
 
@@ -24,12 +26,20 @@ constexpr double Z_RETURN = 0.5e-3;    // world.rs:22
 constexpr int R_SPLIT = 0, R_COMBINE = 10, R_LOST = 11, R_BACK = 12, R_DETECTED = 13;
 constexpr int kNC = 21;                 // counters per port (mq_port_counts)
 
+using namespace mqf;
+
 struct TSpec { double qmdt, s_ion, mr, nsd; };
 
 struct TPort {                  // one port's channel grid and drive
     int32_t kn[3], idle;
     double kh, inv_kh, lim[3];   // spacing [m], its correctly rounded reciprocal, box limits
     const float4 *rf, *ac, *dc, *gate;
+};
+
+// Cube geometry in FP32 (mm, growth 0), for the filter that settles all but the points near a surface
+struct CubeF {
+    float size, c0, pitch, half_d, t_pcb, gap, ptd, stem_r, clear_r, rod_hole, l_ext, cap_reach, cap_r, ap_r;
+    int32_t n, array, ent_axis, ent_side, ent_cell0, ent_cell1, ext_axis, ext_side, ext_cell0, ext_cell1;
 };
 
 struct TConst {
@@ -43,6 +53,10 @@ struct TConst {
     double mouth[9][2];
     double ent_b, ent_c;   // entrance axis centre (mm): along z, along x
     TSpec sp[8];
+    CubeF F;
+    // high words of the positions (m) that are out of reach of every cube face and short of the seam
+    int32_t in_lo;
+    uint32_t in_n[3];
 };
 
 struct Tracks {
@@ -51,103 +65,59 @@ struct Tracks {
     int32_t *sp, *region, *last;
 };
 
-__device__ __forceinline__ double clampd(double v, double lo, double hi) { return v < lo ? lo : (v > hi ? hi : v); }
-
-// cube_field: trilinear RF * rf + combined DC at a point (lib.rs:70-88, fields.rs:89-96)
-__device__ void cube_field(const TConst& C, const float4* dc, const double x[3], double rf, double e[3]) {
-    int c[3];
-    double w[3];
-    for (int a = 0; a < 3; ++a) {
-        const double p = x[a] * 1000.0;
-        const double f = clampd(mqp::div_rn(p - C.clo[a], C.ch_mm, C.inv_ch_mm), 0.0, (double)(C.cn[a] - 1) - 1e-9);
-        c[a] = f > 0.0 ? (int)floor(f) : 0;   // NaN -> 0 as Rust's `as usize`
-        w[a] = f - (double)c[a];
-    }
-    e[0] = e[1] = e[2] = 0.0;
-    for (int k = 0; k < 2; ++k)
-        for (int j = 0; j < 2; ++j)
-            for (int i = 0; i < 2; ++i) {
-                size_t q = (size_t)(c[0] + i) + (size_t)C.cn[0] * ((size_t)(c[1] + j) + (size_t)C.cn[1] * (size_t)(c[2] + k));
-                q = MQ_CHK(q, (size_t)C.cn[0] * (size_t)C.cn[1] * (size_t)C.cn[2], MQ_SITE_TDM_CUBE);
-                const double wt = (i == 1 ? w[0] : 1.0 - w[0]) * (j == 1 ? w[1] : 1.0 - w[1]) * (k == 1 ? w[2] : 1.0 - w[2]);
-                const float4 r = C.crf[q], d = dc[q];
-                e[0] += wt * (rf * (double)r.x + (double)d.x);
-                e[1] += wt * (rf * (double)r.y + (double)d.y);
-                e[2] += wt * (rf * (double)r.z + (double)d.z);
-            }
+constexpr float kNear = 2e-3f;   // mm: over ten times what the FP32 distances are off by
+__device__ __forceinline__ float latf(const CubeF& G, int i) { return G.c0 + G.pitch * (float)i; }
+__device__ __forceinline__ float hypf2(float u, float v) { return sqrtf(u * u + v * v); }
+// v < t, noting in `unsure` when the two are too close to tell
+__device__ __forceinline__ bool below(float v, float t, bool& unsure) {
+    unsure |= !(fabsf(v - t) >= kNear);   // NaN too
+    return v < t;
 }
-
-// channel fields_at (world.rs:265-288) and gate_delta (world.rs:291-302) on the port's grid
-__device__ void chan_field(const TPort& P, double gate_v, const double x[3], double rf, double ac, double e[3]) {
-    const double h = P.kh;
-    const double g[3] = {mqp::div_rn(x[0], h, P.inv_kh), mqp::div_rn(x[1], h, P.inv_kh), mqp::div_rn(x[2], h, P.inv_kh)};
-    const int32_t i0 = mqp::cell_lo(g[0], P.kn[0]), j0 = mqp::cell_lo(g[1], P.kn[1]), k0 = mqp::cell_lo(g[2], P.kn[2]);
-    const double tx = g[0] - (double)i0, ty = g[1] - (double)j0, tz = g[2] - (double)k0;
-    double er[3] = {0, 0, 0}, ea[3] = {0, 0, 0}, ed[3] = {0, 0, 0};
-    const size_t nx = (size_t)P.kn[0], ny = (size_t)P.kn[1];
-    for (int di = 0; di < 2; ++di) {
-        const double wx = di ? tx : 1.0 - tx;
-        for (int dj = 0; dj < 2; ++dj) {
-            const double wy = dj ? ty : 1.0 - ty;
-            for (int dk = 0; dk < 2; ++dk) {
-                const double wz = dk ? tz : 1.0 - tz;
-                size_t q = (size_t)(i0 + di) + nx * ((size_t)(j0 + dj) + ny * (size_t)(k0 + dk));
-                q = MQ_CHK(q, nx * ny * (size_t)P.kn[2], MQ_SITE_TDM_PORT);
-                const double w = wx * wy * wz;
-                const float4 r = P.rf[q], a = P.ac[q], d = P.dc[q];
-                er[0] += w * (double)r.x; er[1] += w * (double)r.y; er[2] += w * (double)r.z;
-                ea[0] += w * (double)a.x; ea[1] += w * (double)a.y; ea[2] += w * (double)a.z;
-                ed[0] += w * (double)d.x; ed[1] += w * (double)d.y; ed[2] += w * (double)d.z;
-            }
+// v.round() clamped to [0, hi]
+__device__ __forceinline__ int round_near(float v, int hi, bool& unsure) {
+    const float r = rintf(v);
+    unsure |= !(fabsf(v - r) <= 0.499f);
+    return r > 0.0f ? (r < (float)hi ? (int)r : hi) : 0;
+}
+// mqc::classify (geometry.rs:136-205) for one face (axis a, side) of the point: does the point lie in
+// an electrode of it?  u: depth below the face, pb / pc: the coordinates along axes a + 1 and a + 2
+__device__ bool face_solid(const CubeF& G, int a, int side, float u, float pb, float pc, bool inside, bool& unsure) {
+    int pid = 0, pc0 = 0, pc1 = 0;
+    if (G.ent_axis == a && G.ent_side == side) { pid = 3; pc0 = G.ent_cell0; pc1 = G.ent_cell1; }
+    else if (G.ext_axis == a && G.ext_side == side) {
+        pid = 4;
+        pc0 = G.ext_cell0; pc1 = G.ext_cell1;
+        if (G.array) {
+            const float first = 0.5f * (latf(G, 2) + latf(G, 3));
+            pc0 = 2 + 2 * round_near((pb - first) / (2.0f * G.pitch), 2, unsure);
+            pc1 = 2 + 2 * round_near((pc - first) / (2.0f * G.pitch), 2, unsure);
         }
     }
-    double bias[3] = {0.0, 0.0, 0.0};
-    if (P.idle) {
-        for (int ii = 0; ii < 2; ++ii)
-            for (int jj = 0; jj < 2; ++jj)
-                for (int kk = 0; kk < 2; ++kk) {
-                    size_t q = (size_t)(i0 + ii) + nx * ((size_t)(j0 + jj) + ny * (size_t)(k0 + kk));
-                    q = MQ_CHK(q, nx * ny * (size_t)P.kn[2], MQ_SITE_TDM_GATE);
-                    const double w = gate_v * (ii == 1 ? tx : 1.0 - tx) * (jj == 1 ? ty : 1.0 - ty) * (kk == 1 ? tz : 1.0 - tz);
-                    const float4 b = P.gate[q];
-                    bias[0] += w * (double)b.x; bias[1] += w * (double)b.y; bias[2] += w * (double)b.z;
-                }
+    const float axis_d = hypf2(pb - 0.5f * (latf(G, pc0) + latf(G, pc0 + 1)), pc - 0.5f * (latf(G, pc1) + latf(G, pc1 + 1)));
+    if (below(u, 0.0f, unsure)) {   // outside the wall: port rods and end cap
+        if (pid == 0) return false;
+        bool hit = false;
+        if (below(u, -G.cap_reach, unsure)) hit = below(axis_d, G.cap_r, unsure);
+        if (!below(u, -G.l_ext, unsure))
+            for (int m = 0; m < 4; ++m)
+                hit |= below(hypf2(pb - latf(G, pc0 + (m >> 1)), pc - latf(G, pc1 + (m & 1))), G.half_d, unsure);
+        return hit;
     }
-    for (int k = 0; k < 3; ++k) e[k] = rf * er[k] + ac * ea[k] + ed[k] + bias[k];
-}
-
-__device__ bool chan_crash(const TPort& P, const double x[3]) {   // world.rs:309-314
-    for (int d = 0; d < 3; ++d)
-        if (x[d] < 0.0 || x[d] > P.lim[d]) return true;
-    const int32_t ni = mqp::node_round(mqp::div_rn(x[0], P.kh, P.inv_kh), P.kn[0]),
-                  nj = mqp::node_round(mqp::div_rn(x[1], P.kh, P.inv_kh), P.kn[1]),
-                  nk = mqp::node_round(mqp::div_rn(x[2], P.kh, P.inv_kh), P.kn[2]);
-    size_t q = (size_t)ni + (size_t)P.kn[0] * ((size_t)nj + (size_t)P.kn[1] * (size_t)nk);
-    q = MQ_CHK(q, (size_t)P.kn[0] * (size_t)P.kn[1] * (size_t)P.kn[2], MQ_SITE_TDM_CRASH);
-    return P.rf[q].w > 0.5f;
-}
-
-__device__ void collide(double v[3], uint64_t* rng, const TSpec& s, double s_gas) {   // world.rs:473-488
-    const double vm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-    const double bound = vm + 6.0 * s_gas;
-    if (mqp::xs_next(rng) < s.nsd * bound) {
-        double vg[3];
-        for (int d = 0; d < 3; ++d) {
-            const double u1 = mqp::xs_next(rng), u2 = mqp::xs_next(rng);
-            vg[d] = s_gas * mqp::gauss(u1, u2);
-        }
-        const double gv[3] = {v[0] - vg[0], v[1] - vg[1], v[2] - vg[2]};
-        const double gl = sqrt(gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2]);
-        if (mqp::xs_next(rng) * bound < gl) {
-            const double c = 2.0 * mqp::xs_next(rng) - 1.0;
-            double sp, cp;
-            mqp::sincos2pi(mqp::xs_next(rng), &sp, &cp);
-            const double omc = 1.0 - c * c;
-            const double sn = sqrt(omc > 0.0 ? omc : 0.0);
-            const double nn[3] = {sn * cp, sn * sp, c};
-            for (int d = 0; d < 3; ++d) v[d] = v[d] - s.mr * gv[d] + s.mr * gl * nn[d];
-        }
+    if (!inside || !below(u, G.ptd, unsure)) return false;
+    const int ib = round_near((pb - G.c0) / G.pitch, G.n - 1, unsure), ic = round_near((pc - G.c0) / G.pitch, G.n - 1, unsure);
+    const bool rim_b = ib == 0 || ib == G.n - 1, rim_c = ic == 0 || ic == G.n - 1;
+    const bool valid = a == 0 ? !rim_b && !rim_c : a == 1 ? !rim_b : true;   // post_valid, geometry.rs:81-86
+    const float dd = hypf2(pb - latf(G, ib), pc - latf(G, ic));
+    const bool rod = pid != 0 && valid && (unsigned)(ib - pc0) <= 1u && (unsigned)(ic - pc1) <= 1u;
+    const bool aperture = pid != 0 && below(axis_d, G.ap_r, unsure);
+    const bool in_post = below(dd, G.half_d, unsure);
+    if (rod && in_post) return true;
+    if (below(u, G.t_pcb, unsure) && !aperture && !(valid && below(dd, rod ? G.rod_hole : G.clear_r, unsure))) return true;
+    if (valid && !rod) {
+        if (below(u, G.t_pcb + G.gap, unsure)) return below(dd, G.stem_r, unsure);
+        return in_post;
     }
+    return false;
 }
 
 // Executed track-steps by region kind (cube, driven port, idle port): one warp-reduced atomic per warp.
@@ -162,104 +132,453 @@ __device__ __forceinline__ void add_steps(unsigned long long* st, uint32_t c, ui
     }
 }
 
-// blockDim.x is a multiple of 32 and no lane returns early, so the warp reductions see full warps.
-__global__ void __launch_bounds__(128) k_tandem(TConst C, Tracks T, uint32_t n, const double* __restrict__ drive,
-                                                uint32_t steps, uint32_t* __restrict__ counts,
-                                                unsigned long long* __restrict__ stepc) {
-    const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t n_cube = 0, n_port = 0, n_idle = 0;
-    if (id < n && T.region[id] < R_LOST) {
-        int reg = T.region[id];
-        double x[3] = {T.x[id], T.y[id], T.z[id]};
-        double v[3] = {T.vx[id], T.vy[id], T.vz[id]};
-        uint64_t rng = T.rng[id];
-        const int sp = T.sp[id];
-        int last = T.last[id];
-        const TSpec S = C.sp[sp];
-        for (uint32_t k = 0; k < steps && reg < R_LOST; ++k) {
-            const double* dr = drive + (size_t)k * 10;   // rf, ac[0..9)
-            const double rf = dr[0];
-            double e[3];
-            if (reg == R_SPLIT || reg == R_COMBINE) {
-                cube_field(C, C.cdc[reg == R_COMBINE ? 1 : 0], x, rf, e);
-                ++n_cube;
+// ---------------------------------------------------------------- the step kernel
+// Bound by GB300's FP64 pipe and by latency, as the channel's FP64 kernel (mq_f64.cu), and shaped like it: a
+// group of G lanes per track, each lane an axis (position, velocity) and one of the eight cell
+// corners (two for G = 4), the sums over the corners side by side in the lanes. With one lane per track
+// a step took 32 us. In the cube the electrode test, some hundreds of FP64 operations, is first made in
+// FP32, one face of the cube per lane, and exactly only within 2 um of a surface; whether a
+// track is at a limit at all is read off the high words of its position. Every operation that counts is the
+// reference's, in its order: results are bit for bit those of one lane per track.
+// G = 16 while the tracks fit one warp per scheduler (two of them in a warp), 4 beyond, where fewer wasted
+// lanes count for more; groups take the next track when theirs has made its steps or is lost.
+// Measured, whole advance call, 180 tracks and 100 steps: 3.48 -> 0.48 ms.
+constexpr int kTBlock = 256;
+constexpr int kTRow = 10;
+constexpr int kTSums = 6 + 12 * kTRow;
+constexpr int kTGroup = kTSums + 12;     // doubles of shared memory per group
+constexpr int kTPad = 120 * 1024;        // one block per SM
+
+template <int G>
+__global__ void __launch_bounds__(kTBlock, 1)
+k_tandem(const __grid_constant__ TConst C, Tracks T, uint32_t n, const double* __restrict__ drive, uint32_t steps,
+         uint32_t* __restrict__ counts, unsigned long long* __restrict__ stepc, uint32_t* __restrict__ head) {
+    constexpr int GPW = 32 / G;
+    constexpr int NC = G == 16 ? 1 : 2;     // corners per lane
+    constexpr int NP = G == 16 ? 6 : 12;    // products per corner: RF, AC, DC, gate of three components; G = 16: half of them
+    constexpr int NS = G == 16 ? 1 : 4;     // sums per lane
+    extern __shared__ __align__(16) double sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gl = lane % G, base = lane - gl;
+    const int d = gl % 3;
+    double* const tw = sm + (size_t)(threadIdx.x / G) * kTGroup;
+    double* const prod = tw + 6;
+    double* const xch = tw + kTSums;
+    const uint32_t first = (uint32_t)((((warp >> 2) * GPW + lane / G) * 4 + (warp & 3)) * gridDim.x + blockIdx.x);
+    const uint32_t groups = gridDim.x * (kTBlock / 32) * GPW;
+    // corner index in the order of the sums: 4 di + 2 dj + dk in a port, di + 2 dj + 4 dk in the cube
+    const int cn = G == 16 ? gl & 7 : gl;
+    const bool upper = G == 16 && gl >= 8;
+    const int chain = G == 16 ? (gl < 12 ? gl : gl - 12) : d;   // sum 3 f + d: RF, AC, DC, gate (cube: the first three)
+
+    bool have = false, drained = false, fresh = true, turn = true;
+    uint32_t id = 0, k = 0;
+    int reg = R_LOST, last = -1, sp = 0;
+    uint64_t rng = 1;
+    double x = 0.0, v = 0.0, q = 0.0, cell = 0.0, qmdt = 0.0;
+    float nsd2 = 0.0f, ub0 = 0.0f;
+    bool cube = true, idle = false;
+    int32_t ci = -1, cj = -1, ck = -1, nd = 2;
+    uint32_t mask = 0, n_cube = 0, n_port = 0, n_idle = 0;
+    double gh = 1.0, ginv = 1.0, glim = 0.0;   // grid spacing, its reciprocal, box limit along the axis (port)
+    size_t nx = 2, ny = 2;
+    const float4 *p_rf = nullptr, *p_ac = nullptr, *p_dc = nullptr, *p_gate = nullptr;
+    double val[NC][NP];
+#pragma unroll
+    for (int c = 0; c < NC; ++c)
+#pragma unroll
+        for (int m = 0; m < NP; ++m) val[c][m] = 0.0;
+
+    // constants of the group's region, and the lane's coordinate on its grid: x / h in a port, mm in the cube
+    auto enter_region = [&](bool go) {
+        if (go) {
+            cube = reg == R_SPLIT || reg == R_COMBINE;
+            if (cube) {
+                nd = C.cn[d]; nx = (size_t)C.cn[0]; ny = (size_t)C.cn[1];
+                p_rf = C.crf; p_dc = C.cdc[reg == R_COMBINE ? 1 : 0];
+                idle = false;
             } else {
-                const int i = reg - 1;
-                chan_field(C.port[i], C.gate_v, x, rf, dr[1 + i], e);
-                if (C.port[i].idle) ++n_idle;
-                else ++n_port;
+                const TPort& P = C.port[reg - 1];
+                nd = P.kn[d]; nx = (size_t)P.kn[0]; ny = (size_t)P.kn[1];
+                p_rf = P.rf; p_ac = P.ac; p_dc = P.dc; p_gate = P.gate;
+                gh = P.kh; ginv = P.inv_kh; glim = P.lim[d];
+                idle = P.idle != 0;
             }
-            // transport_step (lib.rs:90-103)
-            for (int d = 0; d < 3; ++d) {
-                v[d] += S.qmdt * e[d];
-                x[d] += v[d] * C.dt;
-            }
-            collide(v, &rng, S, C.s_gas);
-            if (reg == R_SPLIT || reg == R_COMBINE) {
-                const double mm[3] = {x[0] * 1000.0, x[1] * 1000.0, x[2] * 1000.0};
-                int sg = 0;
-                if (mqc::classify(C.cube, mm, 0.0, &sg) != mqc::ID_FREE) { reg = R_LOST; continue; }
-                if (x[2] > C.seam) {
-                    const int i = mqc::nearest_port(C.cube, mm[0], mm[1]);
-                    const double* c = C.mouth[i];
-                    if (mqc::dist2d(x[0] - c[0], x[1] - c[1]) < C.ap_r * 0.001) {
-                        // enter (lib.rs:338-367)
-                        uint32_t* cnt = counts + (size_t)i * kNC;
-                        x[0] += C.axis - c[0];
-                        x[1] += C.axis - c[1];
-                        const double depth = x[2] - C.seam;
-                        if (reg == R_SPLIT) {
-                            x[2] = Z_RETURN + depth;
-                            atomicAdd(cnt + 0, 1u);
-                            if (last >= 0) {
-                                atomicAdd(cnt + 3, 1u);
-                                atomicAdd(cnt + 5 + last, 1u);
-                                if (last != i) atomicAdd(cnt + 4, 1u);
+            ci = -1;
+        }
+    };
+    auto coordinate = [&](bool go) {
+        if (__any_sync(FULL, go && cube)) { const double qc = x * 1000.0; if (go && cube) q = qc; }
+        if (__any_sync(FULL, go && !cube)) { const double qp = mqp::div_rn(x, gh, ginv); if (go && !cube) q = qp; }
+    };
+    // cell and fractions; corner values of the groups in `go` that changed cell
+    auto locate = [&](bool go) -> double {
+        double f = q;
+        if (__any_sync(FULL, go && cube)) {   // fields.rs:89-96: clamped to the grid, short of its last node
+            const double fc = mqp::div_rn(q - C.clo[d], C.ch_mm, C.inv_ch_mm);
+            const double top = (double)(C.cn[d] - 1) - 1e-9;
+            const long long b = __double_as_longlong(fc);
+            if (cube) f = lt_zero(b) ? 0.0 : gt_pos(b, __double_as_longlong(top)) ? top : fc;
+        }
+        double t = f - cell;
+        const bool stay = ci >= 0 && (unsigned)__double2hiint(t) < 0x3ff00000u;
+        if (__any_sync(FULL, go && gl < 3 && !stay)) {
+            const int32_t ca = cell_lo_bits(f, nd, __double_as_longlong(i2d_bits(nd - 2)));
+            const double cd = i2d_bits(ca);
+            if (go) { cell = cd; t = f - cd; }
+            const int32_t ni = __shfl_sync(FULL, ca, base), nj = __shfl_sync(FULL, ca, base + 1), nk = __shfl_sync(FULL, ca, base + 2);
+            const bool move = go && (ni != ci || nj != cj || nk != ck);
+            bool c0 = false, c1 = false;
+            if (move) {
+                ci = ni; cj = nj; ck = nk;
+                float r[NC][12], solid[2] = {0.0f, 0.0f};
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const int m = cn + 4 * c;   // G = 4: corners cn and cn + 4
+                    const int lo = m & 1, mid = (m >> 1) & 1, hi = m >> 2;
+                    const size_t o = (size_t)(ci + (cube ? lo : hi)) + nx * ((size_t)(cj + mid) + ny * (size_t)(ck + (cube ? hi : lo)));
+                    const size_t w = cube ? MQ_CHK(o, (size_t)C.cn[0] * (size_t)C.cn[1] * (size_t)C.cn[2], MQ_SITE_TDM_CUBE)
+                                          : MQ_CHK(o, nx * ny * (size_t)C.port[reg - 1].kn[2], MQ_SITE_TDM_PORT);
+#pragma unroll
+                    for (int z = 0; z < 12; ++z) r[c][z] = 0.0f;
+                    // G = 16: lower lanes RF and AC (cube: RF and DC), upper lanes DC and gate
+                    if (G == 16) {
+                        if (!(cube && upper)) {
+                            const float4 u = __ldg((upper ? p_dc : p_rf) + w);
+                            r[c][0] = u.x; r[c][1] = u.y; r[c][2] = u.z;
+                            solid[c] = upper || cube ? 0.0f : u.w;
+                            if (!upper || idle) {
+                                const float4 y = __ldg((cube ? p_dc : upper ? p_gate : p_ac) + w);
+                                r[c][3] = y.x; r[c][4] = y.y; r[c][5] = y.z;
                             }
-                        } else {
-                            x[2] = Z_EXIT - depth;
-                            v[2] *= -1.0;
-                            atomicAdd(cnt + 14, 1u);
                         }
-                        reg = 1 + i;
-                        continue;
-                    }
-                    if (x[2] > C.size) { reg = R_LOST; continue; }
-                }
-                if (x[1] > C.size) {
-                    if (mqc::dist2d(mm[0] - C.ent_c, mm[2] - C.ent_b) >= C.ap_r) { reg = R_LOST; continue; }
-                }
-                if (x[1] > C.size + C.l_ext_m) reg = (reg == R_SPLIT) ? R_BACK : R_DETECTED;
-                else if (x[0] < 0.0 || x[1] < 0.0 || x[2] < 0.0 || x[0] > C.size) reg = R_LOST;
-            } else {
-                const int i = reg - 1;
-                uint32_t* cnt = counts + (size_t)i * kNC;
-                if (chan_crash(C.port[i], x)) { reg = R_LOST; atomicAdd(cnt + 15, 1u); }
-                else if (x[2] < Z_RETURN || x[2] > Z_EXIT) {
-                    // leave (lib.rs:368-385)
-                    const double* c = C.mouth[i];
-                    x[0] += c[0] - C.axis;
-                    x[1] += c[1] - C.axis;
-                    if (x[2] < Z_RETURN) {
-                        x[2] = C.seam + x[2] - Z_RETURN;
-                        reg = R_SPLIT;
-                        last = i;
-                        atomicAdd(cnt + 1, 1u);
                     } else {
-                        x[2] = C.seam - (x[2] - Z_EXIT);
-                        v[2] *= -1.0;
-                        reg = R_COMBINE;
-                        last = -1;
-                        atomicAdd(cnt + 2, 1u);
-                        atomicAdd(cnt + 16 + sp, 1u);
+                        const float4 u = __ldg(p_rf + w), y = __ldg((cube ? p_dc : p_ac) + w);
+                        r[c][0] = u.x; r[c][1] = u.y; r[c][2] = u.z; r[c][3] = y.x; r[c][4] = y.y; r[c][5] = y.z;
+                        solid[c] = cube ? 0.0f : u.w;
+                        if (!cube) {
+                            const float4 z = __ldg(p_dc + w);
+                            r[c][6] = z.x; r[c][7] = z.y; r[c][8] = z.z;
+                            if (idle) { const float4 g = __ldg(p_gate + w); r[c][9] = g.x; r[c][10] = g.y; r[c][11] = g.z; }
+                        }
+                    }
+                }
+                bool odd = false;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+#pragma unroll
+                    for (int m = 0; m < NP; ++m) val[c][m] = mqp::widen_normal(r[c][m], odd);
+                if (odd)
+#pragma unroll
+                    for (int c = 0; c < NC; ++c)
+#pragma unroll
+                        for (int m = 0; m < NP; ++m) val[c][m] = (double)r[c][m];
+                c0 = solid[0] > 0.5f;
+                c1 = solid[1] > 0.5f;
+            }
+            const unsigned m0 = __ballot_sync(FULL, c0), m1 = NC == 2 ? __ballot_sync(FULL, c1) : 0u;
+            if (move) mask = NC == 2 ? (((m0 >> base) & 15u) | (((m1 >> base) & 15u) << 4)) : ((m0 >> base) & 255u);
+        }
+        return t;
+    };
+
+    for (;;) {
+        if (turn) {
+            bool got = false;
+            for (;;) {   // groups without a track take the next one
+                const unsigned need = __ballot_sync(FULL, !have && !drained && gl == 0);
+                if (!need) break;
+                uint32_t slot = first;
+                const unsigned later = __ballot_sync(FULL, !have && !drained && gl == 0 && !fresh);
+                if (later) {
+                    uint32_t o = 0;
+                    const int leader = __ffs(later) - 1;
+                    if (lane == leader) o = atomicAdd(head, (uint32_t)__popc(later));
+                    o = __shfl_sync(FULL, o, leader) + groups;
+                    if (!fresh) slot = o + __popc(later & ((1u << base) - 1u));
+                }
+                if (!have && !drained) {
+                    fresh = false;
+                    if (slot >= n) drained = true;
+                    else {
+                        id = slot;
+                        reg = T.region[id];
+                        if (reg < R_LOST) {
+                            have = got = true;
+                            k = 0;
+                            x = d == 0 ? T.x[id] : d == 1 ? T.y[id] : T.z[id];
+                            v = d == 0 ? T.vx[id] : d == 1 ? T.vy[id] : T.vz[id];
+                            rng = T.rng[id]; sp = T.sp[id]; last = T.last[id];
+                            qmdt = C.sp[sp].qmdt;
+                            const double nsd = C.sp[sp].nsd;
+                            const float nsd_up = nsd == 0.0 ? 0.0f : mag_up(nsd);
+                            nsd2 = __fmul_ru(__fmul_ru(nsd_up, nsd_up), 1.00001f);
+                            ub0 = __fmul_ru(__fmul_ru(nsd_up, mag_up(6.0 * C.s_gas)), 1.00001f);
+                        }
+                    }
+                }
+            }
+            if (!__any_sync(FULL, have)) break;
+            if (__any_sync(FULL, got)) {
+                enter_region(got);
+                coordinate(got);
+                const double t = locate(got);
+                if (got && gl < 3) { tw[2 * gl] = 1.0 - t; tw[2 * gl + 1] = t; }
+                __syncwarp();
+            }
+            turn = false;
+        }
+        // ---- field at the current position (lib.rs:70-88, world.rs:265-302)
+        const double* dr = drive + (size_t)(have ? k : 0u) * 10;
+        const double rf = dr[0], ac = dr[have && !cube ? reg : 0];
+        const uint64_t r1 = xs_step(rng);
+        const bool any_cube = __any_sync(FULL, have && cube), any_port = __any_sync(FULL, have && !cube);
+        const bool any_idle = __any_sync(FULL, have && idle);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int m = cn + 4 * c, lo = m & 1, mid = (m >> 1) & 1, hi = m >> 2;
+            const double wx = tw[cube ? lo : hi], wy = tw[2 + mid], wz = tw[4 + (cube ? hi : lo)];
+            const double w = wx * wy * wz;
+            double wg = 0.0;
+            if (any_idle) wg = C.gate_v * wx * wy * wz;
+            if (any_port) {
+                if (!cube) {
+                    if (G == 16) {
+#pragma unroll
+                        for (int z = 0; z < 6; ++z) prod[((upper ? 6 : 0) + z) * kTRow + m] = (upper && z >= 3 ? wg : w) * val[c][z % NP];
+                    } else {
+#pragma unroll
+                        for (int z = 0; z < 9; ++z) prod[z * kTRow + m] = w * val[c][z % NP];
+                        if (any_idle)
+#pragma unroll
+                            for (int z = 9; z < 12; ++z) prod[z * kTRow + m] = wg * val[c][z % NP];
+                    }
+                }
+            }
+            if (any_cube) {
+                if (cube && !upper)
+#pragma unroll
+                    for (int z = 0; z < 3; ++z) prod[z * kTRow + m] = w * (rf * val[c][z % NP] + val[c][(z + 3) % NP]);
+            }
+        }
+        __syncwarp();
+        double acc[NS];
+#pragma unroll
+        for (int f = 0; f < NS; ++f) {
+            acc[f] = 0.0;
+            if (f == 0 || (f < 3 && any_port) || any_idle) {
+                const double2* row = reinterpret_cast<const double2*>(prod + (chain + 3 * f) * kTRow);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const double2 p = row[c];
+                    acc[f] = c == 0 ? plus_zero(p.x) : acc[f] + p.x;
+                    acc[f] = acc[f] + p.y;
+                }
+            }
+        }
+        double e;
+        if (G == 16) {
+            if (any_port) {
+                const int f = chain / 3;
+                const double m = (f == 0 ? rf : ac) * acc[0];
+                if (gl < 12) xch[gl] = cube || f >= 2 ? acc[0] : m;
+                __syncwarp();
+                e = xch[d] + xch[3 + d] + xch[6 + d];
+                e = idle ? e + xch[9 + d] : plus_zero(e);   // + 0.0 where there is no gate
+                if (cube) e = xch[d];
+            } else {
+                e = shfl_d(acc[0], base + d);
+            }
+        } else {
+            e = rf * acc[0] + ac * acc[1 % NS] + acc[2 % NS];
+            e = idle ? e + acc[3 % NS] : plus_zero(e);
+            if (cube) e = acc[0];
+        }
+        // ---- transport_step (lib.rs:90-103)
+        v += qmdt * e;
+        x += v * C.dt;
+        if (have) {
+            if (cube) ++n_cube;
+            else if (idle) ++n_idle;
+            else ++n_port;
+            k += 1;
+        }
+        // ---- thermal collisions (world.rs:473-488): first against an FP32 bound, as in mq_f64.cu
+        {
+            const float vf = mag_up(v), sq = __fmul_ru(vf, vf);
+            const float s2 = __fadd_ru(__shfl_sync(FULL, sq, base), __fadd_ru(__shfl_sync(FULL, sq, base + 1), __shfl_sync(FULL, sq, base + 2)));
+            const float du = __fadd_rd((float)(uint32_t)(r1 >> 40) * 0x1.0p-24f, -ub0);
+            rng = r1;
+            const bool maybe = have && !(du >= 0.0f && __fmul_rd(du, du) >= __fmul_ru(nsd2, s2));
+            if (__any_sync(FULL, maybe)) {
+                const TSpec& S = C.sp[sp];
+                const double v0 = shfl_d(v, base), v1 = shfl_d(v, base + 1), v2 = shfl_d(v, base + 2);
+                const double vm = sqrt(v0 * v0 + v1 * v1 + v2 * v2);
+                const double bound = vm + 6.0 * C.s_gas;
+                const bool cand = maybe && xs_unit(r1) < S.nsd * bound;
+                if (__any_sync(FULL, cand)) {
+                    uint64_t r = r1, ra = 0, rb = 0;
+#pragma unroll
+                    for (int z = 0; z < 3; ++z) {
+                        r = xs_step(r);
+                        if (z == d) ra = r;
+                        r = xs_step(r);
+                        if (z == d) rb = r;
+                    }
+                    const double vg = C.s_gas * mqp::gauss(xs_unit(ra), xs_unit(rb));
+                    const double gv = v - vg;
+                    const double g0 = shfl_d(gv, base), g1 = shfl_d(gv, base + 1), g2 = shfl_d(gv, base + 2);
+                    const double gm = sqrt(g0 * g0 + g1 * g1 + g2 * g2);
+                    r = xs_step(r);
+                    const bool hit = cand && xs_unit(r) * bound < gm;
+                    if (cand) rng = r;
+                    if (__any_sync(FULL, hit)) {
+                        r = xs_step(r);
+                        const double c = 2.0 * xs_unit(r) - 1.0;
+                        r = xs_step(r);
+                        double sn_, cs_;
+                        mqp::sincos2pi(xs_unit(r), &sn_, &cs_);
+                        const double omc = 1.0 - c * c;
+                        const double sn = sqrt(omc > 0.0 ? omc : 0.0);
+                        const double nn = d == 2 ? c : sn * (d == 0 ? cs_ : sn_);
+                        const double vn = v - S.mr * gv + S.mr * gm * nn;
+                        if (hit) { v = vn; rng = r; }
                     }
                 }
             }
         }
-        T.x[id] = x[0]; T.y[id] = x[1]; T.z[id] = x[2];
-        T.vx[id] = v[0]; T.vy[id] = v[1]; T.vz[id] = v[2];
-        T.rng[id] = rng; T.region[id] = reg; T.last[id] = last;
+        // ---- routing (lib.rs:212-272)
+        coordinate(have);
+        bool changed = false;   // the track is in another region now
+        const int xhi = __double2hiint(x);
+        if (any_cube) {
+            // inside the posts' reach of no face, before the seam: nothing can happen
+            const bool off = have && cube && gl < 3 && (unsigned)(xhi - C.in_lo) >= C.in_n[d];
+            if (__any_sync(FULL, off)) {
+                const double x0 = shfl_d(x, base), x1 = shfl_d(x, base + 1), x2 = shfl_d(x, base + 2);
+                const double m0 = shfl_d(q, base), m1 = shfl_d(q, base + 1), m2 = shfl_d(q, base + 2);
+                const float p0 = (float)m0, p1 = (float)m1, p2 = (float)m2;
+                bool unsure = false, solid = false;
+                {
+                    const float l = C.F.size;
+                    bool far = false;   // within kNear of a face plane the FP32 `inside` is not to be trusted
+                    const bool inside = !below(p0, 0.0f, far) && !below(p1, 0.0f, far) && !below(p2, 0.0f, far) && below(p0, l, far) &&
+                                        below(p1, l, far) && below(p2, l, far);
+                    unsure = far;
+                    for (int f = gl; f < 6; f += G) {
+                        const int a = f >> 1, side = f & 1;
+                        const float pa = a == 0 ? p0 : a == 1 ? p1 : p2, pb = a == 0 ? p1 : a == 1 ? p2 : p0, pc = a == 0 ? p2 : a == 1 ? p0 : p1;
+                        bool un = false;
+                        if (face_solid(C.F, a, side, side == 0 ? pa : l - pa, pb, pc, inside, un) && !un) solid = true;
+                        unsure |= un;
+                    }
+                }
+                constexpr unsigned GM = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+                const bool g_solid = ((__ballot_sync(FULL, solid) >> base) & GM) != 0u, g_unsure = ((__ballot_sync(FULL, unsure) >> base) & GM) != 0u;
+                const bool go = have && cube;   // a group that is well inside finds just that
+                if (go) {
+                    bool blocked = g_solid;
+                    if (g_unsure) {
+                        const double mm[3] = {m0, m1, m2};
+                        int sg = 0;
+                        blocked = mqc::classify(C.cube, mm, 0.0, &sg) != mqc::ID_FREE;
+                    }
+                    bool done = false;
+                    if (blocked) { reg = R_LOST; done = true; }
+                    if (!done && x2 > C.seam) {
+                        const int i = mqc::nearest_port(C.cube, m0, m1);
+                        const double* c = C.mouth[i];
+                        if (mqc::dist2d(x0 - c[0], x1 - c[1]) < C.ap_r * 0.001) {
+                            // enter (lib.rs:338-367)
+                            uint32_t* cnt = counts + (size_t)i * kNC;
+                            const double depth = x2 - C.seam;
+                            if (d < 2) x += C.axis - c[d];
+                            if (reg == R_SPLIT) {
+                                if (d == 2) x = Z_RETURN + depth;
+                                if (gl == 0) {
+                                    atomicAdd(cnt + 0, 1u);
+                                    if (last >= 0) {
+                                        atomicAdd(cnt + 3, 1u);
+                                        atomicAdd(cnt + 5 + last, 1u);
+                                        if (last != i) atomicAdd(cnt + 4, 1u);
+                                    }
+                                }
+                            } else {
+                                if (d == 2) { x = Z_EXIT - depth; v *= -1.0; }
+                                if (gl == 0) atomicAdd(cnt + 14, 1u);
+                            }
+                            reg = 1 + i;
+                            changed = done = true;
+                        } else if (x2 > C.size) { reg = R_LOST; done = true; }
+                    }
+                    if (!done && x1 > C.size && mqc::dist2d(m0 - C.ent_c, m2 - C.ent_b) >= C.ap_r) { reg = R_LOST; done = true; }
+                    if (!done) {
+                        if (x1 > C.size + C.l_ext_m) reg = (reg == R_SPLIT) ? R_BACK : R_DETECTED;
+                        else if (x0 < 0.0 || x1 < 0.0 || x2 < 0.0 || x0 > C.size) reg = R_LOST;
+                    }
+                }
+            }
+        }
+        double t = locate(have && !changed && reg < R_LOST);
+        if (any_port) {
+            // is_crash (world.rs:309-314): outside the box, or the nearest node is a conductor
+            const bool port = have && !cube;
+            const long long bx = __double_as_longlong(x);
+            const unsigned th = (unsigned)__double2hiint(t);
+            const unsigned out = (__ballot_sync(FULL, lt_zero(bx) || gt_pos(bx, __double_as_longlong(glim))) >> base) & 7u;
+            const unsigned hb = (__ballot_sync(FULL, th >= 0x3fe00000u && th < 0x7ff00000u) >> base) & 7u;   // t >= 0.5
+            const unsigned zf = __shfl_sync(FULL, (lt_pos(bx, __double_as_longlong(Z_RETURN)) ? 1u : 0u) |
+                                                      (gt_pos(bx, __double_as_longlong(Z_EXIT)) ? 2u : 0u), base + 2);
+            const unsigned near = ((hb & 1u) << 2) | (hb & 2u) | ((hb >> 2) & 1u);
+            if (port) {
+                const int i = reg - 1;
+                uint32_t* cnt = counts + (size_t)i * kNC;
+                if (out || ((mask >> near) & 1u)) {
+                    reg = R_LOST;
+                    if (gl == 0) atomicAdd(cnt + 15, 1u);
+                } else if (zf) {
+                    // leave (lib.rs:368-385)
+                    const double* c = C.mouth[i];
+                    if (d < 2) x += c[d] - C.axis;
+                    if (zf & 1u) {
+                        if (d == 2) x = C.seam + x - Z_RETURN;
+                        reg = R_SPLIT;
+                        last = i;
+                        if (gl == 0) atomicAdd(cnt + 1, 1u);
+                    } else {
+                        if (d == 2) { x = C.seam - (x - Z_EXIT); v *= -1.0; }
+                        reg = R_COMBINE;
+                        last = -1;
+                        if (gl == 0) { atomicAdd(cnt + 2, 1u); atomicAdd(cnt + 16 + sp, 1u); }
+                    }
+                    changed = true;
+                }
+            }
+        }
+        if (__any_sync(FULL, changed)) {
+            enter_region(changed);
+            coordinate(changed);
+            const double t2 = locate(changed);
+            if (changed) t = t2;
+        }
+        {
+            const double omt = 1.0 - t;
+            if (gl < 3) { tw[2 * gl] = omt; tw[2 * gl + 1] = t; }
+        }
+        __syncwarp();
+        const bool put = have && (reg >= R_LOST || k >= steps);
+        if (__any_sync(FULL, put)) {
+            turn = true;
+            if (put) {
+                if (gl < 3) {
+                    (gl == 0 ? T.x : gl == 1 ? T.y : T.z)[id] = x;
+                    (gl == 0 ? T.vx : gl == 1 ? T.vy : T.vz)[id] = v;
+                }
+                if (gl == 0) { T.rng[id] = rng; T.region[id] = reg; T.last[id] = last; }
+                have = false;
+            }
+        }
     }
+    if (gl != 0) n_cube = n_port = n_idle = 0;
     add_steps(stepc, n_cube, n_port, n_idle);
 }
 
@@ -277,7 +596,7 @@ struct mq_tandem {
     size_t drive_cap = 0;
     uint32_t* counts = nullptr;
     unsigned long long* stepc = nullptr;   // executed track-steps: cube, driven port, idle port; mixed engine's
-                                           // cell-cache fills: cube, port
+                                           // cell-cache fills: cube, port; queue head of the FP64 kernel
     mqtm::State* mix = nullptr;            // the mixed-precision engine (MQ_PREC_MIXED)
     cudaStream_t st = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -364,7 +683,7 @@ mq_status mq_tandem_create(const mq_tandem_desc* d, int32_t device, mq_tandem** 
         P.idle = p.tone_khz == 0.0;
     }
     if (cudaMalloc(&t->counts, 9 * kNC * sizeof(uint32_t)) != cudaSuccess) return bail(MQ_ERR_NOMEM);
-    if (cudaMalloc(&t->stepc, 5 * sizeof(unsigned long long)) != cudaSuccess) return bail(MQ_ERR_NOMEM);
+    if (cudaMalloc(&t->stepc, 6 * sizeof(unsigned long long)) != cudaSuccess) return bail(MQ_ERR_NOMEM);
     C.cube = d->cube;
     for (int a = 0; a < 3; ++a) { C.cn[a] = d->cube_dims[a]; C.clo[a] = d->cube_lo_mm[a]; }
     C.ch_mm = d->cube_h_mm;
@@ -380,6 +699,29 @@ mq_status mq_tandem_create(const mq_tandem_desc* d, int32_t device, mq_tandem** 
     C.l_ext_m = d->cube.l_ext * 0.001;
     C.dt = d->dt;
     C.gate_v = d->gate_bias_v;
+    {   // the FP32 face filter and the range that needs none
+        const mq_cube_geom& g = d->cube;
+        CubeF& F = C.F;
+        F.size = (float)mqc::size(g); F.c0 = (float)mqc::c0(g); F.pitch = (float)g.pitch; F.half_d = (float)(g.d / 2.0);
+        F.t_pcb = (float)g.t_pcb; F.gap = (float)g.gap; F.ptd = (float)mqc::post_top_depth(g); F.stem_r = (float)g.stem_r;
+        F.clear_r = (float)g.clear_r; F.rod_hole = (float)(g.d / 2.0 + g.rod_clear_extra); F.l_ext = (float)g.l_ext;
+        F.cap_reach = (float)(g.l_ext + g.cap_gap); F.cap_r = (float)g.cap_r; F.ap_r = (float)g.ap_r;
+        F.n = g.n; F.array = g.array;
+        F.ent_axis = g.ent_axis; F.ent_side = g.ent_side; F.ent_cell0 = g.ent_cell[0]; F.ent_cell1 = g.ent_cell[1];
+        F.ext_axis = g.ext_axis; F.ext_side = g.ext_side; F.ext_cell0 = g.ext_cell[0]; F.ext_cell1 = g.ext_cell[1];
+        auto word = [](double v) {
+            int64_t b;
+            std::memcpy(&b, &v, 8);
+            return (int32_t)(b >> 32);
+        };
+        const double lo = mqc::post_top_depth(g) + 0.01, hi = mqc::size(g) - lo, zhi = std::fmin(hi, C.seam * 1000.0 - 0.01);
+        C.in_lo = word(lo * 1e-3) + 1;
+        for (int a = 0; a < 3; ++a) {
+            const double top = (a == 2 ? zhi : hi) * 1e-3;
+            const int32_t up = top > 0.0 ? word(top) : 0;
+            C.in_n[a] = lo > 0.0 && up > C.in_lo ? (uint32_t)(up - C.in_lo) : 0u;
+        }
+    }
     const double mg = 28.0 * mqp::AMU;
     const double ngas = d->pressure_pa / (mqp::KB * d->temp_k);
     C.s_gas = sqrt(mqp::KB * d->temp_k / mg);
@@ -471,6 +813,12 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
         TCK(cudaMalloc(&t->drive, tab * 10 * 8), "drive table");
         t->drive_cap = tab * 10 * 8;
     }
+    int sms = 0;
+    if (!t->mix) {   // one block of the FP64 kernel per SM: the shared memory asked for lets no second one in
+        TCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, t->dev), "device attributes");
+        TCK(cudaFuncSetAttribute(k_tandem<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTPad), "tandem kernel");
+        TCK(cudaFuncSetAttribute(k_tandem<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTPad), "tandem kernel");
+    }
     uint64_t per = n ? ((uint64_t)1 << 27) / n : tab;
     per = per < 32 ? 32 : (per > 4096 ? 4096 : per);
     std::vector<double> dtab(tab * 10);
@@ -501,8 +849,14 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
         }
         for (uint64_t q = 0; q < k && n; q += per, ++launches) {
             const uint64_t m = k - q < per ? k - q : per;
-            k_tandem<<<(unsigned)((n + 127) / 128), 128, 0, t->st>>>(t->C, T, (uint32_t)n, (const double*)t->drive + q * 10,
-                                                                    (uint32_t)m, t->counts, t->stepc);
+            uint32_t* head = reinterpret_cast<uint32_t*>(t->stepc + 5);
+            TCK(cudaMemsetAsync(head, 0, sizeof(*head), t->st), "queue head");
+            if (n <= 8 * (size_t)sms)
+                k_tandem<16><<<sms, kTBlock, kTPad, t->st>>>(t->C, T, (uint32_t)n, (const double*)t->drive + q * 10, (uint32_t)m,
+                                                             t->counts, t->stepc, head);
+            else
+                k_tandem<4><<<sms, kTBlock, kTPad, t->st>>>(t->C, T, (uint32_t)n, (const double*)t->drive + q * 10, (uint32_t)m,
+                                                            t->counts, t->stepc, head);
             TCK(cudaGetLastError(), "tandem kernel");
         }
     }

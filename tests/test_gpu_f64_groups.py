@@ -53,3 +53,26 @@ def test_groups_equal_oracle(coarse, name, n):
         assert st.ion_steps == R.run(G, b, jobs, ref)
     _assert_bitequal(ions, ref, f"{name} n={n}: to completion")
     assert (ions.status != 0).all()
+
+
+@pytest.mark.parametrize("mouth", [True, False])
+@pytest.mark.parametrize("n", [1, 17, 1216, 1217, 5003])
+def test_tandem_groups_equal_oracle(tandem_small, n, mouth):
+    """The FP64 tandem kernel at the sizes where its lane groups change width or refill, tracks of every
+    region side by side (a first advance spreads them; some are then set lost), in two advances."""
+    from oracle import mqtandem as O
+    m = tandem_small(n=n, seed=77, mouth_start=mouth)
+    d = O.desc_from(m.desc)
+    ref = O.inject(d, 77, mouth, n)
+    cnt = np.zeros((9, O.NC), np.uint32)
+    for s0, k in ((0, 2999), (2999, 1)):
+        m.advance(k)
+        O.advance(d, ref, s0, k, counts=cnt)
+        if n > 1:
+            m.tracks.region[3::17] = 11
+            ref.region[3::17] = 11
+    for k, _ in O.TRACK_FIELDS:
+        a, b = getattr(m.tracks, k), getattr(ref, k)
+        assert np.array_equal(a.view(np.uint8), b.view(np.uint8)), k
+    assert np.array_equal(m.counts_array(), cnt)
+    m.close()
