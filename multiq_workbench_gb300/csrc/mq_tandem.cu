@@ -25,6 +25,9 @@ constexpr double Z_EXIT = 18.6e-3;     // world.rs:21
 constexpr double Z_RETURN = 0.5e-3;    // world.rs:22
 constexpr int R_SPLIT = 0, R_COMBINE = 10, R_LOST = 11, R_BACK = 12, R_DETECTED = 13;
 constexpr int kNC = 21;                 // counters per port (mq_port_counts)
+constexpr size_t kCntBytes = (9 * kNC * 4 + 7) / 8 * 8;               // port counters, then six 8-byte step counters
+constexpr size_t kTail = kCntBytes + 6 * sizeof(unsigned long long);
+constexpr size_t kStageMax = 256 * 1024;
 
 using namespace mqf;
 
@@ -148,6 +151,22 @@ constexpr int kTRow = 10;
 constexpr int kTSums = 6 + 12 * kTRow;
 constexpr int kTGroup = kTSums + 12;     // doubles of shared memory per group
 constexpr int kTPad = 120 * 1024;        // one block per SM
+
+// drive of global steps [s0, s0 + k): rf = V_rf sin(2 pi f_rf t), ac_i = V_ac sin(2 pi f_i t), t = s dt
+// (lib.rs:178-182); one thread per step and tone. On the host, a microsecond a step, it took a tenth of
+// a large advance. `Out` is float for the mixed engine (no FP64 conversions in its step loop).
+struct Tones { double f[10], v[10], dt; };
+template <class Out>
+__global__ void k_drive(const __grid_constant__ Tones tn, uint64_t s0, uint32_t k, Out* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= k * 10u) return;
+    const uint32_t q = i / 10u, c = i % 10u;
+    const double t = (double)(s0 + q) * tn.dt;
+    const double p = tn.f[c] * t;
+    double s, co;
+    mqp::sincos2pi(p - floor(p), &s, &co);
+    out[i] = (Out)(tn.v[c] * s);
+}
 
 template <int G>
 __global__ void __launch_bounds__(kTBlock, 1)
@@ -597,6 +616,7 @@ struct mq_tandem {
     uint32_t* counts = nullptr;
     unsigned long long* stepc = nullptr;   // executed track-steps: cube, driven port, idle port; mixed engine's
                                            // cell-cache fills: cube, port; queue head of the FP64 kernel
+    char* stage = nullptr;                 // pinned: a small call's tracks, then the counters
     mqtm::State* mix = nullptr;            // the mixed-precision engine (MQ_PREC_MIXED)
     cudaStream_t st = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -608,22 +628,6 @@ mq_status tfail(mq_tandem* t, mq_status c, const std::string& m) {
     return c;
 }
 #define TCK(call, what) do { cudaError_t c_ = (call); if (c_ != cudaSuccess) return tfail(t, c_ == cudaErrorMemoryAllocation ? MQ_ERR_NOMEM : MQ_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(c_)); } while (0)
-
-// drive of global steps [s0, s0 + k): rf = V_rf sin(2 pi f_rf t), ac_i = V_ac sin(2 pi f_i t), t = s dt (lib.rs:178-182)
-void drive_table(const mq_tandem_desc& d, uint64_t s0, uint64_t k, double* out) {
-    for (uint64_t q = 0; q < k; ++q) {
-        const double t = (double)(s0 + q) * d.dt;
-        double s, c;
-        double p = d.f_rf * t;
-        mqp::sincos2pi(p - floor(p), &s, &c);
-        out[10 * q] = d.v_rf * s;
-        for (int i = 0; i < 9; ++i) {
-            p = d.port[i].tone_khz * 1000.0 * t;
-            mqp::sincos2pi(p - floor(p), &s, &c);
-            out[10 * q + 1 + i] = d.port[i].v_ac * s;
-        }
-    }
-}
 }  // namespace
 
 extern "C" {
@@ -682,8 +686,8 @@ mq_status mq_tandem_create(const mq_tandem_desc* d, int32_t device, mq_tandem** 
         P.inv_kh = 1.0 / p.h;
         P.idle = p.tone_khz == 0.0;
     }
-    if (cudaMalloc(&t->counts, 9 * kNC * sizeof(uint32_t)) != cudaSuccess) return bail(MQ_ERR_NOMEM);
-    if (cudaMalloc(&t->stepc, 6 * sizeof(unsigned long long)) != cudaSuccess) return bail(MQ_ERR_NOMEM);
+    if (cudaMalloc(&t->counts, kTail) != cudaSuccess) return bail(MQ_ERR_NOMEM);
+    t->stepc = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(t->counts) + kCntBytes);
     C.cube = d->cube;
     for (int a = 0; a < 3; ++a) { C.cn[a] = d->cube_dims[a]; C.clo[a] = d->cube_lo_mm[a]; }
     C.ch_mm = d->cube_h_mm;
@@ -758,7 +762,7 @@ void mq_tandem_destroy(mq_tandem* t) {
     if (t->tr) cudaFree(t->tr);
     if (t->drive) cudaFree(t->drive);
     if (t->counts) cudaFree(t->counts);
-    if (t->stepc) cudaFree(t->stepc);
+    if (t->stage) cudaFreeHost(t->stage);
     if (t->mix) mqtm::destroy(t->mix);
     for (auto& e : t->ev) if (e) cudaEventDestroy(e);
     if (t->st) cudaStreamDestroy(t->st);
@@ -798,11 +802,26 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
         if (tr->sp[i] < 0 || tr->sp[i] >= t->desc.nspecies || tr->region[i] < 0 || tr->region[i] > R_DETECTED ||
             tr->last[i] < -1 || tr->last[i] > 8)
             return tfail(t, MQ_ERR_INVALID, "track " + std::to_string(i) + " has an invalid species, region or last port");
-    for (int k = 0; k < 10; ++k) TCK(cudaMemcpyAsync(dev[k], host[k], sz[k] * n, cudaMemcpyHostToDevice, t->st), "track upload");
-    std::vector<uint32_t> cnt(9 * kNC);
-    for (int i = 0; i < 9; ++i) std::memcpy(&cnt[(size_t)i * kNC], &counts[i], sizeof(mq_port_counts));
-    TCK(cudaMemcpyAsync(t->counts, cnt.data(), cnt.size() * 4, cudaMemcpyHostToDevice, t->st), "counter upload");
-    TCK(cudaMemsetAsync(t->stepc, 0, 5 * sizeof(unsigned long long), t->st), "step counters");
+    // Few tracks go through one pinned block, in one copy each way: ten copies of pageable arrays cost
+    // 5 us each whatever their size. Many are copied array by array, which the driver does as fast as a
+    // host memcpy would stage them.
+    if (!t->stage && cudaMallocHost(&t->stage, kStageMax + kTail) != cudaSuccess) {
+        cudaGetLastError();
+        return tfail(t, MQ_ERR_NOMEM, "pinned staging");
+    }
+    TCK(cudaStreamSynchronize(t->st), "tandem");   // a call that failed may have left copies of the block under way
+    const bool staged = tb <= kStageMax;
+    char* const tail = t->stage + kStageMax;   // port counters, then step counters: their device order
+    if (staged) {
+        size_t o = 0;
+        for (int k = 0; k < 10; ++k) { std::memcpy(t->stage + o, host[k], sz[k] * n); o += sz[k] * n; }
+        TCK(cudaMemcpyAsync(base, t->stage, tb, cudaMemcpyHostToDevice, t->st), "track upload");
+    } else {
+        for (int k = 0; k < 10; ++k) TCK(cudaMemcpyAsync(dev[k], host[k], sz[k] * n, cudaMemcpyHostToDevice, t->st), "track upload");
+    }
+    for (int i = 0; i < 9; ++i) std::memcpy(tail + (size_t)i * kNC * 4, &counts[i], sizeof(mq_port_counts));
+    std::memset(tail + kCntBytes, 0, kTail - kCntBytes);
+    TCK(cudaMemcpyAsync(t->counts, tail, kTail, cudaMemcpyHostToDevice, t->st), "counter upload");
     // Drive table: up to kTab steps per upload; kernels of `per` steps each, about 2^27 track-steps
     // per launch so that no single launch runs for long.
     const uint64_t kTab = 65536;
@@ -821,24 +840,22 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
     }
     uint64_t per = n ? ((uint64_t)1 << 27) / n : tab;
     per = per < 32 ? 32 : (per > 4096 ? 4096 : per);
-    std::vector<double> dtab(tab * 10);
-    std::vector<float> ftab(t->mix ? tab * 10 : 0);
+    Tones tones;
+    tones.f[0] = t->desc.f_rf; tones.v[0] = t->desc.v_rf; tones.dt = t->desc.dt;
+    for (int i = 0; i < 9; ++i) { tones.f[1 + i] = t->desc.port[i].tone_khz * 1000.0; tones.v[1 + i] = t->desc.port[i].v_ac; }
     uint32_t launches = 0;
-    uint64_t h2d = tb + cnt.size() * 4;
+    const uint64_t h2d = tb + 9 * kNC * 4;
     for (uint64_t s = 0; s < steps || s == 0; s += tab) {
         const uint64_t k = steps - s < tab ? steps - s : tab;
-        drive_table(t->desc, step0 + s, k, dtab.data());
-        // pageable source: the call returns once the host buffer has been staged, so it may be refilled next
-        if (t->mix) {   // the mixed engine reads the drive as FP32 (no FP64 conversions in its step loop)
-            for (uint64_t q = 0; q < k * 10; ++q) ftab[q] = (float)dtab[q];
-            if (k) TCK(cudaMemcpyAsync(t->drive, ftab.data(), k * 10 * 4, cudaMemcpyHostToDevice, t->st), "drive upload");
-            h2d += k * 10 * 4;
-        } else {
-            if (k) TCK(cudaMemcpyAsync(t->drive, dtab.data(), k * 10 * 8, cudaMemcpyHostToDevice, t->st), "drive upload");
-            h2d += k * 10 * 8;
+        if (k) {
+            const unsigned blocks = (unsigned)((k * 10 + 127) / 128);
+            if (t->mix) k_drive<float><<<blocks, 128, 0, t->st>>>(tones, step0 + s, (uint32_t)k, (float*)t->drive);
+            else k_drive<double><<<blocks, 128, 0, t->st>>>(tones, step0 + s, (uint32_t)k, (double*)t->drive);
+            TCK(cudaGetLastError(), "drive kernel");
+            ++launches;
         }
         if (s == 0) {
-            TCK(cudaEventRecord(t->ev[0], t->st), "event");   // times the kernels (and later table blocks)
+            TCK(cudaEventRecord(t->ev[0], t->st), "event");   // times the step kernels (and later table blocks)
             if (t->mix) TCK(mqtm::load(t->mix, T64, (uint32_t)n, t->st, &launches), "mixed tandem load");
         }
         if (!steps) break;
@@ -862,12 +879,18 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
     }
     if (t->mix) TCK(mqtm::store(t->mix, T64, (uint32_t)n, t->st, &launches), "mixed tandem store");
     TCK(cudaEventRecord(t->ev[1], t->st), "event");
-    for (int k = 0; k < 10; ++k) TCK(cudaMemcpyAsync(host[k], dev[k], sz[k] * n, cudaMemcpyDeviceToHost, t->st), "track download");
-    TCK(cudaMemcpyAsync(cnt.data(), t->counts, cnt.size() * 4, cudaMemcpyDeviceToHost, t->st), "counter download");
-    unsigned long long sc[5] = {0, 0, 0, 0, 0};
-    TCK(cudaMemcpyAsync(sc, t->stepc, sizeof(sc), cudaMemcpyDeviceToHost, t->st), "step counters");
+    if (staged) TCK(cudaMemcpyAsync(t->stage, base, tb, cudaMemcpyDeviceToHost, t->st), "track download");
+    else
+        for (int k = 0; k < 10; ++k) TCK(cudaMemcpyAsync(host[k], dev[k], sz[k] * n, cudaMemcpyDeviceToHost, t->st), "track download");
+    TCK(cudaMemcpyAsync(tail, t->counts, kTail, cudaMemcpyDeviceToHost, t->st), "counter download");
     TCK(cudaStreamSynchronize(t->st), "tandem");
-    for (int i = 0; i < 9; ++i) std::memcpy(&counts[i], &cnt[(size_t)i * kNC], sizeof(mq_port_counts));
+    if (staged) {
+        size_t o = 0;
+        for (int k = 0; k < 10; ++k) { std::memcpy(host[k], t->stage + o, sz[k] * n); o += sz[k] * n; }
+    }
+    for (int i = 0; i < 9; ++i) std::memcpy(&counts[i], tail + (size_t)i * kNC * 4, sizeof(mq_port_counts));
+    unsigned long long sc[5];
+    std::memcpy(sc, tail + kCntBytes, sizeof(sc));
     if (stats) {
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, t->ev[0], t->ev[1]);
@@ -880,7 +903,7 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
         stats->kernel_ms = ms;
         stats->launches = launches;
         stats->h2d_bytes = h2d;
-        stats->d2h_bytes = tb + cnt.size() * 4 + sizeof(sc);
+        stats->d2h_bytes = tb + 9 * kNC * 4 + sizeof(sc);
     }
     return MQ_OK;
 }
