@@ -265,8 +265,11 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
         if (em && lane == 0) atomicSub(&ctr->open, (uint32_t)__popc(em));
         ended = false;
         if ((iter & 31u) == 0u && __any_sync(FULL, drained)) {
+            // (lanes beyond the warp's share are drained from the start, and blocks may come after others have
+            // ended, so that the queue is empty is read off its head)
             const uint32_t open = __shfl_sync(FULL, *(volatile uint32_t*)&ctr->open, 0);
-            if (open <= hand_at) {
+            const uint32_t head = __shfl_sync(FULL, *(volatile uint32_t*)&ctr->head, 0);
+            if (open <= hand_at && head >= count) {
                 if (have) {
                     hand[MQ_CHK(atomicAdd(&ctr->handed[0], 1u), hand_at, MQ_SITE_MIX_HAND)] = make_uint2(id, done);
                     put_ion(io, keep, n_all, id, n, ncoll, leg, 0, xh, xl, uh, ul);

@@ -53,3 +53,25 @@ def test_groups_equal_one_lane_kernel(coarse, name, wide):
     m = jid < 5
     for f in FIELDS:
         assert np.array_equal(getattr(whole, f)[m].view(np.uint8), getattr(cut, f).view(np.uint8)), f"{name}: 37-step launches, {f}"
+
+
+def test_two_engines_at_once(coarse):
+    """Blocks of one batch that start only after others have ended (another engine's kernels hold their SMs):
+    no ion is left behind when the last ones are handed over."""
+    from concurrent.futures import ThreadPoolExecutor
+    mq = _mq()
+    ph = _variants()["half_kick_gauss"]
+    jobs = [mq.Job(mq.Species(499.0, 1.0, 2.95 * 499.0 ** (2 / 3)), mq.RfAc(100.0, 500e3, 0.5, 100e3), n, 5) for n in (23878, 31000)]
+    engines = [mq.Engine(coarse, mq.PREC_MIXED) for _ in jobs]
+    try:
+        alone = [e.run_batch_ions([j], DC, ph)[0] for e, j in zip(engines, jobs)]
+        with ThreadPoolExecutor(2) as pool:
+            for _ in range(4):
+                both = [f.result()[0] for f in [pool.submit(e.run_batch_ions, [j], DC, ph) for e, j in zip(engines, jobs)]]
+                for a, b in zip(alone, both):
+                    assert (b.status != 0).all()
+                    for f in FIELDS:
+                        assert np.array_equal(getattr(a, f).view(np.uint8), getattr(b, f).view(np.uint8)), f
+    finally:
+        for e in engines:
+            e.close()
