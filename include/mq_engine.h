@@ -132,7 +132,8 @@ uint64_t    mq_fnv1a64(const void* data, size_t bytes, uint64_t h);
  * fixed by #defines and environment variables: simulation/chsim/src/tiled.rs:10-29). */
 typedef struct mq_tuning {
     int32_t threads_per_block;   /* fixed at 128                                          */
-    int32_t blocks_per_sm;       /* resident blocks per SM of the persistent grid (1..3)   */
+    int32_t blocks_per_sm;       /* resident blocks per SM of the persistent grid (1..3);
+                                    1 with 48-byte records is two below 3.5 GB of them     */
     uint32_t chunk;              /* steps per ion per launch (compaction interval)         */
     int32_t use_graph;           /* replay the launch sequence as one CUDA graph           */
     int32_t prefetch;            /* L1-prefetch the cell each ion is heading for           */

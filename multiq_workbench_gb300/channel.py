@@ -337,7 +337,7 @@ class Engine:
     def set_tuning(self, blocks_per_sm: int | None = None, chunk: int | None = None, use_graph: bool | None = None,
                    prefetch: bool | None = None, wide_records: bool | None = None, sort_cells: bool | None = None) -> None:
         """Override the mixed engine's launch shape; ``wide_records`` picks 96-byte node records read
-        with 256-bit loads (the default on grids below 1 GB of 48-byte records) over 48-byte ones;
+        with 256-bit loads (the default on grids below 0.55 GB of 48-byte records) over 48-byte ones;
         ``sort_cells`` puts every launch's live ions in the Morton order of their cells."""
         cur = self.tuning()
         t = N.mq_tuning(128, int(blocks_per_sm if blocks_per_sm is not None else cur["blocks_per_sm"]),

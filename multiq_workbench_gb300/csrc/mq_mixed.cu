@@ -95,8 +95,16 @@ __device__ __forceinline__ void rotate(float& s, float& c, float cw, float sw) {
 //           a lane of a group), and the values come in the pairs that two-at-a-time arithmetic takes.
 // Wide records are faster where the cell reloads hit L2, slower on fine grids whose gathers reach HBM
 // and pay for twice the footprint.
+// Narrow: a corner lies in the slot of its node's parity, not of its place in the cell, so a move to the next
+// cell along an axis replaces the far face's four slots and leaves the near face where it is; the order of
+// an axis's two slots goes into the interpolation. These grids' fills are bound by L1 (24 reads of 16 bytes for
+// each lane, every other step), and 92 in 100 moves are along one axis: 0.050 mm study of a million ions 40.6 ms
+// with whole fills, which want neighbours' lines in L1 and so one block per SM, 39.1 with half fills, 30.5
+// with two blocks of 255 registers (three of 168 spill: 33.9). Wide records come from L2 past L1, and there
+// the slots' extra instructions cost more than half the reads give (sweep 55.8 -> 60.8 ms).
 struct Cell {
-    float R[3][8], D[3][8], A[3][8];   // corner values per field and component, corner q = a + 2b + 4c
+    float R[3][8], D[3][8], A[3][8];   // corner values per field and component, corner or slot q = a + 2b + 4c
+    uint32_t bits[8];                   // narrow: conductor bits of the cell based at each slot's node
     int32_t ci, cj, ck;
     float fci, fcj, fck;                // the same cell as floats (no int -> float conversion per step)
     uint32_t mask;                      // conductor bit per corner
@@ -114,20 +122,29 @@ __device__ __forceinline__ void ld256_na(const float4* p, float4& a, float4& b) 
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p));
 }
 
+// 16 bytes of a narrow record, where p is set
+__device__ __forceinline__ void ld_narrow(const float4* n, bool p, float& r, float& d, float& a, uint32_t& bits) {
+    asm("{.reg .pred p; setp.ne.u32 p, %4, 0; @p ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%5];}"
+        : "+f"(r), "+f"(d), "+f"(a), "+r"(bits) : "r"((uint32_t)p), "l"(n));
+}
+
 // NEAREST (the reference's legacy field mode: the field of the cell's lowest corner, t = 0) reads
 // only that corner's record, which also holds the cell's conductor bits: one record per fill.
+// A narrow fill reads the slots that hold another node than the new cell's, and leaves the conductor bits to
+// cell_mask (so that nothing waits for the reads here).
 template <bool WIDE, bool NEAREST>
 __device__ __forceinline__ void load_cell(const float4* __restrict__ nodes, const MixBatch& B, int32_t ci, int32_t cj,
                                           int32_t ck, Cell& c) {
     const uint32_t sy = (uint32_t)B.nx, sz = (uint32_t)B.nx * (uint32_t)B.ny;
-    const uint32_t base = node_of(B, ci, cj, ck);
+    uint32_t base = node_of(B, ci, cj, ck);
     uint32_t m = 0;
     if (WIDE) {
+        base = (uint32_t)MQ_CHK_SPAN(base, NEAREST ? 1u : sy + 2u, (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
+        const float4* const p0 = nodes + (size_t)6 * base;
+        const float4* const p2 = p0 + (size_t)6 * sy;
 #pragma unroll
         for (int q = 0; q < (NEAREST ? 1 : 4); ++q) {
-            uint32_t o = base + (uint32_t)(q & 1) + ((q & 2) ? sy : 0u);
-            o = (uint32_t)MQ_CHK(o, (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
-            const float4* p = nodes + (size_t)6 * o;
+            const float4* p = ((q & 2) ? p2 : p0) + 6 * (q & 1);
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 float4 u, v;
@@ -140,21 +157,38 @@ __device__ __forceinline__ void load_cell(const float4* __restrict__ nodes, cons
                 if (q == 0 && d == 0) m = __float_as_uint(v.z);   // conductor bits of the cell's corners
             }
         }
+    } else if (NEAREST) {
+        const uint32_t o = (uint32_t)MQ_CHK_SPAN(3u * base, 3u, 3u * (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
+        const float4 x = __ldg(nodes + o), y = __ldg(nodes + o + 1), z = __ldg(nodes + o + 2);
+        c.R[0][0] = x.x; c.R[1][0] = y.x; c.R[2][0] = z.x;
+        c.D[0][0] = x.y; c.D[1][0] = y.y; c.D[2][0] = z.y;
+        c.A[0][0] = x.z; c.A[1][0] = y.z; c.A[2][0] = z.z;
+        m = __float_as_uint(x.w);
     } else {
+        // nodes of each parity along the axes, and whether the slots hold others
+        const int32_t i0 = ci + (ci & 1), i1 = ci | 1, j0 = cj + (cj & 1), j1 = cj | 1, k0 = ck + (ck & 1), k1 = ck | 1;
+        const bool sx0 = i0 != c.ci + (c.ci & 1), sx1 = i1 != (c.ci | 1), sy0 = j0 != c.cj + (c.cj & 1), sy1 = j1 != (c.cj | 1);
+        const bool sz0 = k0 != c.ck + (c.ck & 1), sz1 = k1 != (c.ck | 1);
 #pragma unroll
-        for (int q = 0; q < (NEAREST ? 1 : 8); ++q) {
-            uint32_t o = 3u * (base + (uint32_t)(q & 1) + ((q & 2) ? sy : 0u) + ((q & 4) ? sz : 0u));
+        for (int q = 0; q < 8; ++q) {
+            const bool p = ((q & 1) ? sx1 : sx0) || ((q & 2) ? sy1 : sy0) || ((q & 4) ? sz1 : sz0);
+            uint32_t o = 3u * node_of(B, (q & 1) ? i1 : i0, (q & 2) ? j1 : j0, (q & 4) ? k1 : k0);
             o = (uint32_t)MQ_CHK_SPAN(o, 3u, 3u * (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
-            // through L1, which these grids' fills depend on: neighbouring cells share a face
-            const float4 x = __ldg(nodes + o), y = __ldg(nodes + o + 1), z = __ldg(nodes + o + 2);
-            c.R[0][q] = x.x; c.R[1][q] = y.x; c.R[2][q] = z.x;
-            c.D[0][q] = x.y; c.D[1][q] = y.y; c.D[2][q] = z.y;
-            c.A[0][q] = x.z; c.A[1][q] = y.z; c.A[2][q] = z.z;
-            if (q == 0) m = __float_as_uint(x.w);
+            ld_narrow(nodes + o, p, c.R[0][q], c.D[0][q], c.A[0][q], c.bits[q]);
+            uint32_t pad;
+            ld_narrow(nodes + o + 1, p, c.R[1][q], c.D[1][q], c.A[1][q], pad);
+            ld_narrow(nodes + o + 2, p, c.R[2][q], c.D[2][q], c.A[2][q], pad);
         }
     }
     c.ci = ci; c.cj = cj; c.ck = ck; c.mask = m;
     c.fci = (float)ci; c.fcj = (float)cj; c.fck = (float)ck;
+}
+
+__device__ __forceinline__ uint32_t cell_mask(const Cell& c) {
+    const bool px = c.ci & 1, py = c.cj & 1, pz = c.ck & 1;
+    const uint32_t m0 = py ? (px ? c.bits[3] : c.bits[2]) : (px ? c.bits[1] : c.bits[0]);
+    const uint32_t m1 = py ? (px ? c.bits[7] : c.bits[6]) : (px ? c.bits[5] : c.bits[4]);
+    return pz ? m1 : m0;
 }
 
 // pull the 4 corner runs of a cell into L1 ahead of use
@@ -176,16 +210,22 @@ __device__ __forceinline__ void prefetch_cell(const float4* nodes, const MixBatc
     }
 }
 
+// lo + t (hi - lo) of an axis's two values. SLOTS: odd says that the second is the lower node's, and t is
+// negative then; hi - lo is the same number but for its sign, so that only a zero's sign can differ.
+template <bool SLOTS>
+__device__ __forceinline__ float lerp2(float t, bool odd, float f0, float f1) { return fmaf(t, f1 - f0, SLOTS && odd ? f1 : f0); }
+
 // E = a_rf RF(t) + DC(t) + a_ac AC(t): corner values combined first, then one trilinear pass
+template <bool SLOTS>
 __device__ __forceinline__ float field_comp(const float R[8], const float D[8], const float A[8], float a_rf, float a_ac,
-                                            float tx, float ty, float tz) {
+                                            float tx, float ty, float tz, bool ox, bool oy, bool oz) {
     float F[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) F[q] = fmaf(a_rf, R[q], fmaf(a_ac, A[q], D[q]));
-    const float c00 = fmaf(tx, F[1] - F[0], F[0]), c10 = fmaf(tx, F[3] - F[2], F[2]);
-    const float c01 = fmaf(tx, F[5] - F[4], F[4]), c11 = fmaf(tx, F[7] - F[6], F[6]);
-    const float c0 = fmaf(ty, c10 - c00, c00), c1 = fmaf(ty, c11 - c01, c01);
-    return fmaf(tz, c1 - c0, c0);
+    const float c00 = lerp2<SLOTS>(tx, ox, F[0], F[1]), c10 = lerp2<SLOTS>(tx, ox, F[2], F[3]);
+    const float c01 = lerp2<SLOTS>(tx, ox, F[4], F[5]), c11 = lerp2<SLOTS>(tx, ox, F[6], F[7]);
+    const float c0 = lerp2<SLOTS>(ty, oy, c00, c10), c1 = lerp2<SLOTS>(ty, oy, c01, c11);
+    return lerp2<SLOTS>(tz, oz, c0, c1);
 }
 
 // (xh + xl) - (th + tl) for a double-float position and threshold, as the sign-exact difference of
@@ -210,7 +250,7 @@ __device__ __forceinline__ void put_ion(const DevIons& io, float* __restrict__ k
 
 // ---------------------------------------------------------------- the persistent worker
 template <bool LEGACY, bool PREFETCH, bool WIDE, bool NEAREST>
-__global__ void __launch_bounds__(128, NEAREST ? 5 : 3)
+__global__ void __launch_bounds__(128, NEAREST ? 5 : WIDE ? 3 : 2)
 k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__ jobs, DevIons io,
         const uint32_t* __restrict__ list_in, uint32_t* __restrict__ list_out, Ctrs* ctr, int in_slot, uint32_t chunk,
         float* __restrict__ keep, const uint64_t* __restrict__ kph, uint32_t n_all, uint2* __restrict__ hand, uint32_t hand_at) {
@@ -230,7 +270,7 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
     // lanes that take ions: all 32 when the list fills the grid, else the warp's even share of it
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     bool have = false, drained = lane >= (count + warps - 1) / warps;
-    uint32_t id = 0, jid = 0, n = 0, done = 0, ncoll = 0;
+    uint32_t id = 0, jid = 0, n = 0, done = 0, stop = 0, ncoll = 0;
     int32_t leg = 0;
     float xh[3], xl[3], uh[3], ul[3];
     uint64_t Prf = 0, Pac = 0, Wac = 0;
@@ -238,7 +278,7 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
     // drive sines advanced by rotation each step and re-evaluated exactly from the
     // fixed-point phases every 4 loop iterations (warp-uniform), so rounding cannot build up
     float srf = 0.f, crf = 1.f, sac = 0.f, cac = 1.f, cw_ac = 1.f, sw_ac = 0.f;
-    float kick = 0.f, v_ac = 0.f, cand_a = 0.f, cand_b = 0.f;
+    float kick = 0.f, v_ac = 0.f, cand_aa = 0.f, cand_b = 0.f;
     uint32_t k0 = 0, k1 = 0;
     // per-step candidate uniforms: Philox block n>>2 (rc) and the next block (rn); rn is
     // refreshed for every lane on a warp-uniform schedule (every 4 loop iterations), so the
@@ -251,6 +291,12 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
 #pragma unroll
     for (int d = 0; d < 3; ++d) { xh[d] = xl[d] = uh[d] = ul[d] = 0.f; }
     c.ci = c.cj = c.ck = -1; c.mask = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        c.bits[q] = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) c.R[d][q] = c.D[d][q] = c.A[d][q] = 0.f;
+    }
     c.fci = c.fcj = c.fck = __int_as_float(0x7fc00000);   // NaN: differs from every floored position
 
     // Queue traffic is warp-synchronous and happens once every 4 iterations: survivors that ended in
@@ -306,7 +352,7 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                     sj_mr[threadIdx.x] = J.mr;
                     sj_floor[threadIdx.x] = J.floor_v;
                     sj_mfp[threadIdx.x] = J.mfp_mean;
-                    kick = J.kick; v_ac = J.use_ac ? J.v_ac : 0.0f; cand_a = J.cand_a; cand_b = J.cand_b;
+                    kick = J.kick; v_ac = J.use_ac ? J.v_ac : 0.0f; cand_aa = J.cand_a * J.cand_a; cand_b = J.cand_b;
                     Wac = ((uint64_t)J.w_ac_hi << 32) | J.w_ac_lo;
                     cw_ac = J.cw_ac; sw_ac = J.sw_ac;
                     n = io.steps[id]; ncoll = io.ncoll[id]; leg = io.leg[id];
@@ -317,8 +363,9 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                     }
                     // phase = offset + n * w (mod 1) in 64-bit fixed point
                     const uint64_t orf = kph[id], oac = kph[(size_t)n_all + id];
-                    Prf = orf + (uint64_t)n * Wrf;
-                    Pac = oac + (uint64_t)n * Wac;
+                    const uint64_t n4 = ((uint64_t)n + 3u) & ~(uint64_t)3u;   // the next exact drive
+                    Prf = orf + n4 * Wrf;
+                    Pac = oac + n4 * Wac;
                     // drive state as an uninterrupted run has it: exact at the last step that is
                     // a multiple of 4, then rotated forward (so re-queued ions continue bitwise).
                     // An ion at a multiple of 4 steps (every fresh ion) first steps on a re-sync
@@ -326,8 +373,8 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                     // neither is done here for it
                     const uint32_t r4 = n & 3u;
                     if (r4) {
-                        turn_sincos(Prf - (uint64_t)r4 * Wrf, srf, crf);
-                        turn_sincos(Pac - (uint64_t)r4 * Wac, sac, cac);
+                        turn_sincos(Prf - 4u * Wrf, srf, crf);
+                        turn_sincos(Pac - 4u * Wac, sac, cac);
                         for (uint32_t q = 0; q < r4; ++q) { rotate(srf, crf, B.cw_rf, B.sw_rf); rotate(sac, cac, cw_ac, sw_ac); }
                     }
                     const uint64_t key = io.rng[id];
@@ -339,10 +386,12 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                         rc = philox(k0, k1, n >> 2, 2u, 0u, 0u);
                         rn = philox(k0, k1, n >> 2, 3u, 0u, 0u);
                     }
+                    c.ck = -4;   // nothing held is of use
                     load_cell<WIDE, NEAREST>(nodes, B, clampi(__float2int_rd(xh[0]), 0, B.nx - 2), clampi(__float2int_rd(xh[1]), 0, B.ny - 2),
                               clampi(__float2int_rd(xh[2]), 0, B.nz - 2), c);
                     ++loads;
                     done = 0;
+                    stop = n >= B.max_steps ? 1u : B.max_steps - n < chunk ? B.max_steps - n : chunk;
                     have = true;
                 } else {
                     drained = true;
@@ -366,7 +415,12 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             rc = philox(k0, k1, n >> 2, 2u, 0u, 0u);
             rn = philox(k0, k1, n >> 2, 3u, 0u, 0u);
         }
-        if ((iter & 3u) == 0u && act) { turn_sincos(Prf, srf, crf); turn_sincos(Pac, sac, cac); }
+        if ((iter & 3u) == 0u && act) {
+            turn_sincos(Prf, srf, crf);
+            turn_sincos(Pac, sac, cac);
+            Prf += 4u * Wrf;
+            Pac += 4u * Wac;
+        }
         ++iter;
         if (act) {
             // ---- field at the current position
@@ -379,10 +433,16 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             const float a_rf = B.v_rf * srf;
             const float a_ac = v_ac * sac;
             float E[3];
+            const bool ox = c.ci & 1, oy = c.cj & 1, oz = c.ck & 1;
+            if (!NEAREST && !WIDE) {
+                tx = ox ? -tx : tx;
+                ty = oy ? -ty : ty;
+                tz = oz ? -tz : tz;
+            }
 #pragma unroll
             for (int d = 0; d < 3; ++d)
                 E[d] = NEAREST ? fmaf(a_rf, c.R[d][0], fmaf(a_ac, c.A[d][0], c.D[d][0]))   // = field_comp at t = 0
-                               : field_comp(c.R[d], c.D[d], c.A[d], a_rf, a_ac, tx, ty, tz);
+                               : field_comp<!WIDE>(c.R[d], c.D[d], c.A[d], a_rf, a_ac, tx, ty, tz, ox, oy, oz);
             // ---- kick (compensated) and drift (compensated)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
@@ -393,8 +453,27 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                 e = __fadd_rn(e, __fadd_rn(xl[d], ul[d]));
                 fast_two_sum(s, e, xh[d], xl[d]);
             }
-            Prf += Wrf;
-            Pac += Wac;
+            // ---- cell of the new position: its records are asked for before the collisions, which move no ion,
+            //      so that their way from L2 is covered by these (55.8 -> 53.0 ms on the sweep); and an L1 prefetch of
+            //      the cell one more step ahead. Cell changes are found on floored floats; an ion outside the box
+            //      (the unclamped cell index leaving [0, n-2]) has ended and needs no cell
+            const float ffi = floorf(xh[0]), ffj = floorf(xh[1]), ffk = floorf(xh[2]);
+            bool out = false;
+            if (ffi != c.fci || ffj != c.fcj || ffk != c.fck) {
+                out = ffi < 0.0f || ffj < 0.0f || ffk < 0.0f || ffi > B.lim_x - 1.0f || ffj > B.lim_y - 1.0f || ffk > B.lim_z - 1.0f;
+                if (!out) {
+                    load_cell<WIDE, NEAREST>(nodes, B, __float2int_rz(ffi), __float2int_rz(ffj), __float2int_rz(ffk), c);
+                    c.fci = ffi; c.fcj = ffj; c.fck = ffk;
+                    ++loads;
+                }
+            }
+            if (PREFETCH && !NEAREST) {
+                const int32_t pi = clampi(__float2int_rd(xh[0] + uh[0]), 0, B.nx - 2);
+                const int32_t pj = clampi(__float2int_rd(xh[1] + uh[1]), 0, B.ny - 2);
+                const int32_t pk = clampi(__float2int_rd(xh[2] + uh[2]), 0, B.nz - 2);
+                if (pi != c.ci || pj != c.cj || pk != c.ck) prefetch_cell<WIDE>(nodes, B, pi, pj, pk);
+            }
+            if (!WIDE && !NEAREST) c.mask = cell_mask(c);
             rotate(srf, crf, B.cw_rf, B.sw_rf);
             rotate(sac, cac, cw_ac, sw_ac);
             const uint32_t nprev = n;
@@ -407,7 +486,7 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                 // (no square root per step); see thermal_partner for why E|V| bounds the rate
                 const float um2 = fmaf(uh[0], uh[0], fmaf(uh[1], uh[1], uh[2] * uh[2]));
                 const float du = u0 - cand_b;
-                if (du < 0.0f || du * du < cand_a * cand_a * um2) {
+                if (du < 0.0f || du * du < cand_aa * um2) {
                     const float um = sqrtf(um2);
                     const float s_gas = sj_sgas[threadIdx.x], mr = sj_mr[threadIdx.x];
                     // two Philox blocks per candidate, drawn side by side: the first for the gas
@@ -476,21 +555,6 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                     leg = due ? nl : leg;
                 }
             }
-            // ---- cell of the new position (refresh the cache before the conductor test), and
-            //      an L1 prefetch of the cell one more step ahead
-            // cell changes are found on floored floats; indices are formed only when one is seen
-            const float ffi = floorf(xh[0]), ffj = floorf(xh[1]), ffk = floorf(xh[2]);
-            if (ffi != c.fci || ffj != c.fcj || ffk != c.fck) {
-                const int32_t ci = clampi(__float2int_rd(xh[0]), 0, B.nx - 2), cj = clampi(__float2int_rd(xh[1]), 0, B.ny - 2),
-                              ck = clampi(__float2int_rd(xh[2]), 0, B.nz - 2);
-                if (ci != c.ci || cj != c.cj || ck != c.ck) { load_cell<WIDE, NEAREST>(nodes, B, ci, cj, ck, c); ++loads; }
-            }
-            if (PREFETCH && !NEAREST) {
-                const int32_t pi = clampi(__float2int_rd(xh[0] + uh[0]), 0, B.nx - 2);
-                const int32_t pj = clampi(__float2int_rd(xh[1] + uh[1]), 0, B.ny - 2);
-                const int32_t pk = clampi(__float2int_rd(xh[2] + uh[2]), 0, B.nz - 2);
-                if (pi != c.ci || pj != c.cj || pk != c.ck) prefetch_cell<WIDE>(nodes, B, pi, pj, pk);
-            }
             // ---- termination tests: exit, return, box, conductor, timeout
             // (the loss-surface planes - exit, return and the crash window - are crossed on the full
             // double-float position against the double-float thresholds; the box test is the
@@ -501,9 +565,7 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             int32_t status = 0;
             if (xh[2] > B.z_exit_near && df_diff(xh[2], xl[2], B.z_exit_h, B.z_exit_l) > 0.0f) status = 3;
             else if (xh[2] < B.z_ret_near && df_diff(xh[2], xl[2], B.z_ret_h, B.z_ret_l) < 0.0f) status = 2;
-            else if (ffi < 0.0f || ffj < 0.0f || ffk < 0.0f || ffi > B.lim_x - 1.0f || ffj > B.lim_y - 1.0f ||
-                     ffk > B.lim_z - 1.0f)
-                status = 4;
+            else if (out) status = 4;
             else {
                 if (c.mask != 0u && df_diff(xh[2], xl[2], B.cz0_h, B.cz0_l) > 0.0f &&
                     df_diff(xh[2], xl[2], B.cz1_h, B.cz1_l) < 0.0f) {
@@ -513,9 +575,9 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                     const uint32_t q = (fx >= 0.5f ? 1u : 0u) | (fy >= 0.5f ? 2u : 0u) | (fz >= 0.5f ? 4u : 0u);
                     if ((c.mask >> q) & 1u) status = 1;
                 }
-                if (status == 0 && n >= B.max_steps) status = 5;
             }
-            if (status != 0 || done >= chunk) {
+            if (status != 0 || done >= stop) {
+                if (status == 0 && n >= B.max_steps) status = 5;
                 // ---- write back: counters to the ion states, position and velocity to the working
                 //      state (k_unstage turns it into the FP64 state when the caller wants that)
                 put_ion(io, keep, n_all, id, n, ncoll, leg, status, xh, xl, uh, ul);
@@ -1291,15 +1353,16 @@ Tuning default_tuning(int device, size_t nodes) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) { cudaGetLastError(); sms = 1; }
     t.sms = sms;
-    // Resident ions per SM by the size of the node records: on grids far larger than L2 the
-    // gathers of fewer ions in flight hit the caches more often than more warps hide latency
-    // (measured on the channel at 0.050 / 0.0333 mm, 2.4 / 8.0 GB of 48-byte records: 15.7 / 11.4
-    // G ion-steps/s at 1 block per SM against 15.0 / 7.1 at 2 and 10.6 / - at 3; the 0.100 mm grid,
-    // 0.30 GB, is best at 3). Wide records only in the first class: they win where the reloads hit
-    // L2 and lose where they reach HBM.
+    // Record width and resident ions per SM by the size of the grid (bytes of its 48-byte records). Wide records
+    // win while the part that the ions see lies in L2, with 3 blocks per SM and near the end with 2; then
+    // narrow ones with 2 blocks, until the gathers of fewer ions in flight hit the caches so much more often that
+    // 1 is better. Batch of 512,000 ions, ms, wide 3 / wide 2 / narrow 2 / narrow 1: 0.30 GB (0.100 mm channel) 10.7 / 12.0 /
+    // 13.3 / 18.5, 0.40 GB 11.3 / 12.1 / 13.4 / -, 0.45 GB 14.7 / 12.4 / 14.0 / -, 0.51 GB 17.6 / 12.8 / 14.3 / -, 0.58 GB
+    // 20.6 / - / 14.5 / 19.9, 1.22 GB 31.5 / - / 15.4 / 20.6, 2.6 GB - / - / 19.4 / 23.0, 3.4 GB - / - / 24.2 / 24.6,
+    // 4.6 GB - / - / 28.9 / 25.9, 8.0 GB - / - / 35.7 / 28.2.
     const double rec = 48.0 * (double)nodes;
-    t.blocks_per_sm = rec < 1.0e9 ? 3 : 1;
-    t.wide = rec < 1.0e9 ? 1 : 0;
+    t.wide = rec < 0.55e9 ? 1 : 0;
+    t.blocks_per_sm = rec < 0.42e9 ? 3 : rec < 0.55e9 ? 2 : 1;   // 1 with narrow records: run() doubles it below 3.5 GB
     return t;
 }
 
@@ -1508,6 +1571,8 @@ cudaError_t run(Scratch& s, const Tuning& t, DevGrid g, uint64_t grid_gen, const
     // resident blocks per SM: the tuning's, except for the nearest-node kernels, which hold no
     // 8-corner cache (about 100 registers instead of 167) and run as many blocks as fit
     int blocks = t.blocks_per_sm;
+    // one block per SM with narrow records is two of them below 3.5 GB (default_tuning has the figures)
+    if (!t.wide && blocks == 1 && 48.0 * (double)mb.nx * mb.ny * mb.nz < 3.5e9) blocks = 2;
     if (mb.nearest) {
         int nb = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_kernel(t, mb), t.tpb, 0) == cudaSuccess && nb > 0)

@@ -75,3 +75,39 @@ def test_two_engines_at_once(coarse):
     finally:
         for e in engines:
             e.close()
+
+
+@pytest.mark.parametrize("wide", [True, False], ids=["wide", "narrow"])
+def test_states_at_the_edges_equal_one_lane_kernel(coarse, wide):
+    """States a caller can hand in: outside the box, on its faces, at and past the step cap, at every
+    residue of the step count; 24,000 of them through the one-lane kernel, and in parts through the groups."""
+    mq = _mq()
+    ph = _variants()["half_kick_gauss"]
+    jobs = [mq.Job(mq.Species(499.0, 1.0, 2.95 * 499.0 ** (2 / 3)), mq.RfAc(100.0, 500e3, 0.5, 100e3), 24000, 9)]
+    rng = np.random.default_rng(3)
+    cap = int(round(ph.t_max / ph.dt))
+    with mq.Engine(coarse, mq.PREC_MIXED) as e:
+        e.set_dc(DC)
+        e.set_tuning(wide_records=wide)
+        st = e.inject(jobs, ph)
+        h = coarse.h
+        for f, n in (("x", coarse.nx), ("y", coarse.ny), ("z", coarse.nz)):
+            v = getattr(st, f)
+            pick = rng.random(v.size)
+            v[:] = np.where(pick < 0.05, h * (n - 1) * rng.choice([-0.01, 0.0, 0.999, 1.0, 1.02], v.size),
+                            np.where(pick < 0.1, h * rng.integers(0, n, v.size), v))
+        st.steps[:] = rng.integers(0, 64, st.steps.size)
+        late = rng.random(st.steps.size) < 0.05
+        st.steps[late] = cap + rng.integers(-3, 3, int(late.sum()))
+
+        def run(i0, i1):
+            s = mq.IonStates.empty(i1 - i0)
+            for f in FIELDS:
+                getattr(s, f)[:] = getattr(st, f)[i0:i1]
+            e.run_ions(jobs, ph, s, max_more=301)
+            return s
+        whole = run(0, 24000)
+        parts = [run(i, i + 6000) for i in range(0, 24000, 6000)]
+    for f in FIELDS:
+        b = np.concatenate([getattr(p, f) for p in parts])
+        assert np.array_equal(getattr(whole, f).view(np.uint8), b.view(np.uint8)), f
