@@ -133,7 +133,8 @@ uint64_t    mq_fnv1a64(const void* data, size_t bytes, uint64_t h);
 typedef struct mq_tuning {
     int32_t threads_per_block;   /* fixed at 128                                          */
     int32_t blocks_per_sm;       /* resident blocks per SM of the persistent grid (1..3);
-                                    1 with 48-byte records is two below 3.5 GB of them     */
+                                    1 with 48-byte records is two below 3.5 GB of them, 3 with
+                                    96-byte records four for lists of 2,048 ions per SM    */
     uint32_t chunk;              /* steps per ion per launch (compaction interval)         */
     int32_t use_graph;           /* replay the launch sequence as one CUDA graph           */
     int32_t prefetch;            /* L1-prefetch the cell each ion is heading for           */

@@ -249,8 +249,15 @@ __device__ __forceinline__ void put_ion(const DevIons& io, float* __restrict__ k
 }
 
 // ---------------------------------------------------------------- the persistent worker
-template <bool LEGACY, bool PREFETCH, bool WIDE, bool NEAREST>
-__global__ void __launch_bounds__(128, NEAREST ? 5 : WIDE ? 3 : 2)
+// What bounds it: with 96-byte records the latency of a step's chain and of the cell fills (on nearly every step of a
+// warp some lane needs one) at 12 or 16 warps per SM; with 48-byte records on larger grids the L1 reads of the
+// fills. So registers are kept for the cell, and all that only every fourth step, a collision or the end of a
+// flight reads lies in shared memory. BLOCKS: blocks per SM that the registers are cut for: 3 with wide records, 4
+// for long lists (run() has the rule), 2 with narrow ones, which then need no spills.
+// Measured, wide with registers only / tables in shared memory at 3 / at 4 blocks: sweep of 4.2 million ions 51.1 / 51.9 /
+// 48.7 ms, 40,000 legacy ions 15.4 / 15.0 / 15.0; narrow, 0.050 mm study 30.5 / 27.6 at 2 blocks (34.4 at 3).
+template <bool LEGACY, bool PREFETCH, bool WIDE, bool NEAREST, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS)
 k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__ jobs, DevIons io,
         const uint32_t* __restrict__ list_in, uint32_t* __restrict__ list_out, Ctrs* ctr, int in_slot, uint32_t chunk,
         float* __restrict__ keep, const uint64_t* __restrict__ kph, uint32_t n_all, uint2* __restrict__ hand, uint32_t hand_at) {
@@ -262,6 +269,19 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
     // refill, so those divergent branches do not wait on a global load (1.5% on the sweep, 5% on the
     // legacy-collision scan, against re-reading the job record there).
     __shared__ float sj_sgas[128], sj_mr[128], sj_floor[128], sj_mfp[128];
+    // What a window of four steps needs besides the positions, made at its first step for all of them: the drive
+    // amplitudes, and the candidates' uniforms or the legacy collisions' words; and what only that and the ends of
+    // a flight read.
+    __shared__ float2 s_amp[4][128];
+    __shared__ float s_uni[LEGACY ? 1 : 4][128];
+    __shared__ uint2 s_word[LEGACY ? 4 : 1][128];
+    __shared__ uint64_t s_ph[3][128];       // phases at the next window's start, AC turns per step
+    __shared__ float4 s_drv[128];           // AC amplitude, rotation
+    __shared__ uint2 s_key[128];
+    __shared__ uint32_t s_id[128], s_n0[128], s_nc[128];
+    __shared__ unsigned long long s_tot[128];
+    const uint32_t tid = threadIdx.x;
+    s_tot[tid] = 0;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t count = ctr->count[in_slot];
     if (count <= hand_at) return;   // the lane-group launch takes them
@@ -270,24 +290,41 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
     // lanes that take ions: all 32 when the list fills the grid, else the warp's even share of it
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     bool have = false, drained = lane >= (count + warps - 1) / warps;
-    uint32_t id = 0, jid = 0, n = 0, done = 0, stop = 0, ncoll = 0;
+    uint32_t n = 0, stop = 0;           // the ion's step count, and the one to put it away at
     int32_t leg = 0;
     float xh[3], xl[3], uh[3], ul[3];
-    uint64_t Prf = 0, Pac = 0, Wac = 0;
     const uint64_t Wrf = ((uint64_t)B.w_rf_hi << 32) | B.w_rf_lo;
-    // drive sines advanced by rotation each step and re-evaluated exactly from the
-    // fixed-point phases every 4 loop iterations (warp-uniform), so rounding cannot build up
-    float srf = 0.f, crf = 1.f, sac = 0.f, cac = 1.f, cw_ac = 1.f, sw_ac = 0.f;
-    float kick = 0.f, v_ac = 0.f, cand_aa = 0.f, cand_b = 0.f;
-    uint32_t k0 = 0, k1 = 0;
-    // per-step candidate uniforms: Philox block n>>2 (rc) and the next block (rn); rn is
-    // refreshed for every lane on a warp-uniform schedule (every 4 loop iterations), so the
-    // 10-round generator runs with all lanes active instead of once per lane-boundary
-    uint4 rc = make_uint4(0, 0, 0, 0), rn = make_uint4(0, 0, 0, 0);
+    float kick = 0.f, cand_aa = 0.f, cand_b = 0.f;
+    // The drive is evaluated exactly from the fixed-point phases at every step that is a multiple of 4 and rotated
+    // in between, so rounding cannot build up, and one Philox block (legacy: two) serves four steps.
+    float2 amp = make_float2(0.f, 0.f);   // drive amplitudes of the next step
+    auto window = [&]() {
+        const uint64_t prf = s_ph[0][tid], pac = s_ph[1][tid], wac = s_ph[2][tid];
+        const float4 dv = s_drv[tid];
+        float s, c, sa, ca;
+        turn_sincos(prf, s, c);
+        turn_sincos(pac, sa, ca);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            s_amp[q][tid] = make_float2(B.v_rf * s, dv.x * sa);
+            if (q < 3) { rotate(s, c, B.cw_rf, B.sw_rf); rotate(sa, ca, dv.y, dv.z); }
+        }
+        s_ph[0][tid] = prf + 4u * Wrf;
+        s_ph[1][tid] = pac + 4u * wac;
+        const uint2 key = s_key[tid];
+        if (!LEGACY) {
+            const uint4 r = philox(key.x, key.y, n >> 2, 0u, 0u, 0u);
+            s_uni[0][tid] = unif(r.x); s_uni[LEGACY ? 0 : 1][tid] = unif(r.y);
+            s_uni[LEGACY ? 0 : 2][tid] = unif(r.z); s_uni[LEGACY ? 0 : 3][tid] = unif(r.w);
+        } else {
+            const uint4 ra = philox(key.x, key.y, n >> 2, 2u, 0u, 0u), rb = philox(key.x, key.y, n >> 2, 3u, 0u, 0u);
+            s_word[0][tid] = make_uint2(ra.x, ra.y); s_word[LEGACY ? 1 : 0][tid] = make_uint2(ra.z, ra.w);
+            s_word[LEGACY ? 2 : 0][tid] = make_uint2(rb.x, rb.y); s_word[LEGACY ? 3 : 0][tid] = make_uint2(rb.z, rb.w);
+        }
+    };
     uint32_t iter = 0;
     uint32_t loads = 0;                 // cell-cache fills of this lane
     Cell c;
-    unsigned long long steps_total = 0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) { xh[d] = xl[d] = uh[d] = ul[d] = 0.f; }
     c.ci = c.cj = c.ck = -1; c.mask = 0;
@@ -317,9 +354,10 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             const uint32_t head = __shfl_sync(FULL, *(volatile uint32_t*)&ctr->head, 0);
             if (open <= hand_at && head >= count) {
                 if (have) {
+                    const uint32_t id = s_id[tid], done = n - s_n0[tid];
                     hand[MQ_CHK(atomicAdd(&ctr->handed[0], 1u), hand_at, MQ_SITE_MIX_HAND)] = make_uint2(id, done);
-                    put_ion(io, keep, n_all, id, n, ncoll, leg, 0, xh, xl, uh, ul);
-                    steps_total += done;
+                    put_ion(io, keep, n_all, id, n, s_nc[tid], leg, 0, xh, xl, uh, ul);
+                    s_tot[tid] += done;
                     have = false;
                 }
                 drained = true;
@@ -332,7 +370,7 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             uint32_t base = 0;
             if ((int)lane == leader) base = atomicAdd(count_out, (uint32_t)__popc(am));
             base = __shfl_sync(FULL, base, leader);
-            if (append) list_out[MQ_CHK(base + __popc(am & ((1u << lane) - 1u)), n_all, MQ_SITE_MIX_LIST_OUT)] = id;
+            if (append) list_out[MQ_CHK(base + __popc(am & ((1u << lane) - 1u)), n_all, MQ_SITE_MIX_LIST_OUT)] = s_id[tid];
         }
         append = false;
         // ---- refill: one warp-aggregated atomic hands out queue slots to lanes without an ion
@@ -345,53 +383,38 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
             if (!have && !drained) {
                 const uint32_t slot = base + __popc(need & ((1u << lane) - 1u));
                 if (slot < count) {
-                    id = (uint32_t)MQ_CHK(__ldg(list_in + slot), n_all, MQ_SITE_MIX_ION);
-                    jid = io.jid[id];
-                    const MixJob J = jobs[jid];
-                    sj_sgas[threadIdx.x] = J.s_gas;
-                    sj_mr[threadIdx.x] = J.mr;
-                    sj_floor[threadIdx.x] = J.floor_v;
-                    sj_mfp[threadIdx.x] = J.mfp_mean;
-                    kick = J.kick; v_ac = J.use_ac ? J.v_ac : 0.0f; cand_aa = J.cand_a * J.cand_a; cand_b = J.cand_b;
-                    Wac = ((uint64_t)J.w_ac_hi << 32) | J.w_ac_lo;
-                    cw_ac = J.cw_ac; sw_ac = J.sw_ac;
-                    n = io.steps[id]; ncoll = io.ncoll[id]; leg = io.leg[id];
+                    const uint32_t id = (uint32_t)MQ_CHK(__ldg(list_in + slot), n_all, MQ_SITE_MIX_ION);
+                    const MixJob J = jobs[io.jid[id]];
+                    sj_sgas[tid] = J.s_gas;
+                    sj_mr[tid] = J.mr;
+                    sj_floor[tid] = J.floor_v;
+                    sj_mfp[tid] = J.mfp_mean;
+                    kick = J.kick; cand_aa = J.cand_a * J.cand_a; cand_b = J.cand_b;
+                    n = io.steps[id]; leg = io.leg[id];
+                    s_id[tid] = id; s_n0[tid] = n; s_nc[tid] = io.ncoll[id];
+                    s_drv[tid] = make_float4(J.use_ac ? J.v_ac : 0.0f, J.cw_ac, J.sw_ac, 0.0f);
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
                         xh[d] = keep[(size_t)(0 + d) * n_all + id]; xl[d] = keep[(size_t)(3 + d) * n_all + id];
                         uh[d] = keep[(size_t)(6 + d) * n_all + id]; ul[d] = keep[(size_t)(9 + d) * n_all + id];
                     }
-                    // phase = offset + n * w (mod 1) in 64-bit fixed point
-                    const uint64_t orf = kph[id], oac = kph[(size_t)n_all + id];
-                    const uint64_t n4 = ((uint64_t)n + 3u) & ~(uint64_t)3u;   // the next exact drive
-                    Prf = orf + n4 * Wrf;
-                    Pac = oac + n4 * Wac;
-                    // drive state as an uninterrupted run has it: exact at the last step that is
-                    // a multiple of 4, then rotated forward (so re-queued ions continue bitwise).
-                    // An ion at a multiple of 4 steps (every fresh ion) first steps on a re-sync
-                    // iteration, which sets its drive exactly and draws its next Philox block, so
-                    // neither is done here for it
-                    const uint32_t r4 = n & 3u;
-                    if (r4) {
-                        turn_sincos(Prf - 4u * Wrf, srf, crf);
-                        turn_sincos(Pac - 4u * Wac, sac, cac);
-                        for (uint32_t q = 0; q < r4; ++q) { rotate(srf, crf, B.cw_rf, B.sw_rf); rotate(sac, cac, cw_ac, sw_ac); }
-                    }
+                    // phase = offset + step * w (mod 1) in 64-bit fixed point, at the start of the ion's window
+                    const uint64_t wac = ((uint64_t)J.w_ac_hi << 32) | J.w_ac_lo;
+                    s_ph[0][tid] = kph[id] + (uint64_t)(n & ~3u) * Wrf;
+                    s_ph[1][tid] = kph[(size_t)n_all + id] + (uint64_t)(n & ~3u) * wac;
+                    s_ph[2][tid] = wac;
                     const uint64_t key = io.rng[id];
-                    k0 = (uint32_t)key; k1 = (uint32_t)(key >> 32);
-                    if (!LEGACY) {
-                        rc = philox(k0, k1, n >> 2, 0u, 0u, 0u);
-                        if (r4) rn = philox(k0, k1, (n >> 2) + 1u, 0u, 0u, 0u);
-                    } else if (r4) {   // the legacy collision words of the current 4-step window
-                        rc = philox(k0, k1, n >> 2, 2u, 0u, 0u);
-                        rn = philox(k0, k1, n >> 2, 3u, 0u, 0u);
+                    s_key[tid] = make_uint2((uint32_t)key, (uint32_t)(key >> 32));
+                    // An ion at a multiple of 4 steps (every fresh ion) first steps on an iteration that makes its window
+                    if (n & 3u) {
+                        window();
+                        if (WIDE) amp = s_amp[n & 3u][tid];
                     }
                     c.ck = -4;   // nothing held is of use
                     load_cell<WIDE, NEAREST>(nodes, B, clampi(__float2int_rd(xh[0]), 0, B.nx - 2), clampi(__float2int_rd(xh[1]), 0, B.ny - 2),
                               clampi(__float2int_rd(xh[2]), 0, B.nz - 2), c);
                     ++loads;
-                    done = 0;
-                    stop = n >= B.max_steps ? 1u : B.max_steps - n < chunk ? B.max_steps - n : chunk;
+                    stop = n >= B.max_steps ? n + 1u : B.max_steps - n < chunk ? B.max_steps : n + chunk;
                     have = true;
                 } else {
                     drained = true;
@@ -407,20 +430,11 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
         // then falls on the same steps of every ion, whatever the scheduling, so per-ion
         // results are reproducible bit for bit.
         const bool act = have && (((iter ^ n) & 3u) == 0u);
-        if (!LEGACY && (iter & 3u) == 0u && act) rn = philox(k0, k1, (n >> 2) + 1u, 0u, 0u, 0u);
-        // legacy collisions draw from two Philox blocks per 4-step window, computed here with every
-        // lane of the warp active (7% on the legacy scan against one block per collision inside
-        // the divergent collision branch); a collision at window step q takes words 2q and 2q + 1
-        if (LEGACY && (iter & 3u) == 0u && act) {
-            rc = philox(k0, k1, n >> 2, 2u, 0u, 0u);
-            rn = philox(k0, k1, n >> 2, 3u, 0u, 0u);
-        }
         if ((iter & 3u) == 0u && act) {
-            turn_sincos(Prf, srf, crf);
-            turn_sincos(Pac, sac, cac);
-            Prf += 4u * Wrf;
-            Pac += 4u * Wac;
+            window();
+            if (WIDE) amp = s_amp[0][tid];
         }
+        const uint32_t now = iter & 3u;
         ++iter;
         if (act) {
             // ---- field at the current position
@@ -430,8 +444,9 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                 ty = __fadd_rn(__fsub_rn(xh[1], c.fcj), xl[1]);
                 tz = __fadd_rn(__fsub_rn(xh[2], c.fck), xl[2]);
             }
-            const float a_rf = B.v_rf * srf;
-            const float a_ac = v_ac * sac;
+            if (!WIDE) amp = s_amp[now][tid];
+            const float a_rf = amp.x, a_ac = amp.y;
+            if (WIDE) amp = s_amp[(now + 1u) & 3u][tid];   // the next step's (at the window's end made anew)
             float E[3];
             const bool ox = c.ci & 1, oy = c.cj & 1, oz = c.ck & 1;
             if (!NEAREST && !WIDE) {
@@ -474,25 +489,23 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                 if (pi != c.ci || pj != c.cj || pk != c.ck) prefetch_cell<WIDE>(nodes, B, pi, pj, pk);
             }
             if (!WIDE && !NEAREST) c.mask = cell_mask(c);
-            rotate(srf, crf, B.cw_rf, B.sw_rf);
-            rotate(sac, cac, cw_ac, sw_ac);
             const uint32_t nprev = n;
             n += 1;
-            done += 1;
             // ---- collisions
             if (!LEGACY) {
-                const float u0 = unif((nprev & 3) == 0 ? rc.x : (nprev & 3) == 1 ? rc.y : (nprev & 3) == 2 ? rc.z : rc.w);
+                const float u0 = s_uni[LEGACY ? 0 : now][tid];
                 // candidate if u0 < cand_a |u| + cand_b = n sigma dt (|v| + E|V|), tested on squares
                 // (no square root per step); see thermal_partner for why E|V| bounds the rate
                 const float um2 = fmaf(uh[0], uh[0], fmaf(uh[1], uh[1], uh[2] * uh[2]));
                 const float du = u0 - cand_b;
                 if (du < 0.0f || du * du < cand_aa * um2) {
                     const float um = sqrtf(um2);
-                    const float s_gas = sj_sgas[threadIdx.x], mr = sj_mr[threadIdx.x];
+                    const float s_gas = sj_sgas[tid], mr = sj_mr[tid];
                     // two Philox blocks per candidate, drawn side by side: the first for the gas
                     // partner and the acceptance, the second for the scattering direction
-                    const uint4 r0 = philox(k0, k1, nprev, 1u, 0u, 0u);
-                    const uint4 r1 = philox(k0, k1, nprev, 2u, 0u, 0u);
+                    const uint2 key = s_key[tid];
+                    const uint4 r0 = philox(key.x, key.y, nprev, 1u, 0u, 0u);
+                    const uint4 r1 = philox(key.x, key.y, nprev, 2u, 0u, 0u);
                     const float u2v = B.u2v_f;
                     float v[3] = {uh[0] * u2v, uh[1] * u2v, uh[2] * u2v};
                     float gv[3], vm_sum;
@@ -510,10 +523,9 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                             float vn = fmaf(mr * gl, nn[d], fmaf(-mr, gv[d], v[d]));
                             uh[d] = vn * v2u; ul[d] = 0.0f;
                         }
-                        ncoll += 1;
+                        s_nc[tid] += 1u;
                     }
                 }
-                if ((n & 3) == 0) rc = rn;   // rn holds block n>>2: refreshed at most 3 iterations ago
             } else {
                 // a collision is due every ~4 steps per ion, so some lane of the warp needs one on
                 // almost every iteration: every lane computes it and keeps it only where it is due,
@@ -521,12 +533,11 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                 leg -= 1;
                 const bool due = leg <= 0;
                 {
-                    const float mr = sj_mr[threadIdx.x], floor_v = sj_floor[threadIdx.x], mfp_mean = sj_mfp[threadIdx.x];
+                    const float mr = sj_mr[tid], floor_v = sj_floor[tid], mfp_mean = sj_mfp[tid];
                     // two 32-bit words of this window step: cos(theta) from the top 24 bits of the
                     // first, the free path from the top 24 of the second, phi from their low bytes
-                    const uint32_t q = nprev & 3u;
-                    const uint32_t wa = q == 0 ? rc.x : q == 1 ? rc.z : q == 2 ? rn.x : rn.z;
-                    const uint32_t wb = q == 0 ? rc.y : q == 1 ? rc.w : q == 2 ? rn.y : rn.w;
+                    const uint2 word = s_word[LEGACY ? now : 0][tid];
+                    const uint32_t wa = word.x, wb = word.y;
                     const float u2v = B.u2v_f;
                     float v[3] = {uh[0] * u2v, uh[1] * u2v, uh[2] * u2v};
                     const float vm = sqrtf(fmaf(v[0], v[0], fmaf(v[1], v[1], v[2] * v[2])));
@@ -544,7 +555,7 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                         uh[d] = hit ? vn * v2u : uh[d];
                         ul[d] = hit ? 0.0f : ul[d];
                     }
-                    ncoll += hit ? 1u : 0u;
+                    if (hit) s_nc[tid] += 1u;
                     const float mfp = -__logf(fmaxf(unif(wb), 1e-7f)) * mfp_mean;
                     const float vn = sqrtf(fmaf(v[0], v[0], fmaf(v[1], v[1], v[2] * v[2])));
                     // free path in steps with the hardware's approximate division (within 2 ulp; the
@@ -576,18 +587,19 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
                     if ((c.mask >> q) & 1u) status = 1;
                 }
             }
-            if (status != 0 || done >= stop) {
+            if (status != 0 || n >= stop) {
                 if (status == 0 && n >= B.max_steps) status = 5;
                 // ---- write back: counters to the ion states, position and velocity to the working
                 //      state (k_unstage turns it into the FP64 state when the caller wants that)
-                put_ion(io, keep, n_all, id, n, ncoll, leg, status, xh, xl, uh, ul);
+                put_ion(io, keep, n_all, s_id[tid], n, s_nc[tid], leg, status, xh, xl, uh, ul);
                 ended = true;
-                steps_total += done;
+                s_tot[tid] += n - s_n0[tid];
                 append = status == 0;
                 have = false;
             }
         }
     }
+    unsigned long long steps_total = s_tot[tid];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         steps_total += __shfl_down_sync(FULL, steps_total, o);
@@ -1395,18 +1407,22 @@ void release(Scratch& s) {
 
 // the stepping kernel for the batch's physics and the tuning (the nearest-node field mode reads one
 // record per fill, so the L1 prefetch of the next cell does not apply to it)
-typedef decltype(&k_mixed<true, true, true, false>) Kernel;
-static Kernel pick_kernel(const Tuning& t, const MixBatch& mb) {
+typedef decltype(&k_mixed<true, true, true, false, 3>) Kernel;
+static Kernel pick_kernel(const Tuning& t, const MixBatch& mb, int blocks) {
     if (mb.nearest) {
-        if (mb.legacy_coll) return t.wide ? k_mixed<true, false, true, true> : k_mixed<true, false, false, true>;
-        return t.wide ? k_mixed<false, false, true, true> : k_mixed<false, false, false, true>;
+        if (mb.legacy_coll) return t.wide ? k_mixed<true, false, true, true, 5> : k_mixed<true, false, false, true, 5>;
+        return t.wide ? k_mixed<false, false, true, true, 5> : k_mixed<false, false, false, true, 5>;
+    }
+    if (t.wide && blocks == 4) {
+        if (mb.legacy_coll) return t.prefetch ? k_mixed<true, true, true, false, 4> : k_mixed<true, false, true, false, 4>;
+        return t.prefetch ? k_mixed<false, true, true, false, 4> : k_mixed<false, false, true, false, 4>;
     }
     if (mb.legacy_coll) {
-        if (t.wide) return t.prefetch ? k_mixed<true, true, true, false> : k_mixed<true, false, true, false>;
-        return t.prefetch ? k_mixed<true, true, false, false> : k_mixed<true, false, false, false>;
+        if (t.wide) return t.prefetch ? k_mixed<true, true, true, false, 3> : k_mixed<true, false, true, false, 3>;
+        return t.prefetch ? k_mixed<true, true, false, false, 2> : k_mixed<true, false, false, false, 2>;
     }
-    if (t.wide) return t.prefetch ? k_mixed<false, true, true, false> : k_mixed<false, false, true, false>;
-    return t.prefetch ? k_mixed<false, true, false, false> : k_mixed<false, false, false, false>;
+    if (t.wide) return t.prefetch ? k_mixed<false, true, true, false, 3> : k_mixed<false, false, true, false, 3>;
+    return t.prefetch ? k_mixed<false, true, false, false, 2> : k_mixed<false, false, false, false, 2>;
 }
 
 typedef decltype(&k_mixed_group<true, true, false>) GroupKernel;
@@ -1474,7 +1490,7 @@ static cudaError_t enqueue_launches(const Scratch& s, const Tuning& t, int block
             li = sorted;
             *kernels += 5;
         }
-        const Kernel kern = pick_kernel(t, mb);
+        const Kernel kern = pick_kernel(t, mb, blocks_per_sm);
         const uint32_t hand_at = hand_entries(t.sms, mb.nearest != 0);
         uint2* hand = reinterpret_cast<uint2*>(ctr + 1);
         if (n > hand_at) {
@@ -1571,11 +1587,14 @@ cudaError_t run(Scratch& s, const Tuning& t, DevGrid g, uint64_t grid_gen, const
     // resident blocks per SM: the tuning's, except for the nearest-node kernels, which hold no
     // 8-corner cache (about 100 registers instead of 167) and run as many blocks as fit
     int blocks = t.blocks_per_sm;
+    // three with wide records are four for a list of eight or more ions a lane, which outlasts its uneven end:
+    // 1,280,000 ions 22.1 -> 21.1 ms, 640,000 13.6 -> 13.2, 320,000 the same, 62,000 (S14 sweep) 39.0 -> 40.4
+    if (t.wide && blocks == 3 && n > 2048u * (uint32_t)t.sms) blocks = 4;
     // one block per SM with narrow records is two of them below 3.5 GB (default_tuning has the figures)
     if (!t.wide && blocks == 1 && 48.0 * (double)mb.nx * mb.ny * mb.nz < 3.5e9) blocks = 2;
     if (mb.nearest) {
         int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_kernel(t, mb), t.tpb, 0) == cudaSuccess && nb > 0)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_kernel(t, mb, 0), t.tpb, 0) == cudaSuccess && nb > 0)
             blocks = nb;
         else
             cudaGetLastError();

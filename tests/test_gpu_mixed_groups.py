@@ -111,3 +111,19 @@ def test_states_at_the_edges_equal_one_lane_kernel(coarse, wide):
     for f in FIELDS:
         b = np.concatenate([getattr(p, f) for p in parts])
         assert np.array_equal(getattr(whole, f).view(np.uint8), b.view(np.uint8)), f
+
+
+@pytest.mark.parametrize("name", ["corrected_disc", "legacy_coll_trilinear", "no_gas_rf_random"])
+def test_long_lists_equal_their_parts(coarse, name):
+    """Lists above 2,048 ions per SM run the one-lane kernel at four blocks per SM, shorter ones at three."""
+    mq = _mq()
+    ph = _variants()[name]
+    sp = mq.Species(499.0 * 5, 5.0, 0.0) if name.startswith("legacy") else mq.Species(499.0, 1.0, 2.95 * 499.0 ** (2 / 3))
+    jobs = [mq.Job(sp, mq.RfAc(100.0, 500e3, 0.5, 100e3 + 1e3 * k), 110000, 5 + k) for k in range(3)]
+    with mq.Engine(coarse, mq.PREC_MIXED) as e:
+        e.set_tuning(chunk=301)
+        whole, jid = e.run_batch_ions(jobs, DC, ph)
+        for k, j in enumerate(jobs):
+            part, _ = e.run_batch_ions([j], DC, ph)
+            for f in FIELDS[:-1]:
+                assert np.array_equal(getattr(whole, f)[jid == k].view(np.uint8), getattr(part, f).view(np.uint8)), f
