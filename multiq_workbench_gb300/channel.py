@@ -164,6 +164,7 @@ class Outcomes(Sequence):
 ION_FIELDS = (("x", np.float64), ("y", np.float64), ("z", np.float64), ("vx", np.float64), ("vy", np.float64),
               ("vz", np.float64), ("ph_rf", np.float64), ("ph_ac", np.float64), ("rng", np.uint64),
               ("steps", np.uint32), ("ncoll", np.uint32), ("leg", np.int32), ("status", np.int32), ("jid", np.uint32))
+_ION_BYTES = sum(np.dtype(dt).itemsize for _, dt in ION_FIELDS)
 
 
 @dataclass
@@ -187,23 +188,37 @@ class IonStates:
 
     @classmethod
     def empty(cls, n: int, pinned: bool = False) -> "IonStates":
-        arrs = {}
-        keep = []
+        if not pinned:
+            return cls._in_block(np.zeros(n * _ION_BYTES, np.uint8), n)
+        import torch   # page-locked host memory for the timed host<->device copies
+        t = torch.empty(n * _ION_BYTES, dtype=torch.uint8, pin_memory=True)
+        out = cls._in_block(t.numpy(), n)
+        out._keep.append(t)
+        return out
+
+    @classmethod
+    def _in_block(cls, block: np.ndarray, n: int) -> "IonStates":
+        """The arrays one after the other in one block, the 8-byte ones first: the engine copies such
+        states in one piece, and one block is given back and had again without its pages being
+        returned to the system in between."""
+        arrs, off = {}, 0
         for name, dt in ION_FIELDS:
-            if pinned:
-                import torch   # page-locked host memory for the timed host<->device copies
-                t = torch.empty(n * np.dtype(dt).itemsize, dtype=torch.uint8, pin_memory=True)
-                keep.append(t)
-                arrs[name] = np.frombuffer(t.numpy(), dtype=dt, count=n)
-            else:
-                arrs[name] = np.zeros(n, dt)
-        return cls(**arrs, _keep=keep)
+            size = n * np.dtype(dt).itemsize
+            arrs[name] = block[off:off + size].view(dt)
+            off += size
+        return cls(**arrs)
 
     def __len__(self) -> int:
         return len(self.x)
 
     def copy(self) -> "IonStates":
-        return IonStates(**{name: getattr(self, name).copy() for name, _ in ION_FIELDS})
+        n = len(self)
+        if any(getattr(self, name).dtype != dt or getattr(self, name).shape != (n,) for name, dt in ION_FIELDS):
+            return IonStates(**{name: getattr(self, name).copy() for name, _ in ION_FIELDS})
+        out = IonStates._in_block(np.empty(n * _ION_BYTES, np.uint8), n)
+        for name, _ in ION_FIELDS:
+            np.copyto(getattr(out, name), getattr(self, name))
+        return out
 
     def native(self) -> N.mq_ions:
         io = N.mq_ions()
@@ -400,7 +415,7 @@ class Engine:
     def run_batch_ions(self, jobs, dc, ph: Physics) -> tuple[IonStates, np.ndarray]:
         """Final per-ion states and the job id of each ion (channel.rs:458-475)."""
         n = _total(jobs)
-        ions = IonStates.empty(n)
+        ions = IonStates._in_block(np.empty(n * _ION_BYTES, np.uint8), n)
         self.run_batch(jobs, dc, ph, ions_out=ions)
         return ions, ions.jid.copy()
 
