@@ -36,7 +36,8 @@ sys.path.insert(0, str(ROOT))
 METRIC = "ion-steps/s, 1 GB300: batched mixed-precision vs plain FP64 at matched outcomes"
 UNIT = "ion-steps/s"
 # Bytes the stepping kernel must move, counted by the kernel itself: every cell-cache fill reads the
-# 8 corners of a cell (8 narrow records of 48 B, or 4 wide ones of 96 B, each with the node above), and every ion it takes from the queue reads its
+# corners of a cell that are not held yet (4 wide records of 96 B, each with the node above, or at least 4
+# narrow ones of 48 B), and every ion it takes from the queue reads its
 # working state and job constants and writes them back (ION_STATE_BYTES).  The 384 B of corner
 # values an ion-step interpolates (8 corners x 3 float4) come from registers between fills.
 CORNERS = 8
@@ -45,9 +46,10 @@ ION_STATE_BYTES = 48 + 16 + 24 + 56 + 64   # double-floats, phase offsets, count
 
 def stepping_bytes(stats, wide: bool, nearest: bool = False) -> float:
     """Algorithmic bytes of the stepping kernel(s) of one call, from the kernel's own counters: cell
-    fills x 8 narrow or 4 wide node records (1 record in the nearest-node field mode, which reads only
-    the cell's lowest corner), plus the state traffic of every ion taken from the work queue."""
-    rec, per_fill = (96, CORNERS // 2) if wide else (48, CORNERS)
+    fills x 4 node records (wide ones hold two layers; of narrow ones a move along one axis reads the
+    far face's 4, so this is a lower bound there; 1 record in the nearest-node field mode, which reads
+    only the cell's lowest corner), plus the state traffic of every ion taken from the work queue."""
+    rec, per_fill = (96 if wide else 48), CORNERS // 2
     return float(stats.cell_loads) * (1 if nearest else per_fill) * rec + float(stats.ions_queued) * ION_STATE_BYTES
 
 
@@ -230,7 +232,7 @@ def run_gridstudy(args, rank: int, world: int):
                          "frac": fin["mixed"]["roofline_frac"], "traffic": None,
                          "peak_source": "measured hbm_gbs" if peaks.get("hbm_gbs") else "fallback",
                          "kernel": "k_mixed",
-                         "algorithmic_bytes": "cell fills counted by the kernel x 8 node records (48 B) + "
+                         "algorithmic_bytes": "cell fills counted by the kernel x 4 node records (48 B) + "
                                               f"{ION_STATE_BYTES} B per ion taken from the queue",
                          "cell_loads_per_ion_step": fin["mixed"]["cell_loads_per_ion_step"]},
             "roofline_l2": {"achieved": fin["mixed"]["achieved_gbs"], "peak": l2, "unit": "GB/s",
@@ -544,10 +546,10 @@ TRACK_STATE_BYTES = 68 + 56   # k_tm_step: a track's working state read and writ
 
 def tandem_moved(st, tracks: int) -> float:
     """Bytes the mixed tandem's step kernel must move, from its own counters: cell-cache fills (cube:
-    8 x 32-byte records; port: 8 x 48-byte records) plus every track's state once per launch (the
+    8 x 32-byte records; port: 4 x 48-byte records, which a move along one axis reads) plus every track's state once per launch (the
     advance's launches are a load, a store, and a bucket + step pair per 256-step chunk)."""
     chunks = max((st.launches - 2) // 2, 0)
-    return st.cell_fills_cube * 8 * 32 + st.cell_fills_port * 8 * 48 + float(tracks) * TRACK_STATE_BYTES * chunks
+    return st.cell_fills_cube * 8 * 32 + st.cell_fills_port * 4 * 48 + float(tracks) * TRACK_STATE_BYTES * chunks
 
 
 def tandem_cpu(m, pulse, steps: int, target_s: float, threads: int) -> dict:
@@ -688,7 +690,7 @@ def run_tandem(args, rank: int, world: int):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": None, "peak_source": "measured hbm_gbs" if peaks.get("hbm_gbs") else "fallback",
                          "kernel": "k_tm_step",
-                         "algorithmic_bytes": "cell fills counted by the kernel x 8 records (cube 32 B, port 48 B) + "
+                         "algorithmic_bytes": "cell fills counted by the kernel x 8 cube records (32 B) or 4 port records (48 B) + "
                                               f"{TRACK_STATE_BYTES} B per track per 256-step launch",
                          "cell_fills_per_track_step": fills},
             "roofline_l2": {"achieved": achieved, "peak": l2, "unit": "GB/s", "frac": achieved / l2 if l2 else None,
@@ -891,7 +893,7 @@ def main():
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                              "traffic": None, "peak_source": f"{peak_src} hbm_gbs",
                              "kernel": "k_mixed",
-                             "algorithmic_bytes": f"cell fills counted by the kernel x {'4 node records (96 B)' if wide else '8 node records (48 B)'} "
+                             "algorithmic_bytes": f"cell fills counted by the kernel x {'4 node records (96 B)' if wide else '4 node records (48 B)'} "
                                                   f"+ {ION_STATE_BYTES} B per ion taken from the queue",
                              "algorithmic_bytes_per_ion_step": moved / max(steps_total, 1),
                              "cell_loads_per_ion_step": loads / max(steps_total, 1)},

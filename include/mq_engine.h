@@ -93,7 +93,8 @@ typedef struct mq_run_stats {
     uint32_t step_kernel_launches;
     uint32_t graph_replays;    /* mixed engine: CUDA graph replays of its launch sequence     */
     uint64_t cell_loads;       /* mixed engine: cell-cache fills of the stepping kernel, each
-                                  the 8 corner node records of one cell                     */
+                                  the 8 corners of one cell (with 48-byte records only those
+                                  are read that the cell before did not hold)               */
     uint64_t ions_queued;      /* mixed engine: ions taken from the work queue, summed over the
                                   launches (each reads and writes its working state once)   */
 } mq_run_stats;

@@ -300,7 +300,7 @@ class RunStats:
     step_kernel_ms: float
     step_kernel_launches: int
     graph_replays: int = 0     # mixed engine: CUDA graph replays of its launch sequence
-    cell_loads: int = 0        # mixed engine: cell-cache fills (8 corner node records each)
+    cell_loads: int = 0        # mixed engine: cell-cache fills (the 8 corners of a cell each)
     ions_queued: int = 0       # mixed engine: ions taken from the work queue over the launches
 
     @classmethod

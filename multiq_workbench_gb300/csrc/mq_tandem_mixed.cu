@@ -154,18 +154,24 @@ __device__ bool solid(const CubeF& G, const float p[3]) {
 }
 
 // ---------------------------------------------------------------- fields
-__device__ __forceinline__ float lerp3(const float F[8], float tx, float ty, float tz) {
-    const float c00 = fmaf(tx, F[1] - F[0], F[0]), c10 = fmaf(tx, F[3] - F[2], F[2]);
-    const float c01 = fmaf(tx, F[5] - F[4], F[4]), c11 = fmaf(tx, F[7] - F[6], F[6]);
-    const float c0 = fmaf(ty, c10 - c00, c00), c1 = fmaf(ty, c11 - c01, c01);
-    return fmaf(tz, c1 - c0, c0);
+// lo + t (hi - lo) of an axis's two values; odd: the second is the lower node's, and t is negative then (hi - lo is the
+// same number but for its sign, so that only a zero's sign can differ)
+__device__ __forceinline__ float lerp2(float t, bool odd, float f0, float f1) { return fmaf(t, f1 - f0, odd ? f1 : f0); }
+__device__ __forceinline__ float lerp3(const float F[8], float tx, float ty, float tz, bool ox, bool oy, bool oz) {
+    const float c00 = lerp2(tx, ox, F[0], F[1]), c10 = lerp2(tx, ox, F[2], F[3]);
+    const float c01 = lerp2(tx, ox, F[4], F[5]), c11 = lerp2(tx, ox, F[6], F[7]);
+    const float c0 = lerp2(ty, oy, c00, c10), c1 = lerp2(ty, oy, c01, c11);
+    return lerp2(tz, oz, c0, c1);
 }
 
-
 // Register cache of the track's cell: the 8 corners x {RF, DC, AC} of its region's grid,
-// reloaded only when the track changes cell or region (cube cells have A = 0).
+// reloaded only when the track changes cell or region (cube cells have A = 0). In a port a corner lies in the slot
+// of its node's parity, not of its place in the cell, so a move to the next cell along an axis (nine of ten)
+// reads the far face's four records and leaves the near face where it is; the order of an axis's two slots goes
+// into the interpolation. Pulse of 262,144 / 1,048,576 tracks, 1,000 steps, whole fills -> half: ports at 0.050 mm
+// 10.4 -> 7.9 / 39.2 -> 28.7 ms, at 0.100 mm the same (6.9 / 25.3; two blocks of 215 registers 8.4 / 31.8).
 struct TCell {
-    float R[3][8], D[3][8], A[3][8];   // corner q = a + 2b + 4c
+    float R[3][8], D[3][8], A[3][8];   // corner or slot q = a + 2b + 4c
     int32_t ci, cj, ck, reg;
     float fci, fcj, fck;                // the cell as floats (no int -> float conversion per step)
     uint32_t mask;                      // port: conductor bit per corner
@@ -208,6 +214,13 @@ __device__ __forceinline__ void region_consts(const TMConst& C, int reg, float q
 }
 
 
+// 16 bytes of a port record, where p is set
+__device__ __forceinline__ void ld_if(const float4* n, bool p, float& x, float& y, float& z) {
+    float w;
+    asm("{.reg .pred p; setp.ne.u32 p, %4, 0; @p ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%5];}"
+        : "+f"(x), "+f"(y), "+f"(z), "=f"(w) : "r"((uint32_t)p), "l"(n));
+}
+
 // the cell of grid position x (clamped to the grid), reloading the cache when it changes; a change
 // is found on floored floats, and indices are formed only when one is seen
 __device__ __forceinline__ void cell_for(const RegK& k, int reg, const float xh[3], TCell& c) {
@@ -231,16 +244,21 @@ __device__ __forceinline__ void cell_for(const RegK& k, int reg, const float xh[
                 c.A[0][q] = c.A[1][q] = c.A[2][q] = 0.0f;
             }
         } else {
+            // nodes of each parity along the axes, and whether the slots hold others
+            const bool all = reg != c.reg;
+            const int32_t i0 = ci + (ci & 1), i1 = ci | 1, j0 = cj + (cj & 1), j1 = cj | 1, k0 = ck + (ck & 1), k1 = ck | 1;
+            const bool sx0 = i0 != c.ci + (c.ci & 1), sx1 = i1 != (c.ci | 1), sy0 = j0 != c.cj + (c.cj & 1), sy1 = j1 != (c.cj | 1);
+            const bool sz0 = all || k0 != c.ck + (c.ck & 1), sz1 = all || k1 != (c.ck | 1);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                uint32_t o = 3u * (base + (uint32_t)(q & 1) + ((q & 2) ? sy : 0u) + ((q & 4) ? sz : 0u));
+                const bool p = ((q & 1) ? sx1 : sx0) || ((q & 2) ? sy1 : sy0) || ((q & 4) ? sz1 : sz0);
+                uint32_t o = 3u * ((uint32_t)((q & 1) ? i1 : i0) + sy * (uint32_t)((q & 2) ? j1 : j0) + sz * (uint32_t)((q & 4) ? k1 : k0));
                 o = (uint32_t)MQ_CHK_SPAN(o, 3, 3 * (size_t)sz * (size_t)k.nz, MQ_SITE_TMX_CELL);
-                const float4 r = __ldg(k.rec + o), d = __ldg(k.rec + o + 1), a = __ldg(k.rec + o + 2);
-                c.R[0][q] = r.x; c.R[1][q] = r.y; c.R[2][q] = r.z;
-                c.D[0][q] = d.x; c.D[1][q] = d.y; c.D[2][q] = d.z;
-                c.A[0][q] = a.x; c.A[1][q] = a.y; c.A[2][q] = a.z;
-                if (q == 0) m = __float_as_uint(d.w);
+                ld_if(k.rec + o, p, c.R[0][q], c.R[1][q], c.R[2][q]);
+                ld_if(k.rec + o + 1, p, c.D[0][q], c.D[1][q], c.D[2][q]);
+                ld_if(k.rec + o + 2, p, c.A[0][q], c.A[1][q], c.A[2][q]);
             }
+            m = __float_as_uint(__ldg(&(k.rec + (uint32_t)MQ_CHK(3u * base + 1u, 3 * (size_t)sz * (size_t)k.nz, MQ_SITE_TMX_CELL))->w));
         }
         c.mask = m;
         if (k.cube) ++c.fills_cube; else ++c.fills_port;
@@ -374,6 +392,10 @@ __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32
         TCell c;
         c.ci = c.cj = c.ck = -1;
         c.reg = -1;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) c.R[d][q] = c.D[d][q] = c.A[d][q] = 0.0f;
         c.fills_cube = c.fills_port = 0;
         c.fci = c.fcj = c.fck = __int_as_float(0x7fc00000);
         cell_for(rk, reg, xh, c);
@@ -393,13 +415,15 @@ __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32
                 if (cube) {   // fields.rs:89-96 clamps the grid coordinate to the grid
                     tx = __saturatef(tx); ty = __saturatef(ty); tz = __saturatef(tz);
                 }
+                const bool ox = !cube && (c.ci & 1), oy = !cube && (c.cj & 1), oz = !cube && (c.ck & 1);
+                tx = ox ? -tx : tx; ty = oy ? -ty : ty; tz = oz ? -tz : tz;
                 const float ac = cube ? 0.0f : __ldg(dr + reg);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     float F[8];
 #pragma unroll
                     for (int q = 0; q < 8; ++q) F[q] = fmaf(rf, c.R[d][q], fmaf(ac, c.A[d][q], c.D[d][q]));
-                    E[d] = lerp3(F, tx, ty, tz);
+                    E[d] = lerp3(F, tx, ty, tz, ox, oy, oz);
                 }
             }
             if (cube) ++n_cube;
@@ -414,23 +438,6 @@ __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32
                 fast_two_sum(xh[d], uh[d], s, e);
                 e = __fadd_rn(e, __fadd_rn(xl[d], ul[d]));
                 fast_two_sum(s, e, xh[d], xl[d]);
-            }
-            // A cell that the position has moved to is asked for before the collisions, which move no track, so
-            // that its records are on their way meanwhile. A port's box is left only by a change of cell, so its
-            // test runs only there; in the cube this holds for the inner box, where no face, mouth or wall is
-            // near and the routing has nothing to do (98 of 100 cube steps). With the cube's cells taking the port's
-            // three-field sum (their AC part is 0) instead of one chosen per corner, a pulse of 262,144 tracks
-            // over 1,000 steps is 9.1 -> 8.4 ms, the kernel 7.5 -> 6.8. Tried and slower: one place for all fills
-            // (10.1), indices without the clamp (10.0), fills of 96-byte records (8.6); chunks of 64, 128, 512 or
-            // 1,024 steps are 8.8, 8.5, 8.5 and 8.8 against 8.4.
-            bool quiet = true, out = false;
-            if (cube) {
-                quiet = xh[0] > C.in_lo[0] && xh[0] < C.in_hi[0] && xh[1] > C.in_lo[1] && xh[1] < C.in_hi[1] && xh[2] > C.in_lo[2] &&
-                        xh[2] < C.in_hi[2];
-                if (quiet) cell_for(rk, reg, xh, c);
-            } else if (floorf(xh[0]) != c.fci || floorf(xh[1]) != c.fcj || floorf(xh[2]) != c.fck) {
-                out = xh[0] < 0.0f || xh[1] < 0.0f || xh[2] < 0.0f || xh[0] > rk.lim0 || xh[1] > rk.lim1 || xh[2] > rk.lim2;
-                if (!out) cell_for(rk, reg, xh, c);
             }
             // null-collision thermal bath (world.rs:473-488) with the majorant |v| + E|V| of
             // thermal_partner: candidate if u0 < nsd (|v| + E|V|)
@@ -461,56 +468,67 @@ __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32
                     }
                 }
             }
-            // routing (lib.rs:212-272)
+            // routing (lib.rs:212-272). In the cube's inner box no face, mouth or wall is near and nothing but the cell can
+            // change (98 of 100 cube steps); in a port the conductor test matters only in cells with a conductor
+            // corner. With the cube's cells taking the port's three-field sum instead of one chosen per corner, a
+            // pulse of 262,144 tracks over 1,000 steps with ports at 0.100 mm is 9.1 -> 8.4 ms, the kernel 7.5 -> 6.8.
+            // Tried and slower: one place for all fills (10.1), indices without the clamp (10.0), 96-byte port
+            // records (8.6), fills before the collisions (the same, and 4% slower at 0.050 mm); chunks of 64, 128,
+            // 512 or 1,024 steps are 8.8, 8.5, 8.5 and 8.8 against 8.4.
             if (cube) {
-                if (quiet) continue;
-                float p[3];
+                const bool quiet = xh[0] > C.in_lo[0] && xh[0] < C.in_hi[0] && xh[1] > C.in_lo[1] && xh[1] < C.in_hi[1] &&
+                                   xh[2] > C.in_lo[2] && xh[2] < C.in_hi[2];
+                if (!quiet) {
+                    float p[3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) p[d] = fmaf(xh[d], C.ch, fmaf(xl[d], C.ch, C.clo[d]));
-                const float lo_in = C.G.ptd, hi_in = C.G.size - C.G.ptd;
-                const bool interior = p[0] > lo_in && p[0] < hi_in && p[1] > lo_in && p[1] < hi_in && p[2] > lo_in &&
-                                      p[2] < hi_in;
-                if (!interior && solid(C.G, p)) { reg = R_LOST; continue; }
-                if (p[2] > C.seam_mm) {
-                    const int i = nearest_portf(C.G, p[0], p[1]);
-                    if (hypf2(p[0] - C.mouth_mm[i][0], p[1] - C.mouth_mm[i][1]) < C.G.ap_r) {
-                        // enter (lib.rs:338-367): straight into the port's grid units
-                        uint32_t* cnt = counts + (size_t)i * kNC;
-                        const bool fwd = reg == R_SPLIT;
-                        const float2 a = C.en_a[i];
-                        df_affine(xh[0], xl[0], a, C.en_b[i][0], xh[0], xl[0]);
-                        df_affine(xh[1], xl[1], a, C.en_b[i][1], xh[1], xl[1]);
-                        df_affine(xh[2], xl[2], fwd ? a : neg2(a), C.en_b[i][fwd ? 2 : 3], xh[2], xl[2]);
-                        const float2 z0 = make_float2(0.0f, 0.0f);
-                        df_affine(uh[0], ul[0], a, z0, uh[0], ul[0]);
-                        df_affine(uh[1], ul[1], a, z0, uh[1], ul[1]);
-                        df_affine(uh[2], ul[2], fwd ? a : neg2(a), z0, uh[2], ul[2]);
-                        if (fwd) {
-                            atomicAdd(cnt + 0, 1u);
-                            if (last >= 0) {
-                                atomicAdd(cnt + 3, 1u);
-                                atomicAdd(cnt + 5 + last, 1u);
-                                if (last != i) atomicAdd(cnt + 4, 1u);
+                    for (int d = 0; d < 3; ++d) p[d] = fmaf(xh[d], C.ch, fmaf(xl[d], C.ch, C.clo[d]));
+                    const float lo_in = C.G.ptd, hi_in = C.G.size - C.G.ptd;
+                    const bool interior = p[0] > lo_in && p[0] < hi_in && p[1] > lo_in && p[1] < hi_in && p[2] > lo_in &&
+                                          p[2] < hi_in;
+                    if (!interior && solid(C.G, p)) { reg = R_LOST; continue; }
+                    if (p[2] > C.seam_mm) {
+                        const int i = nearest_portf(C.G, p[0], p[1]);
+                        if (hypf2(p[0] - C.mouth_mm[i][0], p[1] - C.mouth_mm[i][1]) < C.G.ap_r) {
+                            // enter (lib.rs:338-367): straight into the port's grid units
+                            uint32_t* cnt = counts + (size_t)i * kNC;
+                            const bool fwd = reg == R_SPLIT;
+                            const float2 a = C.en_a[i];
+                            df_affine(xh[0], xl[0], a, C.en_b[i][0], xh[0], xl[0]);
+                            df_affine(xh[1], xl[1], a, C.en_b[i][1], xh[1], xl[1]);
+                            df_affine(xh[2], xl[2], fwd ? a : neg2(a), C.en_b[i][fwd ? 2 : 3], xh[2], xl[2]);
+                            const float2 z0 = make_float2(0.0f, 0.0f);
+                            df_affine(uh[0], ul[0], a, z0, uh[0], ul[0]);
+                            df_affine(uh[1], ul[1], a, z0, uh[1], ul[1]);
+                            df_affine(uh[2], ul[2], fwd ? a : neg2(a), z0, uh[2], ul[2]);
+                            if (fwd) {
+                                atomicAdd(cnt + 0, 1u);
+                                if (last >= 0) {
+                                    atomicAdd(cnt + 3, 1u);
+                                    atomicAdd(cnt + 5 + last, 1u);
+                                    if (last != i) atomicAdd(cnt + 4, 1u);
+                                }
+                            } else {
+                                atomicAdd(cnt + 14, 1u);
                             }
-                        } else {
-                            atomicAdd(cnt + 14, 1u);
+                            reg = 1 + i;
+                            region_consts(C, reg, qmdt2, nsd, rk);
+                            cell_for(rk, reg, xh, c);
+                            continue;
                         }
-                        reg = 1 + i;
-                        region_consts(C, reg, qmdt2, nsd, rk);
-                        cell_for(rk, reg, xh, c);
-                        continue;
+                        if (p[2] > C.G.size) { reg = R_LOST; continue; }
                     }
-                    if (p[2] > C.G.size) { reg = R_LOST; continue; }
+                    if (p[1] > C.G.size && hypf2(p[0] - C.ent_c, p[2] - C.ent_b) >= C.G.ap_r) { reg = R_LOST; continue; }
+                    if (p[1] > C.G.size + C.lext_mm) reg = reg == R_SPLIT ? 12 : 13;
+                    else if (p[0] < 0.0f || p[1] < 0.0f || p[2] < 0.0f || p[0] > C.G.size) reg = R_LOST;
+                    if (reg > R_COMBINE) continue;
                 }
-                if (p[1] > C.G.size && hypf2(p[0] - C.ent_c, p[2] - C.ent_b) >= C.G.ap_r) { reg = R_LOST; continue; }
-                if (p[1] > C.G.size + C.lext_mm) reg = reg == R_SPLIT ? 12 : 13;
-                else if (p[0] < 0.0f || p[1] < 0.0f || p[2] < 0.0f || p[0] > C.G.size) reg = R_LOST;
-                else cell_for(rk, reg, xh, c);
+                cell_for(rk, reg, xh, c);
             } else {
                 const int i = reg - 1;
                 // is_crash (world.rs:309-314): outside the box, or the nearest node is a conductor
-                bool crash = out;
-                if (!out && c.mask != 0u) {
+                bool crash = xh[0] < 0.0f || xh[1] < 0.0f || xh[2] < 0.0f || xh[0] > rk.lim0 || xh[1] > rk.lim1 || xh[2] > rk.lim2;
+                if (!crash) cell_for(rk, reg, xh, c);
+                if (!crash && c.mask != 0u) {
                     const uint32_t qn = (__fadd_rn(__fsub_rn(xh[0], c.fci), xl[0]) >= 0.5f ? 1u : 0u) |
                                         (__fadd_rn(__fsub_rn(xh[1], c.fcj), xl[1]) >= 0.5f ? 2u : 0u) |
                                         (__fadd_rn(__fsub_rn(xh[2], c.fck), xl[2]) >= 0.5f ? 4u : 0u);
