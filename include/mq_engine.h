@@ -187,7 +187,7 @@ mq_status   mq_check_selftest(int32_t device);
  * the path because those calls synchronise the device.  Such a caller owns the field arrays
  * and the ion states in device memory and passes pointers to them; this call advances the
  * states exactly like mq_run_ions with MQ_PREC_F64 (same kernel, same results bit for bit)
- * and allocates nothing: its working memory (the per-job constant table and two counters)
+ * and allocates nothing: its working memory (the per-job constant table and its counters)
  * is a fixed array in the library's static device memory, MQ_NOALLOC_SCRATCH_BYTES bytes,
  * which every GPU that loads the library holds until the process exits.
  *

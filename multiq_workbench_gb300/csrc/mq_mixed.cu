@@ -622,8 +622,8 @@ k_mixed(const float4* __restrict__ nodes, MixBatch B, const MixJob* __restrict__
 // and, with many ions to a warp, the reload of some ion's cell on nearly every step; so the chain is kept
 // short (one vote clears most steps) and registers few. A step takes 0.27 us for up to 608 ions,
 // 0.44 for 4,864 and 0.57 for 19,456 (S14 grid), where the one-lane kernel takes 0.8 to 1.1; from there
-// on the one-lane kernel's 58,368 ions in flight win (1.15 us a step), so longer lists start with it.
-// Measured, whole run_batch calls, one-lane kernel with 64-byte records -> now: 1,000 ions at one point
+// on the one-lane kernel's 58,368 ions in flight win (0.86 us a step for 26,000), so longer lists start with it.
+// Measured when these groups came, whole run_batch calls, without -> with them: 1,000 ions at one point
 // 2.25 -> 1.04 ms; mass scan of 25,000 short-lived ions 1.26 -> 0.82; Fig. 4 legacy scan 21.2 -> 10.8;
 // S14 sweep of 62,000 ions 76.7 -> 39.9; sweep of 4.2 million ions 63.7 -> 55.6.
 // One block per SM, as many warps as the registers hold (16 at 128 a thread; 24 at 80 where the nearest
