@@ -17,10 +17,10 @@
 // chains of additions: 32 rows are summed side by side from shared memory while other warps form the
 // next terms. The host sets nothing up: mask, coarse masks and initial iterate are formed here, and its
 // part of an iteration is one synchronisation.
-// Measured on the 0.100 mm channel (160 x 160 x 242, 10 iterations), per basis, before -> now: kernels 24 -> 11.9 ms
-// (half sweeps 9.4 -> 5.5, of which one of the finest level is 35 us; prolongation 2.7 -> 0.6; ordered sums and S p
-// 3.7 -> 2.0; coarsest level 2.1 -> 0.9 with two levels more in the same launch; restriction 2.0 -> 0.8; residuals
-// 1.2 -> 0.7), the whole call 55 -> 13 ms, of which 30 were the host's part.
+// Measured on the 0.100 mm channel (160 x 160 x 242, 10 iterations), per basis, before -> now: kernels 24 -> 9.9 ms
+// (half sweeps 9.4 -> 3.6, of which one of the finest level is 22 us; prolongation 2.7 -> 0.5; ordered sums and S p
+// 3.7 -> 2.0; coarsest level 2.1 -> 0.9 with two levels more in the same launch; restriction 2.0 -> 0.7; residuals
+// 1.2 -> 0.5), the whole call 55 -> 11.5 ms, of which 30 were the host's part.
 #include <sys/mman.h>
 #include <unistd.h>
 
@@ -45,6 +45,8 @@ struct DLevel {
     int nx, ny, nz;
     uint8_t* fix;
     double *u, *rhs, *r;
+    uint32_t* list[2];   // free nodes by colour, or null (k_list)
+    uint32_t cnt[2];
     size_t n() const { return (size_t)nx * ny * nz; }
 };
 
@@ -103,13 +105,47 @@ __device__ __forceinline__ bool colour_node(unsigned t, int k, int col, int nx, 
     return colour_node(t, k, col, nx, ny, q, i, j);
 }
 
+// The free nodes of a colour, in runs of up to 256 neighbours. Half of a channel's nodes lie in electrodes, and its rows
+// cross them: warps over all nodes of a colour have 60 in 100 lanes at work, warps over this list all of them,
+// and the FP64 pipe's time goes by warps (half sweep of the finest level of the 0.100 mm channel 35 -> 22 us, the list once a
+// solve 20 us).
+__global__ void __launch_bounds__(kT) k_list(const uint8_t* __restrict__ fix, int nx, int ny, int nz, int col, uint32_t* __restrict__ list,
+                                             uint32_t* __restrict__ cnt) {
+    __shared__ uint32_t warp_n[kT / 32], base;
+    const int k = 1 + block_plane();
+    size_t q = 0;
+    const bool f = k <= nz - 2 && colour_node(blockIdx.x * kT + threadIdx.x, k, col, nx, ny, q) && !fix[q];
+    const unsigned b = __ballot_sync(0xffffffffu, f), lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    if (lane == 0) warp_n[w] = (uint32_t)__popc(b);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t n = 0;
+        for (int x = 0; x < kT / 32; ++x) { const uint32_t m = warp_n[x]; warp_n[x] = n; n += m; }
+        base = n ? atomicAdd(cnt, n) : 0u;
+    }
+    __syncthreads();
+    if (f) list[base + warp_n[w] + (uint32_t)__popc(b & ((1u << lane) - 1u))] = (uint32_t)q;
+}
+// node of this thread: the list's, or where there is none (grids of 2^32 nodes and more) the colour's free nodes in turn
+__device__ __forceinline__ bool free_node(const uint32_t* __restrict__ list, uint32_t cnt, const uint8_t* __restrict__ fix, int col, int nx,
+                                          int ny, int nz, size_t& q) {
+    const unsigned t = blockIdx.x * kT + threadIdx.x;
+    if (list) {
+        if (t >= cnt) return false;
+        q = list[t];
+        return true;
+    }
+    const int k = 1 + block_plane();
+    return k <= nz - 2 && colour_node(t, k, col, nx, ny, q) && !fix[q];
+}
+
 // RES: also the residual at the nodes updated, whose neighbours stay as they are here
 template <bool RES>
 __global__ void __launch_bounds__(kT) k_gs(double* __restrict__ u, const double* __restrict__ rhs, const uint8_t* __restrict__ fix,
-                                           double* __restrict__ r, int nx, int ny, int nz, int col) {
-    const int k = 1 + block_plane();
+                                           double* __restrict__ r, int nx, int ny, int nz, int col, const uint32_t* __restrict__ list,
+                                           uint32_t cnt) {
     size_t q;
-    if (k > nz - 2 || !colour_node(blockIdx.x * kT + threadIdx.x, k, col, nx, ny, q) || fix[q]) return;
+    if (!free_node(list, cnt, fix, col, nx, ny, nz, q)) return;
     const size_t sy = nx, sz = (size_t)nx * ny;
     const double s = u[q - 1] + u[q + 1] + u[q - sy] + u[q + sy] + u[q - sz] + u[q + sz];
     const double a = rhs[q] + s, v = div6(a);
@@ -117,15 +153,12 @@ __global__ void __launch_bounds__(kT) k_gs(double* __restrict__ u, const double*
     if (RES) r[q] = a - 6.0 * v;
 }
 
-// u = 0 and the first half sweep (colour 0) on it: the neighbours' sum is 0
+// the first half sweep (colour 0) on u = 0: the neighbours' sum is 0. Colour 1's nodes are not read before they are
+// set anew, and fixed ones are 0 from the start.
 __global__ void __launch_bounds__(kT) k_gs_first(double* __restrict__ u, const double* __restrict__ rhs, const uint8_t* __restrict__ fix,
-                                                 int nx, int ny, int nz) {
-    const unsigned t = blockIdx.x * kT + threadIdx.x, n = (unsigned)nx * (unsigned)ny, k = (unsigned)block_plane();
-    if (t >= n || k >= (unsigned)nz) return;
-    const unsigned i = t % (unsigned)nx, j = t / (unsigned)nx;
-    const size_t q = (size_t)t + (size_t)n * k;
-    // colour 0: i + j + k even (interior nodes; all others are fixed)
-    u[q] = ((i + j + k) & 1u) == 0u && !fix[q] ? div6(plus_zero(rhs[q])) : 0.0;
+                                                 int nx, int ny, int nz, const uint32_t* __restrict__ list, uint32_t cnt) {
+    size_t q;
+    if (free_node(list, cnt, fix, 0, nx, ny, nz, q)) u[q] = div6(plus_zero(rhs[q]));
 }
 
 // A coarsest level too large for k_bottom (a long thin grid's, the hierarchy ends below 5 nodes on one
@@ -156,10 +189,10 @@ __global__ void __launch_bounds__(1024) k_coarse(double* u, const double* rhs, c
 // ---------------------------------------------------------------- grid transfer
 // residual at the free nodes of colour 0 (k_gs<true> has left colour 1's; it stays 0 at fixed nodes)
 __global__ void __launch_bounds__(kT) k_residual(const double* __restrict__ u, const double* __restrict__ rhs,
-                                                 const uint8_t* __restrict__ fix, double* __restrict__ r, int nx, int ny, int nz) {
-    const int k = 1 + block_plane();
+                                                 const uint8_t* __restrict__ fix, double* __restrict__ r, int nx, int ny, int nz,
+                                                 const uint32_t* __restrict__ list, uint32_t cnt) {
     size_t q;
-    if (k > nz - 2 || !colour_node(blockIdx.x * kT + threadIdx.x, k, 0, nx, ny, q) || fix[q]) return;
+    if (!free_node(list, cnt, fix, 0, nx, ny, nz, q)) return;
     const size_t sy = nx, sz = (size_t)nx * ny;
     const double s = u[q - 1] + u[q + 1] + u[q - sy] + u[q + sy] + u[q - sz] + u[q + sz];
     r[q] = rhs[q] + s - 6.0 * u[q];
@@ -183,12 +216,23 @@ __device__ __forceinline__ double restrict_node(const double* f, I sy, I sz) {
     return down2(s, 1);
 }
 __global__ void __launch_bounds__(kT) k_restrict(const double* __restrict__ fr, int fnx, int fny, double* __restrict__ crhs,
-                                                 const uint8_t* __restrict__ cfix, int cnx, int cny, int cnz) {
-    const unsigned t = blockIdx.x * kT + threadIdx.x, n = (unsigned)cnx * (unsigned)cny, K = (unsigned)block_plane();
-    if (t >= n || K >= (unsigned)cnz) return;
-    const unsigned I = t % (unsigned)cnx, J = t / (unsigned)cnx;
-    const size_t qc = (size_t)t + (size_t)n * K;
-    if (cfix[qc]) { crhs[qc] = 0.0; return; }
+                                                 const uint8_t* __restrict__ cfix, int cnx, int cny, int cnz,
+                                                 const uint32_t* __restrict__ l0, uint32_t n0, const uint32_t* __restrict__ l1, uint32_t n1) {
+    const unsigned t = blockIdx.x * kT + threadIdx.x, n = (unsigned)cnx * (unsigned)cny;
+    unsigned I, J, K;
+    size_t qc;
+    if (l0) {   // free nodes only: nothing reads the others' right-hand side
+        if (t >= n0 + n1) return;
+        const unsigned x = t < n0 ? l0[t] : l1[t - n0], y = x / (unsigned)cnx;
+        I = x % (unsigned)cnx; J = y % (unsigned)cny; K = y / (unsigned)cny;
+        qc = x;
+    } else {
+        K = (unsigned)block_plane();
+        if (t >= n || K >= (unsigned)cnz) return;
+        I = t % (unsigned)cnx; J = t / (unsigned)cnx;
+        qc = (size_t)t + (size_t)n * K;
+        if (cfix[qc]) { crhs[qc] = 0.0; return; }
+    }
     const size_t sy = fnx, sz = (size_t)fnx * fny;
     crhs[qc] = restrict_node(fr + (size_t)(2 * I) + sy * (size_t)(2 * J) + sz * (size_t)(2 * K), (ptrdiff_t)sy, (ptrdiff_t)sz);
 }
@@ -231,11 +275,17 @@ __device__ __forceinline__ double prolong_node(const double* c, I sy, I sz, bool
 
 // fu += P cu at colour 0: the half sweep over colour 1 that follows reads no value of its own colour
 __global__ void __launch_bounds__(kT) k_prolong(const double* __restrict__ cu, int cnx, int cny, double* __restrict__ fu,
-                                                const uint8_t* __restrict__ ffix, int fnx, int fny, int fnz) {
-    const int k = 1 + block_plane();
+                                                const uint8_t* __restrict__ ffix, int fnx, int fny, int fnz,
+                                                const uint32_t* __restrict__ list, uint32_t cnt) {
     size_t q;
-    int i, j;
-    if (k > fnz - 2 || !colour_node(blockIdx.x * kT + threadIdx.x, k, 0, fnx, fny, q, i, j) || ffix[q]) return;
+    if (!free_node(list, cnt, ffix, 0, fnx, fny, fnz, q)) return;
+    int i, j, k;
+    if (list) {
+        const unsigned x = (unsigned)q, y = x / (unsigned)fnx;
+        i = (int)(x % (unsigned)fnx); j = (int)(y % (unsigned)fny); k = (int)(y / (unsigned)fny);
+    } else {
+        i = (int)(q % (size_t)fnx); j = (int)(q / (size_t)fnx % (size_t)fny); k = (int)(q / ((size_t)fnx * fny));
+    }
     const size_t sy = cnx, sz = (size_t)cnx * cny;
     fu[q] += prolong_node(cu + (size_t)(i / 2) + sy * (size_t)(j / 2) + sz * (size_t)(k / 2), sy, sz, i & 1, j & 1, k & 1);
 }
@@ -498,13 +548,17 @@ __global__ void __launch_bounds__(32) k_planes(const double* __restrict__ rowsum
     }
 }
 
-// phi += alpha p, r -= alpha q, max |r|; nothing if p q is not positive
+// phi += alpha p, r -= alpha q, max |r|; nothing if p q is not positive. p, q and r are 0 at fixed nodes, where only the
+// first update (`all`) changes anything: a potential of -0 to +0 (70 -> 60 us; in the sums and the direction the look
+// at the mask costs what it saves).
 __global__ void __launch_bounds__(kT) k_cg_update(double* __restrict__ phi, double* __restrict__ r, const double* __restrict__ p,
-                                                  const double* __restrict__ qv, size_t n, Scal* __restrict__ sc) {
+                                                  const double* __restrict__ qv, const uint8_t* __restrict__ fix, size_t n, bool all,
+                                                  Scal* __restrict__ sc) {
     if (!(sc->pq > 0)) return;
     const double alpha = sc->alpha;
     unsigned long long m = 0;
     for (size_t q = (size_t)blockIdx.x * kT + threadIdx.x; q < n; q += (size_t)gridDim.x * kT) {
+        if (!all && fix[q]) continue;
         phi[q] += alpha * p[q];
         const double v = r[q] - alpha * qv[q];
         r[q] = v;
@@ -629,13 +683,18 @@ struct Problem {
     std::vector<DLevel> L;
     double *phi, *r, *p, *qv, *rowsum, *plane;
     Scal* sc;
+    uint32_t* cnts;
     size_t n() const { return (size_t)nx * ny * nz; }
+    static bool listed(const std::vector<mqlv::Dims>& dims) { return mqlv::count(dims[0]) < ((size_t)1 << 32); }
+    static size_t half(const mqlv::Dims& d) { return (size_t)((d.nx - 1) / 2) * (d.ny - 2) * (d.nz - 2); }   // nodes of a colour, at most
     static size_t bytes(const std::vector<mqlv::Dims>& dims) {
         size_t b = 0;
         for (size_t l = 0; l < dims.size(); ++l) {
             const size_t m = mqlv::count(dims[l]);
             b += Arena::up(m) + (l ? 3 : 2) * Arena::up(8 * m);   // the finest level's right-hand side is the residual
+            if (listed(dims)) b += 2 * Arena::up(4 * half(dims[l]));
         }
+        b += Arena::up(8 * dims.size());
         const mqlv::Dims& f = dims[0];
         b += 4 * Arena::up(8 * mqlv::count(f)) + Arena::up(8 * (size_t)f.ny * f.nz) + Arena::up(8 * (size_t)f.nz) + Arena::up(sizeof(Scal));
         return b;
@@ -653,7 +712,9 @@ struct Problem {
             v.u = A.take<double>(v.n());
             v.r = A.take<double>(v.n());
             v.rhs = l ? A.take<double>(v.n()) : r;
+            for (int c = 0; c < 2; ++c) { v.list[c] = listed(d) ? A.take<uint32_t>(half(d[l])) : nullptr; v.cnt[c] = 0; }
         }
+        cnts = A.take<uint32_t>(2 * d.size());
     }
 };
 
@@ -681,7 +742,20 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
         const DLevel &f = P.L[l - 1], &c = P.L[l];
         k_coarse_fix<<<plane_blocks((size_t)c.nx * c.ny, c.nz), kT, 0, st>>>(f.fix, f.nx, f.ny, f.nz, c.fix, c.nx, c.ny, c.nz);
     }
+    std::vector<uint32_t> cnts(2 * P.L.size(), 0u);
+    if (P.L[0].list[0]) {
+        if (cudaMemsetAsync(P.cnts, 0, cnts.size() * sizeof(uint32_t), st) != cudaSuccess) return MQ_ERR_CUDA;
+        for (size_t l = 0; l < P.L.size(); ++l)
+            for (int c = 0; c < 2; ++c) {
+                const DLevel& v = P.L[l];
+                k_list<<<plane_blocks((size_t)((v.nx - 1) / 2) * (v.ny - 2), v.nz - 2), kT, 0, st>>>(v.fix, v.nx, v.ny, v.nz, c, v.list[c],
+                                                                                                  P.cnts + 2 * l + c);
+            }
+        if (cudaMemcpyAsync(cnts.data(), P.cnts, cnts.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
+    }
     if (!read()) return MQ_ERR_CUDA;
+    for (size_t l = 0; l < P.L.size(); ++l)
+        for (int c = 0; c < 2; ++c) P.L[l].cnt[c] = cnts[2 * l + c];
     double scale = std::fmax(as_double(h.rmax), std::fabs(outer_bc));
     if (!(scale > 0)) scale = 1.0;
     const double target = tol * scale;
@@ -697,10 +771,17 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
     const int bottom_bytes = (int)(25 * nodes + 8);
     if (cudaFuncSetAttribute(k_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, 25 * kBottomNodes + 8) != cudaSuccess) return MQ_ERR_CUDA;
     for (size_t l = 0; l < low; ++l)
-        if (cudaMemsetAsync(P.L[l].r, 0, P.L[l].n() * sizeof(double), st) != cudaSuccess) return MQ_ERR_CUDA;
+        if (cudaMemsetAsync(P.L[l].r, 0, P.L[l].n() * sizeof(double), st) != cudaSuccess ||
+            cudaMemsetAsync(P.L[l].u, 0, P.L[l].n() * sizeof(double), st) != cudaSuccess)
+            return MQ_ERR_CUDA;
 
-    auto half = [](const DLevel& lv) { return plane_blocks((size_t)((lv.nx - 1) / 2) * (lv.ny - 2), lv.nz - 2); };
-    auto gs = [&](DLevel& lv, int col) { k_gs<false><<<half(lv), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, nullptr, lv.nx, lv.ny, lv.nz, col); };
+    // (a level without a free node of a colour still launches one block)
+    auto half = [](const DLevel& lv, int c) {
+        return lv.list[c] ? dim3(blocks(lv.cnt[c] ? lv.cnt[c] : 1)) : plane_blocks((size_t)((lv.nx - 1) / 2) * (lv.ny - 2), lv.nz - 2);
+    };
+    auto gs = [&](DLevel& lv, int col) {
+        k_gs<false><<<half(lv, col), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, nullptr, lv.nx, lv.ny, lv.nz, col, lv.list[col], lv.cnt[col]);
+    };
     // symmetric V-cycle from u = 0 (Solver::vcycle of the host solver): L0.u = M^-1 r
     std::function<void(size_t)> vcycle = [&](size_t l) {
         DLevel& lv = P.L[l];
@@ -712,15 +793,17 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
             k_coarse<<<1, 1024, 0, st>>>(lv.u, lv.rhs, lv.fix, lv.nx, lv.ny, lv.nz, 60);
             return;
         }
-        k_gs_first<<<plane_blocks((size_t)lv.nx * lv.ny, lv.nz), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, lv.nx, lv.ny, lv.nz);
+        k_gs_first<<<half(lv, 0), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, lv.nx, lv.ny, lv.nz, lv.list[0], lv.cnt[0]);
         gs(lv, 1);
         gs(lv, 0);
-        k_gs<true><<<half(lv), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, lv.r, lv.nx, lv.ny, lv.nz, 1);
-        k_residual<<<half(lv), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, lv.r, lv.nx, lv.ny, lv.nz);
+        k_gs<true><<<half(lv, 1), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, lv.r, lv.nx, lv.ny, lv.nz, 1, lv.list[1], lv.cnt[1]);
+        k_residual<<<half(lv, 0), kT, 0, st>>>(lv.u, lv.rhs, lv.fix, lv.r, lv.nx, lv.ny, lv.nz, lv.list[0], lv.cnt[0]);
         DLevel& c = P.L[l + 1];
-        k_restrict<<<plane_blocks((size_t)c.nx * c.ny, c.nz), kT, 0, st>>>(lv.r, lv.nx, lv.ny, c.rhs, c.fix, c.nx, c.ny, c.nz);
+        const uint32_t cn = c.cnt[0] + c.cnt[1];
+        k_restrict<<<c.list[0] ? dim3(blocks(cn ? cn : 1)) : plane_blocks((size_t)c.nx * c.ny, c.nz), kT, 0, st>>>(
+            lv.r, lv.nx, lv.ny, c.rhs, c.fix, c.nx, c.ny, c.nz, c.list[0], c.cnt[0], c.list[1], c.cnt[1]);
         vcycle(l + 1);
-        k_prolong<<<half(lv), kT, 0, st>>>(c.u, c.nx, c.ny, lv.u, lv.fix, lv.nx, lv.ny, lv.nz);
+        k_prolong<<<half(lv, 0), kT, 0, st>>>(c.u, c.nx, c.ny, lv.u, lv.fix, lv.nx, lv.ny, lv.nz, lv.list[0], lv.cnt[0]);
         for (int s = 0; s < 2; ++s) { gs(lv, 1); gs(lv, 0); }
     };
     auto true_residual = [&]() -> bool {
@@ -747,7 +830,7 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
         while (it < max_it) {
             k_rows<true><<<rb, kT + 32, 0, st>>>(P.p, nullptr, P.L[0].fix, P.qv, nx, ny, rows, P.rowsum);
             k_planes<<<nz, 32, 0, st>>>(P.rowsum, ny, P.plane, P.sc, ALPHA);
-            k_cg_update<<<wide, kT, 0, st>>>(P.phi, P.r, P.p, P.qv, n, P.sc);
+            k_cg_update<<<wide, kT, 0, st>>>(P.phi, P.r, P.p, P.qv, P.L[0].fix, n, it == 0, P.sc);
             if (!read()) return MQ_ERR_CUDA;
             if (!(h.pq > 0)) break;
             rmax = as_double(h.rmax);

@@ -34,6 +34,7 @@ def test_any_size_bitwise(built, dims, scale):
     n = dims[0] * dims[1] * dims[2]
     mask = (rng.random(n) < 0.04).astype(np.uint8)
     fixed = np.where(mask, scale * rng.uniform(-1, 1, n), 0.0)
+    fixed[(mask != 0) & (rng.random(n) < 0.1)] = -0.0
     host, dev = _both(dims, mask, fixed, 0.25 * scale, 1e-8)
     assert host[:4] == dev[:4] and np.array_equal(host[4], dev[4])
 
