@@ -209,20 +209,27 @@ mq_status grow_ions(mq_engine* e, size_t n) {
 // The states to or from the host: one copy where the host's arrays lie one after the other as the device's do
 // (as IonStates lays them out), since each copy costs 5 to 8 us besides its bytes; else one per array. 65,537
 // states there and back, 500 steps: 1.31 -> 1.10 ms; mass scan of 25,000
-// ions whose states come back 0.79 -> 0.62.
+// ions whose states come back 0.79 -> 0.62. Arrays that lie so may still be memory of different kinds (some of them
+// page-locked by the caller): the runtime refuses to copy across such a border, and they go one by one.
 mq_status copy_ions(mq_engine* e, const mq_ions* io, size_t n, bool to_device, uint64_t* bytes) {
+    auto copy = [&](int k, size_t b) {
+        void *hp = host_field(io, k), *dp = e->ions.as<char>() + ion_off(k, n);
+        return to_device ? cudaMemcpyAsync(dp, hp, b, cudaMemcpyHostToDevice, e->st)
+                         : cudaMemcpyAsync(hp, dp, b, cudaMemcpyDeviceToHost, e->st);
+    };
     bool whole = true;
     for (int k = 0; k < 14; ++k) {
         if (!host_field(io, k)) return fail(e, MQ_ERR_INVALID, "ion state array missing");
         whole = whole && static_cast<char*>(host_field(io, k)) == reinterpret_cast<char*>(io->x) + ion_off(k, n);
     }
-    for (int k = 0; k < (whole ? 1 : 14); ++k) {
-        void *hp = host_field(io, k), *dp = e->ions.as<char>() + ion_off(k, n);
-        const size_t b = (whole ? kIonSum : kIonBytes[k]) * n;
-        if (to_device) CK(cudaMemcpyAsync(dp, hp, b, cudaMemcpyHostToDevice, e->st), "ion upload");
-        else CK(cudaMemcpyAsync(hp, dp, b, cudaMemcpyDeviceToHost, e->st), "ion download");
-        if (bytes) *bytes += b;
+    if (whole) {
+        const cudaError_t c = copy(0, kIonSum * n);
+        if (c == cudaErrorInvalidValue) { cudaGetLastError(); whole = false; }
+        else CK(c, to_device ? "ion upload" : "ion download");
     }
+    if (!whole)
+        for (int k = 0; k < 14; ++k) CK(copy(k, kIonBytes[k] * n), to_device ? "ion upload" : "ion download");
+    if (bytes) *bytes += kIonSum * n;
     return MQ_OK;
 }
 
