@@ -42,6 +42,7 @@ struct TPort {                  // one port's channel grid and drive
 // Cube geometry in FP32 (mm, growth 0), for the filter that settles all but the points near a surface
 struct CubeF {
     float size, c0, pitch, half_d, t_pcb, gap, ptd, stem_r, clear_r, rod_hole, l_ext, cap_reach, cap_r, ap_r;
+    float near, round_max;   // distances [mm] closer than this, and fractions beyond this, are left to the exact test
     int32_t n, array, ent_axis, ent_side, ent_cell0, ent_cell1, ext_axis, ext_side, ext_cell0, ext_cell1;
 };
 
@@ -68,18 +69,17 @@ struct Tracks {
     int32_t *sp, *region, *last;
 };
 
-constexpr float kNear = 2e-3f;   // mm: over ten times what the FP32 distances are off by
 __device__ __forceinline__ float latf(const CubeF& G, int i) { return G.c0 + G.pitch * (float)i; }
 __device__ __forceinline__ float hypf2(float u, float v) { return sqrtf(u * u + v * v); }
 // v < t, noting in `unsure` when the two are too close to tell
-__device__ __forceinline__ bool below(float v, float t, bool& unsure) {
-    unsure |= !(fabsf(v - t) >= kNear);   // NaN too
+__device__ __forceinline__ bool below(const CubeF& G, float v, float t, bool& unsure) {
+    unsure |= !(fabsf(v - t) >= G.near);   // NaN too
     return v < t;
 }
 // v.round() clamped to [0, hi]
-__device__ __forceinline__ int round_near(float v, int hi, bool& unsure) {
+__device__ __forceinline__ int round_near(const CubeF& G, float v, int hi, bool& unsure) {
     const float r = rintf(v);
-    unsure |= !(fabsf(v - r) <= 0.499f);
+    unsure |= !(fabsf(v - r) <= G.round_max);
     return r > 0.0f ? (r < (float)hi ? (int)r : hi) : 0;
 }
 // mqc::classify (geometry.rs:136-205) for one face (axis a, side) of the point: does the point lie in
@@ -92,32 +92,32 @@ __device__ bool face_solid(const CubeF& G, int a, int side, float u, float pb, f
         pc0 = G.ext_cell0; pc1 = G.ext_cell1;
         if (G.array) {
             const float first = 0.5f * (latf(G, 2) + latf(G, 3));
-            pc0 = 2 + 2 * round_near((pb - first) / (2.0f * G.pitch), 2, unsure);
-            pc1 = 2 + 2 * round_near((pc - first) / (2.0f * G.pitch), 2, unsure);
+            pc0 = 2 + 2 * round_near(G, (pb - first) / (2.0f * G.pitch), 2, unsure);
+            pc1 = 2 + 2 * round_near(G, (pc - first) / (2.0f * G.pitch), 2, unsure);
         }
     }
     const float axis_d = hypf2(pb - 0.5f * (latf(G, pc0) + latf(G, pc0 + 1)), pc - 0.5f * (latf(G, pc1) + latf(G, pc1 + 1)));
-    if (below(u, 0.0f, unsure)) {   // outside the wall: port rods and end cap
+    if (below(G, u, 0.0f, unsure)) {   // outside the wall: port rods and end cap
         if (pid == 0) return false;
         bool hit = false;
-        if (below(u, -G.cap_reach, unsure)) hit = below(axis_d, G.cap_r, unsure);
-        if (!below(u, -G.l_ext, unsure))
+        if (below(G, u, -G.cap_reach, unsure)) hit = below(G, axis_d, G.cap_r, unsure);
+        if (!below(G, u, -G.l_ext, unsure))
             for (int m = 0; m < 4; ++m)
-                hit |= below(hypf2(pb - latf(G, pc0 + (m >> 1)), pc - latf(G, pc1 + (m & 1))), G.half_d, unsure);
+                hit |= below(G, hypf2(pb - latf(G, pc0 + (m >> 1)), pc - latf(G, pc1 + (m & 1))), G.half_d, unsure);
         return hit;
     }
-    if (!inside || !below(u, G.ptd, unsure)) return false;
-    const int ib = round_near((pb - G.c0) / G.pitch, G.n - 1, unsure), ic = round_near((pc - G.c0) / G.pitch, G.n - 1, unsure);
+    if (!inside || !below(G, u, G.ptd, unsure)) return false;
+    const int ib = round_near(G, (pb - G.c0) / G.pitch, G.n - 1, unsure), ic = round_near(G, (pc - G.c0) / G.pitch, G.n - 1, unsure);
     const bool rim_b = ib == 0 || ib == G.n - 1, rim_c = ic == 0 || ic == G.n - 1;
     const bool valid = a == 0 ? !rim_b && !rim_c : a == 1 ? !rim_b : true;   // post_valid, geometry.rs:81-86
     const float dd = hypf2(pb - latf(G, ib), pc - latf(G, ic));
     const bool rod = pid != 0 && valid && (unsigned)(ib - pc0) <= 1u && (unsigned)(ic - pc1) <= 1u;
-    const bool aperture = pid != 0 && below(axis_d, G.ap_r, unsure);
-    const bool in_post = below(dd, G.half_d, unsure);
+    const bool aperture = pid != 0 && below(G, axis_d, G.ap_r, unsure);
+    const bool in_post = below(G, dd, G.half_d, unsure);
     if (rod && in_post) return true;
-    if (below(u, G.t_pcb, unsure) && !aperture && !(valid && below(dd, rod ? G.rod_hole : G.clear_r, unsure))) return true;
+    if (below(G, u, G.t_pcb, unsure) && !aperture && !(valid && below(G, dd, rod ? G.rod_hole : G.clear_r, unsure))) return true;
     if (valid && !rod) {
-        if (below(u, G.t_pcb + G.gap, unsure)) return below(dd, G.stem_r, unsure);
+        if (below(G, u, G.t_pcb + G.gap, unsure)) return below(G, dd, G.stem_r, unsure);
         return in_post;
     }
     return false;
@@ -140,7 +140,7 @@ __device__ __forceinline__ void add_steps(unsigned long long* st, uint32_t c, ui
 // group of G lanes per track, each lane an axis (position, velocity) and one of the eight cell
 // corners (two for G = 4), the sums over the corners side by side in the lanes. With one lane per track
 // a step took 32 us. In the cube the electrode test, some hundreds of FP64 operations, is first made in
-// FP32, one face of the cube per lane, and exactly only within 2 um of a surface; whether a
+// FP32, one face of the cube per lane, and exactly only near a surface (CubeF::near); whether a
 // track is at a limit at all is read off the high words of its position. Every operation that counts is the
 // reference's, in its order: results are bit for bit those of one lane per track.
 // G = 16 while the tracks fit one warp per scheduler (two of them in a warp), 4 beyond, where fewer wasted
@@ -479,9 +479,9 @@ k_tandem(const __grid_constant__ TConst C, Tracks T, uint32_t n, const double* _
                 bool unsure = false, solid = false;
                 {
                     const float l = C.F.size;
-                    bool far = false;   // within kNear of a face plane the FP32 `inside` is not to be trusted
-                    const bool inside = !below(p0, 0.0f, far) && !below(p1, 0.0f, far) && !below(p2, 0.0f, far) && below(p0, l, far) &&
-                                        below(p1, l, far) && below(p2, l, far);
+                    bool far = false;   // close to a face plane the FP32 `inside` is not to be trusted
+                    const bool inside = !below(C.F, p0, 0.0f, far) && !below(C.F, p1, 0.0f, far) && !below(C.F, p2, 0.0f, far) &&
+                                        below(C.F, p0, l, far) && below(C.F, p1, l, far) && below(C.F, p2, l, far);
                     unsure = far;
                     for (int f = gl; f < 6; f += G) {
                         const int a = f >> 1, side = f & 1;
@@ -710,6 +710,12 @@ mq_status mq_tandem_create(const mq_tandem_desc* d, int32_t device, mq_tandem** 
         F.t_pcb = (float)g.t_pcb; F.gap = (float)g.gap; F.ptd = (float)mqc::post_top_depth(g); F.stem_r = (float)g.stem_r;
         F.clear_r = (float)g.clear_r; F.rod_hole = (float)(g.d / 2.0 + g.rod_clear_extra); F.l_ext = (float)g.l_ext;
         F.cap_reach = (float)(g.l_ext + g.cap_gap); F.cap_r = (float)g.cap_r; F.ap_r = (float)g.ap_r;
+        // Coordinates near a surface are at most m, and an FP32 distance of two of them is off by about 10 * 2^-24 m;
+        // 2^-17 m is over ten times that. In the cube as built (m = 126 mm) it would be 1 um; 2 um is the least taken.
+        const double m = mqc::size(g) + 2.0 * (std::fabs(g.l_ext) + std::fabs(g.cap_gap) + std::fabs(g.cap_r));
+        const double near = std::fmax(2e-3, m * 0x1.0p-17);
+        F.near = (float)near;
+        F.round_max = (float)std::fmin(0.499, 0.5 - near / std::fabs(g.pitch));
         F.n = g.n; F.array = g.array;
         F.ent_axis = g.ent_axis; F.ent_side = g.ent_side; F.ent_cell0 = g.ent_cell[0]; F.ent_cell1 = g.ent_cell[1];
         F.ext_axis = g.ext_axis; F.ext_side = g.ext_side; F.ext_cell0 = g.ext_cell[0]; F.ext_cell1 = g.ext_cell[1];
