@@ -133,9 +133,12 @@ uint64_t    mq_fnv1a64(const void* data, size_t bytes, uint64_t h);
  * fixed by #defines and environment variables: simulation/chsim/src/tiled.rs:10-29). */
 typedef struct mq_tuning {
     int32_t threads_per_block;   /* fixed at 128                                          */
-    int32_t blocks_per_sm;       /* resident blocks per SM of the persistent grid (1..3);
-                                    1 with 48-byte records is two below 3.5 GB of them, 3 with
-                                    96-byte records four for lists of 2,048 ions per SM    */
+    int32_t blocks_per_sm;       /* resident blocks per SM of the persistent grid, 1..3; 3 with
+                                    48-byte records are the two that fit.  Set: 0 leaves them as
+                                    they are.  An engine that was given none chooses for each
+                                    call by the grid and the number of ions (mq_engine_blocks);
+                                    what get_tuning says then is its class of grid, 3 below
+                                    0.42 GB of 48-byte records, 2 below 0.55 GB, else 1     */
     uint32_t chunk;              /* steps per ion per launch (compaction interval)         */
     int32_t use_graph;           /* replay the launch sequence as one CUDA graph           */
     int32_t prefetch;            /* L1-prefetch the cell each ion is heading for           */
@@ -146,6 +149,9 @@ typedef struct mq_tuning {
 } mq_tuning;
 mq_status   mq_engine_get_tuning(mq_engine* e, mq_tuning* t);
 mq_status   mq_engine_set_tuning(mq_engine* e, const mq_tuning* t);
+/* Blocks per SM that a call over `ions` live ions launches with the engine's present tuning and
+ * trilinear fields; 0 where the ions are so few that the lane groups take them alone. */
+mq_status   mq_engine_blocks(mq_engine* e, uint64_t ions, int32_t* blocks);
 /* Autotuner: times every candidate shape on a sample of the batch (the first
  * sample_per_job ions of each job), keeps the fastest as the engine's tuning and returns
  * it with its rate in ion-steps/s.  Mixed engine only. */

@@ -353,15 +353,25 @@ class Engine:
                    prefetch: bool | None = None, wide_records: bool | None = None, sort_cells: bool | None = None) -> None:
         """Override the mixed engine's launch shape; ``wide_records`` picks 96-byte node records read
         with 256-bit loads (the default on grids below 0.55 GB of 48-byte records) over 48-byte ones;
-        ``sort_cells`` puts every launch's live ions in the Morton order of their cells."""
+        ``sort_cells`` puts every launch's live ions in the Morton order of their cells. Without
+        ``blocks_per_sm`` the blocks stay as they are: the engine's choice for each call, or what was given
+        before."""
         cur = self.tuning()
-        t = N.mq_tuning(128, int(blocks_per_sm if blocks_per_sm is not None else cur["blocks_per_sm"]),
+        blocks = 0 if blocks_per_sm is None else int(blocks_per_sm) or -1   # 0 says "as they are" to the library, not here
+        t = N.mq_tuning(128, blocks,
                         int(chunk if chunk is not None else cur["chunk"]),
                         int(use_graph if use_graph is not None else cur["use_graph"]),
                         int(prefetch if prefetch is not None else cur["prefetch"]),
                         int(wide_records if wide_records is not None else cur["wide_records"]),
                         int(sort_cells if sort_cells is not None else cur["sort_cells"]))
         N.check(N.lib().mq_engine_set_tuning(self._h, C.byref(t)), "mq_engine_set_tuning", self._h)
+
+    def blocks_per_sm(self, ions: int) -> int:
+        """Blocks per SM that a call over so many live ions launches (trilinear fields); 0 where the lane
+        groups take them alone."""
+        b = C.c_int32(0)
+        N.check(N.lib().mq_engine_blocks(self._h, int(ions), C.byref(b)), "mq_engine_blocks", self._h)
+        return int(b.value)
 
     def autotune(self, jobs, dc, ph: Physics, sample_per_job: int = 2048) -> tuple[dict, float]:
         """Time candidate launch shapes on a sample of the batch and keep the fastest."""

@@ -648,17 +648,27 @@ mq_status mq_engine_get_tuning(mq_engine* e, mq_tuning* t) {
 
 mq_status mq_engine_set_tuning(mq_engine* e, const mq_tuning* t) {
     if (!e || !t) return MQ_ERR_INVALID;
-    if (t->threads_per_block != 128 || t->blocks_per_sm < 1 || t->blocks_per_sm > 3 || t->chunk == 0)
-        return fail(e, MQ_ERR_INVALID, "tuning: 128 threads per block, 1..3 blocks per SM, chunk > 0");
+    if (t->threads_per_block != 128 || t->blocks_per_sm < 0 || t->blocks_per_sm > 3 || t->chunk == 0)
+        return fail(e, MQ_ERR_INVALID, "tuning: 128 threads per block, 1..3 blocks per SM (0: as they are), chunk > 0");
     if (t->wide_records && 4 * e->nnodes >= ((size_t)1 << 32))
         return fail(e, MQ_ERR_INVALID, "tuning: wide node records need 4 x nodes below 2^32");
     e->tune.tpb = t->threads_per_block;
-    e->tune.blocks_per_sm = t->blocks_per_sm;
+    if (t->blocks_per_sm) {
+        e->tune.blocks_per_sm = t->blocks_per_sm;
+        e->tune.auto_blocks = 0;
+    }
     e->tune.chunk = t->chunk;
     e->tune.use_graph = t->use_graph ? 1 : 0;
     e->tune.prefetch = t->prefetch ? 1 : 0;
     e->tune.wide = t->wide_records ? 1 : 0;
     e->tune.sort_cells = t->sort_cells ? 1 : 0;
+    return MQ_OK;
+}
+
+mq_status mq_engine_blocks(mq_engine* e, uint64_t ions, int32_t* blocks) {
+    if (!e || !blocks) return MQ_ERR_INVALID;
+    if (e->prec != MQ_PREC_MIXED) return fail(e, MQ_ERR_INVALID, "the mixed engine has a launch shape");
+    *blocks = ions > mqmix::group_ions(e->tune, false) ? mqmix::resident_blocks(e->tune, e->nnodes, (size_t)ions) : 0;
     return MQ_OK;
 }
 
@@ -726,18 +736,23 @@ mq_status mq_engine_autotune(mq_engine* e, const mq_job* jobs, size_t njobs, con
     const mqmix::Tuning keep = e->tune;
     mqmix::Tuning top = keep;
     double top_rate = -1.0;
-    const int blocks[] = {1, 2, 3};
+    // blocks per SM: each number that runs as such, and (0) the engine's own choice where that is another
+    size_t n = 0;
+    for (const auto& j : sj) n += j.n;
     const uint32_t chunks[] = {2048, 8192, 20000};
     const int widths = 4 * e->nnodes < ((size_t)1 << 32) ? 2 : 1;
     for (int wd = 0; wd < widths; ++wd)
     for (int pf = 0; pf < 2; ++pf)
-    for (int bl : blocks)
+    for (int bl = 3; bl >= 0; --bl)
         for (uint32_t ch : chunks) {
             e->tune = keep;
-            e->tune.blocks_per_sm = bl;
+            e->tune.wide = wd;
+            e->tune.auto_blocks = bl == 0;
+            e->tune.blocks_per_sm = bl ? bl : mqmix::default_tuning(e->dev, e->nnodes).blocks_per_sm;
+            const int runs = mqmix::resident_blocks(e->tune, e->nnodes, n);
+            if (bl ? runs != bl : runs <= 3) continue;
             e->tune.chunk = ch;
             e->tune.prefetch = pf;
-            e->tune.wide = wd;
             mq_run_stats st;
             // first call warms the graph and caches; the second is timed
             if ((s = mq_run_batch(e, sj.data(), njobs, dc, ph, out.data(), nullptr, &st)) != MQ_OK) { e->tune = keep; return s; }

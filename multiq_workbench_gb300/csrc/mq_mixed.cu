@@ -1380,13 +1380,23 @@ Tuning default_tuning(int device, size_t nodes) {
     // 4.6 GB - / - / 28.9 / 25.9, 8.0 GB - / - / 35.7 / 28.2.
     const double rec = 48.0 * (double)nodes;
     t.wide = rec < 0.55e9 ? 1 : 0;
-    t.blocks_per_sm = rec < 0.42e9 ? 3 : rec < 0.55e9 ? 2 : 1;   // 1 with narrow records: run() doubles it below 3.5 GB
+    t.blocks_per_sm = rec < 0.42e9 ? 3 : rec < 0.55e9 ? 2 : 1;
     return t;
+}
+
+int resident_blocks(const Tuning& t, size_t nodes, size_t n) {
+    constexpr int kNarrow = 2;   // what the narrow kernel's registers leave room for
+    if (!t.auto_blocks) return t.wide || t.blocks_per_sm < kNarrow ? t.blocks_per_sm : kNarrow;
+    if (!t.wide) return 48.0 * (double)nodes < 3.5e9 ? kNarrow : 1;   // default_tuning has the figures
+    // three with wide records are four for a list of eight or more ions a lane, which outlasts its uneven end:
+    // 1,280,000 ions 22.1 -> 21.1 ms, 640,000 13.6 -> 13.2, 320,000 the same, 62,000 (S14 sweep) 39.0 -> 40.4
+    return t.blocks_per_sm == 3 && n > 2048 * (size_t)t.sms ? 4 : t.blocks_per_sm;
 }
 
 // Ions that the lane groups hold at once: a list of up to so many is stepped by them alone, a longer
 // one's last so many are handed to them.
 static uint32_t hand_entries(int sms, bool nearest) { return (uint32_t)sms * (uint32_t)(group_block(nearest) / 4); }
+uint32_t group_ions(const Tuning& t, bool nearest) { return hand_entries(t.sms, nearest); }
 
 // Steps of the lane-group launches of one round of `chunk` steps. Between them the ions that are left are
 // spread over full warps again: worth its 10 us where warps hold many ions each and these end one by one
@@ -1592,12 +1602,7 @@ cudaError_t run(Scratch& s, const Tuning& t, DevGrid g, uint64_t grid_gen, const
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // resident blocks per SM: the tuning's, except for the nearest-node kernels, which hold no
     // 8-corner cache (about 100 registers instead of 167) and run as many blocks as fit
-    int blocks = t.blocks_per_sm;
-    // three with wide records are four for a list of eight or more ions a lane, which outlasts its uneven end:
-    // 1,280,000 ions 22.1 -> 21.1 ms, 640,000 13.6 -> 13.2, 320,000 the same, 62,000 (S14 sweep) 39.0 -> 40.4
-    if (t.wide && blocks == 3 && n > 2048u * (uint32_t)t.sms) blocks = 4;
-    // one block per SM with narrow records is two of them below 3.5 GB (default_tuning has the figures)
-    if (!t.wide && blocks == 1 && 48.0 * (double)mb.nx * mb.ny * mb.nz < 3.5e9) blocks = 2;
+    int blocks = resident_blocks(t, (size_t)mb.nx * mb.ny * mb.nz, n);
     if (mb.nearest) {
         int nb = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_kernel(t, mb, 0), t.tpb, 0) == cudaSuccess && nb > 0)

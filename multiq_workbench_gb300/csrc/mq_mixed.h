@@ -40,8 +40,9 @@ struct MixBatch {      // per-batch constants (device-resident parameter block)
 
 struct Tuning {
     int tpb = 128;             // threads per block
-    int blocks_per_sm = 3;     // resident blocks per SM for the persistent grid (3 at most; run() makes 3 with
-                               // wide records 4 for long lists, and 1 with narrow ones 2 below 3.5 GB); the nearest-node kernels (about 100 registers) run as many as fit instead
+    int blocks_per_sm = 3;     // blocks per SM of the persistent grid, as the caller gave it (resident_blocks()); the
+                               // nearest-node kernels (about 100 registers) run as many as fit instead
+    int auto_blocks = 1;       // the caller gave none: resident_blocks() chooses, from blocks_per_sm with wide records
     uint32_t chunk = 20000;    // steps per ion per launch (compaction interval)
     int use_graph = 1;         // replay the launch sequence as one CUDA graph
     int prefetch = 0;          // L1-prefetch the cell an ion is heading for
@@ -88,6 +89,10 @@ MixBatch make_mix_batch(const mqp::Batch& b);
 // device injection of a batch for the mixed engine: the FP64 injection's draws with FP32 transforms
 cudaError_t launch_inject(const mqp::Batch& b, mqd::JobTable jt, mqd::DevIons io, uint32_t n, cudaStream_t st);
 Tuning default_tuning(int device, size_t nodes);
+// Blocks per SM that run() launches k_mixed with for n ions on a grid of so many nodes (trilinear fields)
+int resident_blocks(const Tuning& t, size_t nodes, size_t n);
+// Ions up to which a call runs in lane groups alone
+uint32_t group_ions(const Tuning& t, bool nearest);
 // write_states = 0 leaves the FP64 position / velocity of the ion states as they were (a caller
 // that wants only the counters, steps, status and collision counts)
 cudaError_t run(Scratch& s, const Tuning& t, mqd::DevGrid g, uint64_t grid_gen, const mqp::Batch& b, const MixJob* jobs,

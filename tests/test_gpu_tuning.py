@@ -1,0 +1,58 @@
+"""The mixed engine's launch shape: what a caller sets is what runs, and an engine that was given no blocks
+per SM keeps choosing them itself whatever else is set. Results do not depend on it."""
+import sys
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, str(Path(__file__).resolve().parent))
+from test_gpu_parity import FIELDS, _mq, _variants  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+DC = [0.0, 5.0, -5.0, 0.0]
+LONG = 2048 * 152 + 1   # ions above which the engine's own choice for wide records is four
+
+
+def _jobs(n, k=1):
+    mq = _mq()
+    return [mq.Job(mq.Species(499.0, 1.0, 2.95 * 499.0 ** (2 / 3)), mq.RfAc(100.0, 500e3, 0.5, 100e3), n, 5 + s) for s in range(k)]
+
+
+def test_given_blocks_run_and_the_engines_choice_stays(coarse):
+    mq = _mq()
+    with mq.Engine(coarse, mq.PREC_MIXED) as e:
+        assert [e.blocks_per_sm(n) for n in (1000, 60000, LONG)] == [0, 3, 4]
+        e.set_tuning(chunk=301, use_graph=False)
+        assert e.tuning()["blocks_per_sm"] == 3 and e.blocks_per_sm(LONG) == 4
+        e.set_tuning(wide_records=False)          # what fits of the narrow kernel
+        assert e.blocks_per_sm(60000) == 2 and e.blocks_per_sm(LONG) == 2
+        for wide, want in ((False, {1: 1, 2: 2, 3: 2}), (True, {1: 1, 2: 2, 3: 3})):
+            for b, w in want.items():
+                e.set_tuning(blocks_per_sm=b, wide_records=wide)
+                assert e.tuning()["blocks_per_sm"] == b
+                e.set_tuning(chunk=400)
+                assert [e.blocks_per_sm(n) for n in (60000, LONG)] == [w, w], (wide, b)
+        for b in (0, 4, 9, -1):
+            with pytest.raises(mq.MqError):
+                e.set_tuning(blocks_per_sm=b)
+    with mq.Engine(coarse, mq.PREC_F64) as e, pytest.raises(mq.MqError):
+        e.blocks_per_sm(1000)
+
+
+def test_any_shape_gives_the_same_ions(coarse):
+    mq = _mq()
+    ph = _variants()["half_kick_gauss"]
+    with mq.Engine(coarse, mq.PREC_MIXED) as e:
+        want, _ = e.run_batch_ions(_jobs(LONG), DC, ph)
+        rate = {}
+        for wide in (True, False):
+            for b in (1, 2, 3):
+                e.set_tuning(blocks_per_sm=b, wide_records=wide)
+                got, _ = e.run_batch_ions(_jobs(LONG), DC, ph)
+                rate[wide, b] = e.last_stats.step_kernel_ms
+                for f in FIELDS:
+                    assert np.array_equal(getattr(want, f).view(np.uint8), getattr(got, f).view(np.uint8)), (wide, b, f)
+    # one block of 128 lanes per SM has half the ions in flight that two have, and does show it
+    assert rate[True, 1] > 1.15 * rate[True, 2] and rate[False, 1] > 1.15 * rate[False, 2], rate
