@@ -154,7 +154,9 @@ mq_status   mq_engine_set_tuning(mq_engine* e, const mq_tuning* t);
 mq_status   mq_engine_blocks(mq_engine* e, uint64_t ions, int32_t* blocks);
 /* Autotuner: times every candidate shape on a sample of the batch (the first
  * sample_per_job ions of each job), keeps the fastest as the engine's tuning and returns
- * it with its rate in ion-steps/s.  Mixed engine only. */
+ * it with its rate in ion-steps/s.  The present shape stays unless another is faster by more than
+ * 2%.  A sample so small that the lane groups take it alone chooses between the record widths
+ * only.  Mixed engine only. */
 mq_status   mq_engine_autotune(mq_engine* e, const mq_job* jobs, size_t njobs, const double dc[4], const mq_physics* ph,
                                uint64_t sample_per_job, mq_tuning* best, double* best_rate);
 

@@ -735,32 +735,48 @@ mq_status mq_engine_autotune(mq_engine* e, const mq_job* jobs, size_t njobs, con
     std::vector<mq_outcome> out(njobs);
     const mqmix::Tuning keep = e->tune;
     mqmix::Tuning top = keep;
-    double top_rate = -1.0;
-    // blocks per SM: each number that runs as such, and (0) the engine's own choice where that is another
+    double top_rate = 0.0;
+    // One candidate: the first call warms the graph and caches, the second is timed. It takes the best one's place only if
+    // it is faster by more than two runs of one shape differ (about 1%), so the engine's present shape stays
+    // where the others do no better.
+    auto time = [&](const mqmix::Tuning& t) -> mq_status {
+        e->tune = t;
+        mq_run_stats st;
+        mq_status r;
+        for (int k = 0; k < 2; ++k)
+            if ((r = mq_run_batch(e, sj.data(), njobs, dc, ph, out.data(), nullptr, &st)) != MQ_OK) return r;
+        const double rate = st.step_kernel_ms > 0 ? (double)st.ion_steps / (st.step_kernel_ms * 1e-3) : 0.0;
+        if (rate > 1.02 * top_rate) { top_rate = rate; top = t; }
+        return MQ_OK;
+    };
     size_t n = 0;
     for (const auto& j : sj) n += j.n;
-    const uint32_t chunks[] = {2048, 8192, 20000};
+    // ions that the lane groups take alone say nothing about the shape of the other kernel: its knobs stay as they are
+    const bool shaped = n > mqmix::group_ions(e->tune, ph->legacy_fields != 0);
+    const int base = mqmix::default_tuning(e->dev, e->nnodes).blocks_per_sm;
     const int widths = 4 * e->nnodes < ((size_t)1 << 32) ? 2 : 1;
-    for (int wd = 0; wd < widths; ++wd)
-    for (int pf = 0; pf < 2; ++pf)
-    for (int bl = 3; bl >= 0; --bl)
-        for (uint32_t ch : chunks) {
-            e->tune = keep;
-            e->tune.wide = wd;
-            e->tune.auto_blocks = bl == 0;
-            e->tune.blocks_per_sm = bl ? bl : mqmix::default_tuning(e->dev, e->nnodes).blocks_per_sm;
-            const int runs = mqmix::resident_blocks(e->tune, e->nnodes, n);
-            if (bl ? runs != bl : runs <= 3) continue;
-            e->tune.chunk = ch;
-            e->tune.prefetch = pf;
-            mq_run_stats st;
-            // first call warms the graph and caches; the second is timed
-            if ((s = mq_run_batch(e, sj.data(), njobs, dc, ph, out.data(), nullptr, &st)) != MQ_OK) { e->tune = keep; return s; }
-            if ((s = mq_run_batch(e, sj.data(), njobs, dc, ph, out.data(), nullptr, &st)) != MQ_OK) { e->tune = keep; return s; }
-            double rate = st.step_kernel_ms > 0 ? (double)st.ion_steps / (st.step_kernel_ms * 1e-3) : 0.0;
-            if (rate > top_rate) { top_rate = rate; top = e->tune; }
+    s = time(keep);
+    for (int wd = 0; wd < widths && s == MQ_OK; ++wd) {
+        mqmix::Tuning t = keep;
+        t.wide = wd;
+        if (!shaped) {
+            if (wd != keep.wide) s = time(t);
+            continue;
         }
-    e->tune = top;
+        // blocks per SM: each number that runs as such, and (0) the engine's own choice where that is another
+        for (int pf = 0; pf < 2; ++pf)
+            for (int bl = 3; bl >= 0; --bl)
+                for (uint32_t ch : {2048u, 8192u, 20000u}) {
+                    t.prefetch = pf;
+                    t.chunk = ch;
+                    t.auto_blocks = bl == 0;
+                    t.blocks_per_sm = bl ? bl : base;
+                    const int runs = mqmix::resident_blocks(t, e->nnodes, n);
+                    if (s == MQ_OK && (bl ? runs == bl : runs > 3)) s = time(t);
+                }
+    }
+    e->tune = s == MQ_OK ? top : keep;
+    if (s != MQ_OK) return s;
     if (best) mq_engine_get_tuning(e, best);
     if (best_rate) *best_rate = top_rate;
     return MQ_OK;

@@ -56,3 +56,31 @@ def test_any_shape_gives_the_same_ions(coarse):
                     assert np.array_equal(getattr(want, f).view(np.uint8), getattr(got, f).view(np.uint8)), (wide, b, f)
     # one block of 128 lanes per SM has half the ions in flight that two have, and does show it
     assert rate[True, 1] > 1.15 * rate[True, 2] and rate[False, 1] > 1.15 * rate[False, 2], rate
+
+
+@pytest.mark.parametrize("n, sample", [(64, 64), (3000, 3000), (48000, 3000)])
+def test_autotune_on_few_ions_leaves_what_it_cannot_time(coarse, n, sample):
+    """A sample that runs in the lane groups alone says nothing about the other kernel's shape, be it the whole batch
+    or the beginning of a long one."""
+    mq = _mq()
+    ph = _variants()["half_kick_gauss"]
+    with mq.Engine(coarse, mq.PREC_MIXED) as e:
+        e.set_tuning(chunk=12345)
+        before = e.tuning()
+        t, rate = e.autotune(_jobs(n, 4), DC, ph, sample_per_job=sample)
+        assert rate > 0 and {**t, "wide_records": before["wide_records"]} == before
+        e.set_tuning(wide_records=True)
+        assert e.blocks_per_sm(LONG) == 4
+
+
+def test_autotune_keeps_no_shape_that_is_slower(built):
+    """60,000 ions on the 0.1 mm channel: the L1 prefetch costs a tenth, narrow records more."""
+    mq = _mq()
+    f = mq.Fields.build(mq.Geom.with_spacing(0.1), bases=[0, 1, 3, 4], cache=False, device=0)
+    ph = _variants()["half_kick_gauss"]
+    got = []
+    for _ in range(4):
+        with mq.Engine(f, mq.PREC_MIXED) as e:
+            t, _ = e.autotune(_jobs(15000, 4), DC, ph, sample_per_job=15000)
+            got.append((t["wide_records"], t["prefetch"]))
+    assert got == [(True, False)] * 4, got
