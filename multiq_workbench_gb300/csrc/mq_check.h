@@ -1,6 +1,7 @@
 // Bounds checks of the debug build.  Compiled with -DMQ_CHECK (build(check=True) makes
-// libmqgb_check.so), every gather whose index is computed from a particle's position, and the
-// work-queue indices of the persistent kernels, go through MQ_CHK / MQ_CHK_SPAN: an index out of
+// libmqgb_check.so), every gather whose index is computed from a particle's position, the
+// work-queue and hand-over indices of the persistent kernels, and the field solve's packed node
+// lists go through MQ_CHK / MQ_CHK_SPAN: an index out of
 // range is recorded (count, site, index, limit) in a per-translation-unit device word and
 // replaced by 0, so the access stays inside the array and the kernel runs on; the host reads the
 // words with mq_check_status.  In the normal build the macros are the bare index.
@@ -69,9 +70,10 @@ __device__ __forceinline__ size_t mq_chk_span(size_t i, size_t span, size_t n, u
 
 // site ids
 enum MqCheckSite : unsigned {
-    MQ_SITE_F64_FIELD = 1, MQ_SITE_F64_CRASH = 2,
+    MQ_SITE_F64_FIELD = 1, MQ_SITE_F64_ION = 3, MQ_SITE_F64_HAND = 4,
     MQ_SITE_MIX_CELL = 10, MQ_SITE_MIX_ION = 11, MQ_SITE_MIX_LIST_OUT = 12, MQ_SITE_MIX_HAND = 13,
-    MQ_SITE_TDM_CUBE = 20, MQ_SITE_TDM_PORT = 21, MQ_SITE_TDM_GATE = 22, MQ_SITE_TDM_CRASH = 23,
+    MQ_SITE_TDM_CUBE = 20, MQ_SITE_TDM_PORT = 21,
     MQ_SITE_TMX_CELL = 30, MQ_SITE_TMX_LIST = 31,
+    MQ_SITE_SOLVE_LIST = 40, MQ_SITE_SOLVE_NODE = 41,
     MQ_SITE_SELFTEST = 99,
 };

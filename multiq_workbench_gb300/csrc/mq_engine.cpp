@@ -687,6 +687,7 @@ extern "C" int mq_check_read_mixed(MqCheckWordC*, int);
 extern "C" int mq_check_read_tandem(MqCheckWordC*, int);
 extern "C" int mq_check_read_tandem_mixed(MqCheckWordC*, int);
 extern "C" int mq_check_read_probe(MqCheckWordC*, int);
+extern "C" int mq_check_read_solve(MqCheckWordC*, int);
 extern "C" int mq_check_selftest_launch(void);
 
 extern "C" {
@@ -699,7 +700,7 @@ mq_status mq_check_status(int32_t device, int32_t reset, int32_t* enabled, uint3
     cudaGetDevice(&prev);
     if (cudaSetDevice(device) != cudaSuccess) { cudaGetLastError(); return MQ_ERR_CUDA; }
     int (*readers[])(MqCheckWordC*, int) = {mq_check_read_f64, mq_check_read_mixed, mq_check_read_tandem,
-                                            mq_check_read_tandem_mixed, mq_check_read_probe};
+                                            mq_check_read_tandem_mixed, mq_check_read_solve, mq_check_read_probe};
     *enabled = 0; *hits = 0; *site = 0; *index = 0; *limit = 0;
     mq_status st = MQ_OK;
     for (auto rd : readers) {

@@ -226,7 +226,7 @@ k_f64_step(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __r
                     else {
                         uint32_t done = 0;
                         id = slot;
-                        if (from_hand) { const uint2 e = hand[slot]; id = e.x; done = e.y; }
+                        if (from_hand) { const uint2 e = hand[slot]; id = (uint32_t)MQ_CHK(e.x, n, MQ_SITE_F64_ION); done = e.y; }
                         if (io.status[id] == 0) {
                             have = got = true;
                             jid = io.jid[id];
@@ -454,7 +454,7 @@ k_f64_step(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __r
                 if (gl == 0) {
                     io.rng[id] = rng; io.steps[id] = age; io.ncoll[id] = ncoll; io.leg[id] = leg; io.status[id] = status;
                     steps_total -= left;
-                    if (give) hand[atomicAdd(&ctr->handed, 1u)] = make_uint2(id, max_more - left);
+                    if (give) hand[MQ_CHK(atomicAdd(&ctr->handed, 1u), hand_at, MQ_SITE_F64_HAND)] = make_uint2(id, max_more - left);
                     else {
                         if (hands) atomicSub(&ctr->open, 1u);
                         live += status == 0 ? 1u : 0u;

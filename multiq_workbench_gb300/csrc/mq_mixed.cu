@@ -714,7 +714,8 @@ k_mixed_group(const float4* __restrict__ nodes, MixBatch B, const MixJob* __rest
         if (!go) return;
         fc = (float)ci;
         ++loads;
-        o = (uint32_t)MQ_CHK(o, (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
+        // the cell's highest record read: with narrow records one layer up, which wide ones hold
+        o = (uint32_t)MQ_CHK_SPAN(o, NEAREST ? 1u : (WIDE ? 0u : sz) + sy + 2u, (size_t)sz * (size_t)B.nz, MQ_SITE_MIX_CELL);
         const float4* const p = nodes + (size_t)(WIDE ? 6u : 3u) * o + (WIDE ? 2 : 1) * d;
 #pragma unroll
         for (int q = 0; q < NQ; ++q) {

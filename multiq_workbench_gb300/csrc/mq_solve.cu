@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "mq_chan_geom.h"
+#include "mq_check.h"
 #include "mq_grid.h"
 #include "mq_levels.h"
 #include "mq_phys.h"
@@ -110,7 +111,7 @@ __device__ __forceinline__ bool colour_node(unsigned t, int k, int col, int nx, 
 // and the FP64 pipe's time goes by warps (half sweep of the finest level of the 0.100 mm channel 35 -> 22 us, the list once a
 // solve 20 us).
 __global__ void __launch_bounds__(kT) k_list(const uint8_t* __restrict__ fix, int nx, int ny, int nz, int col, uint32_t* __restrict__ list,
-                                             uint32_t* __restrict__ cnt) {
+                                             [[maybe_unused]] size_t room, uint32_t* __restrict__ cnt) {
     __shared__ uint32_t warp_n[kT / 32], base;
     const int k = 1 + block_plane();
     size_t q = 0;
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(kT) k_list(const uint8_t* __restrict__ fix, in
         base = n ? atomicAdd(cnt, n) : 0u;
     }
     __syncthreads();
-    if (f) list[base + warp_n[w] + (uint32_t)__popc(b & ((1u << lane) - 1u))] = (uint32_t)q;
+    if (f) list[MQ_CHK(base + warp_n[w] + (uint32_t)__popc(b & ((1u << lane) - 1u)), room, MQ_SITE_SOLVE_LIST)] = (uint32_t)q;
 }
 // node of this thread: the list's, or where there is none (grids of 2^32 nodes and more) the colour's free nodes in turn
 __device__ __forceinline__ bool free_node(const uint32_t* __restrict__ list, uint32_t cnt, const uint8_t* __restrict__ fix, int col, int nx,
@@ -132,7 +133,7 @@ __device__ __forceinline__ bool free_node(const uint32_t* __restrict__ list, uin
     const unsigned t = blockIdx.x * kT + threadIdx.x;
     if (list) {
         if (t >= cnt) return false;
-        q = list[t];
+        q = MQ_CHK(list[t], (size_t)nx * ny * nz, MQ_SITE_SOLVE_NODE);
         return true;
     }
     const int k = 1 + block_plane();
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(kT) k_restrict(const double* __restrict__ fr, 
     size_t qc;
     if (l0) {   // free nodes only: nothing reads the others' right-hand side
         if (t >= n0 + n1) return;
-        const unsigned x = t < n0 ? l0[t] : l1[t - n0], y = x / (unsigned)cnx;
+        const unsigned x = (unsigned)MQ_CHK(t < n0 ? l0[t] : l1[t - n0], (size_t)n * cnz, MQ_SITE_SOLVE_NODE), y = x / (unsigned)cnx;
         I = x % (unsigned)cnx; J = y % (unsigned)cny; K = y / (unsigned)cny;
         qc = x;
     } else {
@@ -749,7 +750,7 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
             for (int c = 0; c < 2; ++c) {
                 const DLevel& v = P.L[l];
                 k_list<<<plane_blocks((size_t)((v.nx - 1) / 2) * (v.ny - 2), v.nz - 2), kT, 0, st>>>(v.fix, v.nx, v.ny, v.nz, c, v.list[c],
-                                                                                                  P.cnts + 2 * l + c);
+                                                                                                  Problem::half(P.dims[l]), P.cnts + 2 * l + c);
             }
         if (cudaMemcpyAsync(cnts.data(), P.cnts, cnts.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
     }
@@ -958,3 +959,5 @@ mq_status mq_channel_basis_device(const mq_geom* g, int32_t basis, double tol, i
     if (cudaMemcpyAsync(e4, e, n * sizeof(float4), cudaMemcpyDeviceToHost, A.st) != cudaSuccess) return MQ_ERR_CUDA;
     return cudaStreamSynchronize(A.st) == cudaSuccess ? MQ_OK : MQ_ERR_CUDA;
 }
+
+MQ_CHECK_READER(mq_check_read_solve)
