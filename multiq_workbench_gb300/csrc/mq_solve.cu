@@ -686,22 +686,24 @@ struct Problem {
     Scal* sc;
     uint32_t* cnts;
     size_t n() const { return (size_t)nx * ny * nz; }
-    static bool listed(const std::vector<mqlv::Dims>& dims) { return mqlv::count(dims[0]) < ((size_t)1 << 32); }
+    bool lists;   // the levels have lists of their free nodes
+    static bool can_list(const std::vector<mqlv::Dims>& dims) { return mqlv::count(dims[0]) < ((size_t)1 << 32); }
     static size_t half(const mqlv::Dims& d) { return (size_t)((d.nx - 1) / 2) * (d.ny - 2) * (d.nz - 2); }   // nodes of a colour, at most
-    static size_t bytes(const std::vector<mqlv::Dims>& dims) {
+    static size_t bytes(const std::vector<mqlv::Dims>& dims, bool lists) {
         size_t b = 0;
         for (size_t l = 0; l < dims.size(); ++l) {
             const size_t m = mqlv::count(dims[l]);
             b += Arena::up(m) + (l ? 3 : 2) * Arena::up(8 * m);   // the finest level's right-hand side is the residual
-            if (listed(dims)) b += 2 * Arena::up(4 * half(dims[l]));
+            if (lists) b += 2 * Arena::up(4 * half(dims[l]));
         }
         b += Arena::up(8 * dims.size());
         const mqlv::Dims& f = dims[0];
         b += 4 * Arena::up(8 * mqlv::count(f)) + Arena::up(8 * (size_t)f.ny * f.nz) + Arena::up(8 * (size_t)f.nz) + Arena::up(sizeof(Scal));
         return b;
     }
-    void carve(Arena& A, const std::vector<mqlv::Dims>& d) {
+    void carve(Arena& A, const std::vector<mqlv::Dims>& d, bool with_lists) {
         dims = d;
+        lists = with_lists;
         nx = d[0].nx; ny = d[0].ny; nz = d[0].nz;
         phi = A.take<double>(n()); r = A.take<double>(n()); p = A.take<double>(n()); qv = A.take<double>(n());
         rowsum = A.take<double>((size_t)ny * nz); plane = A.take<double>((size_t)nz); sc = A.take<Scal>(1);
@@ -713,7 +715,7 @@ struct Problem {
             v.u = A.take<double>(v.n());
             v.r = A.take<double>(v.n());
             v.rhs = l ? A.take<double>(v.n()) : r;
-            for (int c = 0; c < 2; ++c) { v.list[c] = listed(d) ? A.take<uint32_t>(half(d[l])) : nullptr; v.cnt[c] = 0; }
+            for (int c = 0; c < 2; ++c) { v.list[c] = lists ? A.take<uint32_t>(half(d[l])) : nullptr; v.cnt[c] = 0; }
         }
         cnts = A.take<uint32_t>(2 * d.size());
     }
@@ -744,7 +746,7 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
         k_coarse_fix<<<plane_blocks((size_t)c.nx * c.ny, c.nz), kT, 0, st>>>(f.fix, f.nx, f.ny, f.nz, c.fix, c.nx, c.ny, c.nz);
     }
     std::vector<uint32_t> cnts(2 * P.L.size(), 0u);
-    if (P.L[0].list[0]) {
+    if (P.lists) {
         if (cudaMemsetAsync(P.cnts, 0, cnts.size() * sizeof(uint32_t), st) != cudaSuccess) return MQ_ERR_CUDA;
         for (size_t l = 0; l < P.L.size(); ++l)
             for (int c = 0; c < 2; ++c) {
@@ -886,6 +888,11 @@ extern "C" {
 
 mq_status mq_laplace_solve_device(int32_t nx, int32_t ny, int32_t nz, const uint8_t* mask, const double* fixed,
                                   double outer_bc, double tol, int32_t device, double* phi, mq_solve_stats* stats) {
+    return mq_laplace_solve_device_lists(nx, ny, nz, mask, fixed, outer_bc, tol, device, 1, phi, stats);
+}
+
+mq_status mq_laplace_solve_device_lists(int32_t nx, int32_t ny, int32_t nz, const uint8_t* mask, const double* fixed, double outer_bc,
+                                        double tol, int32_t device, int32_t lists, double* phi, mq_solve_stats* stats) {
     if (nx < 3 || ny < 3 || nz < 3 || !mask || !fixed || !phi || !(tol > 0)) return MQ_ERR_INVALID;
     if (!have_device(device)) return MQ_ERR_NO_DEVICE;
     if (cudaSetDevice(device) != cudaSuccess) return MQ_ERR_CUDA;
@@ -894,9 +901,10 @@ mq_status mq_laplace_solve_device(int32_t nx, int32_t ny, int32_t nz, const uint
     const size_t n = mqlv::count(dims[0]);
     Arena A;
     Problem P;
-    mq_status s = A.open(Problem::bytes(dims) + Arena::up(n));
+    const bool listed = lists && Problem::can_list(dims);
+    mq_status s = A.open(Problem::bytes(dims, listed) + Arena::up(n));
     if (s != MQ_OK) return s;
-    P.carve(A, dims);
+    P.carve(A, dims, listed);
     uint8_t* dmask = A.take<uint8_t>(n);
     if (cudaMemcpyAsync(dmask, mask, n, cudaMemcpyHostToDevice, A.st) != cudaSuccess) return MQ_ERR_CUDA;
     if (cudaMemcpyAsync(P.p, fixed, n * sizeof(double), cudaMemcpyHostToDevice, A.st) != cudaSuccess) return MQ_ERR_CUDA;
@@ -925,9 +933,10 @@ mq_status mq_channel_basis_device(const mq_geom* g, int32_t basis, double tol, i
     const double outer = basis == MQ_BASIS_DC_BOX ? 1.0 : 0.0;
     Arena A;
     Problem P;
-    mq_status s = A.open(Problem::bytes(dims) + Arena::up(n));
+    const bool listed = Problem::can_list(dims);
+    mq_status s = A.open(Problem::bytes(dims, listed) + Arena::up(n));
     if (s != MQ_OK) return s;
-    P.carve(A, dims);
+    P.carve(A, dims, listed);
     uint8_t* mask = A.take<uint8_t>(n);
     if (cudaMemsetAsync(P.sc, 0, sizeof(Scal), A.st) != cudaSuccess) return MQ_ERR_CUDA;
     k_channel<<<grid_blocks(device), kT, 0, A.st>>>(*g, mqgeo::layers_of(g), basis, outer, d[0], d[1], d[2], mask, P.L[0].fix, P.phi, P.sc);
