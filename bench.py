@@ -47,10 +47,10 @@ ION_STATE_BYTES = 48 + 16 + 24 + 56 + 64   # double-floats, phase offsets, count
 def stepping_bytes(stats, wide: bool, nearest: bool = False) -> float:
     """Algorithmic bytes of the stepping kernel(s) of one call, from the kernel's own counters: cell
     fills x 4 node records (wide ones hold two layers; of narrow ones a move along one axis reads the
-    far face's 4, so this is a lower bound there; 1 record in the nearest-node field mode, which reads
-    only the cell's lowest corner), plus the state traffic of every ion taken from the work queue."""
-    rec, per_fill = (96 if wide else 48), CORNERS // 2
-    return float(stats.cell_loads) * (1 if nearest else per_fill) * rec + float(stats.ions_queued) * ION_STATE_BYTES
+    far face's 4, so this is a lower bound there; in the nearest-node field mode the 48 bytes of one
+    node, of which a wide record holds two), plus the state traffic of every ion taken from the work queue."""
+    per_fill = 48 if nearest else CORNERS // 2 * (96 if wide else 48)
+    return float(stats.cell_loads) * per_fill + float(stats.ions_queued) * ION_STATE_BYTES
 
 
 def cpu_model() -> str:
@@ -155,7 +155,7 @@ def run_gridstudy(args, rank: int, world: int):
         t_solve = time.perf_counter() - t0
         with mq.Engine(f, mq.PREC_MIXED, device=local) as eng:
             apply_tuning(eng, args)
-            tuned = eng.tuning()   # the default launch shape (a sampled autotune picks worse ones here)
+            tuned = {**eng.tuning(), "blocks_launched": eng.blocks_per_sm(n)}   # the default launch shape
             for _ in range(args.warmup):
                 eng.run_batch(table, dc, ph)
             if h == spacings[-1]:
@@ -345,7 +345,7 @@ def run_legacy(args, rank: int, world: int):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": None, "peak_source": "measured hbm_gbs" if peaks.get("hbm_gbs") else "fallback",
                          "kernel": "k_mixed (legacy collisions, nearest-node fields)",
-                         "algorithmic_bytes": f"cell fills counted by the kernel x 1 node record ({96 if tuned['wide_records'] else 48} B) "
+                         "algorithmic_bytes": f"cell fills counted by the kernel x 1 node (48 B) "
                                               f"+ {ION_STATE_BYTES} B per ion taken from the queue",
                          "cell_loads_per_ion_step": loads / max(steps, 1)},
             "roofline_l2": {"achieved": achieved, "peak": l2, "unit": "GB/s", "frac": achieved / l2 if l2 else None},
@@ -544,11 +544,12 @@ def tandem_bytes(st, kind: str = "mixed") -> float:
 TRACK_STATE_BYTES = 68 + 56   # k_tm_step: a track's working state read and written once per launch
 
 
-def tandem_moved(st, tracks: int) -> float:
+def tandem_moved(st, tracks: int, steps: int) -> float:
     """Bytes the mixed tandem's step kernel must move, from its own counters: cell-cache fills (cube:
-    8 x 32-byte records; port: 4 x 48-byte records, which a move along one axis reads) plus every track's state once per launch (the
-    advance's launches are a load, a store, and a bucket + step pair per 256-step chunk)."""
-    chunks = max((st.launches - 2) // 2, 0)
+    8 x 32-byte records; port: 4 x 48-byte records, which a move along one axis reads) plus every track's state once per
+    launch of the step kernel: one per 256 steps or rest of a 65,536-step drive table."""
+    tables, rest = divmod(steps, 65536)
+    chunks = tables * (65536 // 256) + -(-rest // 256)
     return st.cell_fills_cube * 8 * 32 + st.cell_fills_port * 4 * 48 + float(tracks) * TRACK_STATE_BYTES * chunks
 
 
@@ -646,7 +647,7 @@ def run_tandem(args, rank: int, world: int):
     peaks = measured_peaks()
     hbm = peaks.get("hbm_gbs") or 6800.0
     l2 = l2_read_gbs(local)
-    achieved = sum(tandem_moved(s, args.tracks) for s in sts) / (sum(s.kernel_ms for s in sts) * 1e-3) / 1e9
+    achieved = sum(tandem_moved(s, args.tracks, args.tandem_steps) for s in sts) / (sum(s.kernel_ms for s in sts) * 1e-3) / 1e9
     fills = sum(s.cell_fills_cube + s.cell_fills_port for s in sts) / max(sum(s.track_steps for s in sts), 1)
     f = m.frame()
     cnt = m.counts_array()
@@ -884,7 +885,8 @@ def main():
                                        f"({len(jobs) * args.ions_per_job:,} ions), "
                                        "0.100 mm channel grid 160x160x242, legacy half-kick, <=20000 steps",
                            "jobs": len(jobs), "ions": sum(j.n for j in jobs), "l2_flush": "256 MB write before every timed step",
-                           "tuning": {**(tuned or eng.tuning()), "use_graph": replays > 0,
+                           "tuning": {**(tuned or eng.tuning()), "blocks_launched": eng.blocks_per_sm(sum(j.n for j in jobs)),
+                                      "use_graph": replays > 0,
                                       "graph_replays_per_step": replays / args.steps,
                                       "step_launches_per_step": step_launches / args.steps}},
                 "ion_steps_per_step": steps_total / args.steps,
