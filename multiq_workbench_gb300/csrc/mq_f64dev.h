@@ -19,7 +19,7 @@ __device__ __forceinline__ bool gt_pos(long long x, long long c) { return x > c 
 __device__ __forceinline__ bool lt_pos(long long x, long long c) { return x < c && !is_nan_bits(x); }
 // x < 0
 __device__ __forceinline__ bool lt_zero(long long x) { return x < 0 && x != (long long)0x8000000000000000ULL && !is_nan_bits(x); }
-// mqp::cell_lo (clamp to [0, n - 2], truncate) from the bits of g; lim = the bits of (double)(n - 2)
+// (g.max(0.0) as usize).min(n - 2) from the bits of g; lim = the bits of (double)(n - 2)
 __device__ __forceinline__ int32_t cell_lo_bits(double g, int32_t n, long long lim) {
     const long long b = __double_as_longlong(g);
     if (b <= 0 || b > 0x7FF0000000000000LL) return 0;   // !(g > 0): zeros, negatives, NaN

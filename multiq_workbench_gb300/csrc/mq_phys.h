@@ -85,22 +85,9 @@ MQ_HD double log_(double x) {
 }
 
 #if defined(__CUDACC__)
-// Exact f32 -> f64 widening built on the integer pipe. GB300's FP64 pipe limits the FP64 channel
-// kernel, and the 72 widenings of a step's field gathers would otherwise take a fifth of its FP64
-// instructions (measured: 14-19% faster, bit-identical states). Normal numbers and zeros are
-// assembled from their bits (exponent rebased by 1023 - 127, the 23-bit fraction moved to the top
-// of the 52-bit one); subnormals, infinities and NaN take the hardware conversion. Either way the
-// value is the same double (checked against the hardware conversion on 6e8 bit patterns).
-__device__ __forceinline__ double widen(float f) {
-    const uint32_t u = __float_as_uint(f);
-    const uint32_t e = (u >> 23) & 0xFFu;
-    if (e - 1u >= 0xFEu && (u & 0x7FFFFFFFu) != 0u) return (double)f;
-    const uint32_t sign = u & 0x80000000u;
-    const uint32_t hi = (u & 0x7FFFFFFFu) ? (sign | ((e + 896u) << 20) | ((u & 0x7FFFFFu) >> 3)) : sign;
-    return __hiloint2double((int)hi, (int)(u << 29));
-}
-
-// the same without a branch for zeros and normal numbers; `odd` is set for any other value
+// Exact f32 -> f64 widening on the integer pipe (the FP64 pipe, which limits the FP64 kernels, also executes conversions): zeros
+// and normal numbers are assembled from their bits, the exponent rebased by 1023 - 127 and the 23-bit fraction moved to
+// the top of the 52-bit one. `odd` is set for any other value, which the caller converts.
 __device__ __forceinline__ double widen_normal(float f, bool& odd) {
     const uint32_t u = __float_as_uint(f), m = u & 0x7FFFFFFFu;
     odd |= m - 0x800000u >= 0x7F000000u && m != 0u;
@@ -217,18 +204,6 @@ MQ_HD void inject_one(const Batch& b, const JobC& j, uint64_t seed, Ion0* o) {
 MQ_HD void phase_at(double w, uint32_t n, double* s, double* c) {
     double p = (double)n * w;
     sincos2pi(p - floor(p), s, c);
-}
-
-MQ_HD int32_t cell_lo(double g, int32_t n) {   // (g.max(0.0) as usize).min(n - 2)
-    if (!(g > 0.0)) return 0;
-    if (g >= (double)(n - 2)) return n - 2;
-    return (int32_t)g;
-}
-MQ_HD int32_t node_round(double g, int32_t n) {   // ((x / h).round() as usize).min(n - 1)
-    double r = round(g);
-    if (!(r > 0.0)) return 0;
-    if (r >= (double)(n - 1)) return n - 1;
-    return (int32_t)r;
 }
 
 }  // namespace mqp
