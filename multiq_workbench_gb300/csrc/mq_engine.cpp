@@ -308,11 +308,11 @@ mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_
     e->fault = MQ_FAULT_NONE;
     if (fault == MQ_FAULT_ALLOC) return fail(e, MQ_ERR_NOMEM, "FP64 engine: injected device allocation failure");
     if (fault == MQ_FAULT_LAUNCH) return fail(e, MQ_ERR_CUDA, "FP64 engine: injected kernel launch failure");
-    // every ion times out at max_steps, so ceil(min(max_more, max_steps) / chunk) launches finish
-    // every ion; one more is allowed before the watchdog calls it
+    // every ion times out at max_steps, so min(max_more, max_steps) steps finish every ion; one more
+    // chunk is allowed before the watchdog calls it
     const uint64_t need = max_more < b.max_steps ? (uint64_t)max_more : (uint64_t)b.max_steps;
-    const uint64_t max_launches = fault == MQ_FAULT_LAUNCH_BUDGET ? 1 : (need + kF64Chunk - 1) / kF64Chunk + 1;
     const uint32_t chunk = fault == MQ_FAULT_LAUNCH_BUDGET ? 16u : kF64Chunk;
+    uint64_t allowed = fault == MQ_FAULT_LAUNCH_BUDGET ? chunk : need + chunk;
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->dev), "device attributes");
     CK(e->misc.grow(256 + sizeof(uint2) * (size_t)mqd::f64_hand_entries(sms)), "counters");
@@ -326,10 +326,11 @@ mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_
     float step_ms = 0.0f;
     for (;;) {
         uint32_t L = budget < chunk ? (uint32_t)budget : chunk;
-        if (L == 0 || launches >= max_launches) break;
+        if (L > allowed) L = (uint32_t)allowed;
+        if (L == 0) break;
         CK(cudaEventRecord(e->ev[2], e->st), "event");
-        CK(mqd::launch_f64_step(dev_grid(e), b, e->jobc.as<JobC>(), rf_tab, ac_tab, tlen, dev_ions(e, n), (uint32_t)n, L,
-                                ctr, hand, e->st, &kernels), "FP64 step kernel");
+        CK(mqd::launch_f64_step(dev_grid(e), b, e->jobc.as<JobC>(), rf_tab, ac_tab, tlen, dev_ions(e, n), (uint32_t)n,
+                                launches ? live : (uint32_t)n, &L, ctr, hand, e->st, &kernels), "FP64 step kernel");
         CK(cudaEventRecord(e->ev[3], e->st), "event");
         live = 0;
         CK(cudaMemcpyAsync(&live, &ctr->live, 4, cudaMemcpyDeviceToHost, e->st), "live count");
@@ -339,6 +340,7 @@ mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_
         step_ms += ms;
         ++launches;
         budget -= L;
+        allowed -= L;
         if (live == 0) break;
     }
     unsigned long long steps = 0;

@@ -75,6 +75,7 @@ __device__ __forceinline__ void table_get(const double2* t, uint32_t tlen, doubl
 constexpr int kBlock = 256;            // 8 warps: two per scheduler, one to fill the other's gaps
 constexpr int kPad = 120 * 1024;       // dynamic shared memory asked for, unused
 constexpr uint32_t kPollSteps = 32;    // steps between looks at the count of open ions
+constexpr uint32_t kLaneRound = 1024;  // steps of one launch of the one-lane kernel
 
 // Shared memory of a group, in doubles: the fractions of the three axes as pairs {1 - t, t}, the
 // products of the nine sums (rows of 8 corners, 10 apart: 16-byte reads of the rows meet no bank
@@ -475,6 +476,144 @@ k_f64_step(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __r
     }
 }
 
+// ---------------------------------------------------------------- one lane per ion
+// For long lists with legacy collisions, which come every few steps: with eight ions to a warp some ion has one on
+// nearly every step and the warp pays its hundred FP64 operations for that ion alone, with 32 ions it pays them
+// once for all that have one. Bound by the FP64 pipe like the groups: 15.7 us a step for up to 128 ions per SM, 13.8 for each
+// further 128 (0.1 mm channel), whether they live or not, where the groups take 1.1 to 1.4 us for each
+// thousand live ones (launch_f64_step has the rule). Every operation is that of the groups, in its order. One kernel of
+// this form stepped all FP64 ions before the groups came.
+// f32 -> f64 as mqp::widen_normal, other values included: as a branch, since a selected conversion is paid on every value
+// (26,000 ions, 2,000 steps 66.6 -> 57.2 ms)
+__device__ __forceinline__ double widen(float f) {
+    const uint32_t u = __float_as_uint(f);
+    const uint32_t e = (u >> 23) & 0xFFu;
+    if (e - 1u >= 0xFEu && (u & 0x7FFFFFFFu) != 0u) return (double)f;
+    const uint32_t sign = u & 0x80000000u;
+    const uint32_t hi = (u & 0x7FFFFFFFu) ? (sign | ((e + 896u) << 20) | ((u & 0x7FFFFFu) >> 3)) : sign;
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+__global__ void __launch_bounds__(128)
+k_f64_lane(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __restrict__ rf_tab, const double2* __restrict__ ac_tab,
+           uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more, F64Ctrs* __restrict__ ctr) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t done = 0;
+    int32_t status = 1;
+    if (i < n && io.status[i] == 0) {
+        const JobC jc = jobs[io.jid[i]];
+        const double2* tac = ac_tab + (size_t)jc.tab * tlen;
+        double x[3] = {io.x[i], io.y[i], io.z[i]};
+        double v[3] = {io.vx[i], io.vy[i], io.vz[i]};
+        uint64_t rng = io.rng[i];
+        uint32_t age = io.steps[i], ncoll = io.ncoll[i];
+        int32_t leg = io.leg[i];
+        status = 0;
+        double rs, rc, as_, ac;
+        mqp::sincos2pi(io.ph_rf[i], &rs, &rc);
+        mqp::sincos2pi(io.ph_ac[i], &as_, &ac);
+        const double dt = b.dt, qmdt = jc.qmdt, h = g.h;
+        const int32_t nn[3] = {g.nx, g.ny, g.nz};
+        const long long top[3] = {__double_as_longlong((double)(g.nx - 2)), __double_as_longlong((double)(g.ny - 2)),
+                                  __double_as_longlong((double)(g.nz - 2))};
+        const size_t nx = (size_t)g.nx, ny = (size_t)g.ny;
+        // the cell of the position and its fractions
+        double t[3];
+        int32_t c[3];
+        auto locate = [&]() {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double gx = mqp::div_rn(x[d], h, g.inv_h);
+                c[d] = cell_lo_bits(gx, nn[d], top[d]);
+                t[d] = gx - i2d_bits(c[d]);
+            }
+        };
+        auto node = [&](int32_t ci, int32_t cj, int32_t ck) {
+            const size_t q = (size_t)ci + nx * ((size_t)cj + ny * (size_t)ck);
+            return (size_t)MQ_CHK(q, nx * ny * (size_t)g.nz, MQ_SITE_F64_FIELD);
+        };
+        locate();
+        while (done < max_more) {
+            double S, Cc, Sa = 0.0, Ca = 0.0;
+            table_get(rf_tab, tlen, b.w_rf, age, &S, &Cc);
+            const double srf = b.v_rf * (S * rc + Cc * rs);
+            double sac = 0.0;
+            if (jc.use_ac) {
+                table_get(tac, tlen, jc.w_ac, age, &Sa, &Ca);
+                sac = jc.v_ac * (Sa * ac + Ca * as_);
+            }
+            // fields_at: one pass over the 8 corners, weights (1-t, t) in order i, j, k
+            if (b.nearest) t[0] = t[1] = t[2] = 0.0;
+            double er[3] = {0.0, 0.0, 0.0}, ea[3] = {0.0, 0.0, 0.0}, ed[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int di = k >> 2, dj = (k >> 1) & 1, dk = k & 1;
+                const double w = (di ? t[0] : 1.0 - t[0]) * (dj ? t[1] : 1.0 - t[1]) * (dk ? t[2] : 1.0 - t[2]);
+                const size_t q = node(c[0] + di, c[1] + dj, c[2] + dk);
+                const float4 r = __ldg(g.rf + q), a = __ldg(g.ac + q), o = __ldg(g.dc + q);
+                er[0] += w * widen(r.x); er[1] += w * widen(r.y); er[2] += w * widen(r.z);
+                ea[0] += w * widen(a.x); ea[1] += w * widen(a.y); ea[2] += w * widen(a.z);
+                ed[0] += w * widen(o.x); ed[1] += w * widen(o.y); ed[2] += w * widen(o.z);
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                v[d] += qmdt * (srf * er[d] + sac * ea[d] + ed[d]);
+                x[d] += v[d] * dt;
+            }
+            age += 1;
+            done += 1;
+            leg -= 1;
+            if (leg <= 0) {
+                const double vm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+                if (vm > jc.floor_v) {
+                    const double cth = 2.0 * mqp::xs_next(&rng) - 1.0;
+                    double sp, cp;
+                    mqp::sincos2pi(mqp::xs_next(&rng), &sp, &cp);
+                    const double omc = 1.0 - cth * cth;
+                    const double sn = sqrt(omc > 0.0 ? omc : 0.0);
+                    const double dd[3] = {sn * cp, sn * sp, cth};
+                    const double k1 = 1.0 - jc.mr, k2 = jc.mr * vm;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) v[d] = v[d] * k1 + k2 * dd[d];
+                    ncoll += 1;
+                }
+                const double u = mqp::xs_next(&rng);
+                const double mfp = -mqp::log_(u > 1e-7 ? u : 1e-7) * jc.mfp_mean;
+                const double vn = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+                double st = floor(mfp / (vn > 1e-3 ? vn : 1e-3) / dt);
+                if (st < 1.0) st = 1.0;
+                leg = !(st < 2147483647.0) ? 2147483647 : (int32_t)st;
+            }
+            const long long bx = __double_as_longlong(x[0]), by = __double_as_longlong(x[1]), bz = __double_as_longlong(x[2]);
+            if (gt_pos(bz, __double_as_longlong(b.z_exit))) status = 3;
+            else if (lt_pos(bz, __double_as_longlong(b.z_return))) status = 2;
+            else if (lt_zero(bx) || lt_zero(by) || lt_zero(bz) || gt_pos(bx, __double_as_longlong(b.lim[0])) ||
+                     gt_pos(by, __double_as_longlong(b.lim[1])) || gt_pos(bz, __double_as_longlong(b.lim[2])))
+                status = 4;
+            else {
+                locate();
+                if (x[2] > b.crash_z0 && x[2] < b.crash_z1) {   // the nearest node is a conductor
+                    const size_t q = node(c[0] + (t[0] >= 0.5), c[1] + (t[1] >= 0.5), c[2] + (t[2] >= 0.5));
+                    if (__ldg(&g.rf[q].w) > 0.5f) status = 1;
+                }
+                if (status == 0 && age >= b.max_steps) status = 5;
+            }
+            if (status != 0) break;
+        }
+        io.x[i] = x[0]; io.y[i] = x[1]; io.z[i] = x[2];
+        io.vx[i] = v[0]; io.vy[i] = v[1]; io.vz[i] = v[2];
+        io.rng[i] = rng; io.steps[i] = age; io.ncoll[i] = ncoll; io.leg[i] = leg; io.status[i] = status;
+    }
+    unsigned long long s = done;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(FULL, s, o);
+    const uint32_t live = __popc(__ballot_sync(FULL, status == 0));
+    if ((threadIdx.x & 31) == 0) {
+        if (s) atomicAdd(&ctr->steps, s);
+        if (live) atomicAdd(&ctr->live, live);
+    }
+}
+
 // counters of one round of launches: n open ions, nothing taken or handed on
 __global__ void k_f64_begin(F64Ctrs* ctr, uint32_t n) {
     ctr->live = ctr->head_a = ctr->head_b = ctr->handed = 0;
@@ -526,7 +665,7 @@ cudaError_t launch_inject(const mqp::Batch& b, JobTable jt, DevIons io, uint32_t
 }
 
 cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc, const double2* rf_tab,
-                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more,
+                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t live, uint32_t* steps,
                             F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels) {
     if (n == 0) return cudaSuccess;
     int dev = 0, sms = 0;
@@ -538,7 +677,16 @@ cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc,
     if ((e = cudaFuncSetAttribute(k_f64_step<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPad)) != cudaSuccess) return e;
     k_f64_begin<<<1, 1, 0, s>>>(ctr, n);
     const uint32_t wide = f64_hand_entries(sms);
-    if (n <= wide) {
+    // Legacy collisions: one ion to a lane while more live than 72 per SM for each 128 per SM in the list, looked at
+    // again every kLaneRound steps. 2,000 steps, groups alone / so: 10,000 ions 29 / 29 ms, 15,000 45 / 33, 26,000 76 /
+    // 57, 40,000 109 / 85; 200 steps of 200,000 ions 44 / 30; 40,000 ions to their end (20,000 steps) 745 / 702.
+    const uint64_t waves = ((uint64_t)n + 128u * (uint32_t)sms - 1u) / (128u * (uint32_t)sms);
+    uint32_t max_more = *steps;
+    if (b.legacy_coll && live > 72u * (uint32_t)sms * waves) {
+        *steps = max_more = max_more < kLaneRound ? max_more : kLaneRound;
+        k_f64_lane<<<blocks_for(n, 128), 128, 0, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr);
+        *kernels += 2;
+    } else if (n <= wide) {
         k_f64_step<16><<<sms, kBlock, kPad, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr, nullptr, 0, 0);
         *kernels += 2;
     } else {

@@ -46,8 +46,9 @@ struct F64Ctrs {
 
 // ---- mq_f64.cu
 cudaError_t launch_inject(const mqp::Batch& b, JobTable jt, DevIons io, uint32_t n, cudaStream_t s);
+// One launch over the list's n ions, of which at most `live` live: *steps steps of each, or so many as it leaves there.
 cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc, const double2* rf_tab,
-                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more,
+                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t live, uint32_t* steps,
                             F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels);
 // Ions that the 16-lane groups of one warp per scheduler hold: up to so many, a call steps them in
 // groups of 16 lanes. A larger call starts in groups of 4, which hand over the last so many of their

@@ -152,14 +152,13 @@ extern "C" mq_status mq_run_ions_device_noalloc(const mq_dev_grid* grid, const m
 
     if (cudaMemsetAsync(ctr, 0, sizeof(*ctr), st) != cudaSuccess) return MQ_ERR_CUDA;   // the scratch keeps old values
     uint64_t budget = max_more;
-    uint32_t kernels = 0;
+    uint32_t kernels = 0, live = (uint32_t)n;
     for (;;) {
-        const uint32_t L = budget < kChunk ? (uint32_t)budget : kChunk;
+        uint32_t L = budget < kChunk ? (uint32_t)budget : kChunk;
         if (L == 0) break;
         // no phase tables (length 0): the kernel evaluates every drive phase directly
-        if (mqd::launch_f64_step(g, b, d_jobs, nullptr, nullptr, 0, d, (uint32_t)n, L, ctr, nullptr, st, &kernels) != cudaSuccess)
+        if (mqd::launch_f64_step(g, b, d_jobs, nullptr, nullptr, 0, d, (uint32_t)n, live, &L, ctr, nullptr, st, &kernels) != cudaSuccess)
             return MQ_ERR_CUDA;
-        uint32_t live = 0;
         if (cudaMemcpyAsync(&live, &ctr->live, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
         if (cudaStreamSynchronize(st) != cudaSuccess) return MQ_ERR_CUDA;
         budget -= L;

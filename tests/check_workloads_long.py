@@ -60,7 +60,7 @@ def main():
             e.run_batch([mq.Job(jobs[0].sp, jobs[0].drive, 2048 * 152 + 1, 3)], DC, variants[0])
         out["loads"] = int(e.last_stats.cell_loads)
     with mq.Engine(f, mq.PREC_F64) as e:
-        short = [mq.Job(j.sp, j.drive, 1700, j.seed) for j in jobs]
+        short = [mq.Job(j.sp, j.drive, 4000, j.seed) for j in jobs]   # with legacy collisions one ion to a lane, else in groups
         for ph in variants:
             e.set_dc(DC)
             e.run_ions(short, ph, edges(e.inject(short, ph), f))
