@@ -340,24 +340,33 @@ __global__ void k_tm_store(TMConst C, Tracks64 T, MTracks M, uint32_t n) {
     T.vx[i] = v[0]; T.vy[i] = v[1]; T.vz[i] = v[2];
 }
 
-// group the live tracks by region: list[r * n + k], one warp-aggregated atomic per region group
-__global__ void k_tm_bucket(const int32_t* __restrict__ region, uint32_t n, uint32_t* __restrict__ list,
-                            uint32_t* __restrict__ bcount) {
+// group the live tracks by region: list[r * n + k], one warp-aggregated atomic per region group; and count those of the
+// cube beyond z_near (grid units), which may come to a mouth within the chunk
+__global__ void k_tm_bucket(const int32_t* __restrict__ region, const float* __restrict__ zh, float z_near, uint32_t n,
+                            uint32_t* __restrict__ list, uint32_t* __restrict__ bcount) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = i < n ? region[i] : R_LOST;
     const bool live = r <= R_COMBINE;
     const unsigned lm = __ballot_sync(FULL, live);
     if (!live) return;
+    const unsigned near = __ballot_sync(lm, (r == R_SPLIT || r == R_COMBINE) && zh[i] > z_near);
     const unsigned peers = __match_any_sync(lm, r);
     const int leader = __ffs(peers) - 1;
     const uint32_t lane = threadIdx.x & 31;
+    if (near && (int)lane == __ffs(lm) - 1) atomicAdd(&bcount[kBuckets], (uint32_t)__popc(near));
     uint32_t base = 0;
     if ((int)lane == leader) base = atomicAdd(&bcount[r], (uint32_t)__popc(peers));
     base = __shfl_sync(peers, base, leader);
     list[MQ_CHK((size_t)r * n + base + __popc(peers & ((1u << lane) - 1u)), (size_t)kBuckets * n, MQ_SITE_TMX_LIST)] = i;
 }
 
-// one chunk of global steps for every live track (one thread per track, grouped by region)
+// One chunk of global steps for every live track (one thread per track, grouped by region). Two forms of it are launched, and
+// the census of the chunk says which of them works: CUBE, where next to all tracks are in the cube and stay there, sums
+// two fields in the cube; the other takes the ports' three-field sum with its slots there too, so that
+// warps whose tracks come and go between cube and ports have one way. Both sides, 300 steps of 600,000 tracks: launched
+// through the entrance (none near a mouth) 7.7 / 8.6 ms, from the mouths 5.6 / 5.0; pulse of 262,144 tracks, 1,000 steps 7.4 / 6.7.
+// (Chosen by a vote of the warp on each step, or by warps in one kernel: 7.8 and 7.1, 7.7 and 7.4.)
+template <bool CUBE>
 __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32_t n, const uint32_t* __restrict__ list,
                                                     const uint32_t* __restrict__ bcount, const float* __restrict__ drive,
                                                     uint64_t g0, uint32_t S, uint32_t* __restrict__ counts,
@@ -366,7 +375,8 @@ __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32
     if (threadIdx.x == 0) {
         uint32_t a = 0;
         for (int r = 0; r < kBuckets; ++r) { off[r] = a; a += bcount[r]; }
-        off[kBuckets] = a;
+        const uint32_t abroad = a - bcount[R_SPLIT] - bcount[R_COMBINE] + bcount[kBuckets];   // in a port, or soon
+        off[kBuckets] = ((uint64_t)abroad * 64u <= a) == CUBE ? a : 0u;
     }
     __syncthreads();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -415,15 +425,25 @@ __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32
                 if (cube) {   // fields.rs:89-96 clamps the grid coordinate to the grid
                     tx = __saturatef(tx); ty = __saturatef(ty); tz = __saturatef(tz);
                 }
-                const bool ox = !cube && (c.ci & 1), oy = !cube && (c.cj & 1), oz = !cube && (c.ck & 1);
-                tx = ox ? -tx : tx; ty = oy ? -ty : ty; tz = oz ? -tz : tz;
-                const float ac = cube ? 0.0f : __ldg(dr + reg);
+                if (CUBE && cube) {
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    float F[8];
+                    for (int d = 0; d < 3; ++d) {
+                        float F[8];
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) F[q] = fmaf(rf, c.R[d][q], fmaf(ac, c.A[d][q], c.D[d][q]));
-                    E[d] = lerp3(F, tx, ty, tz, ox, oy, oz);
+                        for (int q = 0; q < 8; ++q) F[q] = fmaf(rf, c.R[d][q], c.D[d][q]);
+                        E[d] = lerp3(F, tx, ty, tz, false, false, false);
+                    }
+                } else {
+                    const bool ox = !cube && (c.ci & 1), oy = !cube && (c.cj & 1), oz = !cube && (c.ck & 1);
+                    tx = ox ? -tx : tx; ty = oy ? -ty : ty; tz = oz ? -tz : tz;
+                    const float ac = cube ? 0.0f : __ldg(dr + reg);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        float F[8];
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) F[q] = fmaf(rf, c.R[d][q], fmaf(ac, c.A[d][q], c.D[d][q]));
+                        E[d] = lerp3(F, tx, ty, tz, ox, oy, oz);
+                    }
                 }
             }
             if (cube) ++n_cube;
@@ -784,7 +804,7 @@ State* create(const mq_tandem_desc& d, const DevFields& f, cudaStream_t st, std:
         C.nsd[k] = (float)(ngas * d.species[k].ccs * 1e-20 * d.dt);
         C.mr[k] = (float)(mg / (m + mg));
     }
-    if ((e = cudaMalloc(&s->bcount, kBuckets * sizeof(uint32_t))) != cudaSuccess) return fail("bucket counters", e);
+    if ((e = cudaMalloc(&s->bcount, (kBuckets + 1) * sizeof(uint32_t))) != cudaSuccess) return fail("bucket counters", e);
     return s;
 }
 
@@ -835,12 +855,15 @@ cudaError_t run(State* s, uint32_t n, const float* drive, uint64_t step0, uint64
     cudaError_t e;
     if (!n) return cudaSuccess;
     const unsigned grid = (n + 127) / 128;
+    // 8 mm, as far as thermal ions of these masses come in a chunk
+    const float z_near = (s->C.seam_mm - 8.0f - s->C.clo[2]) / s->C.ch;
     for (uint64_t q = 0; q < k; q += kChunk) {
         const uint32_t S = (uint32_t)(k - q < kChunk ? k - q : kChunk);
-        if ((e = cudaMemsetAsync(s->bcount, 0, kBuckets * sizeof(uint32_t), st)) != cudaSuccess) return e;
-        k_tm_bucket<<<grid, 128, 0, st>>>(s->M.region, n, s->list, s->bcount);
-        k_tm_step<<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc);
-        *launches += 2;
+        if ((e = cudaMemsetAsync(s->bcount, 0, (kBuckets + 1) * sizeof(uint32_t), st)) != cudaSuccess) return e;
+        k_tm_bucket<<<grid, 128, 0, st>>>(s->M.region, s->M.xh + 2 * (size_t)n, z_near, n, s->list, s->bcount);
+        k_tm_step<false><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc);
+        k_tm_step<true><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc);
+        *launches += 3;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;
