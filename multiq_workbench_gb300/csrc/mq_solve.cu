@@ -745,10 +745,14 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
         const DLevel &f = P.L[l - 1], &c = P.L[l];
         k_coarse_fix<<<plane_blocks((size_t)c.nx * c.ny, c.nz), kT, 0, st>>>(f.fix, f.nx, f.ny, f.nz, c.fix, c.nx, c.ny, c.nz);
     }
+    // the levels from `low` on run in one block
+    size_t low = P.L.size(), nodes = 0;
+    while (low > 0 && P.L.size() - low < (size_t)kBottomLevels && nodes + P.L[low - 1].n() <= (size_t)kBottomNodes) nodes += P.L[--low].n();
+    // lists for the levels that have kernels of their own, and for the first below, whose right-hand side these form
     std::vector<uint32_t> cnts(2 * P.L.size(), 0u);
-    if (P.lists) {
+    if (P.lists && low > 0) {
         if (cudaMemsetAsync(P.cnts, 0, cnts.size() * sizeof(uint32_t), st) != cudaSuccess) return MQ_ERR_CUDA;
-        for (size_t l = 0; l < P.L.size(); ++l)
+        for (size_t l = 0; l < P.L.size() && l <= low; ++l)
             for (int c = 0; c < 2; ++c) {
                 const DLevel& v = P.L[l];
                 k_list<<<plane_blocks((size_t)((v.nx - 1) / 2) * (v.ny - 2), v.nz - 2), kT, 0, st>>>(v.fix, v.nx, v.ny, v.nz, c, v.list[c],
@@ -763,9 +767,6 @@ mq_status solve(Problem& P, double outer_bc, double tol, int device, cudaStream_
     if (!(scale > 0)) scale = 1.0;
     const double target = tol * scale;
 
-    // the levels from `low` on run in one block
-    size_t low = P.L.size(), nodes = 0;
-    while (low > 0 && P.L.size() - low < (size_t)kBottomLevels && nodes + P.L[low - 1].n() <= (size_t)kBottomNodes) nodes += P.L[--low].n();
     Bottom B{};
     for (size_t l = low; l < P.L.size(); ++l) {
         const int x = B.levels++;
