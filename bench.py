@@ -155,7 +155,7 @@ def run_gridstudy(args, rank: int, world: int):
         t_solve = time.perf_counter() - t0
         with mq.Engine(f, mq.PREC_MIXED, device=local) as eng:
             apply_tuning(eng, args)
-            tuned = {**eng.tuning(), "blocks_launched": eng.blocks_per_sm(n)}   # the default launch shape
+            tuned = {**eng.tuning(), "blocks_launched": eng.blocks_per_sm(n, ph)}   # the default launch shape
             for _ in range(args.warmup):
                 eng.run_batch(table, dc, ph)
             if h == spacings[-1]:
@@ -885,7 +885,7 @@ def main():
                                        f"({len(jobs) * args.ions_per_job:,} ions), "
                                        "0.100 mm channel grid 160x160x242, legacy half-kick, <=20000 steps",
                            "jobs": len(jobs), "ions": sum(j.n for j in jobs), "l2_flush": "256 MB write before every timed step",
-                           "tuning": {**(tuned or eng.tuning()), "blocks_launched": eng.blocks_per_sm(sum(j.n for j in jobs)),
+                           "tuning": {**(tuned or eng.tuning()), "blocks_launched": eng.blocks_per_sm(sum(j.n for j in jobs), ph),
                                       "use_graph": replays > 0,
                                       "graph_replays_per_step": replays / args.steps,
                                       "step_launches_per_step": step_launches / args.steps}},

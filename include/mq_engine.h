@@ -134,7 +134,9 @@ uint64_t    mq_fnv1a64(const void* data, size_t bytes, uint64_t h);
 typedef struct mq_tuning {
     int32_t threads_per_block;   /* fixed at 128                                          */
     int32_t blocks_per_sm;       /* resident blocks per SM of the persistent grid, 1..3; 3 with
-                                    48-byte records are the two that fit.  Set: 0 leaves them as
+                                    48-byte records and thermal collisions are the two that fit,
+                                    and with nearest-node fields any number is what fits.  Set: 0
+                                    leaves them as
                                     they are.  An engine that was given none chooses for each
                                     call by the grid and the number of ions (mq_engine_blocks);
                                     what get_tuning says then is its class of grid, 3 below
@@ -149,9 +151,9 @@ typedef struct mq_tuning {
 } mq_tuning;
 mq_status   mq_engine_get_tuning(mq_engine* e, mq_tuning* t);
 mq_status   mq_engine_set_tuning(mq_engine* e, const mq_tuning* t);
-/* Blocks per SM that a call over `ions` live ions launches with the engine's present tuning and
- * trilinear fields; 0 where the ions are so few that the lane groups take them alone. */
-mq_status   mq_engine_blocks(mq_engine* e, uint64_t ions, int32_t* blocks);
+/* Blocks per SM that a call over `ions` live ions with this physics launches with the engine's
+ * present tuning; 0 where the ions are so few that the lane groups take them alone. */
+mq_status   mq_engine_blocks(mq_engine* e, const mq_physics* ph, uint64_t ions, int32_t* blocks);
 /* Autotuner: times every candidate shape on a sample of the batch (the first
  * sample_per_job ions of each job), keeps the fastest as the engine's tuning and returns
  * it with its rate in ion-steps/s.  The present shape stays unless another is faster by more than

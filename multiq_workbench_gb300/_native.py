@@ -327,7 +327,7 @@ def _declare_engine(L) -> None:
     L.mq_engine_get_tuning.restype = C.c_int32
     L.mq_engine_set_tuning.argtypes = [C.c_void_p, P(mq_tuning)]
     L.mq_engine_set_tuning.restype = C.c_int32
-    L.mq_engine_blocks.argtypes = [C.c_void_p, C.c_uint64, P(C.c_int32)]
+    L.mq_engine_blocks.argtypes = [C.c_void_p, P(mq_physics), C.c_uint64, P(C.c_int32)]
     L.mq_engine_blocks.restype = C.c_int32
     L.mq_engine_autotune.argtypes = [C.c_void_p, P(mq_job), C.c_size_t, P(C.c_double), P(mq_physics), C.c_uint64,
                                      P(mq_tuning), P(C.c_double)]

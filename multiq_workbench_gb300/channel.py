@@ -366,11 +366,12 @@ class Engine:
                         int(sort_cells if sort_cells is not None else cur["sort_cells"]))
         N.check(N.lib().mq_engine_set_tuning(self._h, C.byref(t)), "mq_engine_set_tuning", self._h)
 
-    def blocks_per_sm(self, ions: int) -> int:
-        """Blocks per SM that a call over so many live ions launches (trilinear fields); 0 where the lane
-        groups take them alone."""
+    def blocks_per_sm(self, ions: int, ph: Physics | None = None) -> int:
+        """Blocks per SM that a call over so many live ions launches (``ph``: trilinear fields and thermal
+        collisions if not given); 0 where the lane groups take them alone."""
         b = C.c_int32(0)
-        N.check(N.lib().mq_engine_blocks(self._h, int(ions), C.byref(b)), "mq_engine_blocks", self._h)
+        N.check(N.lib().mq_engine_blocks(self._h, C.byref((ph or Physics()).native()), int(ions), C.byref(b)), "mq_engine_blocks",
+                self._h)
         return int(b.value)
 
     def autotune(self, jobs, dc, ph: Physics, sample_per_job: int = 2048) -> tuple[dict, float]:

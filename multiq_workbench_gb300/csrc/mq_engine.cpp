@@ -667,10 +667,12 @@ mq_status mq_engine_set_tuning(mq_engine* e, const mq_tuning* t) {
     return MQ_OK;
 }
 
-mq_status mq_engine_blocks(mq_engine* e, uint64_t ions, int32_t* blocks) {
-    if (!e || !blocks) return MQ_ERR_INVALID;
+mq_status mq_engine_blocks(mq_engine* e, const mq_physics* ph, uint64_t ions, int32_t* blocks) {
+    if (!e || !ph || !blocks) return MQ_ERR_INVALID;
     if (e->prec != MQ_PREC_MIXED) return fail(e, MQ_ERR_INVALID, "the mixed engine has a launch shape");
-    *blocks = ions > mqmix::group_ions(e->tune, false) ? mqmix::resident_blocks(e->tune, e->nnodes, (size_t)ions) : 0;
+    if (cudaSetDevice(e->dev) != cudaSuccess) return fail(e, MQ_ERR_CUDA, "cudaSetDevice");
+    const bool legacy = ph->legacy_collisions != 0, nearest = ph->legacy_fields != 0;
+    *blocks = ions > mqmix::group_ions(e->tune, nearest) ? mqmix::resident_blocks(e->tune, e->nnodes, (size_t)ions, legacy, nearest) : 0;
     return MQ_OK;
 }
 
@@ -774,7 +776,7 @@ mq_status mq_engine_autotune(mq_engine* e, const mq_job* jobs, size_t njobs, con
                     t.chunk = ch;
                     t.auto_blocks = bl == 0;
                     t.blocks_per_sm = bl ? bl : base;
-                    const int runs = mqmix::resident_blocks(t, e->nnodes, n);
+                    const int runs = mqmix::resident_blocks(t, e->nnodes, n, ph->legacy_collisions != 0, false);
                     if (s == MQ_OK && (bl ? runs == bl : runs > 3)) s = time(t);
                 }
     }

@@ -1387,15 +1387,6 @@ Tuning default_tuning(int device, size_t nodes) {
     return t;
 }
 
-int resident_blocks(const Tuning& t, size_t nodes, size_t n) {
-    constexpr int kNarrow = 2;   // what the narrow kernel's registers leave room for
-    if (!t.auto_blocks) return t.wide || t.blocks_per_sm < kNarrow ? t.blocks_per_sm : kNarrow;
-    if (!t.wide) return 48.0 * (double)nodes < 3.5e9 ? kNarrow : 1;   // default_tuning has the figures
-    // three with wide records are four for a list of eight or more ions a lane, which outlasts its uneven end:
-    // 1,280,000 ions 22.1 -> 21.1 ms, 640,000 13.6 -> 13.2, 320,000 the same, 62,000 (S14 sweep) 39.0 -> 40.4
-    return t.blocks_per_sm == 3 && n > 2048 * (size_t)t.sms ? 4 : t.blocks_per_sm;
-}
-
 // Ions that the lane groups hold at once: a list of up to so many is stepped by them alone, a longer
 // one's last so many are handed to them.
 static uint32_t hand_entries(int sms, bool nearest) { return (uint32_t)sms * (uint32_t)(group_block(nearest) / 4); }
@@ -1427,21 +1418,41 @@ void release(Scratch& s) {
 // the stepping kernel for the batch's physics and the tuning (the nearest-node field mode reads one
 // record per fill, so the L1 prefetch of the next cell does not apply to it)
 typedef decltype(&k_mixed<true, true, true, false, 3>) Kernel;
-static Kernel pick_kernel(const Tuning& t, const MixBatch& mb, int blocks) {
-    if (mb.nearest) {
-        if (mb.legacy_coll) return t.wide ? k_mixed<true, false, true, true, 5> : k_mixed<true, false, false, true, 5>;
+static Kernel pick_kernel(const Tuning& t, bool legacy, bool nearest, int blocks) {
+    if (nearest) {
+        if (legacy) return t.wide ? k_mixed<true, false, true, true, 5> : k_mixed<true, false, false, true, 5>;
         return t.wide ? k_mixed<false, false, true, true, 5> : k_mixed<false, false, false, true, 5>;
     }
     if (t.wide && blocks == 4) {
-        if (mb.legacy_coll) return t.prefetch ? k_mixed<true, true, true, false, 4> : k_mixed<true, false, true, false, 4>;
+        if (legacy) return t.prefetch ? k_mixed<true, true, true, false, 4> : k_mixed<true, false, true, false, 4>;
         return t.prefetch ? k_mixed<false, true, true, false, 4> : k_mixed<false, false, true, false, 4>;
     }
-    if (mb.legacy_coll) {
+    if (legacy) {
         if (t.wide) return t.prefetch ? k_mixed<true, true, true, false, 3> : k_mixed<true, false, true, false, 3>;
+        if (blocks == 3) return t.prefetch ? k_mixed<true, true, false, false, 3> : k_mixed<true, false, false, false, 3>;
         return t.prefetch ? k_mixed<true, true, false, false, 2> : k_mixed<true, false, false, false, 2>;
     }
     if (t.wide) return t.prefetch ? k_mixed<false, true, true, false, 3> : k_mixed<false, false, true, false, 3>;
     return t.prefetch ? k_mixed<false, true, false, false, 2> : k_mixed<false, false, false, false, 2>;
+}
+
+int resident_blocks(const Tuning& t, size_t nodes, size_t n, bool legacy, bool nearest) {
+    if (nearest) {   // no 8-corner cache (about 100 registers instead of 167): as many blocks as fit
+        int nb = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_kernel(t, legacy, true, 0), t.tpb, 0) == cudaSuccess && nb > 0) return nb;
+        cudaGetLastError();
+        return t.blocks_per_sm;
+    }
+    // What the narrow kernels' registers leave room for: three with legacy collisions, cut to 168 registers without spills, two
+    // with thermal ones. Three are worth it on small grids for more ions than two hold: legacy collisions, 3,000 steps at 2 / 3
+    // blocks, 0.100 mm 30,000 ions 3.6 / 4.1 ms, 40,000 4.9 / 4.2, 80,000 8.6 / 7.9, 400,000 38.8 / 32.3; 0.050 mm 400,000 52.5 / 54.2.
+    const int narrow = legacy ? 3 : 2;
+    if (!t.auto_blocks) return t.wide || t.blocks_per_sm < narrow ? t.blocks_per_sm : narrow;
+    if (!t.wide && legacy && t.blocks_per_sm == 3 && n > 256 * (size_t)t.sms) return 3;
+    if (!t.wide) return 48.0 * (double)nodes < 3.5e9 ? 2 : 1;   // default_tuning has the figures
+    // three with wide records are four for a list of eight or more ions a lane, which outlasts its uneven end:
+    // 1,280,000 ions 22.1 -> 21.1 ms, 640,000 13.6 -> 13.2, 320,000 the same, 62,000 (S14 sweep) 39.0 -> 40.4
+    return t.blocks_per_sm == 3 && n > 2048 * (size_t)t.sms ? 4 : t.blocks_per_sm;
 }
 
 typedef decltype(&k_mixed_group<true, true, false>) GroupKernel;
@@ -1509,7 +1520,7 @@ static cudaError_t enqueue_launches(const Scratch& s, const Tuning& t, int block
             li = sorted;
             *kernels += 5;
         }
-        const Kernel kern = pick_kernel(t, mb, blocks_per_sm);
+        const Kernel kern = pick_kernel(t, mb.legacy_coll != 0, mb.nearest != 0, blocks_per_sm);
         const uint32_t hand_at = hand_entries(t.sms, mb.nearest != 0);
         uint2* hand = reinterpret_cast<uint2*>(ctr + 1);
         if (n > hand_at) {
@@ -1603,16 +1614,7 @@ cudaError_t run(Scratch& s, const Tuning& t, DevGrid g, uint64_t grid_gen, const
     k_init_list<<<(n + 255) / 256, 256, 0, st>>>(io, n, static_cast<uint32_t*>(s.lists), ctr, mb, keep, kph, staged);
     info->kernel_launches += 1;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // resident blocks per SM: the tuning's, except for the nearest-node kernels, which hold no
-    // 8-corner cache (about 100 registers instead of 167) and run as many blocks as fit
-    int blocks = resident_blocks(t, (size_t)mb.nx * mb.ny * mb.nz, n);
-    if (mb.nearest) {
-        int nb = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_kernel(t, mb, 0), t.tpb, 0) == cudaSuccess && nb > 0)
-            blocks = nb;
-        else
-            cudaGetLastError();
-    }
+    const int blocks = resident_blocks(t, (size_t)mb.nx * mb.ny * mb.nz, n, mb.legacy_coll != 0, mb.nearest != 0);
     cudaEventRecord(s.ev[0], st);
     uint32_t kernels = 0;
     const bool graph = t.use_graph && launches > 1;

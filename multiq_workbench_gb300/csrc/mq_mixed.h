@@ -89,8 +89,8 @@ MixBatch make_mix_batch(const mqp::Batch& b);
 // device injection of a batch for the mixed engine: the FP64 injection's draws with FP32 transforms
 cudaError_t launch_inject(const mqp::Batch& b, mqd::JobTable jt, mqd::DevIons io, uint32_t n, cudaStream_t st);
 Tuning default_tuning(int device, size_t nodes);
-// Blocks per SM that run() launches k_mixed with for n ions on a grid of so many nodes (trilinear fields)
-int resident_blocks(const Tuning& t, size_t nodes, size_t n);
+// Blocks per SM that run() launches k_mixed with for n ions on a grid of so many nodes
+int resident_blocks(const Tuning& t, size_t nodes, size_t n, bool legacy, bool nearest);
 // Ions up to which a call runs in lane groups alone
 uint32_t group_ions(const Tuning& t, bool nearest);
 // write_states = 0 leaves the FP64 position / velocity of the ion states as they were (a caller

@@ -20,20 +20,25 @@ def _jobs(n, k=1):
     return [mq.Job(mq.Species(499.0, 1.0, 2.95 * 499.0 ** (2 / 3)), mq.RfAc(100.0, 500e3, 0.5, 100e3), n, 5 + s) for s in range(k)]
 
 
-def test_given_blocks_run_and_the_engines_choice_stays(coarse):
+@pytest.mark.parametrize("name, narrow", [("half_kick_gauss", 2), ("legacy_coll_trilinear", 3)])
+def test_given_blocks_run_and_the_engines_choice_stays(coarse, name, narrow):
     mq = _mq()
+    ph = _variants()[name]
     with mq.Engine(coarse, mq.PREC_MIXED) as e:
-        assert [e.blocks_per_sm(n) for n in (1000, 60000, LONG)] == [0, 3, 4]
+        def runs(*ions):
+            return [e.blocks_per_sm(n, ph) for n in ions]
+        assert runs(1000, 60000, LONG) == [0, 3, 4]
         e.set_tuning(chunk=301, use_graph=False)
-        assert e.tuning()["blocks_per_sm"] == 3 and e.blocks_per_sm(LONG) == 4
+        assert e.tuning()["blocks_per_sm"] == 3 and runs(LONG) == [4]
         e.set_tuning(wide_records=False)          # what fits of the narrow kernel
-        assert e.blocks_per_sm(60000) == 2 and e.blocks_per_sm(LONG) == 2
-        for wide, want in ((False, {1: 1, 2: 2, 3: 2}), (True, {1: 1, 2: 2, 3: 3})):
-            for b, w in want.items():
+        assert runs(256 * 152, 60000, LONG) == [2, narrow, narrow]
+        for wide, most in ((False, narrow), (True, 3)):
+            for b in (1, 2, 3):
                 e.set_tuning(blocks_per_sm=b, wide_records=wide)
                 assert e.tuning()["blocks_per_sm"] == b
                 e.set_tuning(chunk=400)
-                assert [e.blocks_per_sm(n) for n in (60000, LONG)] == [w, w], (wide, b)
+                assert runs(60000, LONG) == [min(b, most)] * 2, (wide, b)
+        assert e.blocks_per_sm(60000, _variants()["legacy_all"]) > 3   # nearest-node fields: as many as fit
         for b in (0, 4, 9, -1):
             with pytest.raises(mq.MqError):
                 e.set_tuning(blocks_per_sm=b)
@@ -41,9 +46,10 @@ def test_given_blocks_run_and_the_engines_choice_stays(coarse):
         e.blocks_per_sm(1000)
 
 
-def test_any_shape_gives_the_same_ions(coarse):
+@pytest.mark.parametrize("name", ["half_kick_gauss", "legacy_coll_trilinear"])
+def test_any_shape_gives_the_same_ions(coarse, name):
     mq = _mq()
-    ph = _variants()["half_kick_gauss"]
+    ph = _variants()[name]
     with mq.Engine(coarse, mq.PREC_MIXED) as e:
         want, _ = e.run_batch_ions(_jobs(LONG), DC, ph)
         rate = {}
