@@ -46,6 +46,8 @@ __device__ __forceinline__ long long order_key(long long b) {
     if (b == (long long)0x8000000000000000ULL) b = 0;
     return b < 0 ? (long long)(0x8000000000000000ULL - (unsigned long long)b) : b;
 }
+// x > c, c given by its key
+__device__ __forceinline__ bool gt_key(long long x, long long key) { return !is_nan_bits(x) && order_key(x) > key; }
 // FP32 upper bound of |v| from the high word of a double; from 2^127 on (infinities and NaN too) a
 // value whose square overflows
 __device__ __forceinline__ float mag_up(double v) {

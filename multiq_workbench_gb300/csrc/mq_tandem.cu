@@ -42,7 +42,9 @@ struct TPort {                  // one port's channel grid and drive
 // Cube geometry in FP32 (mm, growth 0), for the filter that settles all but the points near a surface
 struct CubeF {
     float size, c0, pitch, half_d, t_pcb, gap, ptd, stem_r, clear_r, rod_hole, l_ext, cap_reach, cap_r, ap_r;
-    float near, round_max;   // distances [mm] closer than this, and fractions beyond this, are left to the exact test
+    float ent_b, ent_c;      // entrance axis: along z, along x
+    float near;              // distances [mm] closer than this are left to the exact test,
+    float round_port, round_post;   // and fractions beyond these
     int32_t n, array, ent_axis, ent_side, ent_cell0, ent_cell1, ext_axis, ext_side, ext_cell0, ext_cell1;
 };
 
@@ -77,9 +79,9 @@ __device__ __forceinline__ bool below(const CubeF& G, float v, float t, bool& un
     return v < t;
 }
 // v.round() clamped to [0, hi]
-__device__ __forceinline__ int round_near(const CubeF& G, float v, int hi, bool& unsure) {
+__device__ __forceinline__ int round_near(float v, int hi, float most, bool& unsure) {
     const float r = rintf(v);
-    unsure |= !(fabsf(v - r) <= G.round_max);
+    unsure |= !(fabsf(v - r) <= most);
     return r > 0.0f ? (r < (float)hi ? (int)r : hi) : 0;
 }
 // mqc::classify (geometry.rs:136-205) for one face (axis a, side) of the point: does the point lie in
@@ -92,8 +94,8 @@ __device__ bool face_solid(const CubeF& G, int a, int side, float u, float pb, f
         pc0 = G.ext_cell0; pc1 = G.ext_cell1;
         if (G.array) {
             const float first = 0.5f * (latf(G, 2) + latf(G, 3));
-            pc0 = 2 + 2 * round_near(G, (pb - first) / (2.0f * G.pitch), 2, unsure);
-            pc1 = 2 + 2 * round_near(G, (pc - first) / (2.0f * G.pitch), 2, unsure);
+            pc0 = 2 + 2 * round_near((pb - first) / (2.0f * G.pitch), 2, G.round_port, unsure);
+            pc1 = 2 + 2 * round_near((pc - first) / (2.0f * G.pitch), 2, G.round_port, unsure);
         }
     }
     const float axis_d = hypf2(pb - 0.5f * (latf(G, pc0) + latf(G, pc0 + 1)), pc - 0.5f * (latf(G, pc1) + latf(G, pc1 + 1)));
@@ -107,7 +109,8 @@ __device__ bool face_solid(const CubeF& G, int a, int side, float u, float pb, f
         return hit;
     }
     if (!inside || !below(G, u, G.ptd, unsure)) return false;
-    const int ib = round_near(G, (pb - G.c0) / G.pitch, G.n - 1, unsure), ic = round_near(G, (pc - G.c0) / G.pitch, G.n - 1, unsure);
+    const int ib = round_near((pb - G.c0) / G.pitch, G.n - 1, G.round_post, unsure);
+    const int ic = round_near((pc - G.c0) / G.pitch, G.n - 1, G.round_post, unsure);
     const bool rim_b = ib == 0 || ib == G.n - 1, rim_c = ic == 0 || ic == G.n - 1;
     const bool valid = a == 0 ? !rim_b && !rim_c : a == 1 ? !rim_b : true;   // post_valid, geometry.rs:81-86
     const float dd = hypf2(pb - latf(G, ib), pc - latf(G, ic));
@@ -201,6 +204,10 @@ k_tandem(const __grid_constant__ TConst C, Tracks T, uint32_t n, const double* _
     double gh = 1.0, ginv = 1.0, glim = 0.0;   // grid spacing, its reciprocal, box limit along the axis (port)
     size_t nx = 2, ny = 2;
     const float4 *p_rf = nullptr, *p_ac = nullptr, *p_dc = nullptr, *p_gate = nullptr;
+    // the lane's limits in the cube: its size, and the seam (z) or the end of the entrance (y), as keys of their order
+    const long long key_size = order_key(__double_as_longlong(C.size));
+    const long long key_end = order_key(__double_as_longlong(d == 2 ? C.seam : C.size + C.l_ext_m));
+    const double cube_top = (double)(C.cn[d] - 1) - 1e-9;
     double val[NC][NP];
 #pragma unroll
     for (int c = 0; c < NC; ++c)
@@ -234,9 +241,8 @@ k_tandem(const __grid_constant__ TConst C, Tracks T, uint32_t n, const double* _
         double f = q;
         if (__any_sync(FULL, go && cube)) {   // fields.rs:89-96: clamped to the grid, short of its last node
             const double fc = mqp::div_rn(q - C.clo[d], C.ch_mm, C.inv_ch_mm);
-            const double top = (double)(C.cn[d] - 1) - 1e-9;
             const long long b = __double_as_longlong(fc);
-            if (cube) f = lt_zero(b) ? 0.0 : gt_pos(b, __double_as_longlong(top)) ? top : fc;
+            if (cube) f = lt_zero(b) ? 0.0 : gt_pos(b, __double_as_longlong(cube_top)) ? cube_top : fc;
         }
         double t = f - cell;
         const bool stay = ci >= 0 && (unsigned)__double2hiint(t) < 0x3ff00000u;
@@ -473,9 +479,11 @@ k_tandem(const __grid_constant__ TConst C, Tracks T, uint32_t n, const double* _
             // inside the posts' reach of no face, before the seam: nothing can happen
             const bool off = have && cube && gl < 3 && (unsigned)(xhi - C.in_lo) >= C.in_n[d];
             if (__any_sync(FULL, off)) {
-                const double x0 = shfl_d(x, base), x1 = shfl_d(x, base + 1), x2 = shfl_d(x, base + 2);
-                const double m0 = shfl_d(q, base), m1 = shfl_d(q, base + 1), m2 = shfl_d(q, base + 2);
-                const float p0 = (float)m0, p1 = (float)m1, p2 = (float)m2;
+                // The look at the walls stays off the FP64 pipe: one conversion a lane, limits by the positions' bits, distances
+                // in FP32 where these decide. The groups' tracks share the pipe's instructions by eight, not by 32 as single
+                // lanes did.
+                const float pm = (float)q;
+                const float p0 = __shfl_sync(FULL, pm, base), p1 = __shfl_sync(FULL, pm, base + 1), p2 = __shfl_sync(FULL, pm, base + 2);
                 bool unsure = false, solid = false;
                 {
                     const float l = C.F.size;
@@ -491,19 +499,33 @@ k_tandem(const __grid_constant__ TConst C, Tracks T, uint32_t n, const double* _
                         unsure |= un;
                     }
                 }
+                // beyond the cube's size | the seam (z) or the entrance's end (y) | below zero
+                const long long bx = __double_as_longlong(x);
+                const unsigned own = (gt_key(bx, key_size) ? 1u : 0u) | (gt_key(bx, key_end) ? 2u : 0u) | (lt_zero(bx) ? 4u : 0u);
+                const unsigned fx = __shfl_sync(FULL, own, base), fy = __shfl_sync(FULL, own, base + 1), fz = __shfl_sync(FULL, own, base + 2);
                 constexpr unsigned GM = G == 32 ? 0xffffffffu : (1u << G) - 1u;
                 const bool g_solid = ((__ballot_sync(FULL, solid) >> base) & GM) != 0u, g_unsure = ((__ballot_sync(FULL, unsure) >> base) & GM) != 0u;
                 const bool go = have && cube;   // a group that is well inside finds just that
-                if (go) {
-                    bool blocked = g_solid;
-                    if (g_unsure) {
+                // off the entrance's axis, where it counts: beyond the cube in y
+                bool un = false;
+                bool off_axis = !below(C.F, hypf2(p0 - C.F.ent_c, p2 - C.F.ent_b), C.F.ap_r, un);
+                const bool beyond = go && (fz & 2u), ask_wall = go && g_unsure, ask_axis = go && (fy & 1u) && un;
+                double x0 = 0.0, x1 = 0.0, x2 = 0.0, m0 = 0.0, m1 = 0.0, m2 = 0.0;
+                bool blocked = g_solid;
+                if (__any_sync(FULL, beyond || ask_wall || ask_axis)) {
+                    x0 = shfl_d(x, base); x1 = shfl_d(x, base + 1); x2 = shfl_d(x, base + 2);
+                    m0 = shfl_d(q, base); m1 = shfl_d(q, base + 1); m2 = shfl_d(q, base + 2);
+                    if (ask_wall) {
                         const double mm[3] = {m0, m1, m2};
                         int sg = 0;
                         blocked = mqc::classify(C.cube, mm, 0.0, &sg) != mqc::ID_FREE;
                     }
+                    if (ask_axis) off_axis = mqc::dist2d(m0 - C.ent_c, m2 - C.ent_b) >= C.ap_r;
+                }
+                if (go) {
                     bool done = false;
                     if (blocked) { reg = R_LOST; done = true; }
-                    if (!done && x2 > C.seam) {
+                    if (!done && beyond) {
                         const int i = mqc::nearest_port(C.cube, m0, m1);
                         const double* c = C.mouth[i];
                         if (mqc::dist2d(x0 - c[0], x1 - c[1]) < C.ap_r * 0.001) {
@@ -527,12 +549,12 @@ k_tandem(const __grid_constant__ TConst C, Tracks T, uint32_t n, const double* _
                             }
                             reg = 1 + i;
                             changed = done = true;
-                        } else if (x2 > C.size) { reg = R_LOST; done = true; }
+                        } else if (fz & 1u) { reg = R_LOST; done = true; }
                     }
-                    if (!done && x1 > C.size && mqc::dist2d(m0 - C.ent_c, m2 - C.ent_b) >= C.ap_r) { reg = R_LOST; done = true; }
+                    if (!done && (fy & 1u) && off_axis) { reg = R_LOST; done = true; }
                     if (!done) {
-                        if (x1 > C.size + C.l_ext_m) reg = (reg == R_SPLIT) ? R_BACK : R_DETECTED;
-                        else if (x0 < 0.0 || x1 < 0.0 || x2 < 0.0 || x0 > C.size) reg = R_LOST;
+                        if (fy & 2u) reg = (reg == R_SPLIT) ? R_BACK : R_DETECTED;
+                        else if (((fx | fy | fz) & 4u) || (fx & 1u)) reg = R_LOST;
                     }
                 }
             }
@@ -715,7 +737,13 @@ mq_status mq_tandem_create(const mq_tandem_desc* d, int32_t device, mq_tandem** 
         const double m = mqc::size(g) + 2.0 * (std::fabs(g.l_ext) + std::fabs(g.cap_gap) + std::fabs(g.cap_r));
         const double near = std::fmax(2e-3, m * 0x1.0p-17);
         F.near = (float)near;
-        F.round_max = (float)std::fmin(0.499, 0.5 - near / std::fabs(g.pitch));
+        const double apart = std::fmin(0.499, 0.5 - near / std::fabs(g.pitch));
+        F.round_port = (float)apart;
+        // Which of two posts is nearer does not matter where both are farther than any radius of theirs, as on the axis
+        // of the entrance, where the tracks come in (200,000 of them, 200 steps: 57 ms with the exact test there).
+        const double radii = std::fmax(std::fmax(g.d / 2.0, g.stem_r), std::fmax(g.clear_r, g.d / 2.0 + g.rod_clear_extra));
+        F.round_post = apart * g.pitch > radii + 4.0 * near ? 1.0f : (float)apart;
+        F.ent_b = (float)C.ent_b; F.ent_c = (float)C.ent_c;
         F.n = g.n; F.array = g.array;
         F.ent_axis = g.ent_axis; F.ent_side = g.ent_side; F.ent_cell0 = g.ent_cell[0]; F.ent_cell1 = g.ent_cell[1];
         F.ext_axis = g.ext_axis; F.ext_side = g.ext_side; F.ext_cell0 = g.ext_cell[0]; F.ext_cell1 = g.ext_cell[1];
