@@ -96,7 +96,8 @@ typedef struct mq_run_stats {
                                   the 8 corners of one cell (with 48-byte records only those
                                   are read that the cell before did not hold)               */
     uint64_t ions_queued;      /* mixed engine: ions taken from the work queue, summed over the
-                                  launches (each reads and writes its working state once)   */
+                                  rounds of launches (each reads and writes its working state
+                                  once, and once more where lane groups take it over)       */
 } mq_run_stats;
 
 int32_t     mq_device_count(void);
@@ -145,7 +146,7 @@ typedef struct mq_tuning {
     int32_t use_graph;           /* replay the launch sequence as one CUDA graph           */
     int32_t prefetch;            /* L1-prefetch the cell each ion is heading for           */
     int32_t wide_records;        /* 96-byte records of a node and the one above it, read with
-                                    256-bit loads (else 48 B; needs 4 x nodes below 2^32)  */
+                                    256-bit loads (else 48 B; needs fewer than 2^30 nodes) */
     int32_t sort_cells;          /* before every launch, put the live ions in the Morton order
                                     of their cells (a counting sort on the device)         */
 } mq_tuning;

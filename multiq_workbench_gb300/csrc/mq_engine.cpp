@@ -652,8 +652,8 @@ mq_status mq_engine_set_tuning(mq_engine* e, const mq_tuning* t) {
     if (!e || !t) return MQ_ERR_INVALID;
     if (t->threads_per_block != 128 || t->blocks_per_sm < 0 || t->blocks_per_sm > 3 || t->chunk == 0)
         return fail(e, MQ_ERR_INVALID, "tuning: 128 threads per block, 1..3 blocks per SM (0: as they are), chunk > 0");
-    if (t->wide_records && 4 * e->nnodes >= ((size_t)1 << 32))
-        return fail(e, MQ_ERR_INVALID, "tuning: wide node records need 4 x nodes below 2^32");
+    if (t->wide_records && 4 * e->nnodes >= ((size_t)1 << 32))   // they alone would take 103 GB
+        return fail(e, MQ_ERR_INVALID, "tuning: wide node records need fewer than 2^30 nodes");
     e->tune.tpb = t->threads_per_block;
     if (t->blocks_per_sm) {
         e->tune.blocks_per_sm = t->blocks_per_sm;

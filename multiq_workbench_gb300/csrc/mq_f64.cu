@@ -73,7 +73,7 @@ __device__ __forceinline__ void table_get(const double2* t, uint32_t tlen, doubl
 // Measured (whole run_batch calls, before -> now): mass scan of 25,000 ions 162 -> 32 ms; S14 point with
 // 20,000 ions and up to 75,000 steps 1,098 -> 197 ms.
 constexpr int kBlock = 256;            // 8 warps: two per scheduler, one to fill the other's gaps
-constexpr int kPad = 120 * 1024;       // dynamic shared memory asked for, unused
+constexpr int kPad = 120 * 1024;       // dynamic shared memory asked for: so much that no second block fits (57 KB are used)
 constexpr uint32_t kPollSteps = 32;    // steps between looks at the count of open ions
 constexpr uint32_t kLaneRound = 1024;  // steps of one launch of the one-lane kernel
 

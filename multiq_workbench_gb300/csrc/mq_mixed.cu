@@ -48,7 +48,7 @@ struct Ctrs {                       // device counters
     uint32_t head_g[kMaxLegs];      // queue heads of the lane-group launches, beyond their first ions
     uint32_t handed[kMaxLegs + 2];  // ions handed to each of them, by k_mixed or by the one before
     unsigned long long steps;       // executed ion-steps
-    unsigned long long cell_loads;  // cell-cache fills (8 node records each)
+    unsigned long long cell_loads;  // cell-cache fills (a cell's 8 corners each)
     unsigned long long queued;      // ions queued over the call's launches
 };
 
@@ -253,7 +253,7 @@ __device__ __forceinline__ void put_ion(const DevIons& io, float* __restrict__ k
 // warp some lane needs one) at 12 or 16 warps per SM; with 48-byte records on larger grids the L1 reads of the
 // fills. So registers are kept for the cell, and all that only every fourth step, a collision or the end of a
 // flight reads lies in shared memory. BLOCKS: blocks per SM that the registers are cut for: 3 with wide records, 4
-// for long lists (run() has the rule), 2 with narrow ones, which then need no spills.
+// for long lists, 2 with narrow ones, which then need no spills, or 3 with legacy collisions (resident_blocks() has the rules).
 // Measured, wide with registers only / tables in shared memory at 3 / at 4 blocks: sweep of 4.2 million ions 51.1 / 51.9 /
 // 48.7 ms, 40,000 legacy ions 15.4 / 15.0 / 15.0; narrow, 0.050 mm study 30.5 / 27.6 at 2 blocks (34.4 at 3).
 template <bool LEGACY, bool PREFETCH, bool WIDE, bool NEAREST, int BLOCKS>
@@ -1374,7 +1374,7 @@ Tuning default_tuning(int device, size_t nodes) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) { cudaGetLastError(); sms = 1; }
     t.sms = sms;
-    // Record width and resident ions per SM by the size of the grid (bytes of its 48-byte records). Wide records
+    // Record width and, with resident_blocks(), ions in flight per SM by the size of the grid (bytes of its 48-byte records). Wide records
     // win while the part that the ions see lies in L2, with 3 blocks per SM and near the end with 2; then
     // narrow ones with 2 blocks, until the gathers of fewer ions in flight hit the caches so much more often that
     // 1 is better. Batch of 512,000 ions, ms, wide 3 / wide 2 / narrow 2 / narrow 1: 0.30 GB (0.100 mm channel) 10.7 / 12.0 /
@@ -1437,7 +1437,7 @@ static Kernel pick_kernel(const Tuning& t, bool legacy, bool nearest, int blocks
 }
 
 int resident_blocks(const Tuning& t, size_t nodes, size_t n, bool legacy, bool nearest) {
-    if (nearest) {   // no 8-corner cache (about 100 registers instead of 167): as many blocks as fit
+    if (nearest) {   // no 8-corner cache (about 96 registers instead of 167): as many blocks as fit
         int nb = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, pick_kernel(t, legacy, true, 0), t.tpb, 0) == cudaSuccess && nb > 0) return nb;
         cudaGetLastError();

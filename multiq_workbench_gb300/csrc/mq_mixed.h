@@ -41,7 +41,7 @@ struct MixBatch {      // per-batch constants (device-resident parameter block)
 struct Tuning {
     int tpb = 128;             // threads per block
     int blocks_per_sm = 3;     // blocks per SM of the persistent grid, as the caller gave it (resident_blocks()); the
-                               // nearest-node kernels (about 100 registers) run as many as fit instead
+                               // nearest-node kernels (about 96 registers) run as many as fit instead
     int auto_blocks = 1;       // the caller gave none: resident_blocks() chooses, from blocks_per_sm with wide records
     uint32_t chunk = 20000;    // steps per ion per launch (compaction interval)
     int use_graph = 1;         // replay the launch sequence as one CUDA graph
@@ -55,7 +55,7 @@ struct Tuning {
 struct Scratch {
     void* lists = nullptr;     // two live-ion lists (ping-pong), u32 each
     size_t list_cap = 0;
-    void* ctrs = nullptr;      // counters: [0] head, [1..2] counts, [4..5] steps (u64), ...
+    void* ctrs = nullptr;      // counters, then the hand-over list
     void* params = nullptr;    // MixBatch
     void* jobs = nullptr;      // MixJob[]
     size_t jobs_cap = 0;
@@ -74,7 +74,7 @@ struct Scratch {
 
 struct RunInfo {
     uint64_t ion_steps = 0;
-    uint64_t cell_loads = 0;   // cell-cache fills of the stepping kernel (8 node records each)
+    uint64_t cell_loads = 0;   // cell-cache fills of the stepping kernel (a cell's 8 corners each)
     uint64_t ions_queued = 0;  // ions taken from the work queue, summed over the launches
     float step_ms = 0.0f;
     uint32_t step_launches = 0;

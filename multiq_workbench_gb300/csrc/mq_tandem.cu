@@ -148,7 +148,8 @@ __device__ __forceinline__ void add_steps(unsigned long long* st, uint32_t c, ui
 // reference's, in its order: results are bit for bit those of one lane per track.
 // G = 16 while the tracks fit one warp per scheduler (two of them in a warp), 4 beyond, where fewer wasted
 // lanes count for more; groups take the next track when theirs has made its steps or is lost.
-// Measured, whole advance call, 180 tracks and 100 steps: 3.48 -> 0.48 ms.
+// Measured, whole advance call, 180 tracks and 100 steps, from the mouths 3.45 -> 0.36 ms; kernel, 200,000 tracks and 200
+// steps, from the mouths 73 -> 41 ms, through the entrance 50 -> 29.5.
 constexpr int kTBlock = 256;
 constexpr int kTRow = 10;
 constexpr int kTSums = 6 + 12 * kTRow;

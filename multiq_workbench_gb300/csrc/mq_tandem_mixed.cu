@@ -175,7 +175,7 @@ struct TCell {
     int32_t ci, cj, ck, reg;
     float fci, fcj, fck;                // the cell as floats (no int -> float conversion per step)
     uint32_t mask;                      // port: conductor bit per corner
-    uint32_t fills_cube, fills_port;    // cache fills of this lane (cube: 8 x 32-byte records; port: 8 x 48)
+    uint32_t fills_cube, fills_port;    // cache fills of this lane (cube: 8 x 32-byte records; port: 4 or 8 x 48)
 };
 
 // Constants of the track's current region, held in registers and refreshed only when the track

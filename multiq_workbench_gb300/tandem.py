@@ -312,7 +312,7 @@ class TandemStats:
     h2d_bytes: int
     d2h_bytes: int
     cell_fills_cube: int = 0   # mixed engine: cell-cache fills in the cube (8 x 32-byte records)
-    cell_fills_port: int = 0   # mixed engine: cell-cache fills in the ports (8 x 48-byte records)
+    cell_fills_port: int = 0   # mixed engine: cell-cache fills in the ports (4 or 8 x 48-byte records)
 
     @property
     def track_steps(self) -> int:
