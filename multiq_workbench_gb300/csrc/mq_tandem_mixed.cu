@@ -363,20 +363,21 @@ __global__ void k_tm_bucket(const int32_t* __restrict__ region, const float* __r
 // One chunk of global steps for every live track (one thread per track, grouped by region). Two forms of it are launched, and
 // the census of the chunk says which of them works: CUBE, where next to all tracks are in the cube and stay there, sums
 // two fields in the cube; the other takes the ports' three-field sum with its slots there too, so that
-// warps whose tracks come and go between cube and ports have one way. Both sides, 300 steps of 600,000 tracks: launched
+// warps whose tracks come and go between cube and ports have one way. (An empty launch costs 10 us at 2,048 blocks, so only
+// calls that may want the cube's form launch both: two_forms().) Both sides, 300 steps of 600,000 tracks: launched
 // through the entrance (none near a mouth) 7.7 / 8.6 ms, from the mouths 5.6 / 5.0; pulse of 262,144 tracks, 1,000 steps 7.4 / 6.7.
 // (Chosen by a vote of the warp on each step, or by warps in one kernel: 7.8 and 7.1, 7.7 and 7.4.)
 template <bool CUBE>
 __global__ void __launch_bounds__(128, 3) k_tm_step(TMConst C, MTracks M, uint32_t n, const uint32_t* __restrict__ list,
                                                     const uint32_t* __restrict__ bcount, const float* __restrict__ drive,
                                                     uint64_t g0, uint32_t S, uint32_t* __restrict__ counts,
-                                                    unsigned long long* __restrict__ stepc) {
+                                                    unsigned long long* __restrict__ stepc, int alone) {
     __shared__ uint32_t off[kBuckets + 1];
     if (threadIdx.x == 0) {
         uint32_t a = 0;
         for (int r = 0; r < kBuckets; ++r) { off[r] = a; a += bcount[r]; }
         const uint32_t abroad = a - bcount[R_SPLIT] - bcount[R_COMBINE] + bcount[kBuckets];   // in a port, or soon
-        off[kBuckets] = ((uint64_t)abroad * 64u <= a) == CUBE ? a : 0u;
+        off[kBuckets] = alone || ((uint64_t)abroad * 64u <= a) == CUBE ? a : 0u;
     }
     __syncthreads();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -649,6 +650,7 @@ struct State {
     uint32_t cap = 0;
     uint32_t* list = nullptr;
     uint32_t* bcount = nullptr;
+    int sms = 0;
 };
 
 static void free_tracks(State* s) {
@@ -671,6 +673,9 @@ State* create(const mq_tandem_desc& d, const DevFields& f, cudaStream_t st, std:
         return nullptr;
     };
     cudaError_t e;
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess || (e = cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return fail("device attributes", e);
     // cube geometry in FP32 (growth 0)
     const mq_cube_geom& g = d.cube;
     CubeF& G = C.G;
@@ -850,20 +855,35 @@ cudaError_t store(State* s, const Tracks64& tr, uint32_t n, cudaStream_t st, uin
     return cudaGetLastError();
 }
 
-cudaError_t run(State* s, uint32_t n, const float* drive, uint64_t step0, uint64_t k, uint32_t* counts,
+constexpr float kReach = 8.0f;   // mm: as far as thermal ions of these masses come in a chunk
+
+int two_forms(const State* s, const mq_tracks& tr, size_t n) {
+    if (n <= 384 * (size_t)s->sms) return 1;
+    const size_t stride = n / 4096 + 1;
+    const double near = ((double)s->C.seam_mm - kReach) * 1e-3;
+    size_t live = 0, abroad = 0;
+    for (size_t i = 0; i < n; i += stride) {
+        const int r = tr.region[i];
+        live += r <= R_COMBINE;
+        abroad += r != R_SPLIT && r != R_COMBINE ? r < R_COMBINE : tr.z[i] > near;
+    }
+    return abroad * 32 <= live ? 2 : 1;
+}
+
+cudaError_t run(State* s, uint32_t n, const float* drive, uint64_t step0, uint64_t k, int forms, uint32_t* counts,
                 unsigned long long* stepc, cudaStream_t st, uint32_t* launches) {
     cudaError_t e;
     if (!n) return cudaSuccess;
     const unsigned grid = (n + 127) / 128;
-    // 8 mm, as far as thermal ions of these masses come in a chunk
-    const float z_near = (s->C.seam_mm - 8.0f - s->C.clo[2]) / s->C.ch;
+    const float z_near = (s->C.seam_mm - kReach - s->C.clo[2]) / s->C.ch;
     for (uint64_t q = 0; q < k; q += kChunk) {
         const uint32_t S = (uint32_t)(k - q < kChunk ? k - q : kChunk);
         if ((e = cudaMemsetAsync(s->bcount, 0, (kBuckets + 1) * sizeof(uint32_t), st)) != cudaSuccess) return e;
         k_tm_bucket<<<grid, 128, 0, st>>>(s->M.region, s->M.xh + 2 * (size_t)n, z_near, n, s->list, s->bcount);
-        k_tm_step<false><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc);
-        k_tm_step<true><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc);
-        *launches += 3;
+        k_tm_step<false><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc, forms < 2);
+        if (forms > 1)
+            k_tm_step<true><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc, 0);
+        *launches += 1u + (uint32_t)forms;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -7,7 +7,7 @@ import pytest
 @pytest.mark.parametrize("steps, chunks", [(0, 0), (1, 1), (256, 1), (1000, 4), (65536, 256), (65537, 257), (200000, 782)])
 def test_tandem_state_is_counted_once_per_step_launch(steps, chunks):
     import bench
-    launches = 2 + 3 * chunks + -(-steps // 65536)   # load, store; bucket and two step kernels; one drive table per 65,536 steps
+    launches = 2 + 2 * chunks + -(-steps // 65536)   # load, store; bucket and step kernel; one drive table per 65,536 steps
     st = SimpleNamespace(launches=launches, cell_fills_cube=3, cell_fills_port=5)
     assert bench.tandem_moved(st, 7, steps) == 3 * 256 + 5 * 192 + 7 * bench.TRACK_STATE_BYTES * chunks
 
