@@ -710,6 +710,7 @@ mq_status mq_tandem_create(const mq_tandem_desc* d, int32_t device, mq_tandem** 
         P.idle = p.tone_khz == 0.0;
     }
     if (cudaMalloc(&t->counts, kTail) != cudaSuccess) return bail(MQ_ERR_NOMEM);
+    if (cudaMallocHost(&t->stage, kStageMax + kTail) != cudaSuccess) { cudaGetLastError(); return bail(MQ_ERR_NOMEM); }   // 0.2 ms: not in an advance
     t->stepc = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(t->counts) + kCntBytes);
     C.cube = d->cube;
     for (int a = 0; a < 3; ++a) { C.cn[a] = d->cube_dims[a]; C.clo[a] = d->cube_lo_mm[a]; }
@@ -839,15 +840,10 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
             return tfail(t, MQ_ERR_INVALID, "track " + std::to_string(i) + " has an invalid species, region or last port");
     // Few tracks go through one pinned block, in one copy each way: ten copies of pageable arrays cost
     // 5 us each whatever their size. Many are copied array by array, which the driver does as fast as a
-    // host memcpy would stage them; they need no block, whose allocation takes 0.2 ms.
+    // host memcpy would stage them; the block holds their counters alone (copied pageable, these cost 30 us).
     const bool staged = tb <= kStageMax;
-    if (staged && !t->stage && cudaMallocHost(&t->stage, kStageMax + kTail) != cudaSuccess) {
-        cudaGetLastError();
-        return tfail(t, MQ_ERR_NOMEM, "pinned staging");
-    }
     TCK(cudaStreamSynchronize(t->st), "tandem");   // a call that failed may have left copies of the block under way
-    char own_tail[kTail];
-    char* const tail = staged ? t->stage + kStageMax : own_tail;   // port counters, then step counters: their device order
+    char* const tail = t->stage + kStageMax;   // port counters, then step counters: their device order
     if (staged) {
         size_t o = 0;
         for (int k = 0; k < 10; ++k) { std::memcpy(t->stage + o, host[k], sz[k] * n); o += sz[k] * n; }
