@@ -875,7 +875,7 @@ mq_status mq_tandem_advance(mq_tandem* t, mq_tracks* tr, size_t n, uint64_t step
     Tones tones;
     tones.f[0] = t->desc.f_rf; tones.v[0] = t->desc.v_rf; tones.dt = t->desc.dt;
     for (int i = 0; i < 9; ++i) { tones.f[1 + i] = t->desc.port[i].tone_khz * 1000.0; tones.v[1 + i] = t->desc.port[i].v_ac; }
-    const int forms = t->mix ? mqtm::two_forms(t->mix, *tr, n) : 0;
+    const int forms = t->mix ? mqtm::two_forms(t->mix, *tr, n, steps) : 0;
     uint32_t launches = 0;
     const uint64_t h2d = tb + 9 * kNC * 4;
     for (uint64_t s = 0; s < steps || s == 0; s += tab) {

@@ -29,9 +29,9 @@ State* create(const mq_tandem_desc& d, const DevFields& f, cudaStream_t st, std:
 void destroy(State* s);
 // FP64 device tracks -> the engine's mixed state (n tracks)
 cudaError_t load(State* s, const Tracks64& tr, uint32_t n, cudaStream_t st, uint32_t* launches);
-// 2 if an advance of the host's tracks is one for both forms of the step kernel (many tracks, next to all of them in the
-// cube and away from its mouths, judged by up to 4,096 of them), else 1; results do not depend on it
-int two_forms(const State* s, const mq_tracks& tr, size_t n);
+// 2 if an advance of the host's tracks is one for both forms of the step kernel (many tracks and steps, next to all
+// tracks in the cube and away from its mouths, judged by up to 256 of them), else 1; results do not depend on it
+int two_forms(const State* s, const mq_tracks& tr, size_t n, uint64_t steps);
 // advance the mixed state by k global steps (drive: k x 10 floats, RF + nine tones) starting at
 // global step step0; counts (9 x 21 u32) and stepc (3 u64) accumulate on the device
 cudaError_t run(State* s, uint32_t n, const float* drive, uint64_t step0, uint64_t k, int forms, uint32_t* counts,

@@ -340,8 +340,8 @@ __global__ void k_tm_store(TMConst C, Tracks64 T, MTracks M, uint32_t n) {
     T.vx[i] = v[0]; T.vy[i] = v[1]; T.vz[i] = v[2];
 }
 
-// group the live tracks by region: list[r * n + k], one warp-aggregated atomic per region group; and count those of the
-// cube beyond z_near (grid units), which may come to a mouth within the chunk
+// group the live tracks by region: list[r * n + k], one warp-aggregated atomic per region group; and, where zh is
+// given, count those of the cube beyond z_near (grid units), which may come to a mouth within the chunk
 __global__ void k_tm_bucket(const int32_t* __restrict__ region, const float* __restrict__ zh, float z_near, uint32_t n,
                             uint32_t* __restrict__ list, uint32_t* __restrict__ bcount) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -349,7 +349,7 @@ __global__ void k_tm_bucket(const int32_t* __restrict__ region, const float* __r
     const bool live = r <= R_COMBINE;
     const unsigned lm = __ballot_sync(FULL, live);
     if (!live) return;
-    const unsigned near = __ballot_sync(lm, (r == R_SPLIT || r == R_COMBINE) && zh[i] > z_near);
+    const unsigned near = zh ? __ballot_sync(lm, (r == R_SPLIT || r == R_COMBINE) && zh[i] > z_near) : 0u;
     const unsigned peers = __match_any_sync(lm, r);
     const int leader = __ffs(peers) - 1;
     const uint32_t lane = threadIdx.x & 31;
@@ -857,9 +857,9 @@ cudaError_t store(State* s, const Tracks64& tr, uint32_t n, cudaStream_t st, uin
 
 constexpr float kReach = 8.0f;   // mm: as far as thermal ions of these masses come in a chunk
 
-int two_forms(const State* s, const mq_tracks& tr, size_t n) {
-    if (n <= 384 * (size_t)s->sms) return 1;
-    const size_t stride = n / 4096 + 1;
+int two_forms(const State* s, const mq_tracks& tr, size_t n, uint64_t steps) {
+    if (n <= 384 * (size_t)s->sms || steps < 64) return 1;
+    const size_t stride = n / 256 + 1;
     const double near = ((double)s->C.seam_mm - kReach) * 1e-3;
     size_t live = 0, abroad = 0;
     for (size_t i = 0; i < n; i += stride) {
@@ -879,7 +879,7 @@ cudaError_t run(State* s, uint32_t n, const float* drive, uint64_t step0, uint64
     for (uint64_t q = 0; q < k; q += kChunk) {
         const uint32_t S = (uint32_t)(k - q < kChunk ? k - q : kChunk);
         if ((e = cudaMemsetAsync(s->bcount, 0, (kBuckets + 1) * sizeof(uint32_t), st)) != cudaSuccess) return e;
-        k_tm_bucket<<<grid, 128, 0, st>>>(s->M.region, s->M.xh + 2 * (size_t)n, z_near, n, s->list, s->bcount);
+        k_tm_bucket<<<grid, 128, 0, st>>>(s->M.region, forms > 1 ? s->M.xh + 2 * (size_t)n : nullptr, z_near, n, s->list, s->bcount);
         k_tm_step<false><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc, forms < 2);
         if (forms > 1)
             k_tm_step<true><<<grid, 128, 0, st>>>(s->C, s->M, n, s->list, s->bcount, drive + q * 10, step0 + q, S, counts, stepc, 0);
