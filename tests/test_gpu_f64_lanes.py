@@ -49,3 +49,17 @@ def test_lanes_equal_oracle(coarse, name, n, dead):
             assert st.ion_steps == R.run(G, b, jobs, ref, **({} if more is None else {"max_more": more}))
             _assert_bitequal(ions, ref, f"{name} n={n}: {more}")
     assert (ions.status != 0).all()
+
+
+def test_allocation_free_entry_takes_the_same_way(coarse):
+    """The same call on device memory of the caller's, whose launches follow the same rule without a hand-over list."""
+    from test_zz_no_alloc import _device_call
+    mq = _mq()
+    ph = _variants()["legacy_all"]
+    jobs = _jobs(LINE // 3 + 1, legacy_species=True)
+    with mq.Engine(coarse, mq.PREC_F64) as e:
+        e.set_dc(DC)
+        ions = e.inject(jobs, ph)
+        got, steps = _device_call(mq, coarse, DC, ph, jobs, ions, 0xFFFFFFFF)
+        assert e.run_ions(jobs, ph, ions).ion_steps == steps
+    _assert_bitequal(got, ions, "allocation-free")
