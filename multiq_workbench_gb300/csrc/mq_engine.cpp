@@ -9,6 +9,7 @@
 #include "mq_internal.h"
 #include "mq_mixed.h"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -302,7 +303,7 @@ mqd::DevGrid dev_grid(const mq_engine* e) {
 
 // FP64 launch loop (chsim run_direct, channel.rs:478-493): relaunch until no ion is live
 // or the step budget is spent.  Each launch advances every live ion by <= kF64Chunk steps.
-mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_t max_more, mq_run_stats* stats,
+mq_status run_f64(mq_engine* e, const Batch& b, size_t njobs, uint32_t tlen, size_t n, uint32_t max_more, mq_run_stats* stats,
                   uint64_t* steps_out) {
     const int32_t fault = e->fault;
     e->fault = MQ_FAULT_NONE;
@@ -323,6 +324,8 @@ mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_
     const double2* ac_tab = rf_tab + tlen;
     uint64_t budget = max_more;
     uint32_t launches = 0, kernels = 0, live = 0;
+    double cand = 0.0;
+    for (size_t k = 0; k < njobs; ++k) cand = std::max(cand, mqd::f64_cand(reinterpret_cast<const JobC*>(e->stage.at(StageLayout(njobs).jc))[k]));
     float step_ms = 0.0f;
     for (;;) {
         uint32_t L = budget < chunk ? (uint32_t)budget : chunk;
@@ -330,7 +333,7 @@ mq_status run_f64(mq_engine* e, const Batch& b, uint32_t tlen, size_t n, uint32_
         if (L == 0) break;
         CK(cudaEventRecord(e->ev[2], e->st), "event");
         CK(mqd::launch_f64_step(dev_grid(e), b, e->jobc.as<JobC>(), rf_tab, ac_tab, tlen, dev_ions(e, n), (uint32_t)n,
-                                launches ? live : (uint32_t)n, &L, ctr, hand, e->st, &kernels), "FP64 step kernel");
+                                launches ? live : (uint32_t)n, cand, &L, ctr, hand, e->st, &kernels), "FP64 step kernel");
         CK(cudaEventRecord(e->ev[3], e->st), "event");
         live = 0;
         CK(cudaMemcpyAsync(&live, &ctr->live, 4, cudaMemcpyDeviceToHost, e->st), "live count");
@@ -555,7 +558,7 @@ mq_status mq_run_ions(mq_engine* e, const mq_job* jobs, size_t njobs, const mq_p
     size_t ntab = 0;
     if ((s = upload_jobs(e, jobs, njobs, *ph, b, false, &tlen, &ntab, &h2d)) != MQ_OK) return s;
     uint64_t steps = 0;
-    if (e->prec == MQ_PREC_F64) s = run_f64(e, b, tlen, n, max_more, stats, &steps);
+    if (e->prec == MQ_PREC_F64) s = run_f64(e, b, njobs, tlen, n, max_more, stats, &steps);
     else s = run_mixed(e, jobs, njobs, *ph, b, n, max_more, 1, stats, &steps);
     if (s == MQ_ERR_WATCHDOG) {   // the states are the checkpoint: hand them back so the caller can resume
         const std::string why = e->err;
@@ -604,7 +607,7 @@ mq_status mq_run_batch(mq_engine* e, const mq_job* jobs, size_t njobs, const dou
     if (e->prec == MQ_PREC_F64) CK(mqd::launch_inject(b, jt, dev_ions(e, n), (uint32_t)n, e->st), "inject kernel");
     else CK(mqmix::launch_inject(b, jt, dev_ions(e, n), (uint32_t)n, e->st), "inject kernel");
     uint64_t steps = 0;
-    if (e->prec == MQ_PREC_F64) s = run_f64(e, b, tlen, n, 0xFFFFFFFFu, stats, &steps);
+    if (e->prec == MQ_PREC_F64) s = run_f64(e, b, njobs, tlen, n, 0xFFFFFFFFu, stats, &steps);
     else s = run_mixed(e, jobs, njobs, *ph, b, n, 0xFFFFFFFFu, ions_out ? 1 : 0, stats, &steps);
     if (s != MQ_OK) return s;
     CK(e->counters.grow(sizeof(unsigned long long) * mqd::kCounters * njobs), "job counters");

@@ -14,6 +14,8 @@
 #include "mq_check.h"
 #include "mq_f64dev.h"
 
+#include <cmath>
+
 namespace mqd {
 namespace {
 
@@ -75,7 +77,7 @@ __device__ __forceinline__ void table_get(const double2* t, uint32_t tlen, doubl
 constexpr int kBlock = 256;            // 8 warps: two per scheduler, one to fill the other's gaps
 constexpr int kPad = 120 * 1024;       // dynamic shared memory asked for: so much that no second block fits (57 KB are used)
 constexpr uint32_t kPollSteps = 32;    // steps between looks at the count of open ions
-constexpr uint32_t kLaneRound = 1024;  // steps of one launch of the one-lane kernel
+constexpr uint32_t kLaneRound = 1024;  // steps of one launch of the one-lane kernel (thermal collisions an eighth of it: fewer ions last)
 
 // Shared memory of a group, in doubles: the fractions of the three axes as pairs {1 - t, t}, the
 // products of the nine sums (rows of 8 corners, 10 apart: 16-byte reads of the rows meet no bank
@@ -477,12 +479,12 @@ k_f64_step(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __r
 }
 
 // ---------------------------------------------------------------- one lane per ion
-// For long lists with legacy collisions, which come every few steps: with eight ions to a warp some ion has one on
-// nearly every step and the warp pays its hundred FP64 operations for that ion alone, with 32 ions it pays them
-// once for all that have one. Bound by the FP64 pipe like the groups: 15.7 us a step for up to 128 ions per SM, 13.8 for each
-// further 128 (0.1 mm channel), whether they live or not, where the groups take 1.1 to 1.4 us for each
-// thousand live ones (launch_f64_step has the rule). Every operation is that of the groups, in its order. One kernel of
-// this form stepped all FP64 ions before the groups came.
+// For long lists with collisions on most steps, legacy ones or those of a dense gas: with eight ions to a warp some ion
+// has one on nearly every step and the warp pays its hundred FP64 operations for that ion alone, with 32 ions it pays them
+// once for all that have one. Bound by the FP64 pipe like the groups: with legacy collisions 15.7 us a step for up to 128
+// ions per SM, 13.8 for each further 128 (0.1 mm channel), whether they live or not, where the groups take 1.1 to 1.4 us for
+// each thousand live ones; with a thermal gas of 5 Pa 25 us, and 1.8 (launch_f64_step has the rules). Every operation is that
+// of the groups, in its order. One kernel of this form stepped all FP64 ions before the groups came.
 // f32 -> f64 as mqp::widen_normal, other values included: as a branch, since a selected conversion is paid on every value
 // (26,000 ions, 2,000 steps 66.6 -> 57.2 ms)
 __device__ __forceinline__ double widen(float f) {
@@ -494,6 +496,7 @@ __device__ __forceinline__ double widen(float f) {
     return __hiloint2double((int)hi, (int)(u << 29));
 }
 
+template <bool LEGACY>
 __global__ void __launch_bounds__(128)
 k_f64_lane(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __restrict__ rf_tab, const double2* __restrict__ ac_tab,
            uint32_t tlen, DevIons io, uint32_t n, uint32_t max_more, F64Ctrs* __restrict__ ctr) {
@@ -562,8 +565,7 @@ k_f64_lane(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __r
             }
             age += 1;
             done += 1;
-            leg -= 1;
-            if (leg <= 0) {
+            if (LEGACY && --leg <= 0) {
                 const double vm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
                 if (vm > jc.floor_v) {
                     const double cth = 2.0 * mqp::xs_next(&rng) - 1.0;
@@ -583,6 +585,31 @@ k_f64_lane(DevGrid g, Batch b, const JobC* __restrict__ jobs, const double2* __r
                 double st = floor(mfp / (vn > 1e-3 ? vn : 1e-3) / dt);
                 if (st < 1.0) st = 1.0;
                 leg = !(st < 2147483647.0) ? 2147483647 : (int32_t)st;
+            }
+            if (!LEGACY) {
+                const double vm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+                const double bound = vm + 6.0 * jc.s_gas;
+                if (mqp::xs_next(&rng) < jc.nsd * bound) {
+                    double gv[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const double u1 = mqp::xs_next(&rng), u2 = mqp::xs_next(&rng);
+                        const double vg = jc.s_gas * mqp::gauss(u1, u2);
+                        gv[d] = v[d] - vg;
+                    }
+                    const double gm = sqrt(gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2]);
+                    if (mqp::xs_next(&rng) * bound < gm) {
+                        const double cth = 2.0 * mqp::xs_next(&rng) - 1.0;
+                        double sp, cp;
+                        mqp::sincos2pi(mqp::xs_next(&rng), &sp, &cp);
+                        const double omc = 1.0 - cth * cth;
+                        const double sn = sqrt(omc > 0.0 ? omc : 0.0);
+                        const double dd[3] = {sn * cp, sn * sp, cth};
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) v[d] = v[d] - jc.mr * gv[d] + jc.mr * gm * dd[d];
+                        ncoll += 1;
+                    }
+                }
             }
             const long long bx = __double_as_longlong(x[0]), by = __double_as_longlong(x[1]), bz = __double_as_longlong(x[2]);
             if (gt_pos(bz, __double_as_longlong(b.z_exit))) status = 3;
@@ -665,8 +692,8 @@ cudaError_t launch_inject(const mqp::Batch& b, JobTable jt, DevIons io, uint32_t
 }
 
 cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc, const double2* rf_tab,
-                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t live, uint32_t* steps,
-                            F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels) {
+                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t live, double cand,
+                            uint32_t* steps, F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels) {
     if (n == 0) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaError_t e;
@@ -677,14 +704,20 @@ cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc,
     if ((e = cudaFuncSetAttribute(k_f64_step<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPad)) != cudaSuccess) return e;
     k_f64_begin<<<1, 1, 0, s>>>(ctr, n);
     const uint32_t wide = f64_hand_entries(sms);
-    // Legacy collisions: one ion to a lane while more live than 72 per SM for each 128 per SM in the list, looked at
-    // again every kLaneRound steps. 2,000 steps, groups alone / so: 10,000 ions 29 / 29 ms, 15,000 45 / 33, 26,000 76 /
-    // 57, 40,000 109 / 85; 200 steps of 200,000 ions 44 / 30; 40,000 ions to their end (20,000 steps) 745 / 702.
+    // One ion to a lane while more live than so many per SM for each 128 per SM in the list, looked at again after a round.
+    // Legacy collisions, 2,000 steps, groups alone / so: 10,000 ions 29 / 29 ms, 15,000 45 / 33, 26,000 76 / 57, 40,000 109 / 85; 200
+    // steps of 200,000 ions 44 / 30; 40,000 ions to their end (20,000 steps) 745 / 702. Thermal collisions: where a resting ion
+    // is a candidate on 14 in 100 steps or more (1.7 Pa for the ions and step of a mass scan; below, the groups are faster), 200,000
+    // ions, 200 steps at 2 Pa 58 / 53 ms, 5 Pa 73 / 53, 30 Pa 80 / 53.
     const uint64_t waves = ((uint64_t)n + 128u * (uint32_t)sms - 1u) / (128u * (uint32_t)sms);
+    const uint64_t line = (b.legacy_coll ? 72u : 78u + (uint32_t)(5.0 / std::fmax(cand, 0.14))) * (uint32_t)sms * waves;
     uint32_t max_more = *steps;
-    if (b.legacy_coll && live > 72u * (uint32_t)sms * waves) {
-        *steps = max_more = max_more < kLaneRound ? max_more : kLaneRound;
-        k_f64_lane<<<blocks_for(n, 128), 128, 0, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr);
+    if ((b.legacy_coll || cand >= 0.14) && live > line) {
+        const uint32_t round = b.legacy_coll ? kLaneRound : kLaneRound / 8;
+        *steps = max_more = max_more < round ? max_more : round;
+        const unsigned blocks = blocks_for(n, 128);
+        if (b.legacy_coll) k_f64_lane<true><<<blocks, 128, 0, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr);
+        else k_f64_lane<false><<<blocks, 128, 0, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr);
         *kernels += 2;
     } else if (n <= wide) {
         k_f64_step<16><<<sms, kBlock, kPad, s>>>(g, b, jc, rf_tab, ac_tab, tlen, io, n, max_more, ctr, nullptr, 0, 0);

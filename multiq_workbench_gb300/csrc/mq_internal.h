@@ -48,8 +48,10 @@ struct F64Ctrs {
 cudaError_t launch_inject(const mqp::Batch& b, JobTable jt, DevIons io, uint32_t n, cudaStream_t s);
 // One launch over the list's n ions, of which at most `live` live: *steps steps of each, or so many as it leaves there.
 cudaError_t launch_f64_step(DevGrid g, const mqp::Batch& b, const mqp::JobC* jc, const double2* rf_tab,
-                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t live, uint32_t* steps,
-                            F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels);
+                            const double2* ac_tab, uint32_t tlen, DevIons io, uint32_t n, uint32_t live, double cand,
+                            uint32_t* steps, F64Ctrs* ctr, uint2* hand, cudaStream_t s, uint32_t* kernels);
+// A resting ion's probability of a thermal collision candidate per step; a batch's `cand` is the largest of its jobs.
+inline double f64_cand(const mqp::JobC& j) { return j.nsd * (6.0 * j.s_gas); }
 // Ions that the 16-lane groups of one warp per scheduler hold: up to so many, a call steps them in
 // groups of 16 lanes. A larger call starts in groups of 4, which hand over the last so many of their
 // ions through a list of that length (null: they finish them themselves).

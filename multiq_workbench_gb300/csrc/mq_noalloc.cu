@@ -11,6 +11,7 @@
 // pointer is what the kernels receive.
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "mq_engine.h"
@@ -130,10 +131,14 @@ extern "C" mq_status mq_run_ions_device_noalloc(const mq_dev_grid* grid, const m
         if (bad != 0) return MQ_ERR_INVALID;
     }
     // job constants, converted on the host in small stack batches and copied into the scratch
+    double cand = 0.0;
     for (size_t k0 = 0; k0 < njobs; k0 += kStage) {
         mqp::JobC buf[kStage];
         const size_t m = njobs - k0 < kStage ? njobs - k0 : kStage;
-        for (size_t k = 0; k < m; ++k) buf[k] = mqd::host_job(jobs[k0 + k], *ph);
+        for (size_t k = 0; k < m; ++k) {
+            buf[k] = mqd::host_job(jobs[k0 + k], *ph);
+            cand = std::max(cand, mqd::f64_cand(buf[k]));
+        }
         // from pageable memory this copy returns once buf has been read, so buf may be reused
         if (cudaMemcpyAsync(d_jobs + k0, buf, m * sizeof(mqp::JobC), cudaMemcpyHostToDevice, st) != cudaSuccess)
             return MQ_ERR_CUDA;
@@ -157,7 +162,7 @@ extern "C" mq_status mq_run_ions_device_noalloc(const mq_dev_grid* grid, const m
         uint32_t L = budget < kChunk ? (uint32_t)budget : kChunk;
         if (L == 0) break;
         // no phase tables (length 0): the kernel evaluates every drive phase directly
-        if (mqd::launch_f64_step(g, b, d_jobs, nullptr, nullptr, 0, d, (uint32_t)n, live, &L, ctr, nullptr, st, &kernels) != cudaSuccess)
+        if (mqd::launch_f64_step(g, b, d_jobs, nullptr, nullptr, 0, d, (uint32_t)n, live, cand, &L, ctr, nullptr, st, &kernels) != cudaSuccess)
             return MQ_ERR_CUDA;
         if (cudaMemcpyAsync(&live, &ctr->live, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return MQ_ERR_CUDA;
         if (cudaStreamSynchronize(st) != cudaSuccess) return MQ_ERR_CUDA;

@@ -3,6 +3,7 @@ hold (so that the one-lane kernel runs, refills, queues ions again and hands its
 FP64 ions and tracks than 16-lane groups take alone, both record widths, the L1 prefetch and the cell sort,
 states that are NaN, outside the box or on its faces in all of these, and device field solves. Run with MQ_LIB
 pointing at libmqgb_check.so (tests/test_gpu_check_long.py does); prints one JSON line with the records."""
+import dataclasses
 import json
 import sys
 from pathlib import Path
@@ -60,8 +61,9 @@ def main():
             e.run_batch([mq.Job(jobs[0].sp, jobs[0].drive, 2048 * 152 + 1, 3)], DC, variants[0])
         out["loads"] = int(e.last_stats.cell_loads)
     with mq.Engine(f, mq.PREC_F64) as e:
-        short = [mq.Job(j.sp, j.drive, 4000, j.seed) for j in jobs]   # with legacy collisions one ion to a lane, else in groups
-        for ph in variants:
+        # with legacy collisions and in the dense gas one ion to a lane, else in groups
+        short = [mq.Job(j.sp, j.drive, 5000, j.seed) for j in jobs]
+        for ph in variants + [dataclasses.replace(variants[0], pressure_pa=5.0)]:
             e.set_dc(DC)
             e.run_ions(short, ph, edges(e.inject(short, ph), f))
     out["channel"] = status(reset=1)

@@ -1,6 +1,8 @@
-"""Legacy collisions on the FP64 engine, where long lists go one ion to a lane: against the CPU oracle, bit for bit, one
-ion above and below the line (72 live ions per SM and wave of 128 per SM; 152 SMs), with a second wave, with so many
-finished ions in the list that the groups take it, and across launches that change from one kernel to the other."""
+"""Collisions on most steps on the FP64 engine, legacy ones and those of a dense gas, where long lists go one ion to a
+lane: against the CPU oracle, bit for bit, one ion above and below the line (72 live ions per SM and wave of 128 per SM with
+legacy collisions, 90 and 80 with the two densities here; 152 SMs), with a second wave, with so many finished ions in the list that the groups take it, and across launches
+that change from one kernel to the other."""
+import dataclasses
 import sys
 from pathlib import Path
 
@@ -16,13 +18,17 @@ DC = [0.0, 5.0, -5.0, 0.0]
 LINE = 72 * 152
 
 
-@pytest.mark.parametrize("n, dead", [(LINE, 0), (LINE + 1, 0), (LINE + 9, 3), (19457, 2), (2 * LINE + 1, 0)])
-@pytest.mark.parametrize("name", ["legacy_all", "legacy_coll_trilinear"])
-def test_lanes_equal_oracle(coarse, name, n, dead):
+@pytest.mark.parametrize("name, pressure, n, dead", [(p, None, n, d) for p in ("legacy_all", "legacy_coll_trilinear") for n, d in (
+    (LINE, 0), (LINE + 1, 0), (LINE + 9, 3), (19457, 2), (2 * LINE + 1, 0))] + [
+    (p, pr, n, d) for p, pr, line in (("half_kick_gauss", 5.0, 90), ("half_kick_gauss", 30.0, 80), ("thermal_nearest", 5.0, 90)) for n, d in (
+        (line * 152, 0), (line * 152 + 153, 0), (line * 152 + 161, 3), (2 * 152 * (line + 1), 0))])
+def test_lanes_equal_oracle(coarse, name, pressure, n, dead):
     mq = _mq()
     from oracle import mqref as R
     ph = _variants()[name]
-    jobs = _jobs((n + 2) // 3, legacy_species=True)
+    if pressure:
+        ph = dataclasses.replace(ph, pressure_pa=pressure)
+    jobs = _jobs((n + 2) // 3, legacy_species=name.startswith("legacy"))
     ions = mq.inject(coarse, jobs, ph)
     for k, _ in mq.channel.ION_FIELDS:
         setattr(ions, k, np.ascontiguousarray(getattr(ions, k)[:n]))
